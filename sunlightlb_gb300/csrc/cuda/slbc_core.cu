@@ -776,23 +776,26 @@ int slbc_create(slbc_lattice **out, int esi, int esj, int esk, int precision) {
   L.npad = (n + 63) / 64 * 64;
   L.par.tau = 0.75; L.par.rho0 = 72.0;
   h->solid_host.assign((size_t)n, 0);
-  cudaError_t e = cudaMalloc(&L.pop, pop_bytes(precision, L.npad));
-  if (e == cudaSuccess) e = cudaMemset(L.pop, 0, pop_bytes(precision, L.npad));
+  // every fill is ordered on the lattice's own stream: it does not wait for
+  // the default stream, where a fill could still be queued (behind other
+  // work of the program) when the geometry kernels already run
+  cudaError_t e = cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking);
+  L.own_stream = e == cudaSuccess;
+  if (e == cudaSuccess) e = cudaMalloc(&L.pop, pop_bytes(precision, L.npad));
+  if (e == cudaSuccess) e = cudaMemsetAsync(L.pop, 0, pop_bytes(precision, L.npad), L.stream);
   if (e == cudaSuccess) e = cudaMalloc(&L.flags, (size_t)n * sizeof(uint16_t));
-  if (e == cudaSuccess) e = cudaMemset(L.flags, 0, (size_t)n * sizeof(uint16_t));
+  if (e == cudaSuccess) e = cudaMemsetAsync(L.flags, 0, (size_t)n * sizeof(uint16_t), L.stream);
   if (e == cudaSuccess) e = cudaMalloc(&L.objidx, (size_t)n * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(L.objidx, 0xff, (size_t)n * sizeof(int));
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(L.objidx, 0xff, (size_t)n * sizeof(int), L.stream);
   if (e == cudaSuccess) e = cudaMallocHost(&L.host_out, 64 * sizeof(double));
   for (int b = 0; b < 2 && e == cudaSuccess && precision == 2; b++) {
     e = cudaMalloc(&L.mom[b], (size_t)L.npad * 4 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMemset(L.mom[b], 0, (size_t)L.npad * 4 * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemsetAsync(L.mom[b], 0, (size_t)L.npad * 4 * sizeof(float), L.stream);
   }
   if (e != cudaSuccess) {
     slbc_destroy(h);
     return fail("slbc_create", e);
   }
-  L.own_stream = true;
   L.layout = SLBC_LAYOUT_N;
   *out = h;
   return 0;
@@ -899,7 +902,7 @@ static int geometry_boundary(Lattice &L, int nobj, const long *bnd_node, const i
     CK(cudaMalloc(&L.bnd_f, 3 * nbnd * sizeof(double)));
     CK(cudaMemcpy(L.bnd_node, nodes.data(), nbnd * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(L.bnd_obj, bnd_obj, nbnd * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemset(L.bnd_f, 0, 3 * nbnd * sizeof(double)));
+    CK(cudaMemsetAsync(L.bnd_f, 0, 3 * nbnd * sizeof(double), L.stream));
   }
   if (nobj > 0) {
     // distribf pieces: each object's run of the list, split into chunks
