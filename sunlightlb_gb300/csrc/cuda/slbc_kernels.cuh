@@ -568,9 +568,12 @@ __device__ __forceinline__ void block_sum(double (&v)[NV]) {
 // deterministic.  The per-node velocity is formed in the population type
 // (FP64: one reciprocal of rho instead of three divisions) and accumulated
 // in FP64.
-template <typename T>
+// The layout is a template argument: only C1 reads neighbours, so the node
+// index is divided into (i, j, k) for that layout alone (1.68 ms at 512^3
+// FP32 with the divisions in every layout).
+template <typename T, int LAYOUT>
 __global__ void __launch_bounds__(kReduceThreads)
-k_vsum(PopArgs<T> p, int layout, double rho0, double fac, int bf_uniform, double b0, double b1,
+k_vsum(PopArgs<T> p, double rho0, double fac, int bf_uniform, double b0, double b1,
        double b2, const T *bf, const double *psi, double *partials) {
   Acc<T> ax, ay, az;
   double wsum = 0.0;
@@ -586,12 +589,15 @@ k_vsum(PopArgs<T> p, int layout, double rho0, double fac, int bf_uniform, double
     const int x = (int)e;
     const uint16_t fl = p.flags[x];
     if (fl & FLAG_SOLID) continue;
-    int i, j, k;
-    decode(x, p.esj, p.esk, i, j, k);
-    const Nbr nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
+    Nbr nb{};
+    if constexpr (LAYOUT == SLBC_LAYOUT_C1) {
+      int i, j, k;
+      decode(x, p.esj, p.esk, i, j, k);
+      nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
+    }
     T t[15];
 #pragma unroll
-    for (int q = 0; q < 15; q++) t[q] = post_value<T>(P, S, layout, q, x, fl, nb);
+    for (int q = 0; q < 15; q++) t[q] = post_value<T>(P, S, LAYOUT, q, x, fl, nb);
     T bx = (T)b0, by = (T)b1, bz = (T)b2;
     if (!bf_uniform) { bx = bf[x]; by = bf[S + x]; bz = bf[2 * S + x]; }
     T rho = r0, nx, ny, nz;
@@ -961,43 +967,82 @@ __global__ void k_move_sphere(PopArgs<T> p, MoveArgs m, T *uw) {
   }
 }
 
+// Constants of the velocity field, FP32 ones as hi + lo pairs split on the
+// host (an FP64 operation per node is what bounded this kernel).
+struct FieldArgs {
+  double rho0, fac, fb[3];          // fb = fac * b (uniform body force)
+  float rho0_h, rho0_l, fac_f, fb_h[3], fb_l[3];
+  int bf_uniform;
+};
+
+// (m + f) / (rho0 + r) of one component in FP32 with every operand a hi + lo
+// pair: one quotient and one exact-remainder correction, about 2^-46.
+__device__ __forceinline__ float ff_quotient(float nh, float nl, float rh, float rl, float rinv) {
+  const float q = nh * rinv;
+  const float rem = __fmaf_rn(-q, rh, nh) + __fmaf_rn(-q, rl, nl);
+  return __fmaf_rn(rem, rinv, q);
+}
+
 // Velocity field u = (sum_q c_q a_q + fac * b) / (rho0 + sum_q a_q) of the
 // post-collision state (any layout) on fluid nodes, 0 on solid nodes, as
-// three FP32 arrays (the per-node form of the accvmean sum).
-template <typename T>
-__global__ void k_velocity(PopArgs<T> p, int layout, double rho0, double fac, int bf_uniform, double b0, double b1,
-                           double b2, const T *bf, float *u, float *drho) {
+// three FP32 arrays (the per-node form of the accvmean sum), and the density
+// deviation.  Bound: HBM (15 populations read, 16 B written).  FP32
+// populations are summed as float-float pairs (TwoSum, 48 bits) and divided
+// with a remainder correction, all on the FP32 pipe: the first form widened
+// every population to FP64 (15 conversions and 45 multiply-adds per node on
+// a pipe 64 times narrower) and took 22.3 ms at 512^3 against 1.5 ms of
+// memory traffic.  One row of k per block row, so no index is divided.
+template <typename T, int LAYOUT>
+__global__ void k_velocity(PopArgs<T> p, FieldArgs f, const T *bf, float *u, float *drho) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y, i = blockIdx.z;
+  if (k >= p.esk) return;
   const long long n = (long long)p.esi * p.esj * p.esk;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)e;
-    const uint16_t fl = p.flags[x];
-    float ux = 0.f, uy = 0.f, uz = 0.f, dr = 0.f;
-    if (!(fl & FLAG_SOLID)) {
-      int i, j, k;
-      decode(x, p.esj, p.esk, i, j, k);
-      const Nbr nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
-      double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+  const Nbr nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
+  const int x = nb.at(0, 0, 0);
+  const uint16_t fl = p.flags[x];
+  float ux = 0.f, uy = 0.f, uz = 0.f, dr = 0.f;
+  if (!(fl & FLAG_SOLID)) {
+    T t[15];
 #pragma unroll
-      for (int q = 0; q < 15; q++) {
-        const double v = (double)post_value<T>(p.pop, p.npad, layout, q, x, fl, nb);
-        r += v;
-        mx += CX(q) * v;
-        my += CY(q) * v;
-        mz += CZ(q) * v;
-      }
-      double bx = b0, by = b1, bz = b2;
-      if (!bf_uniform) { bx = bf[x]; by = bf[p.npad + x]; bz = bf[2 * p.npad + x]; }
-      const double inv = 1.0 / (rho0 + r);
-      ux = (float)((mx + fac * bx) * inv);
-      uy = (float)((my + fac * by) * inv);
-      uz = (float)((mz + fac * bz) * inv);
-      dr = (float)r;
+    for (int q = 0; q < 15; q++) t[q] = post_value<T>(p.pop, p.npad, LAYOUT, q, x, fl, nb);
+    Acc<T> r, mx, my, mz;
+#pragma unroll
+    for (int q = 0; q < 15; q++) {
+      r.add(t[q]);
+      if (CX(q)) mx.add(CX(q) > 0 ? t[q] : -t[q]);
+      if (CY(q)) my.add(CY(q) > 0 ? t[q] : -t[q]);
+      if (CZ(q)) mz.add(CZ(q) > 0 ? t[q] : -t[q]);
     }
-    u[x] = ux;
-    u[n + x] = uy;
-    u[2 * n + x] = uz;
-    if (drho) drho[x] = dr;
+    if constexpr (sizeof(T) == 8) {
+      double bx = f.fb[0], by = f.fb[1], bz = f.fb[2];
+      if (!f.bf_uniform) { bx = f.fac * bf[x]; by = f.fac * bf[p.npad + x]; bz = f.fac * bf[2 * p.npad + x]; }
+      const double inv = 1.0 / (f.rho0 + r.s);
+      ux = (float)((mx.s + bx) * inv);
+      uy = (float)((my.s + by) * inv);
+      uz = (float)((mz.s + bz) * inv);
+      dr = (float)r.s;
+    } else {
+      dr = r.hi + r.lo;
+      Acc<float> rho = r;
+      rho.add(f.rho0_h);
+      rho.add(f.rho0_l);
+      const float rh = rho.hi + rho.lo, rl = rho.lo - (rh - rho.hi), rinv = 1.0f / rh;
+      if (f.bf_uniform) {
+        mx.add(f.fb_h[0]); my.add(f.fb_h[1]); mz.add(f.fb_h[2]);
+        mx.lo += f.fb_l[0]; my.lo += f.fb_l[1]; mz.lo += f.fb_l[2];
+      } else {  // fac is +-1/2 or 0: the products are exact
+        mx.add(f.fac_f * bf[x]); my.add(f.fac_f * bf[p.npad + x]); mz.add(f.fac_f * bf[2 * p.npad + x]);
+      }
+      ux = ff_quotient(mx.hi, mx.lo, rh, rl, rinv);
+      uy = ff_quotient(my.hi, my.lo, rh, rl, rinv);
+      uz = ff_quotient(mz.hi, mz.lo, rh, rl, rinv);
+    }
   }
+  u[x] = ux;
+  u[n + x] = uy;
+  u[2 * n + x] = uz;
+  if (drho) drho[x] = dr;
 }
 
 }  // namespace slbc

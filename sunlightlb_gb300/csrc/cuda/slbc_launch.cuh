@@ -261,9 +261,13 @@ cudaError_t SLBC_FN(launch_force)(Lattice &L) {
 
 cudaError_t SLBC_FN(launch_vsum)(Lattice &L, double fac, const double *psi, double *partials,
                                  int nblocks) {
-  k_vsum<T_><<<nblocks, kReduceThreads, 0, L.stream>>>(
-      pop_args(L), L.layout, L.par.rho0, fac, L.bf_uniform, L.bf_const[0], L.bf_const[1],
-      L.bf_const[2], (const T_ *)L.bf, psi, partials);
+  const auto go = [&](auto kernel) {
+    kernel<<<nblocks, kReduceThreads, 0, L.stream>>>(pop_args(L), L.par.rho0, fac, L.bf_uniform, L.bf_const[0],
+                                                     L.bf_const[1], L.bf_const[2], (const T_ *)L.bf, psi, partials);
+  };
+  if (L.layout == SLBC_LAYOUT_N) go(k_vsum<T_, SLBC_LAYOUT_N>);
+  else if (L.layout == SLBC_LAYOUT_C0) go(k_vsum<T_, SLBC_LAYOUT_C0>);
+  else go(k_vsum<T_, SLBC_LAYOUT_C1>);
   count_launch();
   return cudaGetLastError();
 }
@@ -355,9 +359,25 @@ cudaError_t SLBC_FN(launch_move_sphere)(Lattice &L, const MoveArgs &m, int with_
 }
 
 cudaError_t SLBC_FN(launch_velocity)(Lattice &L, double fac, float *u, float *drho) {
-  const int blocks = (int)std::min<long long>((L.nnodes + 255) / 256, 152LL * 16);
-  k_velocity<T_><<<blocks, 256, 0, L.stream>>>(pop_args(L), L.layout, L.par.rho0, fac, L.bf_uniform, L.bf_const[0],
-                                               L.bf_const[1], L.bf_const[2], (const T_ *)L.bf, u, drho);
+  FieldArgs f;
+  f.rho0 = L.par.rho0;
+  f.fac = fac;
+  f.fac_f = (float)fac;
+  f.rho0_h = (float)f.rho0;
+  f.rho0_l = (float)(f.rho0 - f.rho0_h);
+  f.bf_uniform = L.bf_uniform;
+  for (int c = 0; c < 3; c++) {
+    f.fb[c] = fac * L.bf_const[c];
+    f.fb_h[c] = (float)f.fb[c];
+    f.fb_l[c] = (float)(f.fb[c] - f.fb_h[c]);
+  }
+  const int bx = L.esk >= 256 ? 256 : L.esk >= 128 ? 128 : L.esk > 32 ? 64 : 32;
+  const auto go = [&](auto kernel) {
+    kernel<<<row_grid(L, bx), bx, 0, L.stream>>>(pop_args(L), f, (const T_ *)L.bf, u, drho);
+  };
+  if (L.layout == SLBC_LAYOUT_N) go(k_velocity<T_, SLBC_LAYOUT_N>);
+  else if (L.layout == SLBC_LAYOUT_C0) go(k_velocity<T_, SLBC_LAYOUT_C0>);
+  else go(k_velocity<T_, SLBC_LAYOUT_C1>);
   count_launch();
   return cudaGetLastError();
 }

@@ -107,8 +107,13 @@ cudaError_t launch(const void *pop, long long npad, int layout, const unsigned s
   p.npad = npad;
   p.flags = (const uint16_t *)flags;
   p.esi = esi; p.esj = esj; p.esk = esk;
-  slbc::k_vsum<T><<<nblocks, slbc::kReduceThreads, 0, st>>>(p, layout, rho0, fac, bf == nullptr,
-                                                             bx, by, bz, (const T *)bf, psi, scratch);
+  const auto go = [&](auto kernel) {
+    kernel<<<nblocks, slbc::kReduceThreads, 0, st>>>(p, rho0, fac, bf == nullptr, bx, by, bz, (const T *)bf, psi,
+                                                     scratch);
+  };
+  if (layout == SLBC_LAYOUT_N) go(slbc::k_vsum<T, SLBC_LAYOUT_N>);
+  else if (layout == SLBC_LAYOUT_C0) go(slbc::k_vsum<T, SLBC_LAYOUT_C0>);
+  else go(slbc::k_vsum<T, SLBC_LAYOUT_C1>);
   slbc::count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
