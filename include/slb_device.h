@@ -321,6 +321,12 @@ int slbc_tc_wgrad(const void *dy0, const void *dy1, const void *dy2, const void 
  * go to dst[t][copy][c][64] (ncopy copies side by side per tile). */
 int slbc_tc_cmajor_tiles(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
                          long long pstride, int shift, int copy, int ncopy, void *dst, void *stream);
+/* The three copies of an output gradient at shifts -1, 0, 1 in one pass over
+ * it: with tiles as K-tile blocks dst[t][3][c][64] (three calls of
+ * slbc_tc_cmajor_tiles), else as channel-major copies nch * B * pstride
+ * elements apart (three of slbc_tc_cmajor). */
+int slbc_tc_cmajor_shifts(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
+                          long long pstride, int tiles, void *dst, void *stream);
 /* slbc_tc_wgrad with dY's three copies as K-tile blocks dyt[t][3][cout][64]
  * (slbc_tc_cmajor_tiles, copy = shift + 1, ncopy 3): one tile's operand is
  * one contiguous block of memory.  cout 32, 64 or 128. */

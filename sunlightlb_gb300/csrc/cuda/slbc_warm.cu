@@ -995,65 +995,99 @@ __global__ void k_sum_splits(const float *partial, long long n, int splits, floa
   }
 }
 
-// Channel-major flat copy of channels [coff, coff + nch) of a padded
+// Channel-major flat copies of channels [coff, coff + nch) of a padded
 // channels-last buffer: dst[c][n * pstride + (z * (H + 2) + y) * Wp + x] =
 // src[n][z][y][x - shift][coff + c] for 0 <= x - shift <= W + 1 (0 beyond;
-// zero_halo: interior voxels only, every halo position 0); with ncopy > 0
-// the 64-position rows go to K-tile blocks instead, dst[t][copy][c][64]
+// zero_halo: interior voxels only, every halo position 0), copy_stride
+// elements apart for the NC copies at shift, shift + 1, ...; with ncopy > 0
+// the 64-position rows go to K-tile blocks instead, dst[t][copy + i][c][64]
 // for t = flat position / 64 (the three x-shifted copies of an output
 // gradient side by side per tile: one contiguous 12 KB block of DRAM per
-// 32-channel tile for the weight gradient's A operand).  A block moves
-// 64 consecutive flat positions x 64 channels through shared memory, so
-// both the channel runs it reads and the position runs it writes are
-// 128-byte rows.
-__global__ void __launch_bounds__(256) k_cmajor(const __nv_bfloat16 *src, int B, int D, int H, int W, int ctot,
-                                                int coff, int nch, int Wp, long long pstride, int shift,
-                                                int zero_halo, int copy, int ncopy, __nv_bfloat16 *dst) {
-  __shared__ __nv_bfloat16 tile[64][64 + 8];
-  const long long plane = (long long)(H + 2) * Wp;
-  const long long per_sample = (long long)(D + 2) * plane;
+// 32-channel tile for the weight gradient's A operand).
+//
+// A block moves 256 consecutive flat positions x 32 channels: the voxels
+// (and one to either side for the shifted copies) come into shared memory as
+// channel rows, 16 bytes per access, and leave through transposing matrix
+// loads whose row addresses carry the shift, so the source is read once for
+// all copies; four lanes exchange their pieces so that each writes 16 bytes
+// of one channel.  Each position's voxel is worked out once per block in
+// 32-bit arithmetic.  Bound: HBM (the copies written).  Before, one copy per
+// launch with 64-bit divisions per access and 2-byte shared stores: 2.75 ms
+// of a training iteration of 4 x 64^3.
+constexpr int kCmPos = 256, kCmPitch = 80;  // bytes per row of 32 channels: 8 rows hit 8 different bank groups
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_cmajor(const __nv_bfloat16 *src, int B, int D, int H, int W, int ctot, int coff,
+                                                int nch, int Wp, int pstride, int shift, int zero_halo, int copy, int ncopy,
+                                                long long copy_stride, __nv_bfloat16 *dst) {
+  __shared__ __align__(16) unsigned char rows[(kCmPos + 3) * kCmPitch];  // positions -1 .. 256, and a row of zeros
+  __shared__ int voxel[kCmPos + 2];
+  __shared__ short xs[kCmPos + 2];
+  constexpr int kZero = kCmPos + 2;
+  const int plane = (H + 2) * Wp, per_sample = (D + 2) * plane;
   const long long total = (long long)B * pstride;
-  const long long ntiles = total / 64;
-  const int nck = (nch + 63) / 64;
-  for (long long work = blockIdx.x; work < ntiles * nck; work += gridDim.x) {
-    const long long t = work / nck;
-    const int c0 = (int)(work % nck) * 64;
-    const int cw = nch - c0 < 64 ? nch - c0 : 64;
-    // load: 64 positions x cw channels, 8 channels (16 B) per thread access
-    for (int a = threadIdx.x; a < 64 * 8; a += blockDim.x) {
-      const int pos = a / 8, cv = a % 8;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (cv * 8 < cw) {
-        const long long e = t * 64 + pos;
-        const int n = (int)(e / pstride);
-        const long long f = e % pstride;
+  const int nblk = (int)((total + kCmPos - 1) / kCmPos), nck = (nch + 31) / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kCmPitch / 4) ((unsigned *)(rows + kZero * kCmPitch))[threadIdx.x] = 0u;
+  for (int work = blockIdx.x; work < nblk * nck; work += gridDim.x) {
+    const int blk = work / nck, c0 = (work - blk * nck) * 32;
+    const int cw = min(32, nch - c0);
+    const long long e0 = (long long)blk * kCmPos;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kCmPos + 2; i += 256) {
+      const long long e = e0 + i - 1;
+      int v = -1, x = -0x4000;  // no voxel there
+      if (e >= 0 && e < total) {
+        const int n = (int)(e / pstride), f = (int)(e - (long long)n * pstride);
         if (f < per_sample) {
-          const int z = (int)(f / plane);
-          const long long r = f % plane;
-          const int y = (int)(r / Wp);
-          const int x = (int)(r % Wp) - shift;
-          bool in = x >= 0 && x <= W + 1;
+          const int z = f / plane, r = f - z * plane, y = r / Wp;
+          x = r - y * Wp;
+          bool in = x <= W + 1;
           if (zero_halo) in = in && x >= 1 && x <= W && y >= 1 && y <= H && z >= 1 && z <= D;
-          if (in)
-            v = *(const uint4 *)(src + ((((long long)n * (D + 2) + z) * (H + 2) + y) * (W + 2) + x) * ctot + coff +
-                                 c0 + cv * 8);
+          if (in) v = ((n * (D + 2) + z) * (H + 2) + y) * (W + 2) + x;
         }
       }
-      const __nv_bfloat16 *vb = (const __nv_bfloat16 *)&v;
+      voxel[i] = v;
+      xs[i] = (short)x;
+    }
+    __syncthreads();
+    for (int a = threadIdx.x; a < (kCmPos + 2) * 4; a += 256) {
+      const int i = a >> 2, cv = a & 3, v = voxel[i];
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (v >= 0 && 8 * cv < cw) u = *(const uint4 *)(src + (long long)v * ctot + coff + c0 + 8 * cv);
+      *(uint4 *)(rows + i * kCmPitch + 16 * cv) = u;
+    }
+    __syncthreads();
+    // warp w transposes positions [32 w, 32 w + 32), 8 channels at a time
 #pragma unroll
-      for (int i = 0; i < 8; i++) tile[cv * 8 + i][pos] = vb[i];
+    for (int i = 0; i < NC; i++) {
+      const int s = shift + i;
+      // this lane's row address: position 32 w + lane, moved by the shift
+      const int p = 32 * warp + lane, xsrc = xs[p + 1] - s;
+      const int row = xsrc >= 0 && xsrc <= W + 1 ? p + 1 - s : kZero;
+      const uint32_t at = tc::smem_u32(rows + row * kCmPitch);
+      for (int cv = 0; 8 * cv < cw; cv++) {
+        unsigned r0, r1, r2, r3;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                     : "r"(at + 16 * cv));
+        // lane 4 c + q holds positions 8 j + 2 q, + 1 of channel c in r_j:
+        // exchange so that it holds positions 8 q .. 8 q + 7
+        const bool q1 = lane & 1, q2 = lane & 2;
+        unsigned a = __shfl_xor_sync(0xffffffffu, q1 ? r0 : r1, 1), b = __shfl_xor_sync(0xffffffffu, q1 ? r2 : r3, 1);
+        if (q1) { r0 = a; r2 = b; } else { r1 = a; r3 = b; }
+        a = __shfl_xor_sync(0xffffffffu, q2 ? r0 : r2, 2);
+        b = __shfl_xor_sync(0xffffffffu, q2 ? r1 : r3, 2);
+        if (q2) { r0 = a; r1 = b; } else { r2 = a; r3 = b; }
+        const int c = c0 + 8 * cv + (lane >> 2);
+        const long long e = e0 + 32 * warp + 8 * (lane & 3);
+        if (e < total) {
+          const long long o = ncopy ? (((e >> 6) * ncopy + copy + i) * nch + c) * 64 + (e & 63)
+                                    : (long long)i * copy_stride + (long long)c * total + e;
+          *(uint4 *)(dst + o) = make_uint4(r0, r1, r2, r3);
+        }
+      }
     }
-    __syncthreads();
-    // store: per channel 64 positions = 128 B, 16 B per thread access
-    for (int a = threadIdx.x; a < 64 * 8; a += blockDim.x) {
-      const int c = a / 8, pv = a % 8;
-      if (c >= cw) continue;
-      // channel-major row, or (ncopy > 0) row c of copy `copy` in the
-      // block of K tile t: [t][copy][c][64]
-      const long long o = ncopy ? ((t * ncopy + copy) * nch + c0 + c) * 64 : (long long)(c0 + c) * total + t * 64;
-      *(uint4 *)(dst + o + pv * 8) = *(const uint4 *)&tile[c][pv * 8];
-    }
-    __syncthreads();
   }
 }
 
@@ -1119,17 +1153,27 @@ bool tile_shape(int D, int H, int W, int &wbox, int &hbox, int &dbox) {
          hbox <= 256 && dbox <= 256;
 }
 
+// nc copies (1 or 3) at shift, shift + 1, ...
 int cmajor_launch(const char *who, const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
-                  long long pstride, int shift, int zero_halo, int copy, int ncopy, void *dst, void *stream) {
+                  long long pstride, int shift, int nc, int zero_halo, int copy, int ncopy, long long copy_stride,
+                  void *dst, void *stream) {
   if (B < 1 || nch < 1 || coff < 0 || coff + nch > ctot || Wp < W + 2 || Wp % 8 || pstride % 64 ||
-      pstride < (long long)(D + 2) * (H + 2) * Wp || shift < -1 || shift > 1)
+      pstride < (long long)(D + 2) * (H + 2) * Wp || shift < -1 || shift + nc - 1 > 1)
     return slbc::set_error(std::string(who) + ": bad geometry"), 1;
   if (nch % 8 || coff % 8 || ctot % 8 || !aligned16(src) || !aligned16(dst))
     return slbc::set_error(std::string(who) + ": channels in multiples of 8, 16-byte aligned buffers"), 1;
-  const long long work = (long long)B * pstride / 64 * ((nch + 63) / 64);
-  const int blocks = (int)std::min<long long>(work, 152LL * 16);
-  k_cmajor<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)src, B, D, H, W, ctot, coff, nch, Wp,
-                                                     pstride, shift, zero_halo, copy, ncopy, (__nv_bfloat16 *)dst);
+  if (pstride >= 1LL << 31 || (long long)B * (D + 2) * (H + 2) * (W + 2) >= 1LL << 31 || W >= 0x3fff)
+    return slbc::set_error(std::string(who) + ": grid too large"), 1;
+  const long long work = ((long long)B * pstride + kCmPos - 1) / kCmPos * ((nch + 31) / 32);
+  if (work >= 1LL << 31) return slbc::set_error(std::string(who) + ": grid too large"), 1;
+  const int blocks = (int)std::min<long long>(work, 152LL * 8);
+  const auto go = [&](auto kernel) {
+    kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)src, B, D, H, W, ctot, coff, nch, Wp,
+                                                     (int)pstride, shift, zero_halo, copy, ncopy, copy_stride,
+                                                     (__nv_bfloat16 *)dst);
+  };
+  if (nc == 3) go(k_cmajor<3>);
+  else go(k_cmajor<1>);
   slbc::count_launch();
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string(who) + ": " + cudaGetErrorString(e)), 1;
@@ -1376,16 +1420,22 @@ int slbc_tc_halo(void *buf, int B, int D, int H, int W, int ctot, int coff, int 
 
 int slbc_tc_cmajor(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
                    long long pstride, int shift, int zero_halo, void *dst, void *stream) {
-  return cmajor_launch("slbc_tc_cmajor", src, B, D, H, W, ctot, coff, nch, Wp, pstride, shift, zero_halo, 0, 0, dst,
-                       stream);
+  return cmajor_launch("slbc_tc_cmajor", src, B, D, H, W, ctot, coff, nch, Wp, pstride, shift, 1, zero_halo, 0, 0, 0,
+                       dst, stream);
 }
 
 int slbc_tc_cmajor_tiles(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
                          long long pstride, int shift, int copy, int ncopy, void *dst, void *stream) {
   if (ncopy < 1 || copy < 0 || copy >= ncopy)
     return slbc::set_error("slbc_tc_cmajor_tiles: copy must lie in [0, ncopy)"), 1;
-  return cmajor_launch("slbc_tc_cmajor_tiles", src, B, D, H, W, ctot, coff, nch, Wp, pstride, shift, 0, copy, ncopy,
-                       dst, stream);
+  return cmajor_launch("slbc_tc_cmajor_tiles", src, B, D, H, W, ctot, coff, nch, Wp, pstride, shift, 1, 0, copy, ncopy,
+                       0, dst, stream);
+}
+
+int slbc_tc_cmajor_shifts(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp,
+                          long long pstride, int tiles, void *dst, void *stream) {
+  return cmajor_launch("slbc_tc_cmajor_shifts", src, B, D, H, W, ctot, coff, nch, Wp, pstride, -1, 3, 0, 0, tiles ? 3 : 0,
+                       (long long)nch * B * pstride, dst, stream);
 }
 
 int slbc_tc_wgrad_splits(int cin, int cout, long long k_tiles, long long max_splits) {

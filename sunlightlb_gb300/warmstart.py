@@ -57,6 +57,7 @@ class Kernels:
             "slbc_nn_up_bwd": [p, i, i, p, i, i, p, i, i] + [i] * 5 + [p],
             "slbc_nn_bias_grad": [p, i, i] + [i] * 5 + [p, p],
             "slbc_nn_wfwd": [p, i, i, p, p],
+            "slbc_tc_cmajor_shifts": [p, i, i, i, i, i, i, i, i, ll, i, p, p],
             "slbc_nn_wdgrad": [p, i, i, i, i, p, p],
             "slbc_nn_adam": [p, p, p, p, ll, f, f, f, f, i, p],
             "slbc_nn_mse": [p, i, p, i, p, i, i, i, i, p, i, p, p],
@@ -276,13 +277,8 @@ class UNet:
         tiles = cout <= 128
         n = cout * self.B * ps
         cm_g = [self.cm_g[i * n:(i + 1) * n] for i in range(3)]
-        for i, shift in enumerate((-1, 0, 1)):
-            if tiles:
-                k.tc_cmajor_tiles(g.data_ptr(), self.B, d, h, w, g.shape[-1], 0, cout, Wp, ps, shift, i, 3,
-                                  self.cm_g.data_ptr(), self.stream)
-            else:
-                k.tc_cmajor(g.data_ptr(), self.B, d, h, w, g.shape[-1], 0, cout, Wp, ps, shift, 0,
-                            cm_g[i].data_ptr(), self.stream)
+        k.tc_cmajor_shifts(g.data_ptr(), self.B, d, h, w, g.shape[-1], 0, cout, Wp, ps, int(tiles),
+                           self.cm_g.data_ptr(), self.stream)
         k.tc_cmajor(x.data_ptr(), self.B, d, h, w, x.shape[-1], x_coff, cin, Wp, ps, 0, 1, self.cm_x.data_ptr(),
                     self.stream)
         splits = k.tc_wgrad_splits(cin, cout, self.B * ps // 64, self.ws_floats // (27 * cout * cin))
