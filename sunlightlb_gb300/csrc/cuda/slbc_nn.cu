@@ -48,139 +48,187 @@ __device__ __forceinline__ void store8(bf16 *p, const float (&v)[8]) {
 
 int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 152LL * 32); }
 
+// The kernels over voxels walk the grid row by row (a row: W voxels times the
+// 16-byte vectors of a voxel): a block takes one long row or several short
+// ones at a time, so a thread divides once per row in 32 bits instead of four
+// times per vector in 64 bits, which bounded these kernels at a third to a
+// fifth of the memory rate.
+struct RowWalk {
+  int row, step, e;  // first row of this thread, rows between its turns, first element in the row
+};
+
+__device__ __forceinline__ RowWalk row_walk(int rowlen) {
+  RowWalk w;
+  if (rowlen >= 256) {
+    w.row = blockIdx.x;
+    w.step = gridDim.x;
+    w.e = threadIdx.x;
+  } else {
+    const int per = 256 / rowlen, sub = (int)threadIdx.x / rowlen;
+    w.e = (int)threadIdx.x - sub * rowlen;
+    w.row = sub < per ? (int)blockIdx.x * per + sub : 0x7fffffff;
+    w.step = (int)gridDim.x * per;
+  }
+  return w;
+}
+
+int rows_grid(long long rows, int rowlen) {
+  const int per = rowlen >= 256 ? 1 : 256 / rowlen;
+  return (int)std::max<long long>(1, std::min<long long>((rows + per - 1) / per, 152LL * 16));
+}
+
+__device__ __forceinline__ void row_of(int row, int D, int H, int &n, int &z, int &y) {
+  const int t = row / H;
+  y = row - t * H;
+  n = t / D;
+  z = t - n * D;
+}
+
 // 2x2x2 average of the fine interior (D, H, W) into the coarse interior
-__global__ void k_pool(Slice in, Slice out, int B, int D, int H, int W, int C) {
-  const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8;
-  const long long total = (long long)B * Dc * Hc * Wc * nv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int cv = (int)(e % nv);
-    long long r = e / nv;
-    const int x = (int)(r % Wc); r /= Wc;
-    const int y = (int)(r % Hc); r /= Hc;
-    const int z = (int)(r % Dc);
-    const int n = (int)(r / Dc);
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+__global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D, int H, int W, int C) {
+  const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
+  const RowWalk w = row_walk(len);
+  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+    int n, z, y;
+    row_of(row, Dc, Hc, n, z, y);
+    const bf16 *src = in.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * in.ctot + in.coff;
+    bf16 *dst = out.p + vox(n, z, y, 0, Dc, Hc, Wc) * out.ctot + out.coff;
+    const long long py = (long long)(W + 2) * in.ctot, pz = (H + 2) * py;
+    for (int e = w.e; e < len; e += 256) {
+      const int x = e / nv, cv = e - x * nv;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      float v[8];
-      load8(in.p + vox(n, 2 * z + (c >> 2), 2 * y + ((c >> 1) & 1), 2 * x + (c & 1), D, H, W) * in.ctot + in.coff +
-                8 * cv,
-            v);
+      for (int c = 0; c < 8; c++) {
+        float v[8];
+        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * in.ctot + 8 * cv, v);
 #pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += v[i];
+        for (int i = 0; i < 8; i++) acc[i] += v[i];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) acc[i] *= 0.125f;
+      store8(dst + (long long)x * out.ctot + 8 * cv, acc);
     }
-#pragma unroll
-    for (int i = 0; i < 8; i++) acc[i] *= 0.125f;
-    store8(out.p + vox(n, z, y, x, Dc, Hc, Wc) * out.ctot + out.coff + 8 * cv, acc);
   }
 }
 
 // gradient of k_pool: dfine = (dcoarse / 8 + add) * (mask > 0); add and mask
 // optional (null pointers)
-__global__ void k_pool_bwd(Slice dcoarse, Slice dfine, Slice add, Slice mask, int B, int D, int H, int W, int C) {
-  const int nv = C / 8;
-  const long long total = (long long)B * D * H * W * nv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int cv = (int)(e % nv);
-    long long r = e / nv;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H); r /= H;
-    const int z = (int)(r % D);
-    const int n = (int)(r / D);
-    float g[8];
-    load8(dcoarse.p + vox(n, z / 2, y / 2, x / 2, D / 2, H / 2, W / 2) * dcoarse.ctot + dcoarse.coff + 8 * cv, g);
+__global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Slice add, Slice mask, int B, int D,
+                                                  int H, int W, int C) {
+  const int nv = C / 8, len = W * nv;
+  const RowWalk w = row_walk(len);
+  for (int row = w.row; row < B * D * H; row += w.step) {
+    int n, z, y;
+    row_of(row, D, H, n, z, y);
+    const bf16 *src = dcoarse.p + vox(n, z / 2, y / 2, 0, D / 2, H / 2, W / 2) * dcoarse.ctot + dcoarse.coff;
+    const long long v0 = vox(n, z, y, 0, D, H, W);
+    for (int e = w.e; e < len; e += 256) {
+      const int x = e / nv, cv = e - x * nv;
+      float g[8];
+      load8(src + (long long)(x / 2) * dcoarse.ctot + 8 * cv, g);
 #pragma unroll
-    for (int i = 0; i < 8; i++) g[i] *= 0.125f;
-    const long long v = vox(n, z, y, x, D, H, W);
-    if (add.p) {
-      float a[8];
-      load8(add.p + v * add.ctot + add.coff + 8 * cv, a);
+      for (int i = 0; i < 8; i++) g[i] *= 0.125f;
+      const long long v = v0 + x;
+      if (add.p) {
+        float a[8];
+        load8(add.p + v * add.ctot + add.coff + 8 * cv, a);
 #pragma unroll
-      for (int i = 0; i < 8; i++) g[i] += a[i];
+        for (int i = 0; i < 8; i++) g[i] += a[i];
+      }
+      if (mask.p) {
+        float m[8];
+        load8(mask.p + v * mask.ctot + mask.coff + 8 * cv, m);
+#pragma unroll
+        for (int i = 0; i < 8; i++) g[i] = m[i] > 0.0f ? g[i] : 0.0f;
+      }
+      store8(dfine.p + v * dfine.ctot + dfine.coff + 8 * cv, g);
     }
-    if (mask.p) {
-      float m[8];
-      load8(mask.p + v * mask.ctot + mask.coff + 8 * cv, m);
-#pragma unroll
-      for (int i = 0; i < 8; i++) g[i] = m[i] > 0.0f ? g[i] : 0.0f;
-    }
-    store8(dfine.p + v * dfine.ctot + dfine.coff + 8 * cv, g);
   }
 }
 
-// nearest upsampling: fine (D, H, W) interior = coarse parent
-__global__ void k_up(Slice in, Slice out, int B, int D, int H, int W, int C) {
-  const int nv = C / 8;
-  const long long total = (long long)B * D * H * W * nv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int cv = (int)(e % nv);
-    long long r = e / nv;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H); r /= H;
-    const int z = (int)(r % D);
-    const int n = (int)(r / D);
-    *(uint4 *)(out.p + vox(n, z, y, x, D, H, W) * out.ctot + out.coff + 8 * cv) =
-        *(const uint4 *)(in.p + vox(n, z / 2, y / 2, x / 2, D / 2, H / 2, W / 2) * in.ctot + in.coff + 8 * cv);
+// nearest upsampling: fine (D, H, W) interior = coarse parent; a thread
+// reads its vector of the parent once and writes the eight children
+__global__ void __launch_bounds__(256) k_up(Slice in, Slice out, int B, int D, int H, int W, int C) {
+  const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
+  const RowWalk w = row_walk(len);
+  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+    int n, z, y;
+    row_of(row, Dc, Hc, n, z, y);
+    const bf16 *src = in.p + vox(n, z, y, 0, Dc, Hc, Wc) * in.ctot + in.coff;
+    bf16 *dst = out.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * out.ctot + out.coff;
+    const long long py = (long long)(W + 2) * out.ctot, pz = (H + 2) * py;
+    for (int e = w.e; e < len; e += 256) {
+      const int x = e / nv, cv = e - x * nv;
+      const uint4 v = *(const uint4 *)(src + (long long)x * in.ctot + 8 * cv);
+#pragma unroll
+      for (int c = 0; c < 8; c++)
+        *(uint4 *)(dst + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * out.ctot + 8 * cv) = v;
+    }
   }
 }
 
 // gradient of k_up: dcoarse = sum of the 8 children * (mask > 0) (coarse mask)
-__global__ void k_up_bwd(Slice dfine, Slice dcoarse, Slice mask, int B, int D, int H, int W, int C) {
-  const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8;
-  const long long total = (long long)B * Dc * Hc * Wc * nv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int cv = (int)(e % nv);
-    long long r = e / nv;
-    const int x = (int)(r % Wc); r /= Wc;
-    const int y = (int)(r % Hc); r /= Hc;
-    const int z = (int)(r % Dc);
-    const int n = (int)(r / Dc);
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+__global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slice mask, int B, int D, int H, int W, int C) {
+  const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
+  const RowWalk w = row_walk(len);
+  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+    int n, z, y;
+    row_of(row, Dc, Hc, n, z, y);
+    const bf16 *src = dfine.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * dfine.ctot + dfine.coff;
+    const long long py = (long long)(W + 2) * dfine.ctot, pz = (H + 2) * py;
+    const long long v0 = vox(n, z, y, 0, Dc, Hc, Wc);
+    for (int e = w.e; e < len; e += 256) {
+      const int x = e / nv, cv = e - x * nv;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      float v[8];
-      load8(dfine.p + vox(n, 2 * z + (c >> 2), 2 * y + ((c >> 1) & 1), 2 * x + (c & 1), D, H, W) * dfine.ctot +
-                dfine.coff + 8 * cv,
-            v);
+      for (int c = 0; c < 8; c++) {
+        float v[8];
+        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * dfine.ctot + 8 * cv, v);
 #pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += v[i];
+        for (int i = 0; i < 8; i++) acc[i] += v[i];
+      }
+      const long long v = v0 + x;
+      if (mask.p) {
+        float m[8];
+        load8(mask.p + v * mask.ctot + mask.coff + 8 * cv, m);
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = m[i] > 0.0f ? acc[i] : 0.0f;
+      }
+      store8(dcoarse.p + v * dcoarse.ctot + dcoarse.coff + 8 * cv, acc);
     }
-    const long long v = vox(n, z, y, x, Dc, Hc, Wc);
-    if (mask.p) {
-      float m[8];
-      load8(mask.p + v * mask.ctot + mask.coff + 8 * cv, m);
-#pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] = m[i] > 0.0f ? acc[i] : 0.0f;
-    }
-    store8(dcoarse.p + v * dcoarse.ctot + dcoarse.coff + 8 * cv, acc);
   }
 }
 
-// db[c] += sum over interior voxels of g.  The grid stride is a multiple of
-// C / 8, so a thread always handles the same 8 channels: it sums in
-// registers and adds to the block's shared sums once.
-__global__ void k_bias_grad(Slice g, int B, int D, int H, int W, int C, float *db) {
+// db[c] += sum over interior voxels of g.  256 is a multiple of C / 8, so a
+// thread always handles the same 8 channels: it sums whole rows in registers,
+// the lanes of a warp with the same channels are added by shuffles, and one
+// of them adds to the block's shared sums.
+__global__ void __launch_bounds__(256) k_bias_grad(Slice g, int B, int D, int H, int W, int C, float *db) {
   extern __shared__ float sh[];
   for (int c = threadIdx.x; c < C; c += blockDim.x) sh[c] = 0.0f;
   __syncthreads();
-  const int nv = C / 8;
-  const long long total = (long long)B * D * H * W * nv;
-  const long long start = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int cv = (int)(start % nv);
+  const int nv = C / 8, cv = threadIdx.x % nv, x0 = threadIdx.x / nv, dx = 256 / nv;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (long long e = start; e < total; e += (long long)gridDim.x * blockDim.x) {
-    long long r = e / nv;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H); r /= H;
-    const int z = (int)(r % D);
-    const int n = (int)(r / D);
-    float v[8];
-    load8(g.p + vox(n, z, y, x, D, H, W) * g.ctot + g.coff + 8 * cv, v);
+  // rows of voxels, several at a time where a row is shorter than the block's reach
+  const int per = W >= dx ? 1 : dx / W, sub = x0 / (W >= dx ? dx : W);
+  if (sub < per)
+    for (int row = (int)blockIdx.x * per + sub; row < B * D * H; row += (int)gridDim.x * per) {
+      int n, z, y;
+      row_of(row, D, H, n, z, y);
+      const bf16 *src = g.p + vox(n, z, y, 0, D, H, W) * g.ctot + g.coff + 8 * cv;
+      for (int x = W >= dx ? x0 : x0 - sub * W; x < W; x += dx) {
+        float v[8];
+        load8(src + (long long)x * g.ctot, v);
 #pragma unroll
-    for (int i = 0; i < 8; i++) acc[i] += v[i];
-  }
+        for (int i = 0; i < 8; i++) acc[i] += v[i];
+      }
+    }
+  for (int o = 16; o >= nv; o >>= 1)
 #pragma unroll
-  for (int i = 0; i < 8; i++) atomicAdd(&sh[8 * cv + i], acc[i]);
+    for (int i = 0; i < 8; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+  if ((int)(threadIdx.x & 31) < nv)
+#pragma unroll
+    for (int i = 0; i < 8; i++) atomicAdd(&sh[8 * cv + i], acc[i]);
   __syncthreads();
   for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&db[c], sh[c]);
 }
@@ -271,26 +319,27 @@ __global__ void k_scale(float *g, long long n, const double *state) {
 // in FP32 channels 0..nch-1 of a padded buffer (ctot_p channels), label
 // [n][D][H][W][nch] FP32; grad (BF16, gctot channels, padded) = d loss /
 // d pred in channels 0..nch-1, 0 in the others.  loss[0] += the sum / count.
-__global__ void k_mse(const float *pred, int ctot_p, const float *label, int nch, const float *sample_w, int B, int D,
-                      int H, int W, bf16 *grad, int gctot, double *loss) {
+__global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, const float *label, int nch,
+                                             const float *sample_w, int B, int D, int H, int W, bf16 *grad, int gctot,
+                                             double *loss) {
   __shared__ double sh[256];
-  const long long total = (long long)B * D * H * W;
-  const double inv = 1.0 / ((double)nch * (double)total);
+  const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   double acc = 0.0;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    long long r = e;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H); r /= H;
-    const int z = (int)(r % D);
-    const int n = (int)(r / D);
-    const long long v = vox(n, z, y, x, D, H, W);
+  const RowWalk w = row_walk(W);
+  for (int row = w.row; row < B * D * H; row += w.step) {
+    int n, z, y;
+    row_of(row, D, H, n, z, y);
+    const long long v0 = vox(n, z, y, 0, D, H, W), e0 = (long long)row * W;
     const float sw = sample_w ? sample_w[n] : 1.0f;
-    bf16 *gp = grad + v * gctot;
-    for (int c = 0; c < gctot; c += 8) *(uint4 *)(gp + c) = make_uint4(0, 0, 0, 0);
-    for (int c = 0; c < nch; c++) {
-      const float d = pred[v * ctot_p + c] - label[e * nch + c];
-      acc += (double)sw * d * d;
-      gp[c] = __float2bfloat16((float)(2.0 * inv) * sw * d);
+    for (int x = w.e; x < W; x += 256) {
+      const long long v = v0 + x;
+      bf16 *gp = grad + v * gctot;
+      for (int c = 0; c < gctot; c += 8) *(uint4 *)(gp + c) = make_uint4(0, 0, 0, 0);
+      for (int c = 0; c < nch; c++) {
+        const float d = pred[v * ctot_p + c] - label[(e0 + x) * nch + c];
+        acc += (double)sw * d * d;
+        gp[c] = __float2bfloat16((float)(2.0 * inv) * sw * d);
+      }
     }
   }
   sh[threadIdx.x] = acc;
@@ -365,55 +414,86 @@ constexpr int kDistR1 = 5, kDistR2 = 12;
 // one-axis passes (a minimum of sums is the nested minimum), each over
 // 2R + 1 neighbours instead of (2R + 1)^3.  Values stay integers, so the
 // result equals the cube search.
-// Pass 1 (along x, stride 1): nearest solid node on the row.
+// Pass 1 (along x): nearest solid node on the row, searched outwards.
 template <int R>
-__global__ void k_dist_x(const unsigned char *solid, long long total, int W, unsigned char *a) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(e % W);
-    const unsigned char *row = solid + (e - x);
-    int best = R * R;
-#pragma unroll
-    for (int dx = -R; dx <= R; dx++)
-      if (dx * dx < best && row[((x + dx) % W + W) % W]) best = dx * dx;
-    a[e] = (unsigned char)best;
+__global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int rows, int W, unsigned char *a) {
+  const RowWalk w = row_walk(W);
+  for (int row = w.row; row < rows; row += w.step) {
+    const unsigned char *src = solid + (long long)row * W;
+    unsigned char *dst = a + (long long)row * W;
+    for (int x = w.e; x < W; x += 256) {
+      int best = src[x] ? 0 : R * R;
+      if (W >= R) {
+        for (int d = 1; d < R && best == R * R; d++) {
+          const int l = x - d < 0 ? x - d + W : x - d, r = x + d >= W ? x + d - W : x + d;
+          if (src[l] | src[r]) best = d * d;
+        }
+      } else {
+        for (int d = 1; d < R && best == R * R; d++)
+          if (src[((x - d) % W + W) % W] | src[(x + d) % W]) best = d * d;
+      }
+      dst[x] = (unsigned char)best;
+    }
   }
 }
 
-// Passes 2 and 3 (along y, stride W, extent H; along z, stride W H,
-// extent D): b = min over |d| <= R of d^2 + a at the node d steps away.
-template <int R>
-__global__ void k_dist_min(const unsigned char *a, long long total, int n, long long stride, unsigned char *b) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)((e / stride) % n);
-    const unsigned char *col = a + (e - (long long)p * stride);
-    int best = R * R;
+// Passes 2 and 3 (along y: n = H rows of `inner` = W bytes; along z: n = D
+// planes of W H): b = min over |d| <= R of d^2 + a at the node d steps away.
+// A thread takes four neighbouring bytes where rows hold whole words (VEC 4;
+// squares up to 144 and values up to 144 add without overflow in a byte
+// under saturation, and the cap of R^2 absorbs it).
+template <int R, int VEC>
+__global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int lines, int n, int inner, unsigned char *b) {
+  const int len = inner / VEC;  // a line: the bytes of one p of one outer block
+  const RowWalk w = row_walk(len);
+  for (int line = w.row; line < lines; line += w.step) {
+    const int outer = line / n, p = line - outer * n;
+    const unsigned char *base = a + (long long)outer * n * inner;
+    for (int e = w.e; e < len; e += 256) {
+      unsigned best = VEC == 4 ? (unsigned)(R * R) * 0x01010101u : (unsigned)(R * R);
 #pragma unroll
-    for (int d = -R; d <= R; d++) best = min(best, d * d + (int)col[(long long)(((p + d) % n + n) % n) * stride]);
-    b[e] = (unsigned char)best;
+      for (int d = -R; d <= R; d++) {
+        int q = p + d;
+        if (n >= R) q = q < 0 ? q + n : q >= n ? q - n : q;
+        else q = (q % n + n) % n;
+        const unsigned char *at = base + (long long)q * inner + VEC * e;
+        if (VEC == 4) best = __vminu4(best, __vaddus4(*(const unsigned *)at, (unsigned)(d * d) * 0x01010101u));
+        else best = min(best, (unsigned)(d * d) + *at);
+      }
+      unsigned char *out = b + (long long)line * inner + VEC * e;
+      if (VEC == 4) *(unsigned *)out = best;
+      else *out = (unsigned char)best;
+    }
   }
 }
 
 // dist2: the squared distances of the passes above (null without features),
 // searched to radius R
-__global__ void k_encode(const unsigned char *solid, const unsigned char *dist2, int R, int B, int D, int H, int W,
-                         bf16 *out, int ctot) {
-  const long long total = (long long)B * D * H * W;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    long long r = e;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H); r /= H;
-    const int z = (int)(r % D);
-    const int n = (int)(r / D);
-    bf16 *p = out + vox(n, z, y, x, D, H, W) * ctot;
-    for (int c = 0; c < ctot; c += 8) *(uint4 *)(p + c) = make_uint4(0, 0, 0, 0);
-    const bool s = solid[e] != 0;
-    p[0] = __float2bfloat16(s ? 1.0f : 0.0f);
-    if (dist2 && !s) {
-      const float dist = sqrtf((float)dist2[e]);
-      const float d = dist * (1.0f / (float)R);
-      p[1] = __float2bfloat16(d);
-      p[2] = __float2bfloat16(d * d);
-      if (R != kDistR1) p[3] = __float2bfloat16(fminf(dist, (float)kDistR1) * (1.0f / kDistR1));
+__global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, const unsigned char *dist2, int R, int B,
+                                                int D, int H, int W, bf16 *out, int ctot) {
+  const int nv = ctot / 8, len = W * nv;
+  const RowWalk w = row_walk(len);
+  for (int row = w.row; row < B * D * H; row += w.step) {
+    int n, z, y;
+    row_of(row, D, H, n, z, y);
+    bf16 *dst = out + vox(n, z, y, 0, D, H, W) * ctot;
+    const long long e0 = (long long)row * W;
+    for (int e = w.e; e < len; e += 256) {
+      const int x = e / nv, cv = e - x * nv;
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (cv == 0) {
+        bf16 *p = (bf16 *)&u;
+        const bool s = solid[e0 + x] != 0;
+        p[0] = __float2bfloat16(s ? 1.0f : 0.0f);
+        if (dist2 && !s) {
+          const float dist = sqrtf((float)dist2[e0 + x]);
+          const float d = dist * (1.0f / (float)R);
+          p[1] = __float2bfloat16(d);
+          p[2] = __float2bfloat16(d * d);
+          if (R != kDistR1) p[3] = __float2bfloat16(fminf(dist, (float)kDistR1) * (1.0f / kDistR1));
+        }
+      }
+      *(uint4 *)(dst + (long long)x * ctot + 8 * cv) = u;
     }
   }
 }
@@ -422,18 +502,23 @@ __global__ void k_encode(const unsigned char *solid, const unsigned char *dist2,
 // nodes into three FP32 arrays u[c * N + e] (0 on solid nodes), the layout
 // of lbsetveldev; shift_x is subtracted from u_x on fluid nodes.  With
 // drho, channel 3 * drho_scale into drho[e] (0 on solid nodes).
-__global__ void k_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H, int W, float scale,
-                         float shift_x, float *u, float drho_scale, float *drho) {
+__global__ void __launch_bounds__(256) k_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H,
+                                                int W, float scale, float shift_x, float *u, float drho_scale,
+                                                float *drho) {
   const long long total = (long long)D * H * W;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    long long r = e;
-    const int x = (int)(r % W); r /= W;
-    const int y = (int)(r % H);
-    const int z = (int)(r / H);
-    const long long v = vox(0, z, y, x, D, H, W);
+  const RowWalk w = row_walk(W);
+  for (int row = w.row; row < D * H; row += w.step) {
+    int n, z, y;
+    row_of(row, D, H, n, z, y);
+    const float *src = pred + vox(0, z, y, 0, D, H, W) * ctot_p;
+    for (int x = w.e; x < W; x += 256) {
+      const long long e = (long long)row * W + x;
+      const float *v = src + (long long)x * ctot_p;
+      const bool s = solid[e] != 0;
 #pragma unroll
-    for (int c = 0; c < 3; c++) u[c * total + e] = solid[e] ? 0.0f : scale * pred[v * ctot_p + c] - (c == 0 ? shift_x : 0.0f);
-    if (drho) drho[e] = solid[e] ? 0.0f : drho_scale * pred[v * ctot_p + 3];
+      for (int c = 0; c < 3; c++) u[c * total + e] = s ? 0.0f : scale * v[c] - (c == 0 ? shift_x : 0.0f);
+      if (drho) drho[e] = s ? 0.0f : drho_scale * v[3];
+    }
   }
 }
 
@@ -454,35 +539,78 @@ __global__ void __launch_bounds__(256) k_plane_sum(const float *u, int D, long l
   if (threadIdx.x == 0) q[i] = sh[0];
 }
 
-// One thread: the harmonic mean qh of the plane fluxes, the scale qh / q[i]
+// One block: the harmonic mean qh of the plane fluxes, the scale qh / q[i]
 // of every plane and the pressure p[i] = sum over the planes before i of
 // force (1 - qh / q) (midpoint rule, zero mean), both times gain; work =
 // [q | scale | p | spread].  Any plane flux <= 0 leaves the planes as they
-// are (scale = gain, p 0).
-__global__ void k_plane_fix(int D, float force, float gain, double *work) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double *q = work, *scale = work + D, *p = work + 2 * D;
+// are (scale = gain, p 0).  Thread t takes a run of consecutive planes; the
+// runs' sums are scanned in thread order (one thread alone spent 127 us on
+// the divisions of 128 planes).
+__global__ void __launch_bounds__(256) k_plane_fix(int D, float force, float gain, double *work) {
+  __shared__ double sa[256], sb[256], lo[256], hi[256];
+  __shared__ int all_ok;
+  const double *q = work;
+  double *scale = work + D, *p = work + 2 * D;
+  const int t = threadIdx.x, run = (D + 255) / 256;
+  const int i0 = min(D, t * run), i1 = min(D, i0 + run);
+  if (t == 0) all_ok = 1;
+  __syncthreads();
+  double inv = 0.0, qsum = 0.0, qmin = q[min(i0, D - 1)], qmax = qmin;
   bool ok = true;
-  double inv = 0.0, qmin = q[0], qmax = q[0], qsum = 0.0;
-  for (int i = 0; i < D; i++) {
+  for (int i = i0; i < i1; i++) {
     ok = ok && q[i] > 0.0;
     inv += 1.0 / q[i];
     qmin = fmin(qmin, q[i]);
     qmax = fmax(qmax, q[i]);
     qsum += q[i];
   }
-  work[3 * D] = ok ? (qmax - qmin) / (qsum / D) : -1.0;
-  const double qh = D / inv;
-  double acc = 0.0, mean = 0.0;
-  for (int i = 0; i < D; i++) {
-    const double g = ok ? (double)force * (1.0 - qh / q[i]) : 0.0;
+  if (!ok) all_ok = 0;
+  sa[t] = inv;
+  sb[t] = qsum;
+  lo[t] = qmin;
+  hi[t] = qmax;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (t < o) {
+      sa[t] += sa[t + o];
+      sb[t] += sb[t + o];
+      lo[t] = fmin(lo[t], lo[t + o]);
+      hi[t] = fmax(hi[t], hi[t + o]);
+    }
+    __syncthreads();
+  }
+  ok = all_ok != 0;
+  const double qh = D / sa[0];
+  if (t == 0) work[3 * D] = ok ? (hi[0] - lo[0]) / (sb[0] / D) : -1.0;
+  __syncthreads();
+  double mine = 0.0;
+  for (int i = i0; i < i1; i++) {
     scale[i] = (ok ? qh / q[i] : 1.0) * gain;
+    mine += ok ? (double)force * (1.0 - qh / q[i]) : 0.0;
+  }
+  sa[t] = mine;
+  __syncthreads();
+  for (int o = 1; o < 256; o <<= 1) {  // inclusive scan of the runs
+    const double add = t >= o ? sa[t - o] : 0.0;
+    __syncthreads();
+    sa[t] += add;
+    __syncthreads();
+  }
+  double acc = t > 0 ? sa[t - 1] : 0.0, mean = 0.0;
+  for (int i = i0; i < i1; i++) {
+    const double g = ok ? (double)force * (1.0 - qh / q[i]) : 0.0;
     p[i] = acc + 0.5 * g;
     acc += g;
     mean += p[i];
   }
-  mean /= D;
-  for (int i = 0; i < D; i++) p[i] = (p[i] - mean) * gain;
+  sb[t] = mean;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (t < o) sb[t] += sb[t + o];
+    __syncthreads();
+  }
+  mean = sb[0] / D;
+  for (int i = i0; i < i1; i++) p[i] = (p[i] - mean) * gain;
 }
 
 // u[c][x] *= scale[i]; drho[x] = gain drho[x] + 3 p[i] on fluid nodes (p = rho / 3)
@@ -588,8 +716,7 @@ int slbc_nn_pool(const void *in, int in_ctot, int in_coff, void *out, int out_ct
                  int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool: channel slices must be multiples of 8 and the grid even");
-  const long long n = (long long)B * (D / 2) * (H / 2) * (W / 2) * (C / 8);
-  k_pool<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
+  k_pool<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
                                                         Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
   return launched("slbc_nn_pool");
 }
@@ -600,8 +727,7 @@ int slbc_nn_pool_bwd(const void *dcoarse, int dc_ctot, int dc_coff, void *dfine,
   if (!ok8(dc_ctot, dc_coff, C) || !ok8(df_ctot, df_coff, C) || (add && !ok8(a_ctot, a_coff, C)) ||
       (mask && !ok8(m_ctot, m_coff, C)) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool_bwd: channel slices must be multiples of 8 and the grid even");
-  const long long n = (long long)B * D * H * W * (C / 8);
-  k_pool_bwd<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(
+  k_pool_bwd<<<rows_grid((long long)B * D * H, W * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
       Slice{(bf16 *)dcoarse, dc_ctot, dc_coff}, Slice{(bf16 *)dfine, df_ctot, df_coff},
       Slice{(bf16 *)add, a_ctot, a_coff}, Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
   return launched("slbc_nn_pool_bwd");
@@ -611,8 +737,7 @@ int slbc_nn_up(const void *in, int in_ctot, int in_coff, void *out, int out_ctot
                int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_up: channel slices must be multiples of 8 and the grid even");
-  const long long n = (long long)B * D * H * W * (C / 8);
-  k_up<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
+  k_up<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
                                                       Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
   return launched("slbc_nn_up");
 }
@@ -622,8 +747,7 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
   if (!ok8(df_ctot, df_coff, C) || !ok8(dc_ctot, dc_coff, C) || (mask && !ok8(m_ctot, m_coff, C)) || D % 2 ||
       H % 2 || W % 2)
     return bad("slbc_nn_up_bwd: channel slices must be multiples of 8 and the grid even");
-  const long long n = (long long)B * (D / 2) * (H / 2) * (W / 2) * (C / 8);
-  k_up_bwd<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)dfine, df_ctot, df_coff},
+  k_up_bwd<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)dfine, df_ctot, df_coff},
                                                           Slice{(bf16 *)dcoarse, dc_ctot, dc_coff},
                                                           Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
   return launched("slbc_nn_up_bwd");
@@ -631,8 +755,7 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
 
 int slbc_nn_bias_grad(const void *g, int ctot, int coff, int B, int D, int H, int W, int C, float *db, void *stream) {
   if (!ok8(ctot, coff, C) || C > 1024 || 256 % (C / 8)) return bad("slbc_nn_bias_grad: bad channel slice");
-  const long long n = (long long)B * D * H * W * (C / 8);
-  k_bias_grad<<<std::min(grid_for(n), 152 * 4), 256, C * sizeof(float), (cudaStream_t)stream>>>(
+  k_bias_grad<<<std::min(rows_grid((long long)B * D * H, W * (C / 8)), 152 * 4), 256, C * sizeof(float), (cudaStream_t)stream>>>(
       Slice{(bf16 *)g, ctot, coff}, B, D, H, W, C, db);
   return launched("slbc_nn_bias_grad");
 }
@@ -678,7 +801,7 @@ int slbc_nn_scale(float *g, long long n, const double *state, void *stream) {
 int slbc_nn_mse(const float *pred, int ctot_p, const float *label, int nch, const float *sample_w, int B, int D, int H,
                 int W, void *grad, int gctot, double *loss, void *stream) {
   if (nch < 1 || ctot_p < nch || gctot % 8 || gctot < 8 || gctot < nch) return bad("slbc_nn_mse: bad channel counts");
-  k_mse<<<std::min(grid_for((long long)B * D * H * W), 152 * 4), 256, 0, (cudaStream_t)stream>>>(
+  k_mse<<<std::min(rows_grid((long long)B * D * H, W), 152 * 8), 256, 0, (cudaStream_t)stream>>>(
       pred, ctot_p, label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss);
   return launched("slbc_nn_mse");
 }
@@ -701,26 +824,32 @@ int slbc_nn_proj(const float *pred, int ctot_p, const float *label, int lch, int
 int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void *out, int ctot, int features,
                    void *stream) {
   if (ctot % 8 || ctot < 8) return bad("slbc_nn_encode: bad channel count");
+  if ((long long)B * D * H >= 1LL << 31) return bad("slbc_nn_encode: too many rows");
   const long long total = (long long)B * D * H * W;
   const cudaStream_t st = (cudaStream_t)stream;
   unsigned char *a = nullptr;
   if (features) {
     // two stream-ordered scratch masks of one byte per voxel
-    const cudaError_t e = cudaMallocAsync((void **)&a, 2 * total, st);
+    const cudaError_t e = cudaMallocAsync((void **)&a, 2 * ((total + 255) / 256 * 256), st);
     if (e != cudaSuccess) return bad((std::string("slbc_nn_encode scratch: ") + cudaGetErrorString(e)).c_str());
-    unsigned char *b = a + total;
+    // the second mask on a word boundary; whole words along x where W holds them
+    unsigned char *b = a + (total + 255) / 256 * 256;
+    const int vec = W % 4 == 0 ? 4 : 1;
+    const auto passes = [&](auto rx, auto ry, auto rz) {
+      rx<<<rows_grid((long long)B * D * H, W), 256, 0, st>>>(solid, B * D * H, W, a);
+      ry<<<rows_grid((long long)B * D * H, W / vec), 256, 0, st>>>(a, B * D * H, H, W, b);
+      rz<<<rows_grid((long long)B * D, W * H / vec), 256, 0, st>>>(b, B * D, D, W * H, a);
+    };
     if (features == 2) {
-      k_dist_x<kDistR2><<<grid_for(total), 256, 0, st>>>(solid, total, W, a);
-      k_dist_min<kDistR2><<<grid_for(total), 256, 0, st>>>(a, total, H, W, b);
-      k_dist_min<kDistR2><<<grid_for(total), 256, 0, st>>>(b, total, D, (long long)W * H, a);
+      if (vec == 4) passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 4>, k_dist_min<kDistR2, 4>);
+      else passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 1>, k_dist_min<kDistR2, 1>);
     } else {
-      k_dist_x<kDistR1><<<grid_for(total), 256, 0, st>>>(solid, total, W, a);
-      k_dist_min<kDistR1><<<grid_for(total), 256, 0, st>>>(a, total, H, W, b);
-      k_dist_min<kDistR1><<<grid_for(total), 256, 0, st>>>(b, total, D, (long long)W * H, a);
+      if (vec == 4) passes(k_dist_x<kDistR1>, k_dist_min<kDistR1, 4>, k_dist_min<kDistR1, 4>);
+      else passes(k_dist_x<kDistR1>, k_dist_min<kDistR1, 1>, k_dist_min<kDistR1, 1>);
     }
     slbc::count_launch(3);
   }
-  k_encode<<<grid_for(total), 256, 0, st>>>(solid, a, features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out,
+  k_encode<<<rows_grid((long long)B * D * H, W * (ctot / 8)), 256, 0, st>>>(solid, a, features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out,
                                             ctot);
   const int rc = launched("slbc_nn_encode");
   if (a) {
@@ -737,7 +866,7 @@ int slbc_nn_plane_flux(float *u, float *drho, const unsigned char *solid, int D,
   const long long plane = (long long)H * W;
   k_plane_sum<<<D, 256, 0, st>>>(u, D, plane, work);
   if (launched("slbc_nn_plane_flux")) return 1;
-  k_plane_fix<<<1, 32, 0, st>>>(D, force, gain, work);
+  k_plane_fix<<<1, 256, 0, st>>>(D, force, gain, work);
   if (launched("slbc_nn_plane_flux")) return 1;
   k_plane_apply<<<grid_for((long long)D * plane), 256, 0, st>>>(u, drho, solid, D, plane, gain, work);
   return launched("slbc_nn_plane_flux");
@@ -757,7 +886,7 @@ int slbc_nn_cross_flux(float *u, int D, int H, int W, double *work, void *stream
 int slbc_nn_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H, int W, float scale,
                    float shift_x, float *u, float drho_scale, float *drho, void *stream) {
   if (ctot_p < (drho ? 4 : 3)) return bad("slbc_nn_decode: bad channel count");
-  k_decode<<<grid_for((long long)D * H * W), 256, 0, (cudaStream_t)stream>>>(pred, ctot_p, solid, D, H, W, scale,
+  k_decode<<<rows_grid((long long)D * H, W), 256, 0, (cudaStream_t)stream>>>(pred, ctot_p, solid, D, H, W, scale,
                                                                                        shift_x, u, drho_scale, drho);
   return launched("slbc_nn_decode");
 }
