@@ -732,6 +732,52 @@ cudaError_t ensure_mp_rinv(Lattice &L) {
   return e;
 }
 
+__global__ void k_mp_ratios(const double *rho64, double rho0, double *rinv, double *ratio, long long n) {
+  const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  const double r = rho64[x];
+  rinv[x] = __drcp_rn(r);
+  ratio[x] = __ddiv_rn(rho0, r);
+}
+
+cudaError_t ensure_mp_ratios(Lattice &L) {
+  if (L.mp_rinv64 && L.mp_ratio64 && L.mp_ratio_gen == L.mp_rho_gen && L.mp_ratio_rho0 == L.par.rho0) return cudaSuccess;
+  if (!L.mp_rho64) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
+  if (!L.mp_rinv64) e = cudaMalloc(&L.mp_rinv64, (size_t)L.nnodes * sizeof(double));
+  if (e == cudaSuccess && !L.mp_ratio64) e = cudaMalloc(&L.mp_ratio64, (size_t)L.nnodes * sizeof(double));
+  if (e != cudaSuccess) return e;
+  k_mp_ratios<<<(int)((L.nnodes + 255) / 256), 256, 0, L.stream>>>(L.mp_rho64, L.par.rho0, L.mp_rinv64, L.mp_ratio64,
+                                                                   L.nnodes);
+  g_launches += 1;
+  e = cudaGetLastError();
+  if (e == cudaSuccess) {
+    L.mp_ratio_gen = L.mp_rho_gen;
+    L.mp_ratio_rho0 = L.par.rho0;
+  }
+  return e;
+}
+
+// The march with the least work in whole waves of resident blocks, a block
+// costing its planes and the two it reads for its halo.  (Up to 8 planes with
+// four blocks per SM before: 96^3 in 864 blocks of 4 + 2 planes, now 288 of
+// 12 + 2 in one wave.)
+int march_planes(const Lattice &L, int blocks_per_sm) {
+  const long long tiles = (long long)((L.esk + kTileK - 1) / kTileK) * ((L.esj + kTileJ - 1) / kTileJ);
+  const long long slots = 152LL * blocks_per_sm;
+  long long best = 0;
+  int planes = 1;
+  for (int chunks = 1; chunks <= L.esi; chunks++) {
+    const int p = (L.esi + chunks - 1) / chunks;
+    const long long waves = (tiles * ((L.esi + p - 1) / p) + slots - 1) / slots, cost = waves * (p + 2);
+    if (best == 0 || cost < best) {
+      best = cost;
+      planes = p;
+    }
+  }
+  return planes;
+}
+
 void count_launch(int n) { g_launches += n; }
 void set_error(const std::string &msg) { g_err = msg; }
 int reduction_blocks(const Lattice &L) {
@@ -817,7 +863,7 @@ void slbc_destroy(slbc_lattice *h) {
   void *bufs[] = {L.pop, L.scratch, L.flags, L.bnd_node, L.bnd_obj, L.bnd_f, L.piece_obj,
                   L.piece_lo, L.piece_hi, L.piece_sum, L.obj_pos, L.obj_ft, L.ads, L.objidx,
                   L.bf, L.uw, L.partials, L.staging, L.mp_rho64, L.mp_rho32, L.mom[0], L.mom[1],
-                  L.ads_links, L.mp_rinv32, L.mp_coef, L.move_buf};
+                  L.ads_links, L.mp_rinv32, L.mp_coef, L.move_buf, L.mp_rinv64, L.mp_ratio64};
   for (void *b : bufs) if (b) cudaFree(b);
   if (L.host_out) cudaFreeHost(L.host_out);
   if (L.graph) cudaGraphExecDestroy(L.graph);

@@ -104,6 +104,11 @@ struct Lattice {
   // changes (mp_rho_gen counts snapshots)
   float *mp_rinv32 = nullptr;
   unsigned long long mp_rho_gen = 1, mp_rinv_gen = 0;
+  // 1/rho and rho0/rho in FP64 for the FP64 tracer update, rebuilt when the
+  // snapshot or rho0 changes
+  double *mp_rinv64 = nullptr, *mp_ratio64 = nullptr;
+  unsigned long long mp_ratio_gen = 0;
+  double mp_ratio_rho0 = 0.0;
   // counts changes of the populations (steps, uploads, phases, warm starts)
   unsigned long long state_version = 0;
   // FP32 tracer on a frozen flow: per-node stencil coefficients
@@ -243,6 +248,10 @@ cudaError_t launch_mp_rhoinit_bf16(Lattice &L);
 // 1/rho of the density snapshot for FP32 tracers, rebuilt when stale
 // (slbc_core.cu)
 cudaError_t ensure_mp_rinv(Lattice &L);
+// 1/rho and rho0/rho of the snapshot for FP64 tracers, likewise
+cudaError_t ensure_mp_ratios(Lattice &L);
+// planes a tracer block marches over
+int march_planes(const Lattice &L, int blocks_per_sm);
 // column sums of the tracer stencil set to 1 (mass conservation)
 cudaError_t launch_mp_coef_norm(Lattice &L);
 // one FP32 tracer update from the lattice's stencil coefficients

@@ -392,15 +392,14 @@ cudaError_t SLBC_FN(launch_mp_rhoinit)(Lattice &L) {
 cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, int tp_f64,
                                     double alpha, double adprob, int moving,
                                     const double *objstate, float *lo_in, float *lo_out, int *lo_live) {
-  // planes per block: the largest of 1..8 that still gives about four
-  // blocks per SM
-  const long long tiles = (long long)((L.esk + kTileK - 1) / kTileK) * ((L.esj + kTileJ - 1) / kTileJ);
-  int planes = 8;
-  while (planes > 1 && tiles * ((L.esi + planes - 1) / planes) < 152 * 4) planes /= 2;
-  const dim3 grid((unsigned)((L.esk + kTileK - 1) / kTileK), (unsigned)((L.esj + kTileJ - 1) / kTileJ),
-                  (unsigned)((L.esi + planes - 1) / planes));
+  int planes = 1;
+  const auto tiling = [&](int blocks_per_sm) {
+    planes = march_planes(L, blocks_per_sm);
+    return dim3((unsigned)((L.esk + kTileK - 1) / kTileK), (unsigned)((L.esj + kTileJ - 1) / kTileJ),
+                (unsigned)((L.esi + planes - 1) / planes));
+  };
   const dim3 block(kTileK, kTileJ);
-  MpArgs m;
+  MpArgs m{};
   m.p_in = p_in; m.p_out = p_out;
   m.rho = tp_f64 ? (const void *)L.mp_rho64 : (const void *)L.mp_rho32;
   m.ads = L.ads; m.ads_links = L.ads_links; m.objidx = L.objidx; m.objstate = objstate; m.moving = moving;
@@ -455,9 +454,11 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
           if (me != cudaSuccess) return me;
         }
         *lo_live = 1;
+        const dim3 grid = tiling(4);
         return launch_mp_apply(L, (const float *)p_in, lo_in, (float *)p_out, lo_out, grid, block, planes);
       }
     }
+    const dim3 grid = tiling(3);
     switch (L.layout * 2 + (moving ? 1 : 0)) {
       case SLBC_LAYOUT_N * 2: k_mp_step_f32<T_, SLBC_LAYOUT_N, false><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
       case SLBC_LAYOUT_N * 2 + 1: k_mp_step_f32<T_, SLBC_LAYOUT_N, true><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
@@ -485,6 +486,18 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
     if (e != cudaSuccess) return e;
     attr_set[tp_f64 ? 1 : 0] |= bit;
   }
+  if (tp_f64) {
+    const cudaError_t e = ensure_mp_ratios(L);
+    if (e == cudaSuccess) {
+      m.rinv = L.mp_rinv64;
+      m.rratio = L.mp_ratio64;
+    } else if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();  // the kernel divides instead
+    } else {
+      return e;
+    }
+  }
+  const dim3 grid = tiling(tp_f64 ? 2 : 3);
   if (tp_f64)
     k_mp_step<T_, double><<<grid, block, mp_bucket_bytes<double>(), L.stream>>>(pop_args(L), L.layout, m, planes);
   else

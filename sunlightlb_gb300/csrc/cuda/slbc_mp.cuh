@@ -20,6 +20,7 @@ struct MpArgs {
   const void *p_in;
   void *p_out;
   const void *rho;  // density snapshot in the tracer type
+  const double *rinv, *rratio;  // 1 / rho and rho0 / rho of the snapshot (FP64 tracers)
   const unsigned char *ads;  // adsorbing nodes (0x4000 of the reference mask)
   const uint16_t *ads_links; // per fluid node: links from adsorbing solids
   const int *objidx;         // object of every node (-1 fluid), moving walls
@@ -81,20 +82,66 @@ struct MpSource {
   TP fac, piece;
 };
 
+// p / rho, correctly rounded, from y = RN(1 / rho): each pair of fused
+// multiply-adds forms the remainder of the quotient and corrects it; after the
+// first the quotient is within one ulp, so the second rounds correctly
+// (Markstein).  Five FP64 operations instead of a division's ten or so.
+// Infinite and undefined quotients pass through.
+__device__ __forceinline__ double mp_quotient(double p, double rho, double y) {
+  const double q0 = __dmul_rn(p, y);
+  if ((__double2hiint(q0) & 0x7ff00000) == 0x7ff00000) return p / rho;
+  const double q1 = __fma_rn(__fma_rn(-rho, q0, p), y, q0);
+  return __fma_rn(__fma_rn(-rho, q1, p), y, q1);
+}
+
+// What a source node's values are made of: p, rho and, for FP64 tracers, the
+// snapshot's 1 / rho and rho0 / rho.
 template <typename TP>
-__device__ __forceinline__ MpSource<TP> mp_source(const MpArgs &m, int y, TP rho0, TP alpha) {
-  const TP rhot = mp_load<TP>(m.rho, y), pt = mp_load<TP>(m.p_in, y);
+struct MpRaw {
+  TP p, rho;
+};
+template <>
+struct MpRaw<double> {
+  double p, rho, rinv, ratio;
+};
+
+template <typename TP>
+__device__ __forceinline__ MpRaw<TP> mp_raw(const MpArgs &m, int y) {
+  MpRaw<TP> r;
+  r.p = mp_load<TP>(m.p_in, y);
+  r.rho = mp_load<TP>(m.rho, y);
+  if constexpr (sizeof(TP) == 8) {
+    if (m.rinv) {
+      r.rinv = m.rinv[y];
+      r.ratio = m.rratio[y];
+    } else {  // no room for the two arrays
+      r.rinv = 1.0 / r.rho;
+      r.ratio = m.rho0 / r.rho;
+    }
+  }
+  return r;
+}
+
+template <typename TP>
+__device__ __forceinline__ MpSource<TP> mp_source(const MpRaw<TP> &v, TP rho0, TP alpha) {
   MpSource<TP> r;
-  r.fac = pt / rhot;
-  r.piece = pt * TP(1.0 / 72.0) * (rho0 / rhot - alpha);
+  if constexpr (sizeof(TP) == 8) {
+    r.fac = mp_quotient(v.p, v.rho, v.rinv);
+    r.piece = v.p * TP(1.0 / 72.0) * (v.ratio - alpha);
+  } else {
+    r.fac = v.p / v.rho;
+    r.piece = v.p * TP(1.0 / 72.0) * (rho0 / v.rho - alpha);
+  }
   return r;
 }
 
 // One tracer update of every node.  A block of 32 (k) x 8 (j) threads walks
 // along i over `planes` planes; fac and piece of every node of three
-// consecutive planes (with a one-node halo) sit in shared memory, so each
-// node's two divisions are done about 1.7 times per update instead of once
-// for each of the up to 15 nodes that gather from it.
+// consecutive planes (with a one-node halo) sit in shared memory, so they are
+// formed about 1.6 times per node and update instead of once for each of the
+// up to 15 nodes that gather from it.  FP64 tracers are bound by the FP64
+// pipe: the snapshot's reciprocal and ratio replace the two divisions, and
+// the products with 8 and 16 (exact) ride in fused multiply-adds.
 template <typename T, typename TP>
 __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_step(PopArgs<T> p, int layout, MpArgs m, int planes) {
   __shared__ MpSource<TP> ring[3][kPlane];
@@ -106,7 +153,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
   const int k0 = blockIdx.x * kTileK, j0 = blockIdx.y * kTileJ, i0 = blockIdx.z * planes;
   const int np = min(planes, p.esi - i0);
   const int plane_nodes = p.esj * p.esk;
-  const TP onebyb = TP(1.0 / 72.0), eightbyb = TP(8.0 / 72.0);
+  const TP eightbyb = TP(8.0 / 72.0);
   const TP alpha = mp_param<TP>(m.alpha, m.alpha_f), rho0 = mp_param<TP>(m.rho0, m.rho0_f);
   const TP Pa = mp_param<TP>(m.adprob, m.adprob_f);
   const bool partial = m.partial != 0;
@@ -123,13 +170,13 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
     const int base = wrap_index(i0 - 1 + h, p.esi) * plane_nodes;
 #pragma unroll
     for (int e = 0; e < kPlaneLoads; e++)
-      if (off[e] >= 0) ring[h][tid + kTileThreads * e] = mp_source<TP>(m, base + off[e], rho0, alpha);
+      if (off[e] >= 0) ring[h][tid + kTileThreads * e] = mp_source<TP>(mp_raw<TP>(m, base + off[e]), rho0, alpha);
   }
   // Register prefetch, one plane ahead of use: p and rho of the halo tile
   // of plane i+1 (for the ring) and the flag word, adsorption byte, p and
   // rho of this thread's own node of plane i, so that only the 15
   // population loads stay on a node's critical path.
-  TP pre_p[kPlaneLoads], pre_r[kPlaneLoads];
+  MpRaw<TP> pre[kPlaneLoads];
   const int j = j0 + tj, k = k0 + tk;
   const bool mine = j < p.esj && k < p.esk;
   const int own = mine ? j * p.esk + k : 0;
@@ -137,7 +184,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
     const int base = wrap_index(plane, p.esi) * plane_nodes;
 #pragma unroll
     for (int e = 0; e < kPlaneLoads; e++)
-      if (off[e] >= 0) { pre_p[e] = mp_load<TP>(m.p_in, base + off[e]); pre_r[e] = mp_load<TP>(m.rho, base + off[e]); }
+      if (off[e] >= 0) pre[e] = mp_raw<TP>(m, base + off[e]);
   };
   uint16_t n_fl = 0, n_al = 0;
   unsigned char n_ads = 0;
@@ -148,7 +195,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
     n_ads = m.ads ? m.ads[x] : 0;
     n_al = m.ads ? m.ads_links[x] : 0;
     n_p = mp_load<TP>(m.p_in, x);
-    n_r = mp_load<TP>(m.rho, x);
+    n_r = sizeof(TP) == 8 && m.rinv ? (TP)m.rratio[x] : rho0 / mp_load<TP>(m.rho, x);  // rho0 / rho
   };
   prefetch_ring(i0 + 1);
   prefetch_node(i0);
@@ -162,10 +209,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
 #pragma unroll
     for (int e = 0; e < kPlaneLoads; e++) {
       if (off[e] < 0) continue;
-      MpSource<TP> r;
-      r.fac = pre_p[e] / pre_r[e];
-      r.piece = pre_p[e] * TP(1.0 / 72.0) * (rho0 / pre_r[e] - alpha);
-      ring[sp][tid + kTileThreads * e] = r;
+      ring[sp][tid + kTileThreads * e] = mp_source<TP>(pre[e], rho0, alpha);
     }
     __syncthreads();
     const uint16_t fl = n_fl, al = n_al;
@@ -182,9 +226,9 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
     const int x = nb.at(0, 0, 0);
     const bool solid = (fl & FLAG_SOLID) != 0;
     if (solid && !ads_x) { pout[x] = TP(0); continue; }
-    // rho0/rho - alpha of x itself, for the axis links that return to x
-    TP h_x = TP(0);
-    if (!solid && (fl & 0x7Eu)) h_x = rho0 / r_x - alpha;
+    // b-weight times p and rho0/rho - alpha of x itself, for the axis links
+    // that return to x
+    const TP axis_x = (eightbyb * pt_x) * (r_x - alpha);
     const MpSource<TP> ex = R[1][c0];
     // Each link q is one of: A fluid y scatters into fluid x; B fluid y
     // scatters into adsorbing solid x; C solid y returns to fluid x what x
@@ -220,14 +264,14 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
       const MpSource<TP> e = R[1 - CX(q)][c0 - CY(q) * kHaloK - CZ(q)];
       TP t;
       if (q == 0) {
-        t = e.fac * av[q] + TP(16.0) * e.piece + alpha * pt_x;
+        t = scale_add(e.piece, TP(16.0), e.fac * av[q]) + alpha * pt_x;
       } else {
         // (b q-weight * p) * (rho0/rho - alpha) of x in case C: for the
-        // diagonals this is the piece of x (the products commute exactly)
+        // diagonals this is the piece of x (the products commute exactly);
+        // else 8 or 1 times the piece of the source
         const TP fac = self_c ? ex.fac : e.fac;
-        const TP pc = self_c ? (q <= 6 ? (eightbyb * pt_x) * h_x : ex.piece)
-                             : (q <= 6 ? TP(8.0) * e.piece : e.piece);
-        t = fac * av[q] + pc;
+        if (q <= 6) t = scale_add(self_c ? axis_x : e.piece, self_c ? TP(1.0) : TP(8.0), fac * av[q]);
+        else t = fac * av[q] + (self_c ? ex.piece : e.piece);
         if (bnd && solid && partial) t = Pa * t;  // case B
         // case C from an adsorbing solid keeps 1 - P (nothing when P = 1);
         // with moving walls this follows the wall term, below
