@@ -31,7 +31,7 @@ struct slbc_tracer {
   slbc_lattice *h = nullptr;
   int f64 = 1;
   void *p = nullptr, *p2 = nullptr;
-  double *acc = nullptr;  // tracer added by fills since creation or the last reset
+  double *acc = nullptr;  // tracer added by fills since creation or the last reset; the fills' block counter
   double *objstate = nullptr;
   int objstate_cap = 0;
   // FP32 tracers: the low part of p (p = hi + lo, |lo| <= half an FP32 ulp
@@ -284,53 +284,69 @@ __device__ __forceinline__ long long plane_node(long long e, int axis, int pos, 
 }
 
 // Tracer injection on the fluid nodes of a region (reference src/mpobjs.c).
-// Kind 2 (a wall) visits only the nodes of its plane.  Each block also
-// writes the sum of (value - old p) over the nodes it set, so the host
-// layer can keep count of the tracer the fills have added.
+// Kind 2 (a wall) visits only the nodes of its plane and needs no
+// coordinates.  Each block leaves the sum of (value - old p) over the nodes
+// it set; the last block to finish adds them to acc[0] in block order, so the
+// host layer can keep count of the tracer the fills have added (a second
+// launch for that sum cost as much as the fill of a plane: a source and an
+// absorbing plane of a 256^3 lattice set again every update took 21 of its
+// 255 us).  done: a counter, zero before and after.
 template <typename TP>
 __global__ void __launch_bounds__(kReduceThreads)
 k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, int kind, double g0, double g1,
-          double g2, double g3, double g4, double g5, double value, long long count, double *partials) {
+          double g2, double g3, double g4, double g5, double value, int count, double *partials, unsigned *done,
+          double *acc) {
   double v[1] = {0.0};
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < count;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long x = kind == 2 ? plane_node(e, (int)g0, (int)g1, esi, esj, esk) : e;
+  const TP nv = (TP)value;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
+    int x = e;
+    if (kind == 2) {
+      const int axis = (int)g0, pos = (int)g1;
+      if (axis == 0) x = pos * esj * esk + e;
+      else if (axis == 1) x = ((e / esk) * esj + pos) * esk + e % esk;
+      else x = e * esk + pos;
+    }
     if (flags[x] & FLAG_SOLID) continue;
-    const int k = (int)(x % esk), r = (int)(x / esk), j = r % esj, i = r / esj;
-    bool in = false;
-    switch (kind) {
-      case 0: in = true; break;
-      case 1: in = i > g0 && i < g1 && j > g2 && j < g3 && k > g4 && k < g5; break;
-      case 2: in = true; break;
-      case 3: {
+    bool in = true;
+    if (kind == 1 || kind == 3 || kind == 4) {
+      const int k = x % esk, r = x / esk, j = r % esj, i = r / esj;
+      if (kind == 1) {
+        in = i > g0 && i < g1 && j > g2 && j < g3 && k > g4 && k < g5;
+      } else if (kind == 3) {
         const double rsq = (i - g1) * (i - g1) + (j - g2) * (j - g2) + (k - g3) * (k - g3);
         in = rsq < g0 * g0;
-      } break;
-      case 4: {
+      } else {
         const int ax = (int)g0;
         const double u = ax == 0 ? j : i, w = ax == 2 ? j : k;
         const double rsq = (u - g3) * (u - g3) + (w - g4) * (w - g4);
         in = rsq < g2 * g2;
         if (g1 != 0.0) in = !in;
-      } break;
+      }
     }
     if (in) {
-      const TP nv = (TP)value;
       v[0] += (double)nv - (double)p[x] - (lo ? (double)lo[x] : 0.0);
       p[x] = nv;
       if (lo) lo[x] = 0.0f;
     }
   }
   block_sum<1>(v);
-  if (threadIdx.x == 0) partials[blockIdx.x] = v[0];
-}
-
-// acc[0] += sum of nb partials, in a fixed order
-__global__ void __launch_bounds__(256) k_sum_into(const double *partials, int nb, double *acc) {
-  double v[1] = {0.0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) v[0] += partials[b];
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = v[0];
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  v[0] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) v[0] += __ldcg(partials + b);
+  __syncthreads();
   block_sum<1>(v);
-  if (threadIdx.x == 0) acc[0] += v[0];
+  if (threadIdx.x == 0) {
+    acc[0] += v[0];
+    *done = 0u;
+  }
 }
 
 // sum of p and number of fluid nodes on one plane
@@ -1538,8 +1554,8 @@ int slbc_mp_create(slbc_lattice *h, slbc_tracer **out, int use_f64) {
   if (e == cudaSuccess) e = cudaMemsetAsync(t->p2, 0, (size_t)L.nnodes * es, L.stream);
   if (e == cudaSuccess && !use_f64) e = cudaMalloc(&t->lo, (size_t)L.nnodes * sizeof(float));
   if (e == cudaSuccess && !use_f64) e = cudaMalloc(&t->lo2, (size_t)L.nnodes * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&t->acc, sizeof(double));
-  if (e == cudaSuccess) e = cudaMemsetAsync(t->acc, 0, sizeof(double), L.stream);
+  if (e == cudaSuccess) e = cudaMalloc(&t->acc, 2 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemsetAsync(t->acc, 0, 2 * sizeof(double), L.stream);
   if (e == cudaSuccess && !L.mp_rho64) {
     e = cudaMalloc(&L.mp_rho64, (size_t)L.nnodes * sizeof(double));
     if (e == cudaSuccess) {
@@ -1607,17 +1623,30 @@ int slbc_mp_put(slbc_tracer *t, const double *p) {
   return 0;
 }
 
+// FP32 tracers are widened on the GPU, a staging buffer at a time, and copied
+// straight to the caller's array (widening 256^3 values on one host core after
+// the copy took 17 ms).
 int slbc_mp_get(slbc_tracer *t, double *p) {
   Lattice &L = t->h->L;
   if (t->f64) {
     CK(cudaMemcpyAsync(p, t->p, (size_t)L.nnodes * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
-    CK(cudaStreamSynchronize(L.stream));
-  } else {
+  } else if (ensure_staging(L, L.nnodes, 4)) {  // no room on the GPU: widened here
+    cudaGetLastError();
     std::vector<float> buf((size_t)L.nnodes);
     CK(cudaMemcpyAsync(buf.data(), t->p, (size_t)L.nnodes * sizeof(float), cudaMemcpyDeviceToHost, L.stream));
     CK(cudaStreamSynchronize(L.stream));
     for (long long x = 0; x < L.nnodes; x++) p[x] = buf[x];
+  } else {
+    const long long chunk = L.staging_nodes;
+    for (long long x0 = 0; x0 < L.nnodes; x0 += chunk) {
+      const long long n = std::min(chunk, L.nnodes - x0);
+      k_convert<double, float><<<blocks_for(n, 256), 256, 0, L.stream>>>(L.staging, (const float *)t->p + x0, n);
+      count_launch();
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(p + x0, L.staging, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
+    }
   }
+  CK(cudaStreamSynchronize(L.stream));
   return 0;
 }
 
@@ -1767,13 +1796,11 @@ int slbc_mp_fill(slbc_tracer *t, int kind, const double *geo, double value) {
   }
   const int nb = (int)std::max<long long>(1, std::min<long long>(blocks_for(count, kReduceThreads), 152 * 4));
   if (ensure_partials(L, nb + 8)) return 1;
+  unsigned *done = (unsigned *)(t->acc + 1);
   if (t->f64)
-    k_mp_fill<double><<<nb, kReduceThreads, 0, L.stream>>>((double *)t->p, nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, count, L.partials);
+    k_mp_fill<double><<<nb, kReduceThreads, 0, L.stream>>>((double *)t->p, nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
   else
-    k_mp_fill<float><<<nb, kReduceThreads, 0, L.stream>>>((float *)t->p, t->lo_live ? t->lo : nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, count, L.partials);
-  count_launch();
-  CK(cudaGetLastError());
-  k_sum_into<<<1, 256, 0, L.stream>>>(L.partials, nb, t->acc);
+    k_mp_fill<float><<<nb, kReduceThreads, 0, L.stream>>>((float *)t->p, t->lo_live ? t->lo : nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
   count_launch();
   CK(cudaGetLastError());
   return 0;

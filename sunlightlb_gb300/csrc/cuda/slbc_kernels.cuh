@@ -390,6 +390,34 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> a, OddOffsets off) {
   }
 }
 
+// One fused update of every node of an FP64 lattice whose rows along k do not
+// fill whole warps: the nodes of a plane are taken as one run, so only its
+// last warp is short.  The FP64 step is bound by the FP64 pipe, where a lane
+// without a node costs as much as one with; the division that finds (j, k)
+// is integer work beside it.  (126 x 110 x 97: rows of 97 in four warps, 407
+// us; as runs of 10,670 nodes 318 us.)
+template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>
+__global__ void __launch_bounds__(128) k_step_run(StepArgs<T> a, OddOffsets off) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.z;
+  const int esj = a.p.esj, esk = a.p.esk;
+  if (e >= esj * esk) return;
+  const int j = e / esk, k = e - j * esk;
+  const unsigned warp_mask = __activemask();
+  const Nbr nb = make_nbr(i, j, k, a.p.esi, esj, esk);
+  const int x = nb.at(0, 0, 0);
+  const uint16_t fl = __ldg(a.p.flags + x);
+  T t[15];
+  const bool inner = ODD && __all_sync(warp_mask, i > 0 && i < a.p.esi - 1 && j > 0 && j < esj - 1 && k > 0 && k < esk - 1);
+  if (inner) {
+    load_pops_inner<T>(a.p.pop, off, x, fl, t);
+    relax_node<T, EXACT, MOVING, BFU>(a, nb, x, fl, t);
+    store_pops_inner<T>(a.p.pop, off, x, fl, t);
+  } else {
+    load_pops<T, ODD, true>(a.p.pop, a.p.npad, nb, x, fl, t);
+    finish_node<T, ODD, EXACT, MOVING, BFU, true>(a, nb, x, fl, t);
+  }
+}
+
 // ---- batches of independent lattices ----------------------------------------
 // One persistent launch advances many lattices ("domains") by nsteps fused
 // steps each (the parity of each domain's first step follows its layout).  Block b owns the domains
