@@ -1932,34 +1932,41 @@ int slbc_batch_step(slbc_batch *b, int nsteps) {
     CK(B.precision == 0 ? launch_batch_f64(B, nsteps) : launch_batch_f32(B, nsteps));
   } else {
     CK(B.precision == 0 ? prepare_tiles_f64(B) : prepare_tiles_f32(B));
-    auto one = [&](int s) { return B.precision == 0 ? launch_tiles_f64(B, s) : launch_tiles_f32(B, s); };
-    // 50 steps (an even number: the parity pattern repeats) per graph replay
-    const int G = 50;
-    int done = 0;
-    if (nsteps >= 2 * G) {
-      cudaGraph_t g;
-      cudaGraphExec_t ge = nullptr;
-      CK(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t ce = cudaSuccess;
-      for (int s = 0; s < G && ce == cudaSuccess; s++) ce = one(s);
-      const cudaError_t ee = cudaStreamEndCapture(B.stream, &g);
-      if (ce != cudaSuccess) return fail("slbc_batch_step: capture", ce);
-      if (ee != cudaSuccess) return fail("slbc_batch_step: cudaStreamEndCapture", ee);
-      const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
-      cudaGraphDestroy(g);
-      if (ie != cudaSuccess) return fail("slbc_batch_step: cudaGraphInstantiate", ie);
-      int nclass = 0;
-      for (int c = 0; c < 4; c++) nclass += (B.class_tiles[c][0] > 0) + (B.class_tiles[c][1] > 0);
-      count_launch(-G * nclass);  // the captured launches run only in the replays
-      for (; done + G <= nsteps; done += G) {
-        const cudaError_t le = cudaGraphLaunch(ge, B.stream);
-        if (le != cudaSuccess) { cudaGraphExecDestroy(ge); return fail("slbc_batch_step: cudaGraphLaunch", le); }
-        count_launch(G * nclass);
+    auto one = [&](const BatchState::Set &set, int s) {
+      return B.precision == 0 ? launch_tiles_f64(B, set, s) : launch_tiles_f32(B, set, s);
+    };
+    for (const BatchState::Set &set : B.sets) {
+      // 50 steps (an even number: the parity pattern repeats) per graph
+      // replay where one set holds the whole batch: its launches may be
+      // shorter than their submission.  Several sets are each near the L2's
+      // size, so theirs are not, and a graph per set would only cost time.
+      const int G = 50;
+      int done = 0;
+      if (B.sets.size() == 1 && nsteps >= 2 * G) {
+        cudaGraph_t g;
+        cudaGraphExec_t ge = nullptr;
+        CK(cudaStreamBeginCapture(B.stream, cudaStreamCaptureModeThreadLocal));
+        cudaError_t ce = cudaSuccess;
+        for (int s = 0; s < G && ce == cudaSuccess; s++) ce = one(set, s);
+        const cudaError_t ee = cudaStreamEndCapture(B.stream, &g);
+        if (ce != cudaSuccess) return fail("slbc_batch_step: capture", ce);
+        if (ee != cudaSuccess) return fail("slbc_batch_step: cudaStreamEndCapture", ee);
+        const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
+        cudaGraphDestroy(g);
+        if (ie != cudaSuccess) return fail("slbc_batch_step: cudaGraphInstantiate", ie);
+        int nclass = 0;
+        for (int c = 0; c < 4; c++) nclass += (set.class_tiles[c][0] > 0) + (set.class_tiles[c][1] > 0);
+        count_launch(-G * nclass);  // the captured launches run only in the replays
+        for (; done + G <= nsteps; done += G) {
+          const cudaError_t le = cudaGraphLaunch(ge, B.stream);
+          if (le != cudaSuccess) { cudaGraphExecDestroy(ge); return fail("slbc_batch_step: cudaGraphLaunch", le); }
+          count_launch(G * nclass);
+        }
+        CK(cudaStreamSynchronize(B.stream));
+        cudaGraphExecDestroy(ge);
       }
-      CK(cudaStreamSynchronize(B.stream));
-      cudaGraphExecDestroy(ge);
+      for (; done < nsteps; done++) CK(one(set, done));
     }
-    for (; done < nsteps; done++) CK(one(done));
   }
   CK(cudaEventRecord(B.done, B.stream));
   for (Lattice *L : B.lats) {

@@ -186,11 +186,16 @@ struct BatchState {
   int nworkers = 0;                 // blocks of the last persistent launch
   void *doms = nullptr;             // BatchDom<T> per lattice
   int *work_off = nullptr, *work = nullptr;  // persistent: lattices of each block (CSR)
-  int2 *tiles = nullptr;            // tiles: (lattice, first cell), grouped by class
+  int2 *tiles = nullptr;            // tiles: (lattice, first cell), grouped by set and class
   long long tiles_cap = 0;
-  // tiles per (class, starting parity): class = 2 * moving + uniform force,
-  // group g holds the domains whose first step has parity g (odd0 = g)
-  int class_tiles[4][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
+  // sets of lattices that go through all steps one set after another: tiles
+  // per (class, starting parity), class = 2 * moving + uniform force, [g] the
+  // domains whose first step has parity g (odd0 = g)
+  struct Set {
+    long long first_tile;
+    int class_tiles[4][2];
+  };
+  std::vector<Set> sets;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
 };
@@ -199,7 +204,7 @@ struct BatchState {
   cudaError_t launch_batch_##SUFFIX(BatchState &B, int nsteps);                 \
   cudaError_t launch_velocity_##SUFFIX(Lattice &L, double fac, float *u, float *drho); \
   cudaError_t prepare_tiles_##SUFFIX(BatchState &B);                             \
-  cudaError_t launch_tiles_##SUFFIX(BatchState &B, int step);                    \
+  cudaError_t launch_tiles_##SUFFIX(BatchState &B, const BatchState::Set &set, int step); \
   cudaError_t launch_step_##SUFFIX(Lattice &L, int odd);                        \
   cudaError_t launch_force_##SUFFIX(Lattice &L);                                \
   cudaError_t launch_vsum_##SUFFIX(Lattice &L, double fac, const double *psi,   \

@@ -314,6 +314,21 @@ __device__ __forceinline__ void finish_node(const StepArgs<T> &a, const Nbr &nb,
   }
 }
 
+// The pull-and-push update of node x in 32-bit indices, any place in the
+// lattice: the element population q is pulled from is the one the population
+// of opp(q) is pushed to (slot opp(q) of x - c_q, or slot q of x across a
+// bounce-back link), so each index is worked out once and kept.
+template <typename T>
+__device__ __forceinline__ void odd_places(unsigned S, const Nbr &nb, int x, uint16_t fl, unsigned (&at)[15]) {
+  at[0] = (unsigned)x;
+#pragma unroll
+  for (int q = 1; q < 15; q++) {
+    const unsigned nbr = (unsigned)OPP(q) * S + (unsigned)nb.at(-CX(q), -CY(q), -CZ(q));
+    const unsigned self = (unsigned)q * S + (unsigned)x;
+    at[q] = ((fl >> q) & 1) ? self : nbr;
+  }
+}
+
 // Fused update (bounce-back + streaming + collision) of node (i, j, k).
 // ODD = false: C1 -> C0 (local), ODD = true: C0 -> C1 (pull and push).
 // MOVING compiles the wall terms in, BFU selects a uniform body force (a
@@ -463,21 +478,42 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(const BatchDom<T> *d
 // updates the tiles of one (moving walls, uniform force, parity) group by
 // one step: the host groups each class's tiles by the parity of their
 // domain's first step, so one launch has one parity (ODD) and carries the
-// code of that parity only (64 registers, four blocks per SM).
+// code of that parity only (64 registers, four blocks per SM).  The domain's
+// arguments come in a word per thread, and the pull-and-push update keeps
+// each 32-bit index for both directions (odd_places): 187 -> 162 us per step
+// of 64 FP32 lattices of sides 24 to 64 with the sets of prepare_tiles.
+// Slower: blocks that walk through the tiles with a barrier per tile (169),
+// all arguments in the tile table (180).
 constexpr int kBatchTile = 256;
 
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(kBatchTile, 4) k_batch_tiles(const BatchDom<T> *doms, const int2 *tiles) {
   __shared__ BatchDom<T> dom;
   const int2 tile = tiles[blockIdx.x];
-  if (threadIdx.x == 0) dom = doms[tile.x];
+  constexpr int kWords = (int)(sizeof(BatchDom<T>) / 4);
+  static_assert(sizeof(BatchDom<T>) % 4 == 0 && kWords <= kBatchTile, "a word per thread");
+  if (threadIdx.x < kWords) ((unsigned *)&dom)[threadIdx.x] = ((const unsigned *)(doms + tile.x))[threadIdx.x];
   __syncthreads();
   const StepArgs<T> &a = dom.a;
   const int esj = a.p.esj, esk = a.p.esk;
   const int e = tile.y + threadIdx.x;
   if (e >= a.p.esi * esj * esk) return;
+  const uint16_t fl = __ldg(a.p.flags + e);
   const int r = e / esk;
-  step_node<T, ODD, EXACT, MOVING, BFU>(a, r / esj, r % esj, e - r * esk);
+  const Nbr nb = make_nbr(r / esj, r % esj, e - r * esk, a.p.esi, esj, esk);
+  T t[15];
+  if (ODD && 15 * a.p.npad <= 0xFFFFFFFFLL) {
+    unsigned at[15];
+    odd_places<T>((unsigned)a.p.npad, nb, e, fl, at);
+#pragma unroll
+    for (int q = 0; q < 15; q++) t[q] = a.p.pop[at[q]];
+    relax_node<T, EXACT, MOVING, BFU>(a, nb, e, fl, t);
+#pragma unroll
+    for (int q = 0; q < 15; q++) a.p.pop[at[OPP(q)]] = t[q];
+  } else {
+    load_pops<T, ODD>(a.p.pop, a.p.npad, nb, e, fl, t);
+    finish_node<T, ODD, EXACT, MOVING, BFU>(a, nb, e, fl, t);
+  }
 }
 
 // Explicitly rounded add / multiply: never contracted into FMA, so the
