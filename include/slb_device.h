@@ -172,6 +172,11 @@ int slbc_get_force(slbc_lattice *h, double *f3);
  * out[0..2] = sum w*u, out[3] = sum w, out[4] = number of fluid nodes, with
  * u the velocity corrected by fac*b and w = psi^2 (psi NULL: w = 1). */
 int slbc_vsum(slbc_lattice *h, double fac, const double *psi, double out[5]);
+/* The same in two halves: begin queues the sums of the state as it is then
+ * into one of three slots, end waits for the lattice's stream and returns
+ * them.  Other reductions of the lattice or its tracers end the slots' life. */
+int slbc_vsum_begin(slbc_lattice *h, double fac, const double *psi, int slot);
+int slbc_vsum_end(slbc_lattice *h, int slot, double out[5]);
 /* Object force and torque (reference src/lbmeasure.c:236-263):
  * pos[3*nobj] in, ft[6*nobj] out (frc xyz, trq xyz). */
 int slbc_distribf(slbc_lattice *h, const double *pos, double *ft);

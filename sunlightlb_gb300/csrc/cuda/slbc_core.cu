@@ -1447,24 +1447,43 @@ int slbc_get_force(slbc_lattice *h, double *f3) {
   return 0;
 }
 
-int slbc_vsum(slbc_lattice *h, double fac, const double *psi, double out[5]) {
-  Lattice &L = h->L;
+// Sums of one slot (0..2), left in L.host_out[5 * slot ..] once the stream has
+// been waited for: a measurement takes three of them around its steps and
+// waits once (three round trips of about 15 us each before).
+static int vsum_enqueue(Lattice &L, double fac, const double *psi, int slot) {
   const int nb = reduction_blocks(L);
-  if (ensure_partials(L, 5 * nb + 8)) return 1;
+  if (ensure_partials(L, 5 * nb + 16)) return 1;
+  double *const res = L.partials + 5 * nb + 5 * slot;
   double *dpsi = nullptr;
   if (psi) {
     CK(cudaMallocAsync(&dpsi, (size_t)L.nnodes * sizeof(double), L.stream));
     CK(cudaMemcpyAsync(dpsi, psi, (size_t)L.nnodes * sizeof(double), cudaMemcpyHostToDevice, L.stream));
   }
   CK(DISPATCH3(L, launch_vsum, L, fac, dpsi, L.partials, nb));
-  k_final_sum_tree<5><<<1, 256, 0, L.stream>>>(L.partials, nb, L.partials + 5 * nb);
+  k_final_sum_tree<5><<<1, 256, 0, L.stream>>>(L.partials, nb, res);
   count_launch();
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(L.host_out, L.partials + 5 * nb, 5 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
+  CK(cudaMemcpyAsync(L.host_out + 5 * slot, res, 5 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
   if (dpsi) CK(cudaFreeAsync(dpsi, L.stream));
-  CK(cudaStreamSynchronize(L.stream));
-  for (int c = 0; c < 5; c++) out[c] = L.host_out[c];
   return 0;
+}
+
+int slbc_vsum_begin(slbc_lattice *h, double fac, const double *psi, int slot) {
+  if (slot < 0 || slot > 2) return fail_msg("slbc_vsum_begin: slot 0, 1 or 2");
+  return vsum_enqueue(h->L, fac, psi, slot);
+}
+
+int slbc_vsum_end(slbc_lattice *h, int slot, double out[5]) {
+  Lattice &L = h->L;
+  if (slot < 0 || slot > 2) return fail_msg("slbc_vsum_end: slot 0, 1 or 2");
+  CK(cudaStreamSynchronize(L.stream));
+  for (int c = 0; c < 5; c++) out[c] = L.host_out[5 * slot + c];
+  return 0;
+}
+
+int slbc_vsum(slbc_lattice *h, double fac, const double *psi, double out[5]) {
+  if (vsum_enqueue(h->L, fac, psi, 0)) return 1;
+  return slbc_vsum_end(h, 0, out);
 }
 
 int slbc_distribf(slbc_lattice *h, const double *pos, double *ft) {

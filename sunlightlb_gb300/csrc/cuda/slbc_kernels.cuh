@@ -410,7 +410,8 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> a, OddOffsets off) {
 // last warp is short.  The FP64 step is bound by the FP64 pipe, where a lane
 // without a node costs as much as one with; the division that finds (j, k)
 // is integer work beside it.  (126 x 110 x 97: rows of 97 in four warps, 407
-// us; as runs of 10,670 nodes 318 us.)
+// us; as runs of 10,670 nodes 310 us.)  Small lattices take blocks of one
+// warp: what counts there is how evenly the nodes spread over the SMs.
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(128) k_step_run(StepArgs<T> a, OddOffsets off) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.z;

@@ -86,8 +86,9 @@ static void step_variant(Lattice &L, const StepArgs<T_> &a, int npt, int bx) {
   // go as runs over whole planes (32-bit indices only)
   if (std::is_same<T_, double>::value && 15LL * L.npad <= 0xFFFFFFFFLL &&
       17 * L.esk < 16 * ((L.esk + 31) / 32 * 32)) {
-    const dim3 run((unsigned)((L.esj * L.esk + 127) / 128), 1, (unsigned)L.esi);
-    k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU><<<run, 128, 0, L.stream>>>(a, odd_offsets(L));
+    const int bs = L.nnodes < 152LL * 128 * 8 ? 32 : 128;
+    const dim3 run((unsigned)((L.esj * L.esk + bs - 1) / bs), 1, (unsigned)L.esi);
+    k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU><<<run, bs, 0, L.stream>>>(a, odd_offsets(L));
     return;
   }
   const dim3 grid((unsigned)((L.esk + bx - 1) / bx), (unsigned)((L.esj + npt - 1) / npt), (unsigned)L.esi);

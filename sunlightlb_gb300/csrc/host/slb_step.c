@@ -207,23 +207,32 @@ void batchsteps(LBBatch b, int n) {
 
 /* ---- measurement: reference src/lbmeasure.c ------------------------------ */
 
-/* reference src/lbmeasure.c:58-106 */
-void accvmean(LBSys lb, LBReal prefac) {
-  double s[5];
-  LBReal fac = 0.0, wfac, uxtot, uytot, uztot;
-  int nfluid;
+/* body force factor of the mean velocity at the present status */
+static LBReal vmean_fac(LBSys lb) {
+  LBReal fac = 0.0;
   if (lb->vel_corrected) switch (lb->status) {
     case POST_PROPAGATE: fac = 0.5; break;
     case POST_COLLIDE: fac = -0.5; break;
     default: printf("Accvmean apparently of position\n"); wrstatus(lb, stdout); break;
   }
-  slb_check(slbc_vsum(slb_device(lb), fac, lb->psi, s), "mean velocity");
-  nfluid = (int)s[4];
-  wfac = nfluid / s[3];
-  uxtot = s[0] * wfac; uytot = s[1] * wfac; uztot = s[2] * wfac;
+  return fac;
+}
+
+static void add_vmean(LBSys lb, LBReal prefac, const double s[5]) {
+  int nfluid = (int)s[4];
+  LBReal wfac = nfluid / s[3];
+  LBReal uxtot = s[0] * wfac, uytot = s[1] * wfac, uztot = s[2] * wfac;
   lb->vmeanx += prefac * uxtot / (lb->nnodes);
   lb->vmeany += prefac * uytot / (lb->nnodes);
   lb->vmeanz += prefac * uztot / (lb->nnodes);
+}
+
+/* reference src/lbmeasure.c:58-106 */
+void accvmean(LBSys lb, LBReal prefac) {
+  double s[5];
+  LBReal fac = vmean_fac(lb);
+  slb_check(slbc_vsum(slb_device(lb), fac, lb->psi, s), "mean velocity");
+  add_vmean(lb, prefac, s);
   slb_trace(lb, "accvmean");
 }
 
@@ -278,19 +287,38 @@ void distribf(LBSys lb) {
 void measure(LBSys lb) {
   int fused = lb->status == POST_COLLIDE;
   if (!fused) out_of_position(lb, "Measurements");
+  else slb_need_relaxed_solids(lb);  /* a change of storage now, not between the sums and their reading */
   /* zeroforce on the device only: the force steps below change the node
    * forces at once, so the host arrays are refreshed by lbpull on demand */
   slb_check(slbc_zero_force(slb_device(lb)), "force reset");
   slb_forces_changed(lb);
   slb_trace(lb, "zeroforce");
   lb->vmeanx = lb->vmeany = lb->vmeanz = 0.0;
-  accvmean(lb, 0.25);
-  if (fused) fused_step(lb, 1); else { bblforce(lb); propagate(lb); collide(lb); }
-  accvmean(lb, 0.5);
-  if (fused) fused_step(lb, 1); else { bblforce(lb); propagate(lb); collide(lb); }
-  accvmean(lb, 0.25);
-  normforce(lb, 0.5);
-  distribf(lb);
+  if (fused) {
+    /* the three sums are queued between the steps and read once */
+    static const LBReal weight[3] = {0.25, 0.5, 0.25};
+    double s[5];
+    int k;
+    for (k = 0; k < 3; k++) {
+      slb_check(slbc_vsum_begin(slb_device(lb), vmean_fac(lb), lb->psi, k), "mean velocity");
+      slb_trace(lb, "accvmean");
+      if (k < 2) fused_step(lb, 1);
+    }
+    normforce(lb, 0.5);
+    distribf(lb);
+    for (k = 0; k < 3; k++) {
+      slb_check(slbc_vsum_end(slb_device(lb), k, s), "mean velocity");
+      add_vmean(lb, weight[k], s);
+    }
+  } else {
+    accvmean(lb, 0.25);
+    bblforce(lb); propagate(lb); collide(lb);
+    accvmean(lb, 0.5);
+    bblforce(lb); propagate(lb); collide(lb);
+    accvmean(lb, 0.25);
+    normforce(lb, 0.5);
+    distribf(lb);
+  }
   slb_trace(lb, "measure");
 }
 
