@@ -136,6 +136,7 @@ constexpr int kPairSmem = kPairSlots * 15 * kPlane * (int)sizeof(float);
 // direction opp(q)), and writes its new state with two 16-byte stores.
 template <bool MOVING, bool BFU>
 __global__ void __launch_bounds__(kTileThreads, 3) k_step_pair(PairArgs a, StepArgs<float> s, int planes) {
+  after_previous();
   extern __shared__ __align__(16) float dec[];  // [slot][q][kPlane]
   const int tk = threadIdx.x, tj = threadIdx.y, tid = tj * kTileK + tk;
   const int k0 = blockIdx.x * kTileK, j0 = blockIdx.y * kTileJ, i0 = blockIdx.z * planes;
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(kTileThreads, 3) k_step_pair(PairArgs a, StepA
 // rounding of the larger, or than 2^-20 of the two populations, is counted
 // in *unpaired (the host then keeps the lattice in FP32)
 __global__ void k_put_pair(PairArgs a, const double *stage, long long x0, long long n, int *unpaired) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -255,6 +257,7 @@ __global__ void k_put_pair(PairArgs a, const double *stage, long long x0, long l
 
 // state -> host AoS staging of the reference's array
 __global__ void k_get_pair(PairArgs a, double *stage, long long x0, long long n) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -266,6 +269,7 @@ __global__ void k_get_pair(PairArgs a, double *stage, long long x0, long long n)
 __global__ void __launch_bounds__(kReduceThreads)
 k_vsum_pair(PairArgs a, double rho0, double fac, int bf_uniform, double b0, double b1, double b2,
             const float *bf, const double *psi, double *partials) {
+  after_previous();
   Acc<float> ax, ay, az;
   double wsum = 0.0;
   int count = 0;
@@ -300,6 +304,7 @@ k_vsum_pair(PairArgs a, double rho0, double fac, int bf_uniform, double b0, doub
 // node forces of one bblforce from reconstructed populations (FP32 terms,
 // compensated sums, FP64 store)
 __global__ void k_force_pair(PairArgs a, int moving, const float *uw, ForceArgs f) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= f.nbnd) return;
   const int s = f.bnd_node[e];
@@ -328,6 +333,7 @@ __global__ void k_force_pair(PairArgs a, int moving, const float *uw, ForceArgs 
 // src/lbstore.c:352-399, as moments and paired stress deviations
 __global__ void k_setvel_pair(PairArgs a, const double *stage, long long x0, long long n, int has_rho,
                               double rho0, int stokes, int skip_solid) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -350,6 +356,7 @@ __global__ void k_setvel_pair(PairArgs a, const double *stage, long long x0, lon
 // collision of the current state in place (the separate collide phase)
 template <bool BFU>
 __global__ void k_collide_pair(PairArgs a, StepArgs<float> s) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= (long long)a.esi * a.esj * a.esk) return;
   const bool solid = (a.flags[x] & FLAG_SOLID) != 0;
@@ -365,6 +372,7 @@ __global__ void k_collide_pair(PairArgs a, StepArgs<float> s) {
 
 // density snapshot of the tracer: rho0 + drho on fluid nodes
 __global__ void k_mp_rhoinit_pair(PairArgs a, double rho0, double *rho64, float *rho32) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= (long long)a.esi * a.esj * a.esk) return;
   double r = rho0;
@@ -455,11 +463,11 @@ cudaError_t launch_pair_step(Lattice &L, int planes) {
     attr_set |= 1ull << (dev & 63);
   }
   if (s.moving) {
-    if (s.bf_uniform) k_step_pair<true, true><<<g, b, kPairSmem, L.stream>>>(a, s, planes);
-    else k_step_pair<true, false><<<g, b, kPairSmem, L.stream>>>(a, s, planes);
+    if (s.bf_uniform) launch_pdl(k_step_pair<true, true>, g, b, kPairSmem, L.stream, a, s, planes);
+    else launch_pdl(k_step_pair<true, false>, g, b, kPairSmem, L.stream, a, s, planes);
   } else {
-    if (s.bf_uniform) k_step_pair<false, true><<<g, b, kPairSmem, L.stream>>>(a, s, planes);
-    else k_step_pair<false, false><<<g, b, kPairSmem, L.stream>>>(a, s, planes);
+    if (s.bf_uniform) launch_pdl(k_step_pair<false, true>, g, b, kPairSmem, L.stream, a, s, planes);
+    else launch_pdl(k_step_pair<false, false>, g, b, kPairSmem, L.stream, a, s, planes);
   }
   count_launch();
   return cudaGetLastError();
@@ -475,19 +483,19 @@ cudaError_t launch_step_bf16(Lattice &L, int /*odd*/) {
 }
 
 cudaError_t launch_put_bf16(Lattice &L, const double *stage, long long x0, long long n, int *unpaired) {
-  k_put_pair<<<fblocks(n, 256), 256, 0, L.stream>>>(pair_args_inplace(L), stage, x0, n, unpaired);
+  launch_pdl(k_put_pair, fblocks(n, 256), 256, 0, L.stream, pair_args_inplace(L), stage, x0, n, unpaired);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_get_bf16(Lattice &L, double *stage, long long x0, long long n) {
-  k_get_pair<<<fblocks(n, 256), 256, 0, L.stream>>>(pair_args(L), stage, x0, n);
+  launch_pdl(k_get_pair, fblocks(n, 256), 256, 0, L.stream, pair_args(L), stage, x0, n);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_vsum_bf16(Lattice &L, double fac, const double *psi, double *partials, int nblocks) {
-  k_vsum_pair<<<nblocks, kReduceThreads, 0, L.stream>>>(pair_args(L), L.par.rho0, fac, L.bf_uniform,
+  launch_pdl(k_vsum_pair, nblocks, kReduceThreads, 0, L.stream, pair_args(L), L.par.rho0, fac, L.bf_uniform,
                                                          L.bf_const[0], L.bf_const[1], L.bf_const[2],
                                                          (const float *)L.bf, psi, partials);
   count_launch();
@@ -498,14 +506,15 @@ cudaError_t launch_force_bf16(Lattice &L) {
   if (L.nbnd == 0) return cudaSuccess;
   ForceArgs f{L.nbnd, L.bnd_node, L.bnd_f};
   const int moving = L.par.objects_moving && L.uw != nullptr;
-  k_force_pair<<<fblocks(L.nbnd, 128), 128, 0, L.stream>>>(pair_args(L), moving, (const float *)L.uw, f);
+  launch_pdl(k_force_pair, fblocks(L.nbnd, 128), 128, 0, L.stream, pair_args(L), moving, (const float *)L.uw, f);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_setvel_bf16(Lattice &L, const double *stage, long long x0, long long n, int has_rho,
                                int skip_solid) {
-  k_setvel_pair<<<fblocks(n, 256), 256, 0, L.stream>>>(pair_args_inplace(L), stage, x0, n, has_rho, L.par.rho0,
+  launch_pdl(k_setvel_pair, fblocks(n, 256), 256, 0, L.stream, pair_args_inplace(L), stage, x0, n, has_rho,
+             L.par.rho0,
                                                        L.par.stokes_flow, skip_solid);
   count_launch();
   return cudaGetLastError();
@@ -517,14 +526,15 @@ cudaError_t launch_collide_bf16(Lattice &L) {
     return cudaErrorInvalidValue;
   }
   const StepArgs<float> s = step_args_f(L);
-  if (s.bf_uniform) k_collide_pair<true><<<fblocks(L.nnodes, 256), 256, 0, L.stream>>>(pair_args_inplace(L), s);
-  else k_collide_pair<false><<<fblocks(L.nnodes, 256), 256, 0, L.stream>>>(pair_args_inplace(L), s);
+  if (s.bf_uniform) launch_pdl(k_collide_pair<true>, fblocks(L.nnodes, 256), 256, 0, L.stream, pair_args_inplace(L),
+                               s);
+  else launch_pdl(k_collide_pair<false>, fblocks(L.nnodes, 256), 256, 0, L.stream, pair_args_inplace(L), s);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t launch_mp_rhoinit_bf16(Lattice &L) {
-  k_mp_rhoinit_pair<<<fblocks(L.nnodes, 256), 256, 0, L.stream>>>(pair_args(L), L.par.rho0, L.mp_rho64,
+  launch_pdl(k_mp_rhoinit_pair, fblocks(L.nnodes, 256), 256, 0, L.stream, pair_args(L), L.par.rho0, L.mp_rho64,
                                                                   L.mp_rho32);
   count_launch();
   return cudaGetLastError();

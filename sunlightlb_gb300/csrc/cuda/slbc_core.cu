@@ -77,6 +77,7 @@ size_t side_size(int precision) { return precision == 0 ? 8 : 4; }
 // Flag words from the object map: solid bit, and bit q when x - c_q differs
 // in solidity from x.
 __global__ void k_flags(const int *objidx, uint16_t *flags, int esi, int esj, int esk) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y, i = blockIdx.z;
   if (k >= esk) return;
@@ -105,6 +106,7 @@ constexpr int kBndChunk = 4096;
 __device__ __forceinline__ bool boundary_solid(uint16_t f) { return (f & FLAG_SOLID) && (f & FLAG_LINKS); }
 
 __global__ void __launch_bounds__(256) k_bnd_count(const uint16_t *flags, long long n, int *counts) {
+  after_previous();
   __shared__ int total;
   if (threadIdx.x == 0) total = 0;
   __syncthreads();
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(256) k_bnd_count(const uint16_t *flags, long l
 
 __global__ void __launch_bounds__(256) k_bnd_write(const uint16_t *flags, long long n, const int *offsets,
                                                    int *out) {
+  after_previous();
   __shared__ int warp_sum[8];
   __shared__ int base;
   if (threadIdx.x == 0) base = offsets[blockIdx.x];
@@ -146,6 +149,7 @@ __global__ void __launch_bounds__(256) k_bnd_write(const uint16_t *flags, long l
 }
 
 __global__ void k_scale(double *v, long long n, double fac) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n) v[e] *= fac;
 }
@@ -154,6 +158,7 @@ __global__ void k_scale(double *v, long long n, double fac) {
 __global__ void k_distrib_piece(const int *bnd_node, const double *f, long long nbnd,
                                 const int *piece_obj, const int *piece_lo, const int *piece_hi,
                                 const double *pos, int esj, int esk, double *piece_sum) {
+  after_previous();
   const int pc = blockIdx.x;
   const int o = piece_obj[pc];
   const double px = pos[3 * o], py = pos[3 * o + 1], pz = pos[3 * o + 2];
@@ -178,6 +183,7 @@ __global__ void k_distrib_piece(const int *bnd_node, const double *f, long long 
 // 5,000 pieces of a 512^3 bed held as one object took 1.17 ms; the warp 15 us).
 __global__ void __launch_bounds__(128) k_distrib_obj(const int *obj_first_piece, const int *obj_npiece,
                                                      const double *piece_sum, int nobj, double *ft) {
+  after_previous();
   const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (o >= nobj) return;
   double v[6] = {0, 0, 0, 0, 0, 0};
@@ -197,6 +203,7 @@ __global__ void __launch_bounds__(128) k_distrib_obj(const int *obj_first_piece,
 // solid node x - c_q has its adsorption byte set).
 __global__ void k_ads_links(const uint16_t *flags, const unsigned char *ads, uint16_t *links, int esi,
                             int esj, int esk) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= (long long)esi * esj * esk) return;
   const uint16_t fl = flags[x];
@@ -216,6 +223,7 @@ __global__ void k_ads_links(const uint16_t *flags, const unsigned char *ads, uin
 // given, the density deviations rho - rho0 (else rho = rho0).
 __global__ void k_stage_velocity(const float *u, const float *drho, long long nnodes, long long x0, long long n,
                                  double *stage) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -230,6 +238,7 @@ template <typename TP>
 __global__ void __launch_bounds__(kReduceThreads)
 k_mp_sums(const TP *p, const uint16_t *flags, const unsigned char *ads, long long n, int esj,
           int esk, int axis, double *partials) {
+  after_previous();
   double v[5] = {0, 0, 0, 0, 0};
   for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < n;
        x += (long long)gridDim.x * blockDim.x) {
@@ -251,6 +260,7 @@ k_mp_sums(const TP *p, const uint16_t *flags, const unsigned char *ads, long lon
 
 template <typename TP>
 __global__ void k_mp_minmax(const TP *p, const uint16_t *flags, long long n, double *partials) {
+  after_previous();
   double lo = 1e300, hi = -1e300;
   for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < n;
        x += (long long)gridDim.x * blockDim.x) {
@@ -296,6 +306,7 @@ __global__ void __launch_bounds__(kReduceThreads)
 k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, int kind, double g0, double g1,
           double g2, double g3, double g4, double g5, double value, int count, double *partials, unsigned *done,
           double *acc) {
+  after_previous();
   double v[1] = {0.0};
   const TP nv = (TP)value;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
@@ -354,6 +365,7 @@ template <typename TP>
 __global__ void __launch_bounds__(kReduceThreads)
 k_mp_plane(const TP *p, const uint16_t *flags, int esi, int esj, int esk, int axis, int pos,
            long long count, double *partials) {
+  after_previous();
   double v[2] = {0.0, 0.0};
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < count;
        e += (long long)gridDim.x * blockDim.x) {
@@ -369,6 +381,7 @@ k_mp_plane(const TP *p, const uint16_t *flags, int esi, int esj, int esk, int ax
 template <typename TP>
 __global__ void k_mp_misc(TP *p, const TP *src, const uint16_t *flags, const unsigned char *ads,
                           long long n, int op, double fac) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n) return;
   const bool solid = flags[x] & FLAG_SOLID;
@@ -379,6 +392,7 @@ __global__ void k_mp_misc(TP *p, const TP *src, const uint16_t *flags, const uns
 
 template <typename TD, typename TS>
 __global__ void k_convert(TD *dst, const TS *src, long long n) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n) dst[e] = (TD)src[e];
 }
@@ -614,6 +628,7 @@ namespace slbc {
 
 // 1/rho of the FP64 density snapshot, for the FP32 tracer update
 __global__ void k_mp_rinv(const double *rho64, float *rinv, long long n) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x < n) rinv[x] = (float)(1.0 / rho64[x]);
 }
@@ -638,6 +653,7 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
 __global__ void __launch_bounds__(kTileThreads, 4)
 k_mp_apply(const float *coef, const float *pin, const float *lin, float *pout, float *lout, int esi, int esj,
            int esk, unsigned npad, int planes) {
+  after_previous();
   __shared__ float2 ring[3][kPlane];
   const int tk = threadIdx.x, tj = threadIdx.y, tid = tj * kTileK + tk;
   const int k0 = blockIdx.x * kTileK, j0 = blockIdx.y * kTileJ, i0 = blockIdx.z * planes;
@@ -707,6 +723,7 @@ k_mp_apply(const float *coef, const float *pin, const float *lin, float *pout, f
 // this pass adds the FP64 residual 1 - sum to C_0(y), so that the stencil
 // conserves mass to the rounding of C_0 alone.
 __global__ void k_mp_coef_norm(float *coef, const uint16_t *flags, int esi, int esj, int esk, unsigned npad) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long long)esi * esj * esk) return;
   const int x = (int)e;
@@ -721,7 +738,7 @@ __global__ void k_mp_coef_norm(float *coef, const uint16_t *flags, int esi, int 
 }
 
 cudaError_t launch_mp_coef_norm(Lattice &L) {
-  k_mp_coef_norm<<<(int)((L.nnodes + 255) / 256), 256, 0, L.stream>>>(L.mp_coef, L.flags, L.esi, L.esj, L.esk,
+  launch_pdl(k_mp_coef_norm, (int)((L.nnodes + 255) / 256), 256, 0, L.stream, L.mp_coef, L.flags, L.esi, L.esj, L.esk,
                                                                       (unsigned)L.npad);
   g_launches += 1;
   return cudaGetLastError();
@@ -729,7 +746,8 @@ cudaError_t launch_mp_coef_norm(Lattice &L) {
 
 cudaError_t launch_mp_apply(Lattice &L, const float *pin, const float *lin, float *pout, float *lout, dim3 grid,
                             dim3 block, int planes) {
-  k_mp_apply<<<grid, block, 0, L.stream>>>(L.mp_coef, pin, lin, pout, lout, L.esi, L.esj, L.esk, (unsigned)L.npad,
+  launch_pdl(k_mp_apply, grid, block, 0, L.stream, L.mp_coef, pin, lin, pout, lout, L.esi, L.esj, L.esk,
+             (unsigned)L.npad,
                                            planes);
   g_launches += 1;
   return cudaGetLastError();
@@ -741,7 +759,7 @@ cudaError_t ensure_mp_rinv(Lattice &L) {
   cudaError_t e = cudaSuccess;
   if (!L.mp_rinv32) e = cudaMalloc(&L.mp_rinv32, (size_t)L.nnodes * sizeof(float));
   if (e != cudaSuccess) return e;
-  k_mp_rinv<<<(int)((L.nnodes + 255) / 256), 256, 0, L.stream>>>(L.mp_rho64, L.mp_rinv32, L.nnodes);
+  launch_pdl(k_mp_rinv, (int)((L.nnodes + 255) / 256), 256, 0, L.stream, L.mp_rho64, L.mp_rinv32, L.nnodes);
   g_launches += 1;
   e = cudaGetLastError();
   if (e == cudaSuccess) L.mp_rinv_gen = L.mp_rho_gen;
@@ -749,6 +767,7 @@ cudaError_t ensure_mp_rinv(Lattice &L) {
 }
 
 __global__ void k_mp_ratios(const double *rho64, double rho0, double *rinv, double *ratio, long long n) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n) return;
   const double r = rho64[x];
@@ -763,7 +782,8 @@ cudaError_t ensure_mp_ratios(Lattice &L) {
   if (!L.mp_rinv64) e = cudaMalloc(&L.mp_rinv64, (size_t)L.nnodes * sizeof(double));
   if (e == cudaSuccess && !L.mp_ratio64) e = cudaMalloc(&L.mp_ratio64, (size_t)L.nnodes * sizeof(double));
   if (e != cudaSuccess) return e;
-  k_mp_ratios<<<(int)((L.nnodes + 255) / 256), 256, 0, L.stream>>>(L.mp_rho64, L.par.rho0, L.mp_rinv64, L.mp_ratio64,
+  launch_pdl(k_mp_ratios, (int)((L.nnodes + 255) / 256), 256, 0, L.stream, L.mp_rho64, L.par.rho0, L.mp_rinv64,
+             L.mp_ratio64,
                                                                    L.nnodes);
   g_launches += 1;
   e = cudaGetLastError();
@@ -946,7 +966,7 @@ static int geometry_flags(Lattice &L, slbc_lattice *h, const int *objidx) {
   CK(cudaMemcpyAsync(L.objidx, objidx, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, L.stream));
   const int bx = L.esk >= 128 ? 128 : 32;
   dim3 grid((L.esk + bx - 1) / bx, L.esj, L.esi);
-  k_flags<<<grid, bx, 0, L.stream>>>(L.objidx, L.flags, L.esi, L.esj, L.esk);
+  launch_pdl(k_flags, grid, bx, 0, L.stream, L.objidx, L.flags, L.esi, L.esj, L.esk);
   count_launch();
   CK(cudaGetLastError());
   return 0;
@@ -1037,7 +1057,7 @@ static int boundary_from_flags(Lattice &L, const int *objidx, int nobj, long **b
   const int nb = (int)((L.nnodes + kBndChunk - 1) / kBndChunk);
   int *counts = nullptr, *list = nullptr;
   CK(cudaMalloc(&counts, (size_t)nb * sizeof(int)));
-  k_bnd_count<<<nb, 256, 0, L.stream>>>(L.flags, L.nnodes, counts);
+  launch_pdl(k_bnd_count, nb, 256, 0, L.stream, L.flags, L.nnodes, counts);
   count_launch();
   std::vector<int> off((size_t)nb);
   cudaError_t e = cudaMemcpyAsync(off.data(), counts, (size_t)nb * sizeof(int), cudaMemcpyDeviceToHost, L.stream);
@@ -1052,7 +1072,7 @@ static int boundary_from_flags(Lattice &L, const int *objidx, int nobj, long **b
   if (e == cudaSuccess && total > 0) e = cudaMalloc(&list, (size_t)total * sizeof(int));
   std::vector<int> nodes((size_t)total);
   if (e == cudaSuccess && total > 0) {
-    k_bnd_write<<<nb, 256, 0, L.stream>>>(L.flags, L.nnodes, counts, list);
+    launch_pdl(k_bnd_write, nb, 256, 0, L.stream, L.flags, L.nnodes, counts, list);
     count_launch();
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(nodes.data(), list, (size_t)total * sizeof(int), cudaMemcpyDeviceToHost, L.stream);
@@ -1170,7 +1190,7 @@ int slbc_move_sphere(slbc_lattice *h, int obj, double rad, const double oldc[3],
   // flag words from the updated map, then the boundary list
   const int bx = L.esk >= 128 ? 128 : 32;
   dim3 grid((L.esk + bx - 1) / bx, L.esj, L.esi);
-  k_flags<<<grid, bx, 0, L.stream>>>(L.objidx, L.flags, L.esi, L.esj, L.esk);
+  launch_pdl(k_flags, grid, bx, 0, L.stream, L.objidx, L.flags, L.esi, L.esj, L.esk);
   count_launch();
   CK(cudaGetLastError());
   return boundary_from_flags(L, objidx_host, nobj, bnd_node_out, bnd_obj_out, nbnd_out);
@@ -1422,7 +1442,7 @@ int slbc_zero_force(slbc_lattice *h) {
 int slbc_scale_force(slbc_lattice *h, double fac) {
   Lattice &L = h->L;
   if (!L.nbnd) return 0;
-  k_scale<<<blocks_for(3 * L.nbnd, 256), 256, 0, L.stream>>>(L.bnd_f, 3 * L.nbnd, fac);
+  launch_pdl(k_scale, blocks_for(3 * L.nbnd, 256), 256, 0, L.stream, L.bnd_f, 3 * L.nbnd, fac);
   count_launch();
   CK(cudaGetLastError());
   return 0;
@@ -1460,7 +1480,7 @@ static int vsum_enqueue(Lattice &L, double fac, const double *psi, int slot) {
     CK(cudaMemcpyAsync(dpsi, psi, (size_t)L.nnodes * sizeof(double), cudaMemcpyHostToDevice, L.stream));
   }
   CK(DISPATCH3(L, launch_vsum, L, fac, dpsi, L.partials, nb));
-  k_final_sum_tree<5><<<1, 256, 0, L.stream>>>(L.partials, nb, res);
+  launch_pdl(k_final_sum_tree<5>, 1, 256, 0, L.stream, L.partials, nb, res);
   count_launch();
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(L.host_out + 5 * slot, res, 5 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
@@ -1491,14 +1511,14 @@ int slbc_distribf(slbc_lattice *h, const double *pos, double *ft) {
   if (L.nobj == 0) return 0;
   CK(cudaMemcpyAsync(L.obj_pos, pos, 3 * (size_t)L.nobj * sizeof(double), cudaMemcpyHostToDevice, L.stream));
   if (L.npiece > 0) {
-    k_distrib_piece<<<L.npiece, 256, 0, L.stream>>>(L.bnd_node, L.bnd_f, L.nbnd, L.piece_obj,
+    launch_pdl(k_distrib_piece, L.npiece, 256, 0, L.stream, L.bnd_node, L.bnd_f, L.nbnd, L.piece_obj,
                                                    L.piece_lo, L.piece_hi, L.obj_pos, L.esj,
                                                    L.esk, L.piece_sum);
     count_launch();
     CK(cudaGetLastError());
   }
   const int *first = (const int *)(L.obj_ft + 6 * L.nobj);
-  k_distrib_obj<<<blocks_for(L.nobj, 4), 128, 0, L.stream>>>(first, first + L.nobj, L.piece_sum,
+  launch_pdl(k_distrib_obj, blocks_for(L.nobj, 4), 128, 0, L.stream, first, first + L.nobj, L.piece_sum,
                                                                L.nobj, L.obj_ft);
   count_launch();
   CK(cudaGetLastError());
@@ -1546,7 +1566,7 @@ int slbc_set_state_dev(slbc_lattice *h, const float *u, const float *drho, int s
   const long long chunk = L.staging_nodes / 4;
   for (long long x0 = 0; x0 < L.nnodes; x0 += chunk) {
     const long long n = std::min(chunk, L.nnodes - x0);
-    k_stage_velocity<<<blocks_for(n, 256), 256, 0, L.stream>>>(u, drho, L.nnodes, x0, n, L.staging);
+    launch_pdl(k_stage_velocity, blocks_for(n, 256), 256, 0, L.stream, u, drho, L.nnodes, x0, n, L.staging);
     count_launch();
     CK(cudaGetLastError());
     CK(DISPATCH3(L, launch_setvel, L, L.staging, x0, n, drho ? 2 : 0, skip_solid));
@@ -1586,7 +1606,8 @@ int slbc_mp_create(slbc_lattice *h, slbc_tracer **out, int use_f64) {
   if (e == cudaSuccess && !use_f64 && !L.mp_rho32) {
     e = cudaMalloc(&L.mp_rho32, (size_t)L.nnodes * sizeof(float));
     if (e == cudaSuccess) {
-      k_convert<float, double><<<blocks_for(L.nnodes, 256), 256, 0, L.stream>>>(L.mp_rho32, L.mp_rho64, L.nnodes);
+      launch_pdl(k_convert<float, double>, blocks_for(L.nnodes, 256), 256, 0, L.stream, L.mp_rho32, L.mp_rho64,
+                 L.nnodes);
       count_launch();
       e = cudaGetLastError();
     }
@@ -1659,7 +1680,8 @@ int slbc_mp_get(slbc_tracer *t, double *p) {
     const long long chunk = L.staging_nodes;
     for (long long x0 = 0; x0 < L.nnodes; x0 += chunk) {
       const long long n = std::min(chunk, L.nnodes - x0);
-      k_convert<double, float><<<blocks_for(n, 256), 256, 0, L.stream>>>(L.staging, (const float *)t->p + x0, n);
+      launch_pdl(k_convert<double, float>, blocks_for(n, 256), 256, 0, L.stream, L.staging,
+                 (const float *)t->p + x0, n);
       count_launch();
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(p + x0, L.staging, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
@@ -1675,7 +1697,8 @@ int slbc_mp_step(slbc_tracer *t, int n, double alpha, double adprob, int moving,
   if (no_bf16(L, "slbc_mp_step")) return 1;
   if (L.ads && L.ads_links_version != L.ads_version) {
     if (!L.ads_links) CK(cudaMalloc(&L.ads_links, (size_t)L.nnodes * sizeof(uint16_t)));
-    k_ads_links<<<blocks_for(L.nnodes, 256), 256, 0, L.stream>>>(L.flags, L.ads, L.ads_links, L.esi, L.esj, L.esk);
+    launch_pdl(k_ads_links, blocks_for(L.nnodes, 256), 256, 0, L.stream, L.flags, L.ads, L.ads_links, L.esi, L.esj,
+               L.esk);
     count_launch();
     CK(cudaGetLastError());
     L.ads_links_version = L.ads_version;
@@ -1705,12 +1728,14 @@ static int mp_reduce(slbc_tracer *t, int axis, double out[5]) {
   const int nb = 152 * 4;
   if (ensure_partials(L, 5 * nb + 8)) return 1;
   if (t->f64)
-    k_mp_sums<double><<<nb, kReduceThreads, 0, L.stream>>>((const double *)t->p, L.flags, L.ads, L.nnodes, L.esj, L.esk, axis, L.partials);
+    launch_pdl(k_mp_sums<double>, nb, kReduceThreads, 0, L.stream, (const double *)t->p, L.flags, L.ads, L.nnodes,
+               L.esj, L.esk, axis, L.partials);
   else
-    k_mp_sums<float><<<nb, kReduceThreads, 0, L.stream>>>((const float *)t->p, L.flags, L.ads, L.nnodes, L.esj, L.esk, axis, L.partials);
+    launch_pdl(k_mp_sums<float>, nb, kReduceThreads, 0, L.stream, (const float *)t->p, L.flags, L.ads, L.nnodes,
+               L.esj, L.esk, axis, L.partials);
   count_launch();
   CK(cudaGetLastError());
-  k_final_sum_tree<5><<<1, 256, 0, L.stream>>>(L.partials, nb, L.partials + 5 * nb);
+  launch_pdl(k_final_sum_tree<5>, 1, 256, 0, L.stream, L.partials, nb, L.partials + 5 * nb);
   count_launch();
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(L.host_out, L.partials + 5 * nb, 5 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
@@ -1725,6 +1750,7 @@ namespace slbc {
 // pass 1 of the tracer velocity autocorrelation: sums of psi P and psi^2
 __global__ void __launch_bounds__(kReduceThreads) k_vacf_mean(const double *p, const uint16_t *flags,
                                                             const double *psi, long long n, double *partials) {
+  after_previous();
   double v[2] = {0.0, 0.0};
   for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (long long)gridDim.x * blockDim.x) {
     if (flags[x] & FLAG_SOLID) continue;
@@ -1753,11 +1779,11 @@ int slbc_mp_vacf(slbc_tracer *t, slbc_tracer *t2, int axis, const double *psi_ho
   }
   double sums[2];
   cudaError_t e = cudaSuccess;
-  k_vacf_mean<<<nb, kReduceThreads, 0, L.stream>>>((const double *)t->p, L.flags, psi, L.nnodes, L.partials);
+  launch_pdl(k_vacf_mean, nb, kReduceThreads, 0, L.stream, (const double *)t->p, L.flags, psi, L.nnodes, L.partials);
   count_launch();
   e = cudaGetLastError();
   if (e == cudaSuccess) {
-    k_final_sum_tree<2><<<1, 256, 0, L.stream>>>(L.partials, nb, L.partials + 2 * nb);
+    launch_pdl(k_final_sum_tree<2>, 1, 256, 0, L.stream, L.partials, nb, L.partials + 2 * nb);
     count_launch();
     e = cudaGetLastError();
   }
@@ -1766,7 +1792,7 @@ int slbc_mp_vacf(slbc_tracer *t, slbc_tracer *t2, int axis, const double *psi_ho
   if (e == cudaSuccess) e = DISPATCH(L, launch_vacf_sums, L, (double *)t->p, (const double *)t2->p, psi, sums[0] / sums[1],
                                      axis, L.partials, nb);
   if (e == cudaSuccess) {
-    k_final_sum_tree<2><<<1, 256, 0, L.stream>>>(L.partials, nb, L.partials + 2 * nb);
+    launch_pdl(k_final_sum_tree<2>, 1, 256, 0, L.stream, L.partials, nb, L.partials + 2 * nb);
     count_launch();
     e = cudaGetLastError();
   }
@@ -1784,8 +1810,9 @@ int slbc_mp_minmax(slbc_tracer *t, double out[2]) {
   Lattice &L = t->h->L;
   const int nb = 152 * 2;
   if (ensure_partials(L, 2 * nb + 8)) return 1;
-  if (t->f64) k_mp_minmax<double><<<nb, 256, 0, L.stream>>>((const double *)t->p, L.flags, L.nnodes, L.partials);
-  else k_mp_minmax<float><<<nb, 256, 0, L.stream>>>((const float *)t->p, L.flags, L.nnodes, L.partials);
+  if (t->f64) launch_pdl(k_mp_minmax<double>, nb, 256, 0, L.stream, (const double *)t->p, L.flags, L.nnodes,
+                         L.partials);
+  else launch_pdl(k_mp_minmax<float>, nb, 256, 0, L.stream, (const float *)t->p, L.flags, L.nnodes, L.partials);
   count_launch();
   CK(cudaGetLastError());
   std::vector<double> part(2 * nb);
@@ -1817,9 +1844,12 @@ int slbc_mp_fill(slbc_tracer *t, int kind, const double *geo, double value) {
   if (ensure_partials(L, nb + 8)) return 1;
   unsigned *done = (unsigned *)(t->acc + 1);
   if (t->f64)
-    k_mp_fill<double><<<nb, kReduceThreads, 0, L.stream>>>((double *)t->p, nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
+    launch_pdl(k_mp_fill<double>, nb, kReduceThreads, 0, L.stream, (double *)t->p, nullptr, L.flags, L.esi, L.esj,
+               L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
   else
-    k_mp_fill<float><<<nb, kReduceThreads, 0, L.stream>>>((float *)t->p, t->lo_live ? t->lo : nullptr, L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
+    launch_pdl(k_mp_fill<float>, nb, kReduceThreads, 0, L.stream, (float *)t->p, t->lo_live ? t->lo : nullptr,
+               L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count,
+               L.partials, done, t->acc);
   count_launch();
   CK(cudaGetLastError());
   return 0;
@@ -1843,12 +1873,14 @@ int slbc_mp_plane(slbc_tracer *t, int axis, int pos, double out[2]) {
   const int nb = (int)std::max<long long>(1, std::min<long long>(blocks_for(count, kReduceThreads), 152 * 2));
   if (ensure_partials(L, 2 * nb + 8)) return 1;
   if (t->f64)
-    k_mp_plane<double><<<nb, kReduceThreads, 0, L.stream>>>((const double *)t->p, L.flags, L.esi, L.esj, L.esk, axis, pos, count, L.partials);
+    launch_pdl(k_mp_plane<double>, nb, kReduceThreads, 0, L.stream, (const double *)t->p, L.flags, L.esi, L.esj,
+               L.esk, axis, pos, count, L.partials);
   else
-    k_mp_plane<float><<<nb, kReduceThreads, 0, L.stream>>>((const float *)t->p, L.flags, L.esi, L.esj, L.esk, axis, pos, count, L.partials);
+    launch_pdl(k_mp_plane<float>, nb, kReduceThreads, 0, L.stream, (const float *)t->p, L.flags, L.esi, L.esj,
+               L.esk, axis, pos, count, L.partials);
   count_launch();
   CK(cudaGetLastError());
-  k_final_sum_tree<2><<<1, 256, 0, L.stream>>>(L.partials, nb, L.partials + 2 * nb);
+  launch_pdl(k_final_sum_tree<2>, 1, 256, 0, L.stream, L.partials, nb, L.partials + 2 * nb);
   count_launch();
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(L.host_out, L.partials + 2 * nb, 2 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
@@ -1865,9 +1897,11 @@ static int mp_misc(slbc_tracer *t, const slbc_tracer *src, int op, double fac) {
   // (at most half an FP32 ulp per node, once)
   t->lo_live = 0;
   if (t->f64)
-    k_mp_misc<double><<<blocks_for(L.nnodes, 256), 256, 0, L.stream>>>((double *)t->p, src ? (const double *)src->p : nullptr, L.flags, L.ads, L.nnodes, op, fac);
+    launch_pdl(k_mp_misc<double>, blocks_for(L.nnodes, 256), 256, 0, L.stream, (double *)t->p,
+               src ? (const double *)src->p : nullptr, L.flags, L.ads, L.nnodes, op, fac);
   else
-    k_mp_misc<float><<<blocks_for(L.nnodes, 256), 256, 0, L.stream>>>((float *)t->p, src ? (const float *)src->p : nullptr, L.flags, L.ads, L.nnodes, op, fac);
+    launch_pdl(k_mp_misc<float>, blocks_for(L.nnodes, 256), 256, 0, L.stream, (float *)t->p,
+               src ? (const float *)src->p : nullptr, L.flags, L.ads, L.nnodes, op, fac);
   count_launch();
   CK(cudaGetLastError());
   return 0;

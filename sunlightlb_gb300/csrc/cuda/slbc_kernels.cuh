@@ -358,6 +358,7 @@ __device__ __forceinline__ void step_node(const StepArgs<T> &a, int i, int j, in
 // runs both forms).
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU, int NPT, bool I32 = false>
 __global__ void __launch_bounds__(256) k_step(StepArgs<T> a, OddOffsets off) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.z;
   if (k >= a.p.esk) return;
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(256) k_step(StepArgs<T> a, OddOffsets off) {
 // warp: what counts there is how evenly the nodes spread over the SMs.
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(128) k_step_run(StepArgs<T> a, OddOffsets off) {
+  after_previous();
   const int e = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.z;
   const int esj = a.p.esj, esk = a.p.esk;
   if (e >= esj * esk) return;
@@ -463,6 +465,7 @@ struct BatchDom {
 template <typename T, bool EXACT, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(const BatchDom<T> *doms, const int *work_off,
                                                             const int *work, int nsteps) {
+  after_previous();
   for (int w = work_off[blockIdx.x]; w < work_off[blockIdx.x + 1]; w++) {
     const StepArgs<T> a = doms[work[w]].a;
     const int odd0 = doms[work[w]].odd0;
@@ -489,6 +492,7 @@ constexpr int kBatchTile = 256;
 
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(kBatchTile, 4) k_batch_tiles(const BatchDom<T> *doms, const int2 *tiles) {
+  after_previous();
   __shared__ BatchDom<T> dom;
   const int2 tile = tiles[blockIdx.x];
   constexpr int kWords = (int)(sizeof(BatchDom<T>) / 4);
@@ -561,6 +565,7 @@ __device__ __forceinline__ T post_value(const T *P, long long S, int layout, int
 // state; the links of a solid node s are those whose far end is fluid.
 template <typename T>
 __global__ void k_force(PopArgs<T> p, int layout, int moving, const T *uw, ForceArgs f) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= f.nbnd) return;
   const int s = f.bnd_node[e];
@@ -649,6 +654,7 @@ template <typename T, int LAYOUT>
 __global__ void __launch_bounds__(kReduceThreads)
 k_vsum(PopArgs<T> p, double rho0, double fac, int bf_uniform, double b0, double b1,
        double b2, const T *bf, const double *psi, double *partials) {
+  after_previous();
   Acc<T> ax, ay, az;
   double wsum = 0.0;
   int count = 0;
@@ -702,6 +708,7 @@ k_vsum(PopArgs<T> p, double rho0, double fac, int bf_uniform, double b0, double 
 // adds a fixed strided subset in order, then a fixed-shape tree.
 template <int NV>
 __global__ void __launch_bounds__(256) k_final_sum_tree(const double *partials, int nb, double *out) {
+  after_previous();
   double v[NV];
 #pragma unroll
   for (int c = 0; c < NV; c++) v[c] = 0.0;
@@ -717,6 +724,7 @@ __global__ void __launch_bounds__(256) k_final_sum_tree(const double *partials, 
 // Host AoS staging (FP64, a[15*x + q]) -> layout N.
 template <typename T>
 __global__ void k_put(PopArgs<T> p, const double *stage, long long x0, long long n) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -727,6 +735,7 @@ __global__ void k_put(PopArgs<T> p, const double *stage, long long x0, long long
 // Any layout -> host AoS staging of the reference's array.
 template <typename T>
 __global__ void k_get(PopArgs<T> p, int layout, double *stage, long long x0, long long n) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const int x = (int)(x0 + e);
@@ -747,6 +756,7 @@ constexpr int kHostTile = 128;
 
 template <typename T>
 __global__ void __launch_bounds__(kHostTile) k_put_host(PopArgs<T> p, const double *host, long long n) {
+  after_previous();
   __shared__ double buf[15 * kHostTile];
   for (long long x0 = (long long)blockIdx.x * kHostTile; x0 < n; x0 += (long long)gridDim.x * kHostTile) {
     const int cnt = (int)(n - x0 < kHostTile ? n - x0 : kHostTile);
@@ -763,6 +773,7 @@ __global__ void __launch_bounds__(kHostTile) k_put_host(PopArgs<T> p, const doub
 
 template <typename T>
 __global__ void __launch_bounds__(kHostTile) k_get_host(PopArgs<T> p, int layout, double *host, long long n) {
+  after_previous();
   __shared__ double buf[15 * kHostTile];
   for (long long x0 = (long long)blockIdx.x * kHostTile; x0 < n; x0 += (long long)gridDim.x * kHostTile) {
     const int cnt = (int)(n - x0 < kHostTile ? n - x0 : kHostTile);
@@ -785,6 +796,7 @@ __global__ void __launch_bounds__(kHostTile) k_get_host(PopArgs<T> p, int layout
 // N <-> C0: swap the slots of opposite populations at every node.
 template <typename T>
 __global__ void k_swap(PopArgs<T> p, long long n) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n) return;
   T *P = p.pop;
@@ -800,6 +812,7 @@ __global__ void k_swap(PopArgs<T> p, long long n) {
 // C1 -> N (out of place into dst).
 template <typename T>
 __global__ void k_c1_to_n(PopArgs<T> p, T *dst) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y, i = blockIdx.z;
   if (k >= p.esk) return;
@@ -814,6 +827,7 @@ __global__ void k_c1_to_n(PopArgs<T> p, T *dst) {
 // solid boundary node swaps each of its fluid links; optional force.
 template <typename T>
 __global__ void k_bbl_n(PopArgs<T> p, int moving, const T *uw, int with_force, ForceArgs f) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= f.nbnd) return;
   const int s = f.bnd_node[e];
@@ -850,6 +864,7 @@ __global__ void k_bbl_n(PopArgs<T> p, int moving, const T *uw, int with_force, F
 // (reference src/lbkernel.c:623-762).
 template <typename T>
 __global__ void k_propagate_n(PopArgs<T> p, T *dst) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y, i = blockIdx.z;
   if (k >= p.esk) return;
@@ -862,6 +877,7 @@ __global__ void k_propagate_n(PopArgs<T> p, T *dst) {
 // Separate collision on layout N (reference src/lbkernel.c:769-877).
 template <typename T, bool EXACT>
 __global__ void k_collide_n(StepArgs<T> a) {
+  after_previous();
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)a.p.esi * a.p.esj * a.p.esk;
   if (x >= n) return;
@@ -885,6 +901,7 @@ __global__ void k_collide_n(StepArgs<T> a) {
 template <typename T, bool EXACT>
 __global__ void k_setvel(PopArgs<T> p, const double *stage, long long x0, long long n, int has_rho,
                          double rho0, int stokes, int skip_solid) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const long long x = x0 + e;
@@ -919,6 +936,7 @@ template <typename T>
 __global__ void __launch_bounds__(kReduceThreads) k_vacf_sums(PopArgs<T> pa, int layout, const double *rho,
                                                             double *p, const double *p2, const double *psi,
                                                             double pmean, int axis, double *partials) {
+  after_previous();
   const long long n = (long long)pa.esi * pa.esj * pa.esk;
   double v[2] = {0.0, 0.0};
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
@@ -977,6 +995,7 @@ struct MoveArgs {
 
 template <typename T, bool EXACT>
 __global__ void k_move_sphere(PopArgs<T> p, MoveArgs m, T *uw) {
+  after_previous();
   const long long nbox = (long long)m.len[0] * m.len[1] * m.len[2];
   const double rr = __dmul_rn(m.rad, m.rad);
   const int L3[3] = {p.esi, p.esj, p.esk};
@@ -1068,6 +1087,7 @@ __device__ __forceinline__ float ff_quotient(float nh, float nl, float rh, float
 // memory traffic.  One row of k per block row, so no index is divided.
 template <typename T, int LAYOUT>
 __global__ void k_velocity(PopArgs<T> p, FieldArgs f, const T *bf, float *u, float *drho) {
+  after_previous();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y, i = blockIdx.z;
   if (k >= p.esk) return;

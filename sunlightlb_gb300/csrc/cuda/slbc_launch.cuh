@@ -78,7 +78,7 @@ static void step_variant(Lattice &L, const StepArgs<T_> &a, int npt, int bx) {
       const dim3 block((unsigned)lanes_k, (unsigned)(kV4Threads / lanes_k));
       const dim3 grid((unsigned)((L.esk / 4 + lanes_k - 1) / lanes_k), (unsigned)((L.esj + block.y - 1) / block.y),
                       (unsigned)L.esi);
-      k_step_v4<ODD, MOVING, BFU><<<grid, block, 0, L.stream>>>(a);
+      launch_pdl(k_step_v4<ODD, MOVING, BFU>, grid, block, 0, L.stream, a);
     }
     return;
   }
@@ -88,7 +88,7 @@ static void step_variant(Lattice &L, const StepArgs<T_> &a, int npt, int bx) {
       17 * L.esk < 16 * ((L.esk + 31) / 32 * 32)) {
     const int bs = L.nnodes < 152LL * 128 * 8 ? 32 : 128;
     const dim3 run((unsigned)((L.esj * L.esk + bs - 1) / bs), 1, (unsigned)L.esi);
-    k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU><<<run, bs, 0, L.stream>>>(a, odd_offsets(L));
+    launch_pdl(k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU>, run, bs, 0, L.stream, a, odd_offsets(L));
     return;
   }
   const dim3 grid((unsigned)((L.esk + bx - 1) / bx), (unsigned)((L.esj + npt - 1) / npt), (unsigned)L.esi);
@@ -96,14 +96,14 @@ static void step_variant(Lattice &L, const StepArgs<T_> &a, int npt, int bx) {
   // about 286 M nodes)
   if (15LL * L.npad <= 0xFFFFFFFFLL) {
     const OddOffsets off = odd_offsets(L);
-    if (npt == 4) k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 4, true><<<grid, bx, 0, L.stream>>>(a, off);
-    else if (npt == 2) k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 2, true><<<grid, bx, 0, L.stream>>>(a, off);
-    else k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 1, true><<<grid, bx, 0, L.stream>>>(a, off);
+    if (npt == 4) launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 4, true>, grid, bx, 0, L.stream, a, off);
+    else if (npt == 2) launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 2, true>, grid, bx, 0, L.stream, a, off);
+    else launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 1, true>, grid, bx, 0, L.stream, a, off);
   } else {
     const OddOffsets off{};
-    if (npt == 4) k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 4, false><<<grid, bx, 0, L.stream>>>(a, off);
-    else if (npt == 2) k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 2, false><<<grid, bx, 0, L.stream>>>(a, off);
-    else k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 1, false><<<grid, bx, 0, L.stream>>>(a, off);
+    if (npt == 4) launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 4, false>, grid, bx, 0, L.stream, a, off);
+    else if (npt == 2) launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 2, false>, grid, bx, 0, L.stream, a, off);
+    else launch_pdl(k_step<T_, ODD, SLBC_EXACT, MOVING, BFU, 1, false>, grid, bx, 0, L.stream, a, off);
   }
 }
 
@@ -162,10 +162,10 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
     const BatchDom<T_> *D = (const BatchDom<T_> *)B.doms;
     const int *O = B.work_off + base_off, *K = B.work + base_work;
     switch (c) {
-      case 0: k_batch<T_, SLBC_EXACT, false, false><<<W, kBatchThreads, 0, B.stream>>>(D, O, K, nsteps); break;
-      case 1: k_batch<T_, SLBC_EXACT, false, true><<<W, kBatchThreads, 0, B.stream>>>(D, O, K, nsteps); break;
-      case 2: k_batch<T_, SLBC_EXACT, true, false><<<W, kBatchThreads, 0, B.stream>>>(D, O, K, nsteps); break;
-      default: k_batch<T_, SLBC_EXACT, true, true><<<W, kBatchThreads, 0, B.stream>>>(D, O, K, nsteps); break;
+      case 0: launch_pdl(k_batch<T_, SLBC_EXACT, false, false>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
+      case 1: launch_pdl(k_batch<T_, SLBC_EXACT, false, true>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
+      case 2: launch_pdl(k_batch<T_, SLBC_EXACT, true, false>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
+      default: launch_pdl(k_batch<T_, SLBC_EXACT, true, true>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
     }
     count_launch();
     e = cudaGetLastError();
@@ -246,14 +246,14 @@ cudaError_t SLBC_FN(launch_tiles)(BatchState &B, const BatchState::Set &set, int
       // domains of group g take an odd step when (step + g) is odd
       const bool odd = ((step + g) & 1) == 1;
       switch (c * 2 + (odd ? 1 : 0)) {
-        case 0: k_batch_tiles<T_, false, SLBC_EXACT, false, false><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 1: k_batch_tiles<T_, true, SLBC_EXACT, false, false><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 2: k_batch_tiles<T_, false, SLBC_EXACT, false, true><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 3: k_batch_tiles<T_, true, SLBC_EXACT, false, true><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 4: k_batch_tiles<T_, false, SLBC_EXACT, true, false><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 5: k_batch_tiles<T_, true, SLBC_EXACT, true, false><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        case 6: k_batch_tiles<T_, false, SLBC_EXACT, true, true><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
-        default: k_batch_tiles<T_, true, SLBC_EXACT, true, true><<<nt, kBatchTile, 0, B.stream>>>(D, t); break;
+        case 0: launch_pdl(k_batch_tiles<T_, false, SLBC_EXACT, false, false>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 1: launch_pdl(k_batch_tiles<T_, true, SLBC_EXACT, false, false>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 2: launch_pdl(k_batch_tiles<T_, false, SLBC_EXACT, false, true>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 3: launch_pdl(k_batch_tiles<T_, true, SLBC_EXACT, false, true>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 4: launch_pdl(k_batch_tiles<T_, false, SLBC_EXACT, true, false>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 5: launch_pdl(k_batch_tiles<T_, true, SLBC_EXACT, true, false>, nt, kBatchTile, 0, B.stream, D, t); break;
+        case 6: launch_pdl(k_batch_tiles<T_, false, SLBC_EXACT, true, true>, nt, kBatchTile, 0, B.stream, D, t); break;
+        default: launch_pdl(k_batch_tiles<T_, true, SLBC_EXACT, true, true>, nt, kBatchTile, 0, B.stream, D, t); break;
       }
       count_launch();
       t += nt;
@@ -287,7 +287,7 @@ cudaError_t SLBC_FN(launch_force)(Lattice &L) {
   ForceArgs f{L.nbnd, L.bnd_node, L.bnd_f};
   const int bs = 128;
   const int moving = L.par.objects_moving && L.uw != nullptr;
-  k_force<T_><<<flat_blocks(L.nbnd, bs), bs, 0, L.stream>>>(pop_args(L), L.layout, moving,
+  launch_pdl(k_force<T_>, flat_blocks(L.nbnd, bs), bs, 0, L.stream, pop_args(L), L.layout, moving,
                                                            (const T_ *)L.uw, f);
   count_launch();
   return cudaGetLastError();
@@ -296,7 +296,8 @@ cudaError_t SLBC_FN(launch_force)(Lattice &L) {
 cudaError_t SLBC_FN(launch_vsum)(Lattice &L, double fac, const double *psi, double *partials,
                                  int nblocks) {
   const auto go = [&](auto kernel) {
-    kernel<<<nblocks, kReduceThreads, 0, L.stream>>>(pop_args(L), L.par.rho0, fac, L.bf_uniform, L.bf_const[0],
+    launch_pdl(kernel, nblocks, kReduceThreads, 0, L.stream, pop_args(L), L.par.rho0, fac, L.bf_uniform,
+               L.bf_const[0],
                                                      L.bf_const[1], L.bf_const[2], (const T_ *)L.bf, psi, partials);
   };
   if (L.layout == SLBC_LAYOUT_N) go(k_vsum<T_, SLBC_LAYOUT_N>);
@@ -307,40 +308,40 @@ cudaError_t SLBC_FN(launch_vsum)(Lattice &L, double fac, const double *psi, doub
 }
 
 cudaError_t SLBC_FN(launch_put)(Lattice &L, const double *stage, long long x0, long long n) {
-  k_put<T_><<<flat_blocks(n, 256), 256, 0, L.stream>>>(pop_args(L), stage, x0, n);
+  launch_pdl(k_put<T_>, flat_blocks(n, 256), 256, 0, L.stream, pop_args(L), stage, x0, n);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_get)(Lattice &L, double *stage, long long x0, long long n) {
-  k_get<T_><<<flat_blocks(n, 256), 256, 0, L.stream>>>(pop_args(L), L.layout, stage, x0, n);
+  launch_pdl(k_get<T_>, flat_blocks(n, 256), 256, 0, L.stream, pop_args(L), L.layout, stage, x0, n);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_put_host)(Lattice &L, const double *host) {
   const int blocks = (int)std::min<long long>((L.nnodes + kHostTile - 1) / kHostTile, 152LL * 16);
-  k_put_host<T_><<<blocks, kHostTile, 0, L.stream>>>(pop_args(L), host, L.nnodes);
+  launch_pdl(k_put_host<T_>, blocks, kHostTile, 0, L.stream, pop_args(L), host, L.nnodes);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_get_host)(Lattice &L, double *host) {
   const int blocks = (int)std::min<long long>((L.nnodes + kHostTile - 1) / kHostTile, 152LL * 16);
-  k_get_host<T_><<<blocks, kHostTile, 0, L.stream>>>(pop_args(L), L.layout, host, L.nnodes);
+  launch_pdl(k_get_host<T_>, blocks, kHostTile, 0, L.stream, pop_args(L), L.layout, host, L.nnodes);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_swap)(Lattice &L) {
-  k_swap<T_><<<flat_blocks(L.nnodes, 256), 256, 0, L.stream>>>(pop_args(L), L.nnodes);
+  launch_pdl(k_swap<T_>, flat_blocks(L.nnodes, 256), 256, 0, L.stream, pop_args(L), L.nnodes);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_to_natural)(Lattice &L) {
   const int bx = L.esk >= 128 ? 128 : 32;
-  k_c1_to_n<T_><<<row_grid(L, bx), bx, 0, L.stream>>>(pop_args(L), (T_ *)L.scratch);
+  launch_pdl(k_c1_to_n<T_>, row_grid(L, bx), bx, 0, L.stream, pop_args(L), (T_ *)L.scratch);
   count_launch();
   return cudaGetLastError();
 }
@@ -349,7 +350,7 @@ cudaError_t SLBC_FN(launch_bbl)(Lattice &L, int with_force) {
   if (L.nbnd == 0) return cudaSuccess;
   ForceArgs f{L.nbnd, L.bnd_node, L.bnd_f};
   const int moving = L.par.objects_moving && L.uw != nullptr;
-  k_bbl_n<T_><<<flat_blocks(L.nbnd, 128), 128, 0, L.stream>>>(pop_args(L), moving,
+  launch_pdl(k_bbl_n<T_>, flat_blocks(L.nbnd, 128), 128, 0, L.stream, pop_args(L), moving,
                                                               (const T_ *)L.uw, with_force, f);
   count_launch();
   return cudaGetLastError();
@@ -357,20 +358,20 @@ cudaError_t SLBC_FN(launch_bbl)(Lattice &L, int with_force) {
 
 cudaError_t SLBC_FN(launch_propagate)(Lattice &L) {
   const int bx = L.esk >= 128 ? 128 : 32;
-  k_propagate_n<T_><<<row_grid(L, bx), bx, 0, L.stream>>>(pop_args(L), (T_ *)L.scratch);
+  launch_pdl(k_propagate_n<T_>, row_grid(L, bx), bx, 0, L.stream, pop_args(L), (T_ *)L.scratch);
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_collide)(Lattice &L) {
-  k_collide_n<T_, SLBC_EXACT><<<flat_blocks(L.nnodes, 256), 256, 0, L.stream>>>(step_args(L));
+  launch_pdl(k_collide_n<T_, SLBC_EXACT>, flat_blocks(L.nnodes, 256), 256, 0, L.stream, step_args(L));
   count_launch();
   return cudaGetLastError();
 }
 
 cudaError_t SLBC_FN(launch_setvel)(Lattice &L, const double *stage, long long x0, long long n,
                                    int has_rho, int skip_solid) {
-  k_setvel<T_, SLBC_EXACT><<<flat_blocks(n, 256), 256, 0, L.stream>>>(
+  launch_pdl(k_setvel<T_, SLBC_EXACT>, flat_blocks(n, 256), 256, 0, L.stream,
       pop_args(L), stage, x0, n, has_rho, L.par.rho0, L.par.stokes_flow, skip_solid);
   count_launch();
   return cudaGetLastError();
@@ -378,7 +379,8 @@ cudaError_t SLBC_FN(launch_setvel)(Lattice &L, const double *stage, long long x0
 
 cudaError_t SLBC_FN(launch_vacf_sums)(Lattice &L, double *p, const double *p2, const double *psi, double pmean,
                                       int axis, double *partials, int nblocks) {
-  k_vacf_sums<T_><<<nblocks, kReduceThreads, 0, L.stream>>>(pop_args(L), L.layout, L.mp_rho64, p, p2, psi, pmean,
+  launch_pdl(k_vacf_sums<T_>, nblocks, kReduceThreads, 0, L.stream, pop_args(L), L.layout, L.mp_rho64, p, p2, psi,
+             pmean,
                                                              axis, partials);
   count_launch();
   return cudaGetLastError();
@@ -387,7 +389,7 @@ cudaError_t SLBC_FN(launch_vacf_sums)(Lattice &L, double *p, const double *p2, c
 cudaError_t SLBC_FN(launch_move_sphere)(Lattice &L, const MoveArgs &m, int with_uw) {
   const long long nbox = (long long)m.len[0] * m.len[1] * m.len[2];
   const int blocks = (int)std::max<long long>(1, std::min<long long>((nbox + 255) / 256, 152LL * 8));
-  k_move_sphere<T_, SLBC_EXACT><<<blocks, 256, 0, L.stream>>>(pop_args(L), m, with_uw ? (T_ *)L.uw : nullptr);
+  launch_pdl(k_move_sphere<T_, SLBC_EXACT>, blocks, 256, 0, L.stream, pop_args(L), m, with_uw ? (T_ *)L.uw : nullptr);
   count_launch();
   return cudaGetLastError();
 }
@@ -407,7 +409,7 @@ cudaError_t SLBC_FN(launch_velocity)(Lattice &L, double fac, float *u, float *dr
   }
   const int bx = L.esk >= 256 ? 256 : L.esk >= 128 ? 128 : L.esk > 32 ? 64 : 32;
   const auto go = [&](auto kernel) {
-    kernel<<<row_grid(L, bx), bx, 0, L.stream>>>(pop_args(L), f, (const T_ *)L.bf, u, drho);
+    launch_pdl(kernel, row_grid(L, bx), bx, 0, L.stream, pop_args(L), f, (const T_ *)L.bf, u, drho);
   };
   if (L.layout == SLBC_LAYOUT_N) go(k_velocity<T_, SLBC_LAYOUT_N>);
   else if (L.layout == SLBC_LAYOUT_C0) go(k_velocity<T_, SLBC_LAYOUT_C0>);
@@ -417,7 +419,7 @@ cudaError_t SLBC_FN(launch_velocity)(Lattice &L, double fac, float *u, float *dr
 }
 
 cudaError_t SLBC_FN(launch_mp_rhoinit)(Lattice &L) {
-  k_mp_rhoinit<T_><<<flat_blocks(L.nnodes, 256), 256, 0, L.stream>>>(
+  launch_pdl(k_mp_rhoinit<T_>, flat_blocks(L.nnodes, 256), 256, 0, L.stream,
       pop_args(L), L.layout, L.par.rho0, L.mp_rho64, L.mp_rho32);
   count_launch();
   return cudaGetLastError();
@@ -468,9 +470,12 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
         if (L.mp_coef) {
           const int nb = (int)((L.nnodes + 255) / 256);
           switch (L.layout) {
-            case SLBC_LAYOUT_N: k_mp_coef<T_, SLBC_LAYOUT_N, false><<<nb, 256, 0, L.stream>>>(pa, m, ri, L.mp_coef); break;
-            case SLBC_LAYOUT_C0: k_mp_coef<T_, SLBC_LAYOUT_C0, false><<<nb, 256, 0, L.stream>>>(pa, m, ri, L.mp_coef); break;
-            default: k_mp_coef<T_, SLBC_LAYOUT_C1, false><<<nb, 256, 0, L.stream>>>(pa, m, ri, L.mp_coef); break;
+            case SLBC_LAYOUT_N: launch_pdl(k_mp_coef<T_, SLBC_LAYOUT_N, false>, nb, 256, 0, L.stream, pa, m, ri,
+                                           L.mp_coef); break;
+            case SLBC_LAYOUT_C0: launch_pdl(k_mp_coef<T_, SLBC_LAYOUT_C0, false>, nb, 256, 0, L.stream, pa, m, ri,
+                                            L.mp_coef); break;
+            default: launch_pdl(k_mp_coef<T_, SLBC_LAYOUT_C1, false>, nb, 256, 0, L.stream, pa, m, ri,
+                                L.mp_coef); break;
           }
           count_launch();
           cudaError_t ce = cudaGetLastError();
@@ -494,12 +499,18 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
     }
     const dim3 grid = tiling(3);
     switch (L.layout * 2 + (moving ? 1 : 0)) {
-      case SLBC_LAYOUT_N * 2: k_mp_step_f32<T_, SLBC_LAYOUT_N, false><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
-      case SLBC_LAYOUT_N * 2 + 1: k_mp_step_f32<T_, SLBC_LAYOUT_N, true><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
-      case SLBC_LAYOUT_C0 * 2: k_mp_step_f32<T_, SLBC_LAYOUT_C0, false><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
-      case SLBC_LAYOUT_C0 * 2 + 1: k_mp_step_f32<T_, SLBC_LAYOUT_C0, true><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
-      case SLBC_LAYOUT_C1 * 2: k_mp_step_f32<T_, SLBC_LAYOUT_C1, false><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
-      default: k_mp_step_f32<T_, SLBC_LAYOUT_C1, true><<<grid, block, 0, L.stream>>>(pa, m, ri, planes); break;
+      case SLBC_LAYOUT_N * 2: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_N, false>, grid, block, 0, L.stream, pa, m,
+                                         ri, planes); break;
+      case SLBC_LAYOUT_N * 2 + 1: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_N, true>, grid, block, 0, L.stream, pa,
+                                             m, ri, planes); break;
+      case SLBC_LAYOUT_C0 * 2: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_C0, false>, grid, block, 0, L.stream, pa, m,
+                                          ri, planes); break;
+      case SLBC_LAYOUT_C0 * 2 + 1: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_C0, true>, grid, block, 0, L.stream, pa,
+                                              m, ri, planes); break;
+      case SLBC_LAYOUT_C1 * 2: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_C1, false>, grid, block, 0, L.stream, pa, m,
+                                          ri, planes); break;
+      default: launch_pdl(k_mp_step_f32<T_, SLBC_LAYOUT_C1, true>, grid, block, 0, L.stream, pa, m, ri,
+                          planes); break;
     }
     if (lo_live) *lo_live = 0;  // p alone holds the tracer
     count_launch();
@@ -533,9 +544,11 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
   }
   const dim3 grid = tiling(tp_f64 ? 2 : 3);
   if (tp_f64)
-    k_mp_step<T_, double><<<grid, block, mp_bucket_bytes<double>(), L.stream>>>(pop_args(L), L.layout, m, planes);
+    launch_pdl(k_mp_step<T_, double>, grid, block, mp_bucket_bytes<double>(), L.stream, pop_args(L), L.layout, m,
+               planes);
   else
-    k_mp_step<T_, float><<<grid, block, mp_bucket_bytes<float>(), L.stream>>>(pop_args(L), L.layout, m, planes);
+    launch_pdl(k_mp_step<T_, float>, grid, block, mp_bucket_bytes<float>(), L.stream, pop_args(L), L.layout, m,
+               planes);
   if (lo_live) *lo_live = 0;  // p alone holds the tracer
   count_launch();
   return cudaGetLastError();

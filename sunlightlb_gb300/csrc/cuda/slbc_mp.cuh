@@ -144,6 +144,7 @@ __device__ __forceinline__ MpSource<TP> mp_source(const MpRaw<TP> &v, TP rho0, T
 // the products with 8 and 16 (exact) ride in fused multiply-adds.
 template <typename T, typename TP>
 __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_step(PopArgs<T> p, int layout, MpArgs m, int planes) {
+  after_previous();
   __shared__ MpSource<TP> ring[3][kPlane];
   // summation order at wrap nodes: 27 x kTileThreads values, dynamic
   // shared memory (mp_bucket_bytes per block)
@@ -364,6 +365,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
 template <typename T, int LAYOUT, bool MOVING>
 __global__ void __launch_bounds__(kTileThreads, 3)
 k_mp_step_f32(PopArgs<T> p, MpArgs m, const float *rinv, int planes) {
+  after_previous();
   __shared__ MpSource<float> ring[3][kPlane];
   const int tk = threadIdx.x, tj = threadIdx.y, tid = tj * kTileK + tk;
   const int k0 = blockIdx.x * kTileK, j0 = blockIdx.y * kTileJ, i0 = blockIdx.z * planes;
@@ -503,6 +505,7 @@ k_mp_step_f32(PopArgs<T> p, MpArgs m, const float *rinv, int planes) {
 // node; the layout is that of the flow when the coefficients were built.
 template <typename T, int LAYOUT, bool MOVING>
 __global__ void __launch_bounds__(256) k_mp_coef(PopArgs<T> p, MpArgs m, const float *rinv, float *coef) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long long)p.esi * p.esj * p.esk) return;
   const int x = (int)e;
@@ -571,6 +574,7 @@ __global__ void __launch_bounds__(256) k_mp_coef(PopArgs<T> p, MpArgs m, const f
 // FP32 tracers exist, in FP32.
 template <typename T>
 __global__ void k_mp_rhoinit(PopArgs<T> p, int layout, double rho0, double *rho64, float *rho32) {
+  after_previous();
   const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long n = (long long)p.esi * p.esj * p.esk;
   if (e >= n) return;

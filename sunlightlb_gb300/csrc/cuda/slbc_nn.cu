@@ -16,6 +16,9 @@
 
 namespace {
 
+using slbc::after_previous;
+using slbc::launch_pdl;
+
 typedef __nv_bfloat16 bf16;
 
 struct Slice {
@@ -86,6 +89,7 @@ __device__ __forceinline__ void row_of(int row, int D, int H, int &n, int &z, in
 
 // 2x2x2 average of the fine interior (D, H, W) into the coarse interior
 __global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D, int H, int W, int C) {
+  after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
   const RowWalk w = row_walk(len);
   for (int row = w.row; row < B * Dc * Hc; row += w.step) {
@@ -115,6 +119,7 @@ __global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D,
 // optional (null pointers)
 __global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Slice add, Slice mask, int B, int D,
                                                   int H, int W, int C) {
+  after_previous();
   const int nv = C / 8, len = W * nv;
   const RowWalk w = row_walk(len);
   for (int row = w.row; row < B * D * H; row += w.step) {
@@ -149,6 +154,7 @@ __global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Sl
 // nearest upsampling: fine (D, H, W) interior = coarse parent; a thread
 // reads its vector of the parent once and writes the eight children
 __global__ void __launch_bounds__(256) k_up(Slice in, Slice out, int B, int D, int H, int W, int C) {
+  after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
   const RowWalk w = row_walk(len);
   for (int row = w.row; row < B * Dc * Hc; row += w.step) {
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(256) k_up(Slice in, Slice out, int B, int D, i
 
 // gradient of k_up: dcoarse = sum of the 8 children * (mask > 0) (coarse mask)
 __global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slice mask, int B, int D, int H, int W, int C) {
+  after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
   const RowWalk w = row_walk(len);
   for (int row = w.row; row < B * Dc * Hc; row += w.step) {
@@ -204,6 +211,7 @@ __global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slic
 // the lanes of a warp with the same channels are added by shuffles, and one
 // of them adds to the block's shared sums.
 __global__ void __launch_bounds__(256) k_bias_grad(Slice g, int B, int D, int H, int W, int C, float *db) {
+  after_previous();
   extern __shared__ float sh[];
   for (int c = threadIdx.x; c < C; c += blockDim.x) sh[c] = 0.0f;
   __syncthreads();
@@ -235,6 +243,7 @@ __global__ void __launch_bounds__(256) k_bias_grad(Slice g, int B, int D, int H,
 
 // forward weights: w[tap][cin/32][cout][32] from master m[tap][cout][cin]
 __global__ void k_wfwd(const float *m, int cout, int cin, bf16 *w) {
+  after_previous();
   const long long n = 27LL * cout * cin;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(e % 32);
@@ -250,6 +259,7 @@ __global__ void k_wfwd(const float *m, int cout, int cin, bf16 *w) {
 // these weights maps dY (cout channels) to dX: w[t][cout/32][nci][32] =
 // m[26 - t][32 ck + j][ci0 + ci]
 __global__ void k_wdgrad(const float *m, int cout, int cin, int ci0, int nci, bf16 *w) {
+  after_previous();
   const long long n = 27LL * nci * cout;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const int j = (int)(e % 32);
@@ -263,6 +273,7 @@ __global__ void k_wdgrad(const float *m, int cout, int cin, int ci0, int nci, bf
 
 __global__ void k_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2,
                        float eps, float c1, float c2) {
+  after_previous();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -278,6 +289,7 @@ __global__ void k_adam(float *p, const float *g, float *m, float *v, long long n
 // gradient tensor (k_sqsum adds to it, k_clip_scale resets it); state[1]:
 // running norm (0 before the first call); state[2]: the scale to apply.
 __global__ void k_sqsum(const float *g, long long n, double *state) {
+  after_previous();
   __shared__ double sh[256];
   double s = 0.0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -295,6 +307,7 @@ __global__ void k_sqsum(const float *g, long long n, double *state) {
 // (1 - decay) * norm * scale.  A non-finite norm gives scale 0 (the
 // gradients are zeroed) and leaves the running norm as it was.
 __global__ void k_clip_scale(double *state, float factor, float decay) {
+  after_previous();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double nrm = sqrt(state[0]);
   state[0] = 0.0;
@@ -309,6 +322,7 @@ __global__ void k_clip_scale(double *state, float factor, float decay) {
 }
 
 __global__ void k_scale(float *g, long long n, const double *state) {
+  after_previous();
   const float sc = (float)state[2];
   if (sc == 1.0f) return;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -322,6 +336,7 @@ __global__ void k_scale(float *g, long long n, const double *state) {
 __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, const float *label, int nch,
                                              const float *sample_w, int B, int D, int H, int W, bf16 *grad, int gctot,
                                              double *loss) {
+  after_previous();
   __shared__ double sh[256];
   const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   double acc = 0.0;
@@ -358,6 +373,7 @@ __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, cons
 // (weight / B) * sum_n s_n^2 to the BF16 gradient and the term to the loss.
 __global__ void k_proj_dot(const float *pred, int ctot_p, const float *label, int lch, int nch, int D, int H, int W,
                            double *dot) {
+  after_previous();
   __shared__ double sh[256];
   const int n = blockIdx.y;
   const long long per = (long long)D * H * W;
@@ -382,6 +398,7 @@ __global__ void k_proj_dot(const float *pred, int ctot_p, const float *label, in
 
 __global__ void k_proj_grad(const float *label, int lch, int nch, const double *lab_sq, const double *dot, int B, int D,
                             int H, int W, float weight, bf16 *grad, int gctot, double *loss) {
+  after_previous();
   const long long per = (long long)D * H * W, total = (long long)B * per;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
     long long r = e;
@@ -417,6 +434,7 @@ constexpr int kDistR1 = 5, kDistR2 = 12;
 // Pass 1 (along x): nearest solid node on the row, searched outwards.
 template <int R>
 __global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int rows, int W, unsigned char *a) {
+  after_previous();
   const RowWalk w = row_walk(W);
   for (int row = w.row; row < rows; row += w.step) {
     const unsigned char *src = solid + (long long)row * W;
@@ -444,6 +462,7 @@ __global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int 
 // under saturation, and the cap of R^2 absorbs it).
 template <int R, int VEC>
 __global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int lines, int n, int inner, unsigned char *b) {
+  after_previous();
   const int len = inner / VEC;  // a line: the bytes of one p of one outer block
   const RowWalk w = row_walk(len);
   for (int line = w.row; line < lines; line += w.step) {
@@ -471,6 +490,7 @@ __global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int li
 // searched to radius R
 __global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, const unsigned char *dist2, int R, int B,
                                                 int D, int H, int W, bf16 *out, int ctot) {
+  after_previous();
   const int nv = ctot / 8, len = W * nv;
   const RowWalk w = row_walk(len);
   for (int row = w.row; row < B * D * H; row += w.step) {
@@ -505,6 +525,7 @@ __global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, cons
 __global__ void __launch_bounds__(256) k_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H,
                                                 int W, float scale, float shift_x, float *u, float drho_scale,
                                                 float *drho) {
+  after_previous();
   const long long total = (long long)D * H * W;
   const RowWalk w = row_walk(W);
   for (int row = w.row; row < D * H; row += w.step) {
@@ -526,6 +547,7 @@ __global__ void __launch_bounds__(256) k_decode(const float *pred, int ctot_p, c
 // index; the flux of x through plane i is q[i] = sum over the plane of u_x).
 // k_plane_sum: one block per plane, a fixed summation order.
 __global__ void __launch_bounds__(256) k_plane_sum(const float *u, int D, long long plane, double *q) {
+  after_previous();
   __shared__ double sh[256];
   const int i = blockIdx.x;
   double acc = 0.0;
@@ -547,6 +569,7 @@ __global__ void __launch_bounds__(256) k_plane_sum(const float *u, int D, long l
 // runs' sums are scanned in thread order (one thread alone spent 127 us on
 // the divisions of 128 planes).
 __global__ void __launch_bounds__(256) k_plane_fix(int D, float force, float gain, double *work) {
+  after_previous();
   __shared__ double sa[256], sb[256], lo[256], hi[256];
   __shared__ int all_ok;
   const double *q = work;
@@ -616,6 +639,7 @@ __global__ void __launch_bounds__(256) k_plane_fix(int D, float force, float gai
 // u[c][x] *= scale[i]; drho[x] = gain drho[x] + 3 p[i] on fluid nodes (p = rho / 3)
 __global__ void k_plane_apply(float *u, float *drho, const unsigned char *solid, int D, long long plane,
                               float gain, const double *work) {
+  after_previous();
   const long long total = (long long)D * plane;
   const double *scale = work + D, *p = work + 2 * D;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
@@ -636,6 +660,7 @@ __global__ void k_plane_apply(float *u, float *drho, const unsigned char *solid,
 // (plane fluxes, y planes then z planes), m[H + W] (plane sums of |u|),
 // delta[H + W].  One block per plane, a fixed summation order.
 __global__ void __launch_bounds__(256) k_cross_sum(const float *u, int D, int H, int W, double *work) {
+  after_previous();
   __shared__ double sq[256], sm[256];
   const int b = blockIdx.x;
   const bool ydir = b < H;
@@ -668,6 +693,7 @@ __global__ void __launch_bounds__(256) k_cross_sum(const float *u, int D, int H,
 }
 
 __global__ void k_cross_fix(int H, int W, double *work) {
+  after_previous();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   const double *q = work, *m = work + H + W;
   double *delta = work + 2 * (H + W);
@@ -680,6 +706,7 @@ __global__ void k_cross_fix(int H, int W, double *work) {
 }
 
 __global__ void k_cross_apply(float *u, int D, int H, int W, const double *work) {
+  after_previous();
   const long long total = (long long)D * H * W;
   const double *delta = work + 2 * (H + W);
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
@@ -716,7 +743,8 @@ int slbc_nn_pool(const void *in, int in_ctot, int in_coff, void *out, int out_ct
                  int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool: channel slices must be multiples of 8 and the grid even");
-  k_pool<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
+  launch_pdl(k_pool, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
+             Slice{(bf16 *)in, in_ctot, in_coff},
                                                         Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
   return launched("slbc_nn_pool");
 }
@@ -727,7 +755,7 @@ int slbc_nn_pool_bwd(const void *dcoarse, int dc_ctot, int dc_coff, void *dfine,
   if (!ok8(dc_ctot, dc_coff, C) || !ok8(df_ctot, df_coff, C) || (add && !ok8(a_ctot, a_coff, C)) ||
       (mask && !ok8(m_ctot, m_coff, C)) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool_bwd: channel slices must be multiples of 8 and the grid even");
-  k_pool_bwd<<<rows_grid((long long)B * D * H, W * (C / 8)), 256, 0, (cudaStream_t)stream>>>(
+  launch_pdl(k_pool_bwd, rows_grid((long long)B * D * H, W * (C / 8)), 256, 0, (cudaStream_t)stream,
       Slice{(bf16 *)dcoarse, dc_ctot, dc_coff}, Slice{(bf16 *)dfine, df_ctot, df_coff},
       Slice{(bf16 *)add, a_ctot, a_coff}, Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
   return launched("slbc_nn_pool_bwd");
@@ -737,7 +765,8 @@ int slbc_nn_up(const void *in, int in_ctot, int in_coff, void *out, int out_ctot
                int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_up: channel slices must be multiples of 8 and the grid even");
-  k_up<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)in, in_ctot, in_coff},
+  launch_pdl(k_up, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
+             Slice{(bf16 *)in, in_ctot, in_coff},
                                                       Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
   return launched("slbc_nn_up");
 }
@@ -747,7 +776,8 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
   if (!ok8(df_ctot, df_coff, C) || !ok8(dc_ctot, dc_coff, C) || (mask && !ok8(m_ctot, m_coff, C)) || D % 2 ||
       H % 2 || W % 2)
     return bad("slbc_nn_up_bwd: channel slices must be multiples of 8 and the grid even");
-  k_up_bwd<<<rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream>>>(Slice{(bf16 *)dfine, df_ctot, df_coff},
+  launch_pdl(k_up_bwd, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
+             Slice{(bf16 *)dfine, df_ctot, df_coff},
                                                           Slice{(bf16 *)dcoarse, dc_ctot, dc_coff},
                                                           Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
   return launched("slbc_nn_up_bwd");
@@ -755,20 +785,22 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
 
 int slbc_nn_bias_grad(const void *g, int ctot, int coff, int B, int D, int H, int W, int C, float *db, void *stream) {
   if (!ok8(ctot, coff, C) || C > 1024 || 256 % (C / 8)) return bad("slbc_nn_bias_grad: bad channel slice");
-  k_bias_grad<<<std::min(rows_grid((long long)B * D * H, W * (C / 8)), 152 * 4), 256, C * sizeof(float), (cudaStream_t)stream>>>(
+  launch_pdl(k_bias_grad, std::min(rows_grid((long long)B * D * H, W * (C / 8)), 152 * 4), 256, C * sizeof(float),
+             (cudaStream_t)stream,
       Slice{(bf16 *)g, ctot, coff}, B, D, H, W, C, db);
   return launched("slbc_nn_bias_grad");
 }
 
 int slbc_nn_wfwd(const float *master, int cout, int cin, void *w, void *stream) {
   if (cin % 32 || cout < 1) return bad("slbc_nn_wfwd: cin must be a multiple of 32");
-  k_wfwd<<<grid_for(27LL * cout * cin), 256, 0, (cudaStream_t)stream>>>(master, cout, cin, (bf16 *)w);
+  launch_pdl(k_wfwd, grid_for(27LL * cout * cin), 256, 0, (cudaStream_t)stream, master, cout, cin, (bf16 *)w);
   return launched("slbc_nn_wfwd");
 }
 
 int slbc_nn_wdgrad(const float *master, int cout, int cin, int ci0, int nci, void *w, void *stream) {
   if (cout % 32 || ci0 < 0 || nci < 1 || ci0 + nci > cin) return bad("slbc_nn_wdgrad: bad channel range");
-  k_wdgrad<<<grid_for(27LL * cout * nci), 256, 0, (cudaStream_t)stream>>>(master, cout, cin, ci0, nci, (bf16 *)w);
+  launch_pdl(k_wdgrad, grid_for(27LL * cout * nci), 256, 0, (cudaStream_t)stream, master, cout, cin, ci0, nci,
+             (bf16 *)w);
   return launched("slbc_nn_wdgrad");
 }
 
@@ -776,32 +808,32 @@ int slbc_nn_adam(float *p, const float *g, float *m, float *v, long long n, floa
                  int t, void *stream) {
   if (t < 1) return bad("slbc_nn_adam: step count starts at 1");
   const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
-  k_adam<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(p, g, m, v, n, lr, b1, b2, eps, c1, c2);
+  launch_pdl(k_adam, grid_for(n), 256, 0, (cudaStream_t)stream, p, g, m, v, n, lr, b1, b2, eps, c1, c2);
   return launched("slbc_nn_adam");
 }
 
 int slbc_nn_sqsum(const float *g, long long n, double *state, void *stream) {
   if (n <= 0) return bad("slbc_nn_sqsum: empty tensor");
-  k_sqsum<<<std::min(grid_for(n), 152 * 4), 256, 0, (cudaStream_t)stream>>>(g, n, state);
+  launch_pdl(k_sqsum, std::min(grid_for(n), 152 * 4), 256, 0, (cudaStream_t)stream, g, n, state);
   return launched("slbc_nn_sqsum");
 }
 
 int slbc_nn_clip(double *state, float factor, float decay, void *stream) {
   if (!(factor > 0.0f) || !(decay >= 0.0f && decay < 1.0f)) return bad("slbc_nn_clip: factor > 0, 0 <= decay < 1");
-  k_clip_scale<<<1, 32, 0, (cudaStream_t)stream>>>(state, factor, decay);
+  launch_pdl(k_clip_scale, 1, 32, 0, (cudaStream_t)stream, state, factor, decay);
   return launched("slbc_nn_clip");
 }
 
 int slbc_nn_scale(float *g, long long n, const double *state, void *stream) {
   if (n <= 0) return bad("slbc_nn_scale: empty tensor");
-  k_scale<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(g, n, state);
+  launch_pdl(k_scale, grid_for(n), 256, 0, (cudaStream_t)stream, g, n, state);
   return launched("slbc_nn_scale");
 }
 
 int slbc_nn_mse(const float *pred, int ctot_p, const float *label, int nch, const float *sample_w, int B, int D, int H,
                 int W, void *grad, int gctot, double *loss, void *stream) {
   if (nch < 1 || ctot_p < nch || gctot % 8 || gctot < 8 || gctot < nch) return bad("slbc_nn_mse: bad channel counts");
-  k_mse<<<std::min(rows_grid((long long)B * D * H, W), 152 * 8), 256, 0, (cudaStream_t)stream>>>(
+  launch_pdl(k_mse, std::min(rows_grid((long long)B * D * H, W), 152 * 8), 256, 0, (cudaStream_t)stream,
       pred, ctot_p, label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss);
   return launched("slbc_nn_mse");
 }
@@ -814,9 +846,10 @@ int slbc_nn_proj(const float *pred, int ctot_p, const float *label, int lch, int
   if (cudaMemsetAsync(dot, 0, sizeof(double) * B, st) != cudaSuccess) return bad("slbc_nn_proj: memset");
   const long long per = (long long)D * H * W;
   const dim3 g1((unsigned)std::min<long long>((per + 255) / 256, 152), (unsigned)B);
-  k_proj_dot<<<g1, 256, 0, st>>>(pred, ctot_p, label, lch, nch, D, H, W, dot);
+  launch_pdl(k_proj_dot, g1, 256, 0, st, pred, ctot_p, label, lch, nch, D, H, W, dot);
   if (launched("slbc_nn_proj")) return 1;
-  k_proj_grad<<<std::min(grid_for((long long)B * per), 152 * 4), 256, 0, st>>>(label, lch, nch, lab_sq, dot, B, D, H,
+  launch_pdl(k_proj_grad, std::min(grid_for((long long)B * per), 152 * 4), 256, 0, st, label, lch, nch, lab_sq, dot,
+             B, D, H,
                                                                                 W, weight, (bf16 *)grad, gctot, loss);
   return launched("slbc_nn_proj");
 }
@@ -836,9 +869,9 @@ int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void 
     unsigned char *b = a + (total + 255) / 256 * 256;
     const int vec = W % 4 == 0 ? 4 : 1;
     const auto passes = [&](auto rx, auto ry, auto rz) {
-      rx<<<rows_grid((long long)B * D * H, W), 256, 0, st>>>(solid, B * D * H, W, a);
-      ry<<<rows_grid((long long)B * D * H, W / vec), 256, 0, st>>>(a, B * D * H, H, W, b);
-      rz<<<rows_grid((long long)B * D, W * H / vec), 256, 0, st>>>(b, B * D, D, W * H, a);
+      launch_pdl(rx, rows_grid((long long)B * D * H, W), 256, 0, st, solid, B * D * H, W, a);
+      launch_pdl(ry, rows_grid((long long)B * D * H, W / vec), 256, 0, st, a, B * D * H, H, W, b);
+      launch_pdl(rz, rows_grid((long long)B * D, W * H / vec), 256, 0, st, b, B * D, D, W * H, a);
     };
     if (features == 2) {
       if (vec == 4) passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 4>, k_dist_min<kDistR2, 4>);
@@ -849,7 +882,8 @@ int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void 
     }
     slbc::count_launch(3);
   }
-  k_encode<<<rows_grid((long long)B * D * H, W * (ctot / 8)), 256, 0, st>>>(solid, a, features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out,
+  launch_pdl(k_encode, rows_grid((long long)B * D * H, W * (ctot / 8)), 256, 0, st, solid, a,
+             features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out,
                                             ctot);
   const int rc = launched("slbc_nn_encode");
   if (a) {
@@ -864,29 +898,30 @@ int slbc_nn_plane_flux(float *u, float *drho, const unsigned char *solid, int D,
   if (D < 1 || H < 1 || W < 1 || D > 65535 || !u || !solid || !work) return bad("slbc_nn_plane_flux: bad arguments");
   const cudaStream_t st = (cudaStream_t)stream;
   const long long plane = (long long)H * W;
-  k_plane_sum<<<D, 256, 0, st>>>(u, D, plane, work);
+  launch_pdl(k_plane_sum, D, 256, 0, st, u, D, plane, work);
   if (launched("slbc_nn_plane_flux")) return 1;
-  k_plane_fix<<<1, 256, 0, st>>>(D, force, gain, work);
+  launch_pdl(k_plane_fix, 1, 256, 0, st, D, force, gain, work);
   if (launched("slbc_nn_plane_flux")) return 1;
-  k_plane_apply<<<grid_for((long long)D * plane), 256, 0, st>>>(u, drho, solid, D, plane, gain, work);
+  launch_pdl(k_plane_apply, grid_for((long long)D * plane), 256, 0, st, u, drho, solid, D, plane, gain, work);
   return launched("slbc_nn_plane_flux");
 }
 
 int slbc_nn_cross_flux(float *u, int D, int H, int W, double *work, void *stream) {
   if (D < 1 || H < 1 || W < 1 || H + W > 65535 || !u || !work) return bad("slbc_nn_cross_flux: bad arguments");
   const cudaStream_t st = (cudaStream_t)stream;
-  k_cross_sum<<<H + W, 256, 0, st>>>(u, D, H, W, work);
+  launch_pdl(k_cross_sum, H + W, 256, 0, st, u, D, H, W, work);
   if (launched("slbc_nn_cross_flux")) return 1;
-  k_cross_fix<<<1, 32, 0, st>>>(H, W, work);
+  launch_pdl(k_cross_fix, 1, 32, 0, st, H, W, work);
   if (launched("slbc_nn_cross_flux")) return 1;
-  k_cross_apply<<<grid_for((long long)D * H * W), 256, 0, st>>>(u, D, H, W, work);
+  launch_pdl(k_cross_apply, grid_for((long long)D * H * W), 256, 0, st, u, D, H, W, work);
   return launched("slbc_nn_cross_flux");
 }
 
 int slbc_nn_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H, int W, float scale,
                    float shift_x, float *u, float drho_scale, float *drho, void *stream) {
   if (ctot_p < (drho ? 4 : 3)) return bad("slbc_nn_decode: bad channel count");
-  k_decode<<<rows_grid((long long)D * H, W), 256, 0, (cudaStream_t)stream>>>(pred, ctot_p, solid, D, H, W, scale,
+  launch_pdl(k_decode, rows_grid((long long)D * H, W), 256, 0, (cudaStream_t)stream, pred, ctot_p, solid, D, H, W,
+             scale,
                                                                                        shift_x, u, drho_scale, drho);
   return launched("slbc_nn_decode");
 }

@@ -40,6 +40,7 @@ __device__ __forceinline__ float f4_get(const float4 &v, int n) {
 
 template <bool ODD, bool MOVING, bool BFU>
 __global__ void __launch_bounds__(kV4Threads, ODD ? (MOVING ? 2 : 3) : 4) k_step_v4(StepArgs<float> a) {
+  after_previous();
   float *__restrict__ P = a.p.pop;
   const long long S = a.p.npad;
   const int esi = a.p.esi, esj = a.p.esj, esk = a.p.esk;

@@ -92,6 +92,7 @@ bool make_map_2d(CUtensorMap *map, const void *ptr, long long rows, long long co
 __global__ void __launch_bounds__(128, 1)
 k_gemm_bf16(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, float *D, int ldd,
             int K, int *err) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
@@ -215,6 +216,7 @@ static_assert(conv_smem(6, 128) <= kConvSmemMax && conv_smem(4, 256) <= kConvSme
 template <int NST>
 __global__ void __launch_bounds__(128, 2)
 k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int *err) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
@@ -391,6 +393,7 @@ template <int COUT, int S>
 __global__ void __launch_bounds__(192, 1)
 k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int items,
          int *err) {
+  after_previous();
   using C = ConvZ<COUT, S>;
   constexpr int NST = C::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -568,6 +571,7 @@ k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
 // for interior z the rows y = 0 and y = H + 1, then for interior z, y the
 // columns x = 0 and x = W + 1.
 __global__ void k_halo(__nv_bfloat16 *buf, int B, int D, int H, int W, int ctot, int coff, int nch) {
+  after_previous();
   const long long Pz = 2LL * (H + 2) * (W + 2), Py = 2LL * D * (W + 2), Px = 2LL * D * H;
   const long long per = Pz + Py + Px;
   const int nv = nch / 8;
@@ -665,6 +669,7 @@ constexpr int kWgSmem = kStages * (kWgTileA + kWgTileB) + 1024;
 __global__ void __launch_bounds__(128, 2)
 k_wgrad(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensorMap a1,
         const __grid_constant__ CUtensorMap a2, const __grid_constant__ CUtensorMap tb, WgradArgs w, int *err) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
@@ -847,6 +852,7 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
           const __grid_constant__ CUtensorMap a2, const __grid_constant__ CUtensorMap tb,
           const __grid_constant__ CUtensorMap a_all, const __grid_constant__ CUtensorMap b_win, WgradNArgs w,
           int *err) {
+  after_previous();
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
@@ -988,6 +994,7 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
 
 // dw[i] = sum over splits of partial[s][i], in split order
 __global__ void k_sum_splits(const float *partial, long long n, int splits, float *dw) {
+  after_previous();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float v = 0.0f;
     for (int s = 0; s < splits; s++) v += partial[(long long)s * n + i];
@@ -1020,6 +1027,7 @@ template <int NC>
 __global__ void __launch_bounds__(256) k_cmajor(const __nv_bfloat16 *src, int B, int D, int H, int W, int ctot, int coff,
                                                 int nch, int Wp, int pstride, int shift, int zero_halo, int copy, int ncopy,
                                                 long long copy_stride, __nv_bfloat16 *dst) {
+  after_previous();
   __shared__ __align__(16) unsigned char rows[(kCmPos + 3) * kCmPitch];  // positions -1 .. 256, and a row of zeros
   __shared__ int voxel[kCmPos + 2];
   __shared__ short xs[kCmPos + 2];
@@ -1168,7 +1176,8 @@ int cmajor_launch(const char *who, const void *src, int B, int D, int H, int W, 
   if (work >= 1LL << 31) return slbc::set_error(std::string(who) + ": grid too large"), 1;
   const int blocks = (int)std::min<long long>(work, 152LL * 8);
   const auto go = [&](auto kernel) {
-    kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)src, B, D, H, W, ctot, coff, nch, Wp,
+    launch_pdl(kernel, blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16 *)src, B, D, H, W, ctot, coff,
+               nch, Wp,
                                                      (int)pstride, shift, zero_halo, copy, ncopy, copy_stride,
                                                      (__nv_bfloat16 *)dst);
   };
@@ -1236,12 +1245,12 @@ int wgrad_launch(const char *who, const void *dy0, const void *dy1, const void *
     if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
     const dim3 grid((unsigned)wgrad_n_ctas(wn), 1, (unsigned)splits);
     const int smem = kStages * (kWgTileA + wn.n_rows * 128) + 1024;
-    k_wgrad_n<<<grid, 128, smem, (cudaStream_t)stream>>>(m0, m1, m2, mb, ma, mw, wn, err);
+    launch_pdl(k_wgrad_n, grid, 128, smem, (cudaStream_t)stream, m0, m1, m2, mb, ma, mw, wn, err);
     slbc::count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
     const long long n = 27LL * cout * cin;
-    k_sum_splits<<<(int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream>>>(
+    launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream,
         partial, n, splits, dw);
     slbc::count_launch();
     e = cudaGetLastError();
@@ -1274,12 +1283,12 @@ int wgrad_launch(const char *who, const void *dy0, const void *dy1, const void *
   const dim3 grid((unsigned)(((27 + w.taps_per_tile - 1) / w.taps_per_tile) * w.co_tiles), (unsigned)(cin / w.ntile),
                   (unsigned)splits);
   const int smem = kStages * (kWgTileA + w.ntile * 128) + 1024;
-  k_wgrad<<<grid, 128, smem, (cudaStream_t)stream>>>(m0, m1, m2, mb, w, err);
+  launch_pdl(k_wgrad, grid, 128, smem, (cudaStream_t)stream, m0, m1, m2, mb, w, err);
   slbc::count_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
   const long long n = 27LL * cout * cin;
-  k_sum_splits<<<(int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream>>>(
+  launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream,
       partial, n, splits, dw);
   slbc::count_launch();
   e = cudaGetLastError();
@@ -1305,7 +1314,7 @@ int slbc_tc_gemm(const void *A, const void *B, float *D, int M, int N, int K, in
   static unsigned long long attr_done = 0;
   cudaError_t e = smem_opt_in((const void *)k_gemm_bf16, kGemmSmem, attr_done);
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_gemm: ") + cudaGetErrorString(e)), 1;
-  k_gemm_bf16<<<dim3(N / kBN, M / kBM), 128, kGemmSmem, (cudaStream_t)stream>>>(ta, tb, D, ldd, K, err);
+  launch_pdl(k_gemm_bf16, dim3(N / kBN, M / kBM), 128, kGemmSmem, (cudaStream_t)stream, ta, tb, D, ldd, K, err);
   slbc::count_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_gemm: ") + cudaGetErrorString(e)), 1;
@@ -1361,7 +1370,7 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
     const auto go = [&](auto kernel, int smem, int slot) {
       cudaError_t e = smem_opt_in((const void *)kernel, smem, attr_z[slot]);
       if (e != cudaSuccess) return e;
-      kernel<<<std::min(items, kConvSms), 192, smem, (cudaStream_t)stream>>>(th, tw, a, items, err);
+      launch_pdl(kernel, std::min(items, kConvSms), 192, smem, (cudaStream_t)stream, th, tw, a, items, err);
       slbc::count_launch();
       return cudaGetLastError();
     };
@@ -1379,11 +1388,11 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
   const dim3 grid((unsigned)((long long)D * H * W / 128), (unsigned)B);
   if (nst == 8)
-    k_conv_fwd<8><<<grid, 128, smem, (cudaStream_t)stream>>>(tx, tw, a, err);
+    launch_pdl(k_conv_fwd<8>, grid, 128, smem, (cudaStream_t)stream, tx, tw, a, err);
   else if (nst == 6)
-    k_conv_fwd<6><<<grid, 128, smem, (cudaStream_t)stream>>>(tx, tw, a, err);
+    launch_pdl(k_conv_fwd<6>, grid, 128, smem, (cudaStream_t)stream, tx, tw, a, err);
   else
-    k_conv_fwd<4><<<grid, 128, smem, (cudaStream_t)stream>>>(tx, tw, a, err);
+    launch_pdl(k_conv_fwd<4>, grid, 128, smem, (cudaStream_t)stream, tx, tw, a, err);
   slbc::count_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
@@ -1411,7 +1420,7 @@ int slbc_tc_halo(void *buf, int B, int D, int H, int W, int ctot, int coff, int 
   const long long per = 2LL * (H + 2) * (W + 2) + 2LL * D * (W + 2) + 2LL * D * H;
   const long long total = (long long)B * per * (nch / 8);
   const int blocks = (int)std::min<long long>((total + 255) / 256, 152LL * 16);
-  k_halo<<<blocks, 256, 0, (cudaStream_t)stream>>>((__nv_bfloat16 *)buf, B, D, H, W, ctot, coff, nch);
+  launch_pdl(k_halo, blocks, 256, 0, (cudaStream_t)stream, (__nv_bfloat16 *)buf, B, D, H, W, ctot, coff, nch);
   slbc::count_launch();
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_halo: ") + cudaGetErrorString(e)), 1;
