@@ -107,16 +107,35 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 enum : uint32_t { kSwizzle128 = 2, kSwizzle64 = 4, kSwizzle32 = 6 };
 
 // Descriptor of a K-major tile: rows of `row_bytes` (the swizzle width),
-// groups of 8 rows `8 * row_bytes` apart; the tile starts on a multiple of
-// the swizzle pattern (8 * row_bytes), so the base offset field is 0.
-__device__ __forceinline__ uint64_t smem_desc(const void *p, uint32_t swizzle, uint32_t row_bytes) {
+// groups of 8 rows `group` bytes apart (8 * row_bytes where the rows follow one
+// another); the buffer starts on a multiple of the swizzle pattern (8 *
+// row_bytes), so the base offset field is 0.
+__device__ __forceinline__ uint64_t smem_desc(const void *p, uint32_t swizzle, uint32_t row_bytes, uint32_t group = 0) {
+  if (!group) group = 8u * row_bytes;
   uint64_t d = 0;
   d |= (uint64_t)((smem_u32(p) & 0x3FFFFu) >> 4);
   d |= (uint64_t)1 << 16;                              // leading offset: unused when swizzled
-  d |= (uint64_t)((8u * row_bytes) >> 4) << 32;        // stride between 8-row groups
+  d |= (uint64_t)(group >> 4) << 32;                   // stride between 8-row groups
   d |= (uint64_t)1 << 46;                              // descriptor version
   d |= (uint64_t)swizzle << 61;
   return d;
+}
+
+// The same from the low word of such a descriptor (start address in 16-byte
+// units), whose start may have been moved by whole 16-byte units.
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo, uint32_t swizzle, uint32_t group) {
+  return ((uint64_t)((group >> 4) | (1u << 14) | (swizzle << 29)) << 32) | lo;
+}
+
+// True in one thread of a converged warp, always the same one.  The loops that
+// issue copies and MMAs are entered on it: knowing that one thread is left,
+// the compiler keeps descriptors in uniform registers.  Measured, cycles per
+// MMA of 128 x N x 16 in such a loop: max(32 + N / 4, N / 2) (40 at N = 32, 56
+// at 96, 96 at 192); entered on a thread index 72 to 140 whatever N.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+  return one != 0;
 }
 
 // D[tmem] (+)= A * B^T for one K = 16 slice (BF16).

@@ -120,7 +120,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUte
   const uint32_t tmem = tmem_base;
   bool ok = true;
   int issued = 0;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = 0; kt < nk; kt++) {
       const int s = kt % kStages;
       if (kt >= kStages && !tc::mbar_wait(&empty[s], ((kt / kStages) - 1) & 1, kWaitLimit)) {
@@ -132,7 +132,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUte
       tc::tma_load_2d(tB + s * kTileB, &tb, &full[s], kt * kBK, n0);
       issued = kt + 1;
     }
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1 && tc::elect_one()) {
     constexpr uint32_t idesc = tc::idesc_bf16(kBM, kBN);
     for (int kt = 0; kt < nk; kt++) {
       const int s = kt % kStages;
@@ -165,7 +165,7 @@ k_gemm_bf16(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUte
     }
   }
   if (!ok || !okd) atomicExch(err, 1);
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     // the loads this thread issued have all landed before the block ends
     for (int kt = issued > kStages ? issued - kStages : 0; kt < issued; kt++)
       if (!tc::mbar_wait(&full[kt % kStages], (kt / kStages) & 1, kWaitLimit)) atomicExch(err, 2);
@@ -250,7 +250,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
   const uint32_t tmem = tmem_base;
   bool ok = true;
   int issued = 0;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     int s = 0, round = 0, ck = 0, dx = 0, dy = 0, dz = 0;
     int c = a.in_coff, wrow = 0;
     for (int kt = 0; kt < nk; kt++) {
@@ -280,7 +280,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
         ++round;
       }
     }
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1 && tc::elect_one()) {
     const uint32_t idesc = tc::idesc_bf16(128, a.cout);
     const uint64_t ad0 = tc::smem_desc(tA, tc::kSwizzle64, 64);
     const uint64_t bd0 = tc::smem_desc(tB, tc::kSwizzle64, 64);
@@ -345,7 +345,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
     }
   }
   if (!ok || !okd) atomicExch(err, 1);
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = issued > NST ? issued - NST : 0; kt < issued; kt++)
       if (!tc::mbar_wait(&full[kt % NST], (kt / NST) & 1, kWaitLimit)) atomicExch(err, 2);
   }
@@ -354,48 +354,339 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
   if (warp == 0) tc::tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
 }
 
-// Convolution of the narrower layers (32, 64 or 128 output channels) with input
-// reuse, one persistent block per SM.  An output tile is 16 (x) x 8 (y) x S
-// (z) voxels.  For each 32-channel chunk and each x-shift dx, one 5-D TMA
-// box brings the input block x0+dx .. x0+dx+15, y0-1 .. y0+8, z0-1 .. z0+S
+// One accumulator row per lane (COUT columns from TMEM address acc) to the
+// voxel at element `at` of the output: bias, ReLU, mask, conversion.
+template <int COUT>
+__device__ __forceinline__ void conv_rows_out(const ConvArgs &a, uint32_t acc, long long at, const float *bias) {
+#pragma unroll 1
+  for (int c = 0; c < COUT; c += 16) {
+    float v[16];
+    tc::tmem_ld16(acc + (uint32_t)c, v);
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] += bias[c + i];
+    if (a.relu) {
+#pragma unroll
+      for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i], 0.0f);
+    }
+    if (a.mask) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const uint4 mv = *(const uint4 *)(a.mask + at + c + 8 * h);
+        const __nv_bfloat16 *mb = (const __nv_bfloat16 *)&mv;
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[8 * h + i] = __bfloat162float(mb[i]) > 0.0f ? v[8 * h + i] : 0.0f;
+      }
+    }
+    if (a.out_f32) {
+      float4 *fd = (float4 *)(a.out_f32 + at + c);
+#pragma unroll
+      for (int h = 0; h < 4; h++) fd[h] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
+    } else {
+      uint4 o[2];
+      __nv_bfloat162 *ob = (__nv_bfloat162 *)o;
+#pragma unroll
+      for (int i = 0; i < 8; i++) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+      uint4 *dst = (uint4 *)(a.out + at + c);
+      dst[0] = o[0];
+      dst[1] = o[1];
+    }
+  }
+}
+
+// Convolution of 32 and 64 output channels, one persistent block per SM, every
+// input voxel staged once per 32-channel chunk.  An output item is 8 (x) x 16
+// (y) x up to S (z) voxels; input planes of 10 x 18 voxels (64-byte rows, x
+// fastest, halo included) go through a ring in shared memory, one TMA box
+// each.  The 128 rows of an MMA are the 16 y-lines of 8 voxels: groups of 8
+// rows at a pitch of 10 rows, so the tap (dx, dy) only moves the start by
+// 10 dy + dx rows (the swizzle is a function of the address, not of the row).
+// Weights come per (chunk, dx); with one chunk they stay for all items.
+//
+// An MMA of 128 x N x 16 takes max(32 + N / 4, N / 2) cycles: its A rows and
+// weights come from shared memory at 128 bytes per cycle.  Input plane zi
+// serves the output slices zi - 2, zi - 1 and zi (dz = 2, 1, 0), whose
+// accumulators are neighbours in TMEM, so the weights of the three dz lie
+// stacked in that order and one MMA of 128 x 3 cout does all three from one
+// read of A.  Every accumulator receives its products in the order chunk, dx,
+// dz, dy.  A plane leaves the ring in the last dx of its chunk, plane by
+// plane, while the next item's come in; two accumulator sets alternate between
+// items, so four warps write item i while the MMAs of item i + 1 run.
+//
+// Bound: the MMAs (75% of the peak for 32 output channels by the formula).
+// Measured at 128^3: 32 -> 32 channels 136 -> 95 us (854 -> 1220 TFLOP/s), 96
+// -> 32 1300 TFLOP/s; 64^3: 64 -> 64 channels 60 -> 44 us (1320 TFLOP/s); before,
+// a stage held the input block of one x-shift (three times the copies), the
+// issuing thread was slower than the tensor core, and a tile had 2 or 4 slices.
+template <int COUT>
+struct ConvR {
+  static constexpr int kS = 256 / COUT;                // slices of an item, at most
+  static constexpr int kPlane = 23 * 512;              // 180 rows of 64 B
+  static constexpr int kPlanes = COUT == 32 ? 14 : 12;
+  static constexpr int kTileB = 9 * COUT * 64;
+  static constexpr int kStagesB = COUT == 32 ? 3 : 2;
+  static constexpr int kSmem = kPlanes * kPlane + kStagesB * kTileB + 1024;
+  static constexpr int kSet = kS * COUT;               // TMEM columns of one accumulator set
+  static_assert(kSmem <= 227 * 1024 - 2048 && 2 * kSet <= 512 && kS + 2 <= kPlanes, "budget");
+};
+
+// The MMAs of one 32-channel chunk of an item, issued by one thread.  The
+// loop over the planes is unrolled for each run length, so that next to the
+// ring position everything is a constant: a plane's six MMAs take some 300
+// cycles of the tensor core, and what the thread does between them must take
+// less (computed with run-time lengths: 350 cycles per plane; the five
+// 32-channel layers of a 128^3 grid 706 us).
+template <int COUT>
+struct ConvRIssue {
+  using C = ConvR<COUT>;
+  uint32_t a_ring, b_ring, d0;    // low descriptor words (16-byte units); accumulator set
+  uint64_t *full_b, *empty_b, *full_p, *empty_p;
+  uint32_t limit = kWaitLimit;    // of a wait; 0 once one has run out
+  int slot = 0, sb = 0;           // ring slot of the chunk's first plane, next weight stage
+  uint32_t phase_p = 0, phase_b = 0;
+  bool keep_b, with_b;
+
+  __device__ __forceinline__ void wait(uint64_t *bar, uint32_t phase) {
+    if (!tc::mbar_wait(bar, phase, limit)) limit = 0;
+  }
+
+  template <int LEN>
+  __device__ __forceinline__ void chunk(uint32_t more) {
+    if constexpr (LEN <= C::kS) {
+      constexpr uint32_t tap = COUT * 64 >> 4, plane = C::kPlane >> 4;
+      int sp = slot;
+      uint32_t ph = phase_p;
+#pragma unroll 1
+      for (int dx = 0; dx < 3; dx++) {
+        if (with_b) {
+          wait(&full_b[sb], phase_b);
+          tc::fence_after_sync();
+        }
+        const uint32_t bx = b_ring + (uint32_t)sb * (C::kTileB >> 4), acc = more | (dx > 0);
+        sp = slot;
+        ph = phase_p;
+#pragma unroll
+        for (int zi = 0; zi < LEN + 2; zi++) {
+          if (dx == 0) {
+            wait(&full_p[sp], ph);
+            tc::fence_after_sync();
+          }
+          // dz of the slices this plane serves
+          const int lo = zi > LEN - 1 ? zi - (LEN - 1) : 0, hi = zi < 2 ? zi : 2;
+          const uint32_t d = d0 + (uint32_t)((zi - hi) * COUT), id = tc::idesc_bf16(128, (hi - lo + 1) * COUT);
+          const uint32_t az = a_ring + (uint32_t)sp * plane + (uint32_t)dx * 4u, bz = bx + (uint32_t)(2 - hi) * tap;
+          const auto mma = [&](uint32_t dst, uint32_t at, uint32_t bt, uint32_t idesc, uint32_t accumulate) {
+            tc::mma_bf16(dst, tc::desc_of(at, tc::kSwizzle64, 10 * 64), tc::desc_of(bt, tc::kSwizzle64, 8 * 64), idesc,
+                         accumulate);
+          };
+          if (lo == 0 && hi > 0 && !acc) {
+            // the first product of the last of these slices (dz = 0) overwrites it
+            mma(d, az, bz, tc::idesc_bf16(128, hi * COUT), 1);
+            mma(d + (uint32_t)(hi * COUT), az, bz + hi * tap, tc::idesc_bf16(128, COUT), 0);
+          } else {
+            mma(d, az, bz, id, lo == 0 && hi == 0 ? acc : 1);
+          }
+          mma(d, az + 2, bz + 2, id, 1);
+          mma(d, az + 40, bz + 3 * tap, id, 1);
+          mma(d, az + 42, bz + 3 * tap + 2, id, 1);
+          mma(d, az + 80, bz + 6 * tap, id, 1);
+          mma(d, az + 82, bz + 6 * tap + 2, id, 1);
+          if (dx == 2) tc::mma_commit(&empty_p[sp]);
+          if (++sp == C::kPlanes) {
+            sp = 0;
+            ph ^= 1u;
+          }
+        }
+        if (with_b && !keep_b) tc::mma_commit(&empty_b[sb]);
+        if (++sb == C::kStagesB) {
+          sb = 0;
+          phase_b ^= 1u;
+        }
+      }
+      slot = sp;
+      phase_p = ph;
+    }
+  }
+};
+
+template <int COUT>
+__global__ void __launch_bounds__(192, 1)
+k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int runs,
+         int items, int *err) {
+  after_previous();
+  using C = ConvR<COUT>;
+  constexpr int NB = C::kStagesB, NP = C::kPlanes;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
+  constexpr uint32_t tap_b = COUT * 64;  // one tap's weights
+  uint8_t *const tB = smem_raw + pad, *const tA = tB + NB * C::kTileB;
+  __shared__ uint64_t full_b[NB], empty_b[NB], full_p[NP], empty_p[NP], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_base;
+  __shared__ float bias[COUT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_x = a.W / 8, tiles_y = a.H / 16, cols = tiles_x * tiles_y;
+  const int nck = a.cin / 32;
+  const bool keep_b = nck == 1 && NB >= 3;  // all weights fit: loaded for the first item only
+  if (warp == 0) {
+    tc::tmem_alloc(&tmem_base, 2 * C::kSet);
+    tc::tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < NB; s++) {
+      tc::mbar_init(&full_b[s], 1);
+      tc::mbar_init(&empty_b[s], 1);
+    }
+    for (int s = 0; s < NP; s++) {
+      tc::mbar_init(&full_p[s], 1);
+      tc::mbar_init(&empty_p[s], 1);
+    }
+    for (int b = 0; b < 2; b++) {
+      tc::mbar_init(&acc_full[b], 1);
+      tc::mbar_init(&acc_empty[b], 4);
+    }
+    tc::fence_mbar_init();
+  }
+  for (int c = threadIdx.x; c < COUT; c += 192) bias[c] = a.bias ? a.bias[c] : 0.0f;
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_base;
+  bool ok = true;
+  // first slice and number of slices of an item; a column is cut into `runs` almost equal runs
+  const auto slices = [&](int item, int &z0) {
+    const int run = (item / cols) % runs;
+    z0 = run * a.D / runs;
+    return (run + 1) * a.D / runs - z0;
+  };
+  if (warp == 0 && tc::elect_one()) {  // copies
+    int nb = 0, np = 0;    // weight stages and planes issued
+    const auto load_b = [&](int ck, int dx) {
+      const int s = nb % NB;
+      if (nb >= NB && !tc::mbar_wait(&empty_b[s], (uint32_t)(nb / NB - 1) & 1u, kWaitLimit)) return false;
+      tc::mbar_expect_tx(&full_b[s], (uint32_t)C::kTileB);
+      for (int dy = 0; dy < 3; dy++)
+        for (int dz = 0; dz < 3; dz++)
+          tc::tma_load_2d(tB + s * C::kTileB + (dy * 3 + 2 - dz) * tap_b, &tw, &full_b[s], 0,
+                          ((dz * 9 + dy * 3 + dx) * nck + ck) * COUT);
+      nb++;
+      return true;
+    };
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      const int x0 = (item % tiles_x) * 8, y0 = ((item / tiles_x) % tiles_y) * 16, n = item / (cols * runs);
+      int z0;
+      const int len = slices(item, z0);
+      const bool with_b = !keep_b || item == (int)blockIdx.x;
+      for (int ck = 0; ck < nck && ok; ck++) {
+        if (with_b) ok = load_b(ck, 0);
+        for (int zi = 0; zi < len + 2 && ok; zi++) {
+          const int s = np % NP;
+          if (np >= NP && !tc::mbar_wait(&empty_p[s], (uint32_t)(np / NP - 1) & 1u, kWaitLimit)) {
+            ok = false;
+            break;
+          }
+          tc::mbar_expect_tx(&full_p[s], 180 * 64);
+          // padded coordinates: interior voxel v is v + 1, the halo before it v
+          tc::tma_load_5d(tA + s * C::kPlane, &tx, &full_p[s], a.in_coff + ck * 32, x0, y0, z0 + zi, n);
+          np++;
+        }
+        if (with_b && ok) ok = load_b(ck, 1);
+        if (with_b && ok) ok = load_b(ck, 2);
+      }
+    }
+    // the copies issued have landed before the block ends
+    for (int i = nb > NB ? nb - NB : 0; i < nb; i++)
+      if (!tc::mbar_wait(&full_b[i % NB], (uint32_t)(i / NB) & 1u, kWaitLimit)) atomicExch(err, 2);
+    for (int i = np > NP ? np - NP : 0; i < np; i++)
+      if (!tc::mbar_wait(&full_p[i % NP], (uint32_t)(i / NP) & 1u, kWaitLimit)) atomicExch(err, 2);
+  } else if (warp == 1 && tc::elect_one()) {  // MMAs
+    ConvRIssue<COUT> m;
+    m.a_ring = (uint32_t)tc::smem_desc(tA, tc::kSwizzle64, 64, 10 * 64);
+    m.b_ring = (uint32_t)tc::smem_desc(tB, tc::kSwizzle64, 64);
+    m.full_b = full_b; m.empty_b = empty_b; m.full_p = full_p; m.empty_p = empty_p;
+    m.keep_b = keep_b;
+    int g = 0;
+    for (int item = blockIdx.x; item < items && m.limit; item += gridDim.x, g++) {
+      const int set = g & 1;
+      int z0;
+      const int len = slices(item, z0);
+      m.with_b = !keep_b || g == 0;
+      if (g >= 2) m.wait(&acc_empty[set], (uint32_t)((g >> 1) - 1) & 1u);
+      tc::fence_after_sync();
+      m.d0 = tmem + (uint32_t)(set * C::kSet);
+      for (int ck = 0; ck < nck; ck++) {
+        const uint32_t more = ck > 0;
+        switch (len) {
+          case 1: m.template chunk<1>(more); break;
+          case 2: m.template chunk<2>(more); break;
+          case 3: m.template chunk<3>(more); break;
+          case 4: m.template chunk<4>(more); break;
+          case 5: m.template chunk<5>(more); break;
+          case 6: m.template chunk<6>(more); break;
+          case 7: m.template chunk<7>(more); break;
+          default: m.template chunk<8>(more); break;
+        }
+      }
+      tc::mma_commit(&acc_full[set]);
+    }
+    ok = m.limit != 0;
+  } else if (warp >= 2) {  // accumulators to memory
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    int g = 0;
+    for (int item = blockIdx.x; item < items; item += gridDim.x, g++) {
+      const int set = g & 1;
+      int z0;
+      const int len = slices(item, z0);
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[set], (uint32_t)(g >> 1) & 1u, kWaitLimit));
+      if (!ok) break;
+      tc::fence_after_sync();
+      const int vx = (item % tiles_x) * 8 + row % 8, vy = ((item / tiles_x) % tiles_y) * 16 + row / 8;
+      const int n = item / (cols * runs);
+#pragma unroll 1
+      for (int sl = 0; sl < len; sl++) {
+        const long long vox = (((long long)n * (a.D + 2) + z0 + sl + 1) * (a.H + 2) + vy + 1) * (a.W + 2) + vx + 1;
+        conv_rows_out<COUT>(a, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * C::kSet + sl * COUT),
+                            vox * a.out_ctot + a.out_coff, bias);
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&acc_empty[set]);
+    }
+  }
+  if (!ok) atomicExch(err, 1);
+  tc::fence_before_sync();
+  __syncthreads();
+  __syncwarp();
+  if (warp == 0) tc::tmem_dealloc(tmem, 2 * C::kSet);
+}
+
+// Convolution of 128 output channels (and of 32 and 64 on grids 8 high),
+// one persistent block per SM.  An output tile is 16 (x) x 8 (y) x 2 (z)
+// voxels.  For each 32-channel chunk and each x-shift dx, one 5-D TMA
+// box brings the input block x0+dx .. x0+dx+15, y0-1 .. y0+8, z0-1 .. z0+2
 // (rows of 64 B, x fastest) into shared memory, with the weights of the nine
 // taps of that dx.  The 128 rows of input plane zi shifted by dy start at row
-// (zi * 10 + dy) * 16, a multiple of 16 rows (1024 B, whole 64-byte swizzle
-// atoms).
-//
-// Up to 64 output channels an MMA of 128 x cout is bound by reading its A
-// rows from shared memory (4 KB per 16 channels; 32 output channels: 40
-// cycles against 16 of arithmetic).  Input plane zi serves the output slices
-// zi - 2, zi - 1 and zi (dz = 2, 1, 0), whose accumulators are neighbours in
-// TMEM, so the weights of the three dz lie stacked in that order and one MMA
-// of 128 x 3 cout does all three from one read of A (56 cycles instead of
-// 120).  Every accumulator still receives its products in the order chunk,
-// dx, dz, dy.
-//
-// Two accumulator sets alternate between tiles, so four warps convert and
-// write tile t while the copies and MMAs of tile t + 1 run.  Measured: the
-// five 32-channel layers of a 128^3 grid 2333 -> 950 us (348 -> 854 TFLOP/s),
-// 64 -> 64 channels at 64^3 97 -> 60 us (600 -> 970 TFLOP/s); before, one
-// block per tile of two slices did its set-up, copies, MMAs and epilogue in
-// sequence, one dz per MMA.
-template <int COUT, int S>
+// (zi * 10 + dy) * 16.  Two accumulator sets alternate between tiles, so four
+// warps convert and write tile t while the copies and MMAs of tile t + 1 run.
+// 128 -> 128 channels: bound by the weights' way into shared memory (74 KB
+// per 2300 cycles of MMAs).
+template <int COUT>
 struct ConvZ {
+  static constexpr int S = 2;
   static constexpr int kTileA = (S + 2) * 160 * 64;
   static constexpr int kTileB = 9 * COUT * 64;
-  static constexpr int kStages = COUT == 32 && S == 2 ? 3 : 2;
+  static constexpr int kStages = COUT == 32 ? 3 : 2;
   static constexpr int kSmem = kStages * (kTileA + kTileB) + 1024;
   static constexpr bool kStack = 3 * COUT <= 256;
   static constexpr int kSet = S * COUT;  // TMEM columns of one accumulator set
   static_assert(kSmem <= 227 * 1024 - 2048 && 2 * kSet <= 512, "stage budget");
 };
 
-template <int COUT, int S>
+template <int COUT>
 __global__ void __launch_bounds__(192, 1)
 k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int items,
          int *err) {
   after_previous();
-  using C = ConvZ<COUT, S>;
-  constexpr int NST = C::kStages;
+  using C = ConvZ<COUT>;
+  constexpr int NST = C::kStages, S = C::S;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
@@ -429,7 +720,7 @@ k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   tc::fence_after_sync();
   const uint32_t tmem = tmem_base;
   bool ok = true;
-  if (threadIdx.x == 0) {  // copies
+  if (warp == 0 && tc::elect_one()) {  // copies
     int s = 0, round = 0;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
       const int x0 = (item % tiles_x) * 16, y0 = ((item / tiles_x) % tiles_y) * 8,
@@ -454,7 +745,7 @@ k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
     const int issued = round * NST + s;
     for (int kt = issued > NST ? issued - NST : 0; kt < issued; kt++)
       if (!tc::mbar_wait(&full[kt % NST], (kt / NST) & 1, kWaitLimit)) atomicExch(err, 2);
-  } else if (threadIdx.x == 32) {  // MMAs
+  } else if (warp == 1 && tc::elect_one()) {  // MMAs
     int s = 0, round = 0, g = 0;
     for (int item = blockIdx.x; item < items && ok; item += gridDim.x, g++) {
       const int set = g & 1;
@@ -519,39 +810,7 @@ k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
       for (int sl = 0; sl < S; sl++) {
         const long long vox = (((long long)n * (a.D + 2) + z0 + sl + 1) * (a.H + 2) + vy + 1) * (a.W + 2) + vx + 1;
         const long long at = vox * a.out_ctot + a.out_coff;
-#pragma unroll 1
-        for (int c = 0; c < COUT; c += 16) {
-          float v[16];
-          tc::tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * C::kSet + sl * COUT + c), v);
-#pragma unroll
-          for (int i = 0; i < 16; i++) v[i] += bias[c + i];
-          if (a.relu) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = fmaxf(v[i], 0.0f);
-          }
-          if (a.mask) {
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              const uint4 mv = *(const uint4 *)(a.mask + at + c + 8 * h);
-              const __nv_bfloat16 *mb = (const __nv_bfloat16 *)&mv;
-#pragma unroll
-              for (int i = 0; i < 8; i++) v[8 * h + i] = __bfloat162float(mb[i]) > 0.0f ? v[8 * h + i] : 0.0f;
-            }
-          }
-          if (a.out_f32) {
-            float4 *fd = (float4 *)(a.out_f32 + at + c);
-#pragma unroll
-            for (int h = 0; h < 4; h++) fd[h] = make_float4(v[4 * h], v[4 * h + 1], v[4 * h + 2], v[4 * h + 3]);
-          } else {
-            uint4 o[2];
-            __nv_bfloat162 *ob = (__nv_bfloat162 *)o;
-#pragma unroll
-            for (int i = 0; i < 8; i++) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            uint4 *dst = (uint4 *)(a.out + at + c);
-            dst[0] = o[0];
-            dst[1] = o[1];
-          }
-        }
+        conv_rows_out<COUT>(a, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * C::kSet + sl * COUT), at, bias);
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -705,7 +964,7 @@ k_wgrad(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensor
   const uint32_t tmem = tmem_base;
   bool ok = true;
   int issued = 0;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = 0; kt < nk; kt++) {
       const int s = kt % kStages;
       if (kt >= kStages && !tc::mbar_wait(&empty[s], ((kt / kStages) - 1) & 1, kWaitLimit)) {
@@ -724,7 +983,7 @@ k_wgrad(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensor
       tc::tma_load_2d(tB + s * tile_b, &tb, &full[s], k0, ci0);
       issued = kt + 1;
     }
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1 && tc::elect_one()) {
     const uint32_t idesc = tc::idesc_bf16(128, w.ntile);
     for (int kt = 0; kt < nk; kt++) {
       const int s = kt % kStages;
@@ -763,7 +1022,7 @@ k_wgrad(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtensor
     }
   }
   if (!ok || !okd) atomicExch(err, 1);
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = issued > kStages ? issued - kStages : 0; kt < issued; kt++)
       if (!tc::mbar_wait(&full[kt % kStages], (kt / kStages) & 1, kWaitLimit)) atomicExch(err, 2);
   }
@@ -894,7 +1153,7 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
   const uint32_t tmem = tmem_base;
   bool ok = true;
   int issued = 0;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = 0; kt < nk; kt++) {
       const int s = kt % kStages;
       if (kt >= kStages && !tc::mbar_wait(&empty[s], ((kt / kStages) - 1) & 1, kWaitLimit)) {
@@ -936,7 +1195,7 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
       }
       issued = kt + 1;
     }
-  } else if (threadIdx.x == 32) {
+  } else if (warp == 1 && tc::elect_one()) {
     const uint32_t idesc = tc::idesc_bf16(128, w.n_mma);
     const int parts = w.n_rows / w.n_mma;
     for (int kt = 0; kt < nk; kt++) {
@@ -983,7 +1242,7 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
     }
   }
   if (!ok || !okd) atomicExch(err, 1);
-  if (threadIdx.x == 0) {
+  if (warp == 0 && tc::elect_one()) {
     for (int kt = issued > kStages ? issued - kStages : 0; kt < issued; kt++)
       if (!tc::mbar_wait(&full[kt % kStages], (kt / kStages) & 1, kWaitLimit)) atomicExch(err, 2);
   }
@@ -1353,20 +1612,46 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
   a.mask = (const __nv_bfloat16 *)mask;
   a.out = out_f32 ? nullptr : (__nv_bfloat16 *)out;
   a.out_f32 = out_f32;
-  if ((cout == 32 || cout == 64 || cout == 128) && W % 16 == 0 && H % 8 == 0 && D % 2 == 0) {
-    // Tiles of 16 x 8 x S voxels.  Four slices per tile read the input's z
-    // halo and the A operand less often, two make twice the tiles: the least
-    // work of the busiest block decides, in units of MMA cycles per chunk
-    // (128 output channels: two, whose accumulator sets fill the TMEM).
-    const long long t2 = (long long)(W / 16) * (H / 8) * (D / 2) * B;
-    const long long w2 = (t2 + kConvSms - 1) / kConvSms * (cout == 32 ? 176 : 224);
-    const long long w4 = (t2 / 2 + kConvSms - 1) / kConvSms * (cout == 32 ? 288 : 416);
-    const int slices = cout <= 64 && D % 4 == 0 && w4 <= w2 ? 4 : 2;
+  if ((cout == 32 || cout == 64) && W % 8 == 0 && H % 16 == 0) {
+    // A column of 8 x 16 voxels is cut into runs along z.  Fewer, longer runs
+    // read fewer halo planes; the count is the one whose busiest block has the
+    // least work, in MMA cycles per chunk and tap pair: 32 per input plane (its
+    // A rows) and cout / 4 per slice and dz (the weights).
+    const int cols = (W / 8) * (H / 16), most = 256 / cout;
+    int runs = (D + most - 1) / most;
+    double best = 0.0;
+    for (int k = runs; k <= D; k++) {
+      const double len = (double)D / k;
+      const double work = (double)(((long long)cols * k * B + kConvSms - 1) / kConvSms) * (32.0 * (len + 2.0) + 0.75 * cout * len);
+      if (k == runs || work < best) {
+        best = work;
+        runs = k;
+      }
+    }
     CUtensorMap th;
-    if (!make_map_act(&th, in, B, D, H, W, in_ctot, 16, 10, slices + 2))
+    if (!make_map_act(&th, in, B, D, H, W, in_ctot, 10, 18, 1))
       return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
-    const int items = (int)(slices == 4 ? t2 / 2 : t2);
-    static unsigned long long attr_z[5] = {0, 0, 0, 0, 0};
+    const int items = cols * runs * B;
+    static unsigned long long attr_r[2] = {0, 0};
+    const auto go = [&](auto kernel, int smem, int slot) {
+      cudaError_t e = smem_opt_in((const void *)kernel, smem, attr_r[slot]);
+      if (e != cudaSuccess) return e;
+      launch_pdl(kernel, std::min(items, kConvSms), 192, smem, (cudaStream_t)stream, th, tw, a, runs, items, err);
+      slbc::count_launch();
+      return cudaGetLastError();
+    };
+    const cudaError_t e = cout == 32 ? go(k_conv_r<32>, ConvR<32>::kSmem, 0) : go(k_conv_r<64>, ConvR<64>::kSmem, 1);
+    if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
+    return 0;
+  }
+  if ((cout == 32 || cout == 64 || cout == 128) && W % 16 == 0 && H % 8 == 0 && D % 2 == 0) {
+    // 128 output channels, whose accumulator sets of two slices fill the TMEM
+    // and whose weights fill the ring's memory, and grids 8 high.
+    CUtensorMap th;
+    if (!make_map_act(&th, in, B, D, H, W, in_ctot, 16, 10, 4))
+      return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
+    const int items = (int)((long long)(W / 16) * (H / 8) * (D / 2) * B);
+    static unsigned long long attr_z[3] = {0, 0, 0};
     const auto go = [&](auto kernel, int smem, int slot) {
       cudaError_t e = smem_opt_in((const void *)kernel, smem, attr_z[slot]);
       if (e != cudaSuccess) return e;
@@ -1375,9 +1660,9 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
       return cudaGetLastError();
     };
     cudaError_t e;
-    if (cout == 128) e = go(k_conv_z<128, 2>, ConvZ<128, 2>::kSmem, 0);
-    else if (cout == 64) e = slices == 4 ? go(k_conv_z<64, 4>, ConvZ<64, 4>::kSmem, 1) : go(k_conv_z<64, 2>, ConvZ<64, 2>::kSmem, 2);
-    else e = slices == 4 ? go(k_conv_z<32, 4>, ConvZ<32, 4>::kSmem, 3) : go(k_conv_z<32, 2>, ConvZ<32, 2>::kSmem, 4);
+    if (cout == 128) e = go(k_conv_z<128>, ConvZ<128>::kSmem, 0);
+    else if (cout == 64) e = go(k_conv_z<64>, ConvZ<64>::kSmem, 1);
+    else e = go(k_conv_z<32>, ConvZ<32>::kSmem, 2);
     if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
     return 0;
   }
