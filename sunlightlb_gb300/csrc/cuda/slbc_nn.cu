@@ -457,31 +457,49 @@ __global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int 
 
 // Passes 2 and 3 (along y: n = H rows of `inner` = W bytes; along z: n = D
 // planes of W H): b = min over |d| <= R of d^2 + a at the node d steps away.
-// A thread takes four neighbouring bytes where rows hold whole words (VEC 4;
-// squares up to 144 and values up to 144 add without overflow in a byte
-// under saturation, and the cap of R^2 absorbs it).
+// A thread takes kDistRun consecutive nodes p of the pass at one place of the
+// line: 2R + kDistRun loads serve them all.  Where lines hold whole words it
+// takes four neighbouring bytes (VEC 4) as two pairs of 16 bits, for which one
+// instruction adds and takes the minimum.  Bound: those instructions.  Measured
+// at 128^3, R = 12: 127 -> 14 us for both passes; before, 25 loads per output,
+// byte-wise minima in some ten instructions each and, along z, one block per
+// plane.
+constexpr int kDistRun = 4;
+
 template <int R, int VEC>
-__global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int lines, int n, int inner, unsigned char *b) {
+__global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int outers, int n, int inner, unsigned char *b) {
   after_previous();
-  const int len = inner / VEC;  // a line: the bytes of one p of one outer block
-  const RowWalk w = row_walk(len);
-  for (int line = w.row; line < lines; line += w.step) {
-    const int outer = line / n, p = line - outer * n;
-    const unsigned char *base = a + (long long)outer * n * inner;
-    for (int e = w.e; e < len; e += 256) {
-      unsigned best = VEC == 4 ? (unsigned)(R * R) * 0x01010101u : (unsigned)(R * R);
+  const unsigned len = (unsigned)inner / VEC, groups = (unsigned)(n + kDistRun - 1) / kDistRun;
+  const unsigned total = (unsigned)outers * groups * len;
+  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+    const unsigned row = i / len, e = i - row * len, outer = row / groups;
+    const int p0 = (int)(row - outer * groups) * kDistRun;
+    const unsigned char *base = a + (long long)outer * n * inner + VEC * e;
+    unsigned lo[kDistRun], hi[kDistRun];
 #pragma unroll
-      for (int d = -R; d <= R; d++) {
-        int q = p + d;
-        if (n >= R) q = q < 0 ? q + n : q >= n ? q - n : q;
-        else q = (q % n + n) % n;
-        const unsigned char *at = base + (long long)q * inner + VEC * e;
-        if (VEC == 4) best = __vminu4(best, __vaddus4(*(const unsigned *)at, (unsigned)(d * d) * 0x01010101u));
-        else best = min(best, (unsigned)(d * d) + *at);
+    for (int t = 0; t < kDistRun; t++) lo[t] = hi[t] = (unsigned)(R * R) * 0x00010001u;
+#pragma unroll
+    for (int k = -R; k < R + kDistRun; k++) {
+      int q = p0 + k;
+      if (n >= R + kDistRun) q = q < 0 ? q + n : q >= n ? q - n : q;
+      else q = (q % n + n) % n;
+      const unsigned char *at = base + (long long)q * inner;
+      const unsigned v = VEC == 4 ? *(const unsigned *)at : *at;
+      const unsigned vl = VEC == 4 ? __byte_perm(v, 0, 0x4140) : v, vh = VEC == 4 ? __byte_perm(v, 0, 0x4342) : 0u;
+#pragma unroll
+      for (int t = 0; t < kDistRun; t++) {
+        const int d = k - t;
+        if (d < -R || d > R) continue;
+        lo[t] = __viaddmin_u16x2(vl, (unsigned)(d * d) * 0x00010001u, lo[t]);
+        if (VEC == 4) hi[t] = __viaddmin_u16x2(vh, (unsigned)(d * d) * 0x00010001u, hi[t]);
       }
-      unsigned char *out = b + (long long)line * inner + VEC * e;
-      if (VEC == 4) *(unsigned *)out = best;
-      else *out = (unsigned char)best;
+    }
+    unsigned char *out = b + ((long long)outer * n + p0) * inner + VEC * e;
+#pragma unroll
+    for (int t = 0; t < kDistRun; t++) {
+      if (p0 + t >= n) break;
+      if (VEC == 4) *(unsigned *)(out + (long long)t * inner) = __byte_perm(lo[t], hi[t], 0x6420);
+      else out[(long long)t * inner] = (unsigned char)lo[t];
     }
   }
 }
@@ -870,8 +888,10 @@ int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void 
     const int vec = W % 4 == 0 ? 4 : 1;
     const auto passes = [&](auto rx, auto ry, auto rz) {
       launch_pdl(rx, rows_grid((long long)B * D * H, W), 256, 0, st, solid, B * D * H, W, a);
-      launch_pdl(ry, rows_grid((long long)B * D * H, W / vec), 256, 0, st, a, B * D * H, H, W, b);
-      launch_pdl(rz, rows_grid((long long)B * D, W * H / vec), 256, 0, st, b, B * D, D, W * H, a);
+      const long long run_y = (long long)B * D * ((H + kDistRun - 1) / kDistRun) * (W / vec);
+      const long long run_z = (long long)B * ((D + kDistRun - 1) / kDistRun) * (W * H / vec);
+      launch_pdl(ry, grid_for(run_y), 256, 0, st, a, B * D, H, W, b);
+      launch_pdl(rz, grid_for(run_z), 256, 0, st, b, B, D, W * H, a);
     };
     if (features == 2) {
       if (vec == 4) passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 4>, k_dist_min<kDistR2, 4>);
