@@ -209,10 +209,12 @@ __host__ __device__ constexpr int conv_smem(int nst, int cout) { return nst * (k
 constexpr int kConvSmemMax = conv_smem(8, 64);
 static_assert(conv_smem(6, 128) <= kConvSmemMax && conv_smem(4, 256) <= kConvSmemMax, "stage budget");
 
-// The producer (thread 0) and the MMA issuer (thread 32) step through
-// (tap, channel chunk, stage, round) with counters instead of divisions:
-// for the narrow layers an MMA pair takes a few tens of cycles, so the
-// single-thread loops set the pace.
+// The producer and the MMA issuer step through (tap, channel chunk, stage,
+// round) with counters instead of divisions: for the narrow layers an MMA pair
+// takes a few tens of cycles, so the single-thread loops set the pace.  On
+// coarse grids, whose 128-voxel tiles are far fewer than the SMs, the output
+// channels are split over the blocks of gridDim.z (a.cout each): the K loop of
+// 27 taps x cin is the same length but its stages are smaller and deeper.
 template <int NST>
 __global__ void __launch_bounds__(128, 2)
 k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int *err) {
@@ -220,7 +222,8 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
   extern __shared__ uint8_t smem_raw[];
   const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
   uint8_t *tA = smem_raw + pad;
-  const uint32_t tile_b = (uint32_t)a.cout * 64u;
+  const uint32_t tile_b = (uint32_t)a.cout * 64u;  // of this block's output channels
+  const int co0 = (int)blockIdx.z * a.cout;
   uint8_t *tB = tA + NST * kConvTileA;
   __shared__ uint64_t full[NST], empty[NST], done;
   __shared__ uint32_t tmem_base;
@@ -252,7 +255,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
   int issued = 0;
   if (warp == 0 && tc::elect_one()) {
     int s = 0, round = 0, ck = 0, dx = 0, dy = 0, dz = 0;
-    int c = a.in_coff, wrow = 0;
+    int c = a.in_coff, wrow = co0;
     for (int kt = 0; kt < nk; kt++) {
       if (round > 0 && !tc::mbar_wait(&empty[s], (uint32_t)(round - 1) & 1u, kWaitLimit)) {
         ok = false;
@@ -262,7 +265,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
       tc::tma_load_5d(tA + s * kConvTileA, &tx, &full[s], c, x0 + dx, y0 + dy, z0 + dz, n);
       tc::tma_load_2d(tB + s * tile_b, &tw, &full[s], 0, wrow);
       issued = kt + 1;
-      wrow += a.cout;
+      wrow += a.cout * (int)gridDim.z;
       c += 32;
       if (++ck == nck) {
         ck = 0;
@@ -311,15 +314,15 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
     const int r = warp * 32 + lane;
     const int vx = x0 + r % a.wbox, vy = y0 + (r / a.wbox) % a.hbox, vz = z0 + r / (a.wbox * a.hbox);
     const long long vox = (((long long)n * (a.D + 2) + vz + 1) * (a.H + 2) + vy + 1) * (a.W + 2) + vx + 1;
-    __nv_bfloat16 *dst = a.out + vox * a.out_ctot + a.out_coff;
-    const __nv_bfloat16 *msk = a.mask ? a.mask + vox * a.out_ctot + a.out_coff : nullptr;
+    __nv_bfloat16 *dst = a.out + vox * a.out_ctot + a.out_coff + co0;
+    const __nv_bfloat16 *msk = a.mask ? a.mask + vox * a.out_ctot + a.out_coff + co0 : nullptr;
 #pragma unroll 1
     for (int c = 0; c < a.cout; c += 8) {
       float v[8];
       tc::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
       if (a.bias) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) v[i] += a.bias[c + i];
+        for (int i = 0; i < 8; i++) v[i] += a.bias[co0 + c + i];
       }
       if (a.relu) {
 #pragma unroll
@@ -332,7 +335,7 @@ k_conv_fwd(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUten
         for (int i = 0; i < 8; i++) v[i] = __bfloat162float(mb[i]) > 0.0f ? v[i] : 0.0f;
       }
       if (a.out_f32) {
-        float4 *fd = (float4 *)(a.out_f32 + vox * a.out_ctot + a.out_coff + c);
+        float4 *fd = (float4 *)(a.out_f32 + vox * a.out_ctot + a.out_coff + co0 + c);
         fd[0] = make_float4(v[0], v[1], v[2], v[3]);
         fd[1] = make_float4(v[4], v[5], v[6], v[7]);
       } else {
@@ -393,7 +396,8 @@ __device__ __forceinline__ void conv_rows_out(const ConvArgs &a, uint32_t acc, l
   }
 }
 
-// Convolution of 32 and 64 output channels, one persistent block per SM, every
+// Convolution of 32 and 64 output channels (and of 32 to 96, the input gradient
+// of the finest level's first decoder layer), one persistent block per SM, every
 // input voxel staged once per 32-channel chunk.  An output item is 8 (x) x 16
 // (y) x up to S (z) voxels; input planes of 10 x 18 voxels (64-byte rows, x
 // fastest, halo included) go through a ring in shared memory, one TMA box
@@ -421,9 +425,9 @@ template <int COUT>
 struct ConvR {
   static constexpr int kS = 256 / COUT;                // slices of an item, at most
   static constexpr int kPlane = 23 * 512;              // 180 rows of 64 B
-  static constexpr int kPlanes = COUT == 32 ? 14 : 12;
+  static constexpr int kPlanes = COUT == 32 ? 14 : COUT == 64 ? 12 : 5;
   static constexpr int kTileB = 9 * COUT * 64;
-  static constexpr int kStagesB = COUT == 32 ? 3 : 2;
+  static constexpr int kStagesB = COUT == 64 ? 2 : 3;
   static constexpr int kSmem = kPlanes * kPlane + kStagesB * kTileB + 1024;
   static constexpr int kSet = kS * COUT;               // TMEM columns of one accumulator set
   static_assert(kSmem <= 227 * 1024 - 2048 && 2 * kSet <= 512 && kS + 2 <= kPlanes, "budget");
@@ -447,6 +451,46 @@ struct ConvRIssue {
 
   __device__ __forceinline__ void wait(uint64_t *bar, uint32_t phase) {
     if (!tc::mbar_wait(bar, phase, limit)) limit = 0;
+  }
+
+  __device__ __forceinline__ static void mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate) {
+    tc::mma_bf16(d, tc::desc_of(a, tc::kSwizzle64, 10 * 64), tc::desc_of(b, tc::kSwizzle64, 8 * 64), idesc, accumulate);
+  }
+
+  // The one chunk of 32 input channels with all weights in shared memory: each
+  // plane is finished, in the order dz, dy, dx, before it leaves the ring.
+  template <int LEN>
+  __device__ __forceinline__ void whole() {
+    if constexpr (LEN <= C::kS) {
+      constexpr uint32_t tap = COUT * 64 >> 4, plane = C::kPlane >> 4, stage = C::kTileB >> 4;
+      if (with_b)
+        for (int dx = 0; dx < 3; dx++) wait(&full_b[dx], 0);
+#pragma unroll
+      for (int zi = 0; zi < LEN + 2; zi++) {
+        wait(&full_p[slot], phase_p);
+        tc::fence_after_sync();
+        const int lo = zi > LEN - 1 ? zi - (LEN - 1) : 0, hi = zi < 2 ? zi : 2;  // dz of the slices this plane serves
+        const uint32_t d = d0 + (uint32_t)((zi - hi) * COUT), id = tc::idesc_bf16(128, (hi - lo + 1) * COUT);
+        const uint32_t az = a_ring + (uint32_t)slot * plane, bz = b_ring + (uint32_t)(2 - hi) * tap;
+#pragma unroll
+        for (int t = 0; t < 18; t++) {
+          const int dy = t / 6, dx = t / 2 % 3, kk = t % 2;
+          const uint32_t at = az + (uint32_t)(dy * 40 + dx * 4 + 2 * kk), bt = bz + (uint32_t)(dx * stage + dy * 3 * tap + 2 * kk);
+          if (t == 0 && lo == 0) {
+            // the first product of the last of these slices (dz = 0) overwrites it
+            if (hi > 0) mma(d, at, bt, tc::idesc_bf16(128, hi * COUT), 1);
+            mma(d + (uint32_t)(hi * COUT), at, bt + hi * tap, tc::idesc_bf16(128, COUT), 0);
+          } else {
+            mma(d, at, bt, id, 1);
+          }
+        }
+        tc::mma_commit(&empty_p[slot]);
+        if (++slot == C::kPlanes) {
+          slot = 0;
+          phase_p ^= 1u;
+        }
+      }
+    }
   }
 
   template <int LEN>
@@ -474,10 +518,6 @@ struct ConvRIssue {
           const int lo = zi > LEN - 1 ? zi - (LEN - 1) : 0, hi = zi < 2 ? zi : 2;
           const uint32_t d = d0 + (uint32_t)((zi - hi) * COUT), id = tc::idesc_bf16(128, (hi - lo + 1) * COUT);
           const uint32_t az = a_ring + (uint32_t)sp * plane + (uint32_t)dx * 4u, bz = bx + (uint32_t)(2 - hi) * tap;
-          const auto mma = [&](uint32_t dst, uint32_t at, uint32_t bt, uint32_t idesc, uint32_t accumulate) {
-            tc::mma_bf16(dst, tc::desc_of(at, tc::kSwizzle64, 10 * 64), tc::desc_of(bt, tc::kSwizzle64, 8 * 64), idesc,
-                         accumulate);
-          };
           if (lo == 0 && hi > 0 && !acc) {
             // the first product of the last of these slices (dz = 0) overwrites it
             mma(d, az, bz, tc::idesc_bf16(128, hi * COUT), 1);
@@ -527,7 +567,7 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   const int nck = a.cin / 32;
   const bool keep_b = nck == 1 && NB >= 3;  // all weights fit: loaded for the first item only
   if (warp == 0) {
-    tc::tmem_alloc(&tmem_base, 2 * C::kSet);
+    tc::tmem_alloc(&tmem_base, 512);
     tc::tmem_relinquish();
   }
   if (threadIdx.x == 32) {
@@ -612,17 +652,22 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
       if (g >= 2) m.wait(&acc_empty[set], (uint32_t)((g >> 1) - 1) & 1u);
       tc::fence_after_sync();
       m.d0 = tmem + (uint32_t)(set * C::kSet);
-      for (int ck = 0; ck < nck; ck++) {
-        const uint32_t more = ck > 0;
-        switch (len) {
-          case 1: m.template chunk<1>(more); break;
-          case 2: m.template chunk<2>(more); break;
-          case 3: m.template chunk<3>(more); break;
-          case 4: m.template chunk<4>(more); break;
-          case 5: m.template chunk<5>(more); break;
-          case 6: m.template chunk<6>(more); break;
-          case 7: m.template chunk<7>(more); break;
-          default: m.template chunk<8>(more); break;
+      if constexpr (COUT > 64) {
+        if (len == 1) m.template whole<1>();
+        else m.template whole<2>();
+      } else {
+        for (int ck = 0; ck < nck; ck++) {
+          const uint32_t more = ck > 0;
+          switch (len) {
+            case 1: m.template chunk<1>(more); break;
+            case 2: m.template chunk<2>(more); break;
+            case 3: m.template chunk<3>(more); break;
+            case 4: m.template chunk<4>(more); break;
+            case 5: m.template chunk<5>(more); break;
+            case 6: m.template chunk<6>(more); break;
+            case 7: m.template chunk<7>(more); break;
+            default: m.template chunk<8>(more); break;
+          }
         }
       }
       tc::mma_commit(&acc_full[set]);
@@ -655,7 +700,7 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   tc::fence_before_sync();
   __syncthreads();
   __syncwarp();
-  if (warp == 0) tc::tmem_dealloc(tmem, 2 * C::kSet);
+  if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
 // Convolution of 128 output channels (and of 32 and 64 on grids 8 high),
@@ -829,35 +874,36 @@ k_conv_z(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
 // are enumerated face by face: the planes z = 0 and z = D + 1 whole, then
 // for interior z the rows y = 0 and y = H + 1, then for interior z, y the
 // columns x = 0 and x = W + 1.
-__global__ void k_halo(__nv_bfloat16 *buf, int B, int D, int H, int W, int ctot, int coff, int nch) {
+// I: 32-bit unless the vectors of all halo voxels do not fit it (64-bit
+// divisions took 4.5 us of a launch where the copies take 2).
+template <typename I>
+__global__ void __launch_bounds__(256) k_halo(__nv_bfloat16 *buf, int B, int D, int H, int W, int ctot, int coff, int nch) {
   after_previous();
-  const long long Pz = 2LL * (H + 2) * (W + 2), Py = 2LL * D * (W + 2), Px = 2LL * D * H;
-  const long long per = Pz + Py + Px;
-  const int nv = nch / 8;
-  const long long total = (long long)B * per * nv;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int cv = (int)(e % nv);
-    const long long h = e / nv;
-    const int n = (int)(h / per);
-    long long r = h % per;
+  const I row = (I)(W + 2), face = (I)(H + 2) * row, side = (I)D * row, wall = (I)D * (I)H;
+  const I per = 2 * (face + side + wall), nv = (I)(nch / 8), total = (I)B * per * nv;
+  for (I e = (I)blockIdx.x * 256 + threadIdx.x; e < total; e += (I)gridDim.x * 256) {
+    const I h = e / nv;
+    const int cv = (int)(e - h * nv), n = (int)(h / per);
+    I r = h - (I)n * per;
     int x, y, z;
-    if (r < Pz) {
-      z = r < Pz / 2 ? 0 : D + 1;
-      r %= Pz / 2;
-      y = (int)(r / (W + 2));
-      x = (int)(r % (W + 2));
-    } else if ((r -= Pz) < Py) {
-      y = r < Py / 2 ? 0 : H + 1;
-      r %= Py / 2;
-      z = 1 + (int)(r / (W + 2));
-      x = (int)(r % (W + 2));
+    if (r < 2 * face) {
+      z = r < face ? 0 : D + 1;
+      if (r >= face) r -= face;
+      y = (int)(r / row);
+      x = (int)(r - (I)y * row);
+    } else if ((r -= 2 * face) < 2 * side) {
+      y = r < side ? 0 : H + 1;
+      if (r >= side) r -= side;
+      z = (int)(r / row);
+      x = (int)(r - (I)z * row);
+      z++;
     } else {
-      r -= Py;
-      x = r < Px / 2 ? 0 : W + 1;
-      r %= Px / 2;
-      z = 1 + (int)(r / H);
-      y = 1 + (int)(r % H);
+      r -= 2 * side;
+      x = r < wall ? 0 : W + 1;
+      if (r >= wall) r -= wall;
+      z = (int)(r / (I)H);
+      y = 1 + (int)(r - (I)z * (I)H);
+      z++;
     }
     const int sx = x == 0 ? W : (x == W + 1 ? 1 : x);
     const int sy = y == 0 ? H : (y == H + 1 ? 1 : y);
@@ -1612,7 +1658,7 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
   a.mask = (const __nv_bfloat16 *)mask;
   a.out = out_f32 ? nullptr : (__nv_bfloat16 *)out;
   a.out_f32 = out_f32;
-  if ((cout == 32 || cout == 64) && W % 8 == 0 && H % 16 == 0) {
+  if ((cout == 32 || cout == 64 || (cout == 96 && cin == 32)) && W % 8 == 0 && H % 16 == 0) {
     // A column of 8 x 16 voxels is cut into runs along z.  Fewer, longer runs
     // read fewer halo planes; the count is the one whose busiest block has the
     // least work, in MMA cycles per chunk and tap pair: 32 per input plane (its
@@ -1632,7 +1678,7 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
     if (!make_map_act(&th, in, B, D, H, W, in_ctot, 10, 18, 1))
       return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
     const int items = cols * runs * B;
-    static unsigned long long attr_r[2] = {0, 0};
+    static unsigned long long attr_r[3] = {0, 0, 0};
     const auto go = [&](auto kernel, int smem, int slot) {
       cudaError_t e = smem_opt_in((const void *)kernel, smem, attr_r[slot]);
       if (e != cudaSuccess) return e;
@@ -1640,7 +1686,9 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
       slbc::count_launch();
       return cudaGetLastError();
     };
-    const cudaError_t e = cout == 32 ? go(k_conv_r<32>, ConvR<32>::kSmem, 0) : go(k_conv_r<64>, ConvR<64>::kSmem, 1);
+    const cudaError_t e = cout == 32   ? go(k_conv_r<32>, ConvR<32>::kSmem, 0)
+                          : cout == 64 ? go(k_conv_r<64>, ConvR<64>::kSmem, 1)
+                                       : go(k_conv_r<96>, ConvR<96>::kSmem, 2);
     if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
     return 0;
   }
@@ -1666,12 +1714,23 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
     if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
     return 0;
   }
+  // as many parts of the output channels as fit one wave, at least 32 each
+  const long long tiles = (long long)D * H * W / 128 * B;
+  int parts = 1;
+  while (cout % (32 * parts) == 0 && cout / (2 * parts) >= 32 && tiles * 2 * parts <= kConvSms) parts *= 2;
+  if (parts > 1) {
+    a.cout = cout / parts;
+    if (!make_map_rows32(&tw, wgt, 27LL * (cin / 32) * cout, a.cout))
+      return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
+    a.tmem_cols = 32;
+    while (a.tmem_cols < a.cout) a.tmem_cols *= 2;
+  }
   static unsigned long long attr_done[3] = {0, 0, 0};
-  const int nst = conv_stages(cout), smem = conv_smem(nst, cout);
+  const int nst = conv_stages(a.cout), smem = conv_smem(nst, a.cout);
   const void *fn = nst == 8 ? (const void *)k_conv_fwd<8> : (nst == 6 ? (const void *)k_conv_fwd<6> : (const void *)k_conv_fwd<4>);
   cudaError_t e = smem_opt_in(fn, kConvSmemMax, attr_done[nst == 8 ? 0 : (nst == 6 ? 1 : 2)]);
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
-  const dim3 grid((unsigned)((long long)D * H * W / 128), (unsigned)B);
+  const dim3 grid((unsigned)((long long)D * H * W / 128), (unsigned)B, (unsigned)parts);
   if (nst == 8)
     launch_pdl(k_conv_fwd<8>, grid, 128, smem, (cudaStream_t)stream, tx, tw, a, err);
   else if (nst == 6)
@@ -1705,7 +1764,11 @@ int slbc_tc_halo(void *buf, int B, int D, int H, int W, int ctot, int coff, int 
   const long long per = 2LL * (H + 2) * (W + 2) + 2LL * D * (W + 2) + 2LL * D * H;
   const long long total = (long long)B * per * (nch / 8);
   const int blocks = (int)std::min<long long>((total + 255) / 256, 152LL * 16);
-  launch_pdl(k_halo, blocks, 256, 0, (cudaStream_t)stream, (__nv_bfloat16 *)buf, B, D, H, W, ctot, coff, nch);
+  const auto go = [&](auto kernel) {
+    launch_pdl(kernel, blocks, 256, 0, (cudaStream_t)stream, (__nv_bfloat16 *)buf, B, D, H, W, ctot, coff, nch);
+  };
+  if (total < (1LL << 31)) go(k_halo<unsigned>);  // the grid's stride may go past the end
+  else go(k_halo<unsigned long long>);
   slbc::count_launch();
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_halo: ") + cudaGetErrorString(e)), 1;

@@ -24,6 +24,8 @@ CONV = [  # B, D, H, W, cin, cout
     (1, 128, 32, 16, 128, 64),
     (1, 32, 8, 16, 64, 64),      # y of 8
     (2, 8, 16, 8, 64, 32),       # x of 8
+    (1, 16, 16, 16, 32, 96),     # two slices per item
+    (4, 7, 32, 16, 64, 128),     # an odd number of planes
 ]
 
 
