@@ -375,6 +375,12 @@ int slbc_nn_wfwd(const float *master, int cout, int cin, void *w, void *stream);
 int slbc_nn_wdgrad(const float *master, int cout, int cin, int ci0, int nci, void *w, void *stream);
 int slbc_nn_adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
                  int t, void *stream);
+/* wfwd (nci[i] = 0) and wdgrad for `count` weight tensors, and adam for `count`
+ * tensors, in one launch per 48 of them (host arrays of device pointers). */
+int slbc_nn_layouts(int count, const float *const *master, const int *cout, const int *cin, const int *ci0,
+                    const int *nci, void *const *w, void *stream);
+int slbc_nn_adam_list(int count, float *const *p, const float *const *g, float *const *m, float *const *v,
+                      const long long *n, float lr, float b1, float b2, float eps, int t, void *stream);
 int slbc_nn_mse(const float *pred, int ctot_p, const float *label, int nch, const float *sample_w, int B, int D, int H,
                 int W, void *grad, int gctot, double *loss, void *stream);
 /* Projection term of the loss, after slbc_nn_mse on the same buffers: per
@@ -394,6 +400,8 @@ int slbc_nn_proj(const float *pred, int ctot_p, const float *label, int lch, int
 int slbc_nn_sqsum(const float *g, long long n, double *state, void *stream);
 int slbc_nn_clip(double *state, float factor, float decay, void *stream);
 int slbc_nn_scale(float *g, long long n, const double *state, void *stream);
+int slbc_nn_sqsum_list(int count, const float *const *g, const long long *n, double *state, void *stream);
+int slbc_nn_scale_list(int count, float *const *g, const long long *n, const double *state, void *stream);
 int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void *out, int ctot, int features,
                    void *stream);
 int slbc_nn_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H, int W, float scale,

@@ -60,6 +60,10 @@ class Kernels:
             "slbc_tc_cmajor_shifts": [p, i, i, i, i, i, i, i, i, ll, i, p, p],
             "slbc_nn_wdgrad": [p, i, i, i, i, p, p],
             "slbc_nn_adam": [p, p, p, p, ll, f, f, f, f, i, p],
+            "slbc_nn_layouts": [i] + [p] * 7,
+            "slbc_nn_adam_list": [i] + [p] * 5 + [f, f, f, f, i, p],
+            "slbc_nn_sqsum_list": [i, p, p, p, p],
+            "slbc_nn_scale_list": [i, p, p, p, p],
             "slbc_nn_mse": [p, i, p, i, p, i, i, i, i, p, i, p, p],
             "slbc_nn_proj": [p, i, p, i, i, p, i, i, i, i, f, p, i, p, p, p],
             "slbc_nn_sqsum": [p, ll, p, p],
@@ -90,6 +94,12 @@ class Kernels:
                 raise RuntimeError(f"{name}: {self.dll.slbc_last_error().decode()}")
             return rc
         return call
+
+
+def pointers(addresses):
+    """A C array of device addresses."""
+    a = list(addresses)
+    return (C.c_void_p * len(a))(*a)
 
 
 def flat_geometry(D, H, W_):
@@ -180,12 +190,13 @@ class UNet:
     def refresh_weights(self):
         """BF16 tensor-core layouts of the FP32 master weights."""
         torch = self.torch
+        jobs = []  # master, cout, cin, first input channel, input channels (0: forward), layout
         for name, lv, cin, cout, *_ in self.layers:
             m = self.params[name]["w"]
             wf = self.wf.get(name)
             if wf is None:
                 wf = self.wf[name] = torch.empty(27 * cin * cout, device=self.dev, dtype=torch.bfloat16)
-            self.k.nn_wfwd(m.data_ptr(), cout, cin, wf.data_ptr(), self.stream)
+            jobs.append((m.data_ptr(), cout, cin, 0, 0, wf.data_ptr()))
             if name == "e0a":
                 continue  # no input gradient needed
             chunks = self.wd.get(name)
@@ -193,8 +204,11 @@ class UNet:
                 nci = cin if cin <= 256 else cin // 2
                 chunks = self.wd[name] = [(c0, nci, torch.empty(27 * nci * cout, device=self.dev,
                                                                  dtype=torch.bfloat16)) for c0 in range(0, cin, nci)]
-            for c0, nci, t in chunks:
-                self.k.nn_wdgrad(m.data_ptr(), cout, cin, c0, nci, t.data_ptr(), self.stream)
+            jobs += [(m.data_ptr(), cout, cin, c0, nci, t.data_ptr()) for c0, nci, t in chunks]
+        m, cout, cin, c0, nci, w = zip(*jobs)
+        n = len(jobs)
+        self.k.nn_layouts(n, pointers(m), (C.c_int * n)(*cout), (C.c_int * n)(*cin), (C.c_int * n)(*c0),
+                          (C.c_int * n)(*nci), pointers(w), self.stream)
 
     def _halo(self, name, coff=0, nch=None):
         t = self.buf[name] if name in self.buf else self.grad[name]
@@ -295,7 +309,9 @@ class UNet:
 
     def _dgrad(self, name, g_name, out_name, mask_name=None):
         """gradient at the input of layer `name` into grad[out_name], times
-        (mask > 0) when the input is a ReLU output mask_name."""
+        (mask > 0) when the input is a ReLU output mask_name.  The halo is
+        filled where a convolution reads it next (not for the sums of pooling
+        and upsampling, gP* and gC*)."""
         k = self.k
         _, lv, cin, cout, *_ = next(l for l in self.layers if l[0] == name)
         d, h, w = self.dims(lv)
@@ -304,7 +320,8 @@ class UNet:
         for c0, nci, wt in self.wd[name]:
             k.tc_conv3d(g.data_ptr(), self.B, d, h, w, g.shape[-1], 0, cout, wt.data_ptr(), None, nci,
                         o.data_ptr(), o.shape[-1], c0, 0, m.data_ptr() if m is not None else None, self.stream)
-        self._halo(out_name)
+        if out_name[:2] not in ("gP", "gC"):
+            self._halo(out_name)
 
     def loss_and_backward(self, labels, sample_w=None, proj=None):
         """labels: device FP32 (B, D, H, W, 3 or 4); sample_w: optional device
@@ -382,19 +399,17 @@ class UNet:
             self.clip_state = self.torch.zeros(3, device=self.dev, dtype=self.torch.float64)
         st = self.clip_state.data_ptr()
         grads = [self.params[name]["g" + key] for name, *_ in self.layers for key in ("w", "b")]
-        for g in grads:
-            self.k.nn_sqsum(g.data_ptr(), g.numel(), st, self.stream)
+        ptr, n = pointers(g.data_ptr() for g in grads), (C.c_longlong * len(grads))(*(g.numel() for g in grads))
+        self.k.nn_sqsum_list(len(grads), ptr, n, st, self.stream)
         self.k.nn_clip(st, factor, decay, self.stream)
-        for g in grads:
-            self.k.nn_scale(g.data_ptr(), g.numel(), st, self.stream)
+        self.k.nn_scale_list(len(grads), ptr, n, st, self.stream)
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.t += 1
-        for name, *_ in self.layers:
-            p = self.params[name]
-            for key in ("w", "b"):
-                self.k.nn_adam(p[key].data_ptr(), p["g" + key].data_ptr(), p["m" + key].data_ptr(),
-                               p["v" + key].data_ptr(), p[key].numel(), lr, b1, b2, eps, self.t, self.stream)
+        tensors = [(self.params[name], key) for name, *_ in self.layers for key in ("w", "b")]
+        lists = [pointers(p[pre + key].data_ptr() for p, key in tensors) for pre in ("", "g", "m", "v")]
+        n = (C.c_longlong * len(tensors))(*(p[key].numel() for p, key in tensors))
+        self.k.nn_adam_list(len(tensors), *lists, n, lr, b1, b2, eps, self.t, self.stream)
         self.refresh_weights()
 
     def status(self):
