@@ -338,6 +338,15 @@ int slbc_tc_cmajor_shifts(const void *src, int B, int D, int H, int W, int ctot,
 int slbc_tc_wgrad_tiles(const void *dyt, const void *xt, int B, int D, int H, int W, int Wp, long long pstride,
                         int cin, int cout, float *partial, long long partial_floats, int splits, float *dw,
                         void *stream);
+/* Flat copies that keep the channels last, dst[n * pstride + (z * (H+2) + y) *
+ * Wp + x][c] = src[n][z][y][x][coff + c] (0 beyond W + 1; zero_halo keeps interior
+ * voxels only), and the weight gradient from such copies of dY (halo kept) and
+ * the input (zero_halo): the same sums in the same order as slbc_tc_wgrad_tiles
+ * with the same splits.  cout 32, 64 or 128, cin a multiple of 32. */
+int slbc_tc_flat(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp, long long pstride,
+                 int zero_halo, void *dst, void *stream);
+int slbc_tc_wgrad_flat(const void *dyf, const void *xf, int B, int D, int H, int W, int Wp, long long pstride, int cin,
+                       int cout, float *partial, long long partial_floats, int splits, float *dw, void *stream);
 /* K splits for slbc_tc_wgrad that fill the current device once (at most
  * k_tiles / 8 and max_splits; k_tiles = B * pstride / 64). */
 int slbc_tc_wgrad_splits(int cin, int cout, long long k_tiles, long long max_splits);

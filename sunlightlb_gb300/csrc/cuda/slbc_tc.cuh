@@ -121,6 +121,23 @@ __device__ __forceinline__ uint64_t smem_desc(const void *p, uint32_t swizzle, u
   return d;
 }
 
+// Both operands MN-major (bits 15 and 16): K is the strided dimension of the
+// tiles.
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) { return idesc_bf16(M, N) | (1u << 15) | (1u << 16); }
+
+// Descriptor of an MN-major tile: rows of K with `row_bytes` (the swizzle width)
+// of M or N each, the next elements of M or N `mn_bytes` further on, groups of 8
+// rows following one another.
+__device__ __forceinline__ uint64_t smem_desc_mn(const void *p, uint32_t swizzle, uint32_t row_bytes, uint32_t mn_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_u32(p) & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(mn_bytes >> 4) << 16;
+  d |= (uint64_t)((8u * row_bytes) >> 4) << 32;
+  d |= (uint64_t)1 << 46;  // descriptor version
+  d |= (uint64_t)swizzle << 61;
+  return d;
+}
+
 // The same from the low word of such a descriptor (start address in 16-byte
 // units), whose start may have been moved by whole 16-byte units.
 __device__ __forceinline__ uint64_t desc_of(uint32_t lo, uint32_t swizzle, uint32_t group) {

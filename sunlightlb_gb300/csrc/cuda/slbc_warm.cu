@@ -1297,6 +1297,175 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
   if (warp == 0) tc::tmem_dealloc(tmem, (uint32_t)w.tmem_cols);
 }
 
+// The same sums, tile by tile and in the same order, from flat copies that keep
+// the channels last (k_flat): position f = (z * (H + 2) + y) * Wp + x of a sample
+// is a row of `ctot` channels.  K is then the row index of the staged tiles (MN-
+// major operands), so a tile of 64 positions is 64 rows of 64 or 128 bytes and
+// the three x-shifted views of dY are one tile of 72 rows read from three
+// starting rows: M block i of the operand begins i rows further on and holds tap
+// dx = 2 - i.  The input's nt windows are boxes of 64 rows x 32 channels.
+//
+// Against k_wgrad_n it stages 40 instead of 48 KB per K tile at 32 channels, and
+// the copies are one pass each without a transpose, one of dY instead of three.
+// Bound: staging (L2 to shared memory).  Measured, the 13 layers of a training
+// iteration of 4 x 64^3: 1228 -> 735 us, their copies 835 -> 451 us.
+constexpr int kWgfTileA = 72 * 128 * 2;
+constexpr int kWgfSmem = kStages * (kWgfTileA + kWgnMaxRows * 128) + 1024;
+
+__global__ void __launch_bounds__(128, 1)
+k_wgrad_f(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+          const __grid_constant__ CUtensorMap b_win, WgradNArgs w, int *err) {
+  after_previous();
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
+  uint8_t *tA = smem_raw + pad;
+  uint8_t *tB = tA + kStages * kWgfTileA;
+  const int tile_b = w.n_rows * 128;  // bytes of one B stage (a multiple of 4096)
+  __shared__ uint64_t full[kStages], empty[kStages], done;
+  __shared__ uint32_t tmem_base;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunk = blockIdx.x % w.ci_chunks;
+  const int g = (blockIdx.x / w.ci_chunks) % w.groups;
+  const int mt = blockIdx.x / (w.ci_chunks * w.groups);
+  const int ci0 = chunk * w.cc;
+  const long long kz = blockIdx.z;  // K tiles kz, kz + splits, ...
+  const int nk = kz < w.k_tiles ? (int)((w.k_tiles - kz + w.splits - 1) / w.splits) : 0;
+  int b_taps = 0;
+  for (int t = 0; t < w.nt; t++) b_taps += g * w.nt + t < 9;
+  const int row_a = w.cout == 32 ? 64 : 128;  // bytes of an A row: 32 or 64 channels
+  const uint32_t bytes = (uint32_t)(72 * w.cout * 2 + b_taps * w.cc * 128);
+  if (warp == 0) {
+    tc::tmem_alloc(&tmem_base, (uint32_t)w.tmem_cols);
+    tc::tmem_relinquish();
+  }
+  if (threadIdx.x == 32) {
+    for (int s = 0; s < kStages; s++) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    tc::mbar_init(&done, 1);
+    tc::fence_mbar_init();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_base;
+  bool ok = true;
+  if (warp == 0 && tc::elect_one()) {
+    int issued = 0;
+    for (int kt = 0; kt < nk; kt++) {
+      const int s = kt % kStages;
+      if (kt >= kStages && !tc::mbar_wait(&empty[s], ((kt / kStages) - 1) & 1, kWaitLimit)) {
+        ok = false;
+        break;
+      }
+      const int k0 = (int)((kz + (long long)kt * w.splits) * 64);
+      tc::mbar_expect_tx(&full[s], bytes);
+      // rows before 0 and past the end are zero
+      tc::tma_load_3d(tA + s * kWgfTileA, &ta, &full[s], 0, k0 - 1, 0);
+      // first window of the group: dy = 0 at the group's first dz
+      const long long xw = (long long)k0 - w.Wp + ((g * w.nt) / 3 - 1) * (long long)w.plane;
+      if (w.b4 && b_taps == w.nt && xw >= 0 && xw + 64 <= w.b4_dim0) {
+        tc::tma_load_5d(tB + s * tile_b, &b_win, &full[s], 0, (int)xw, ci0 / 32, 0, 0);
+      } else {
+        for (int t = 0; t < b_taps; t++) {
+          const int yz = g * w.nt + t, dy = yz % 3, dz = yz / 3;
+          tc::tma_load_3d(tB + s * tile_b + t * w.cc * 128, &tb, &full[s], 0, k0 + (dy - 1) * w.Wp + (dz - 1) * w.plane,
+                          ci0 / 32);
+        }
+      }
+      issued = kt + 1;
+    }
+    for (int kt = issued > kStages ? issued - kStages : 0; kt < issued; kt++)
+      if (!tc::mbar_wait(&full[kt % kStages], (kt / kStages) & 1, kWaitLimit)) atomicExch(err, 2);
+  } else if (warp == 1 && tc::elect_one()) {
+    // columns in one MMA or two, whole blocks of 32 each
+    const int n1 = w.n_rows <= 256 ? w.n_rows : (w.n_rows / 64 + 1) / 2 * 64 > 256 ? 256 : (w.n_rows / 64 + 1) / 2 * 64;
+    const int n2 = w.n_rows - n1;
+    const uint32_t id1 = tc::idesc_bf16_mn(128, n1), id2 = tc::idesc_bf16_mn(128, n2);
+    // the M blocks: one row further on for the next dx, or (128 output
+    // channels) the other 64 channels
+    const uint32_t mn = w.cout == 128 ? 72 * 128 : row_a;
+    const uint64_t a0 = tc::smem_desc_mn(tA, w.cout == 32 ? tc::kSwizzle64 : tc::kSwizzle128, row_a, mn) +
+                        (uint64_t)(mt * w.dpm * (row_a >> 4));
+    const uint64_t b0 = tc::smem_desc_mn(tB, tc::kSwizzle64, 64, 64 * 64);
+    for (int kt = 0; kt < nk; kt++) {
+      const int s = kt % kStages;
+      if (!tc::mbar_wait(&full[s], (kt / kStages) & 1, kWaitLimit)) {
+        ok = false;
+        break;
+      }
+      tc::fence_after_sync();
+      const uint64_t ad = a0 + (uint64_t)(s * (kWgfTileA >> 4)), bd = b0 + (uint64_t)(s * (tile_b >> 4));
+#pragma unroll
+      for (int kk = 0; kk < 4; kk++)
+        tc::mma_bf16(tmem, ad + (uint64_t)(kk * row_a), bd + (uint64_t)(kk * 64), id1, (kt | kk) != 0);
+      if (n2) {
+        const uint64_t be = bd + (uint64_t)(n1 / 32 * (64 * 64 >> 4));
+#pragma unroll
+        for (int kk = 0; kk < 4; kk++)
+          tc::mma_bf16(tmem + (uint32_t)n1, ad + (uint64_t)(kk * row_a), be + (uint64_t)(kk * 64), id2, (kt | kk) != 0);
+      }
+      tc::mma_commit(&empty[s]);
+    }
+    tc::mma_commit(&done);
+  }
+  __syncwarp();
+  const bool okd = __all_sync(0xffffffffu, tc::mbar_wait(&done, 0, kWaitLimit));
+  tc::fence_after_sync();
+  if (okd) {
+    const int r = warp * 32 + lane, d = r / w.cout, co = r % w.cout, off = mt * w.dpm + d;
+    const bool row_ok = d < w.dpm && off < 3;
+#pragma unroll 1
+    for (int c = 0; c < w.n_rows; c += 8) {
+      float v[8];
+      tc::tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);  // whole warp
+      if (nk == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = 0.0f;
+      }
+      const int yz = g * w.nt + c / w.cc;
+      if (row_ok && yz < 9) {
+        const int tap = yz / 3 * 9 + yz % 3 * 3 + 2 - off;
+        float *dst = w.partial + (((long long)blockIdx.z * 27 + tap) * w.cout + co) * w.cin + ci0 + c % w.cc;
+        ((float4 *)dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+        ((float4 *)dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+      }
+    }
+  }
+  if (!ok || !okd) atomicExch(err, 1);
+  tc::fence_before_sync();
+  __syncthreads();
+  __syncwarp();
+  if (warp == 0) tc::tmem_dealloc(tmem, (uint32_t)w.tmem_cols);
+}
+
+// Flat copies of channels [coff, coff + nch) with the row pitch Wp:
+// dst[n * pstride + (z * (H + 2) + y) * Wp + x][c] = src[n][z][y][x][coff + c], 0
+// beyond x = W + 1 (zero_halo: interior voxels only).  A warp takes a row of
+// positions at a time (the last `row` of a sample: what is left of its stride).
+// Bound: HBM.
+__global__ void __launch_bounds__(256) k_flat(const __nv_bfloat16 *src, int B, int D, int H, int W, int ctot, int coff,
+                                              int nch, int Wp, int pstride, int zero_halo, __nv_bfloat16 *dst) {
+  after_previous();
+  const int rows = (D + 2) * (H + 2), nv = nch / 8, tail = pstride - rows * Wp;
+  const int lane = threadIdx.x & 31, step = (int)gridDim.x * 8;
+  for (int q = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5); q < B * (rows + 1); q += step) {
+    const int n = q / (rows + 1), row = q - n * (rows + 1), z = row / (H + 2), y = row - z * (H + 2);
+    const bool in = row < rows && (!zero_halo || (z >= 1 && z <= D && y >= 1 && y <= H));
+    const int len = (row < rows ? Wp : tail) * nv, lo = zero_halo ? 1 : 0, hi = zero_halo ? W : W + 1;
+    const __nv_bfloat16 *from = src + ((long long)n * rows + row) * (W + 2) * ctot + coff;
+    uint4 *to = (uint4 *)(dst + ((long long)n * pstride + (long long)row * Wp) * nch);
+#pragma unroll 4
+    for (int i = lane; i < len; i += 32) {
+      const int x = (int)((unsigned)i / (unsigned)nv), cv = i - x * nv;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (in && x >= lo && x <= hi) v = *(const uint4 *)(from + (long long)x * ctot + 8 * cv);
+      to[i] = v;
+    }
+  }
+}
+
 // dw[i] = sum over splits of partial[s][i], in split order
 __global__ void k_sum_splits(const float *partial, long long n, int splits, float *dw) {
   after_previous();
@@ -1453,6 +1622,36 @@ bool make_map_windows(CUtensorMap *map, const void *ptr, long long rows, long lo
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, estr,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Flat channels-last copies of `rows` positions x nch channels: boxes of box_ch
+// (32 or 64) channels x box_rows positions x box_chunks, and (ny, nz > 1) the
+// windows of such boxes Wp and plane positions apart.
+bool make_map_flat(CUtensorMap *map, const void *ptr, long long rows, int nch, int box_ch, int box_rows, int box_chunks) {
+  EncodeTiled enc = encode_fn();
+  if (!enc) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)box_ch, (cuuint64_t)rows, (cuuint64_t)(nch / box_ch)};
+  const cuuint64_t strides[2] = {(cuuint64_t)nch * 2, (cuuint64_t)box_ch * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)box_ch, (cuuint32_t)box_rows, (cuuint32_t)box_chunks};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, box_ch == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool make_map_flat_windows(CUtensorMap *map, const void *ptr, long long rows, int nch, int box_chunks, int Wp,
+                           long long plane, int ny, int nz, long long &dim0) {
+  EncodeTiled enc = encode_fn();
+  if (!enc) return false;
+  dim0 = rows - (ny - 1) * (long long)Wp - (nz - 1) * plane;
+  if (dim0 < 64) return false;
+  const cuuint64_t pos = (cuuint64_t)nch * 2;
+  const cuuint64_t dims[5] = {32, (cuuint64_t)dim0, (cuuint64_t)(nch / 32), (cuuint64_t)ny, (cuuint64_t)nz};
+  const cuuint64_t strides[4] = {pos, 64, pos * Wp, pos * (cuuint64_t)plane};
+  const cuuint32_t box[5] = {32, 64, (cuuint32_t)box_chunks, (cuuint32_t)ny, (cuuint32_t)nz};
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(ptr), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1793,6 +1992,70 @@ int slbc_tc_cmajor_shifts(const void *src, int B, int D, int H, int W, int ctot,
                           long long pstride, int tiles, void *dst, void *stream) {
   return cmajor_launch("slbc_tc_cmajor_shifts", src, B, D, H, W, ctot, coff, nch, Wp, pstride, -1, 3, 0, 0, tiles ? 3 : 0,
                        (long long)nch * B * pstride, dst, stream);
+}
+
+int slbc_tc_flat(const void *src, int B, int D, int H, int W, int ctot, int coff, int nch, int Wp, long long pstride,
+                 int zero_halo, void *dst, void *stream) {
+  if (B < 1 || nch < 8 || coff < 0 || coff + nch > ctot || Wp < W + 2 || Wp % 8 || pstride % 64 ||
+      pstride < (long long)(D + 2) * (H + 2) * Wp || (long long)B * ((long long)(D + 2) * (H + 2) + 1) >= 1LL << 30 ||
+      pstride >= 1LL << 31)
+    return slbc::set_error("slbc_tc_flat: bad geometry"), 1;
+  if (nch % 8 || coff % 8 || ctot % 8 || !aligned16(src) || !aligned16(dst))
+    return slbc::set_error("slbc_tc_flat: channels must be multiples of 8 and buffers 16-byte aligned"), 1;
+  const long long warps = (long long)B * ((long long)(D + 2) * (H + 2) + 1);
+  launch_pdl(k_flat, (int)std::min<long long>((warps + 7) / 8, 152LL * 8), 256, 0, (cudaStream_t)stream,
+             (const __nv_bfloat16 *)src, B, D, H, W, ctot, coff, nch, Wp, (int)pstride, zero_halo, (__nv_bfloat16 *)dst);
+  slbc::count_launch();
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_flat: ") + cudaGetErrorString(e)), 1;
+  return 0;
+}
+
+int slbc_tc_wgrad_flat(const void *dyf, const void *xf, int B, int D, int H, int W, int Wp, long long pstride, int cin,
+                       int cout, float *partial, long long partial_floats, int splits, float *dw, void *stream) {
+  const std::string me = "slbc_tc_wgrad_flat";
+  WgradNArgs w;
+  if (cin % 32 || !wgrad_n_plan(cin, cout, w) || w.cc % 32)
+    return slbc::set_error(me + ": cout must be 32, 64 or 128, cin a multiple of 32"), 1;
+  const long long rows = (long long)B * pstride;
+  if (B < 1 || Wp < W + 2 || Wp % 8 || pstride % 64 || pstride < (long long)(D + 2) * (H + 2) * Wp || splits < 1 ||
+      rows >= 1LL << 31)
+    return slbc::set_error(me + ": bad geometry"), 1;
+  const long long n = 27LL * cout * cin;
+  if (partial_floats < splits * n) return slbc::set_error(me + ": partial buffer too small"), 1;
+  if (!aligned16(dyf) || !aligned16(xf) || !aligned16(partial) || !aligned16(dw))
+    return slbc::set_error(me + ": buffers must be 16-byte aligned"), 1;
+  int *err = tc_err_flag();
+  if (!err) return slbc::set_error(me + ": no device error flag"), 1;
+  w.Wp = Wp;
+  w.plane = (H + 2) * Wp;
+  w.k_tiles = rows / 64;
+  w.splits = splits;
+  w.partial = partial;
+  w.a3 = w.a_tiles = 0;
+  CUtensorMap ta, tb, win;
+  const int ch = cout == 32 ? 32 : 64;
+  if (!make_map_flat(&ta, dyf, rows, cout, ch, 72, cout / ch) || !make_map_flat(&tb, xf, rows, cin, 32, 64, w.cc / 32))
+    return slbc::set_error(me + ": tensor map encoding failed"), 1;
+  w.b4_dim0 = 0;
+  w.b4 = (w.nt == 9 || w.nt == 3) &&
+         make_map_flat_windows(&win, xf, rows, cin, w.cc / 32, Wp, w.plane, 3, w.nt / 3, w.b4_dim0);
+  if (!w.b4) win = tb;
+  static unsigned long long attr_done = 0;
+  cudaError_t e = smem_opt_in((const void *)k_wgrad_f, kWgfSmem, attr_done);
+  if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
+  const int smem = kStages * (kWgfTileA + w.n_rows * 128) + 1024;
+  launch_pdl(k_wgrad_f, dim3((unsigned)wgrad_n_ctas(w), 1, (unsigned)splits), 128, smem, (cudaStream_t)stream, ta, tb, win,
+             w, err);
+  slbc::count_launch();
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
+  launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream, partial, n,
+             splits, dw);
+  slbc::count_launch();
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
+  return 0;
 }
 
 int slbc_tc_wgrad_splits(int cin, int cout, long long k_tiles, long long max_splits) {

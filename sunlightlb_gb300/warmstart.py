@@ -51,6 +51,8 @@ class Kernels:
             "slbc_tc_wgrad": [p] * 4 + [i] * 5 + [ll, i, i, p, ll, i, p, p],
             "slbc_tc_cmajor_tiles": [p] + [i] * 8 + [ll, i, i, i, p, p],
             "slbc_tc_wgrad_tiles": [p] * 2 + [i] * 5 + [ll, i, i, p, ll, i, p, p],
+            "slbc_tc_flat": [p] + [i] * 8 + [ll, i, p, p],
+            "slbc_tc_wgrad_flat": [p] * 2 + [i] * 5 + [ll, i, i, p, ll, i, p, p],
             "slbc_nn_pool": [p, i, i, p, i, i] + [i] * 5 + [p],
             "slbc_nn_pool_bwd": [p, i, i, p, i, i, p, i, i, p, i, i] + [i] * 5 + [p],
             "slbc_nn_up": [p, i, i, p, i, i] + [i] * 5 + [p],
@@ -267,8 +269,8 @@ class UNet:
         Wp, ps = flat_geometry(self.D, self.H, self.W)
         maxc = max(c for _, c in self.buf_spec.values())
         self.cm_x = torch.empty(maxc * self.B * ps, device=self.dev, dtype=torch.bfloat16)
-        # the three x-shifted copies of an output gradient: K-tile blocks
-        # (cout <= 128), else three equally spaced channel-major copies
+        # the flat copy of an output gradient (cout <= 128), else three
+        # channel-major copies, one per x shift
         self.cm_g = torch.empty(3 * w3 * self.B * ps, device=self.dev, dtype=torch.bfloat16)
         self.ws_floats = 1 << 26
         self.ws = torch.empty(self.ws_floats, device=self.dev, dtype=torch.float32)
@@ -288,22 +290,21 @@ class UNet:
         Wp, ps = flat_geometry(d, h, w)
         g = self.grad[g_name]
         x = self.buf[x_name]
-        tiles = cout <= 128
-        n = cout * self.B * ps
-        cm_g = [self.cm_g[i * n:(i + 1) * n] for i in range(3)]
-        k.tc_cmajor_shifts(g.data_ptr(), self.B, d, h, w, g.shape[-1], 0, cout, Wp, ps, int(tiles),
-                           self.cm_g.data_ptr(), self.stream)
-        k.tc_cmajor(x.data_ptr(), self.B, d, h, w, x.shape[-1], x_coff, cin, Wp, ps, 0, 1, self.cm_x.data_ptr(),
-                    self.stream)
-        splits = k.tc_wgrad_splits(cin, cout, self.B * ps // 64, self.ws_floats // (27 * cout * cin))
         p = self.params[name]
-        if tiles:
-            k.tc_wgrad_tiles(self.cm_g.data_ptr(), self.cm_x.data_ptr(), self.B, d, h, w, Wp, ps, cin, cout,
-                             self.ws.data_ptr(), self.ws_floats, splits, p["gw"].data_ptr(), self.stream)
+        splits = k.tc_wgrad_splits(cin, cout, self.B * ps // 64, self.ws_floats // (27 * cout * cin))
+        geom = (self.B, d, h, w)
+        out = (self.ws.data_ptr(), self.ws_floats, splits, p["gw"].data_ptr(), self.stream)
+        if cout <= 128:
+            k.tc_flat(g.data_ptr(), *geom, g.shape[-1], 0, cout, Wp, ps, 0, self.cm_g.data_ptr(), self.stream)
+            k.tc_flat(x.data_ptr(), *geom, x.shape[-1], x_coff, cin, Wp, ps, 1, self.cm_x.data_ptr(), self.stream)
+            k.tc_wgrad_flat(self.cm_g.data_ptr(), self.cm_x.data_ptr(), *geom, Wp, ps, cin, cout, *out)
         else:
-            k.tc_wgrad(cm_g[0].data_ptr(), cm_g[1].data_ptr(), cm_g[2].data_ptr(), self.cm_x.data_ptr(),
-                       self.B, d, h, w, Wp, ps, cin, cout, self.ws.data_ptr(), self.ws_floats, splits,
-                       p["gw"].data_ptr(), self.stream)
+            n = cout * self.B * ps
+            cm_g = [self.cm_g[i * n:(i + 1) * n] for i in range(3)]
+            k.tc_cmajor_shifts(g.data_ptr(), *geom, g.shape[-1], 0, cout, Wp, ps, 0, self.cm_g.data_ptr(), self.stream)
+            k.tc_cmajor(x.data_ptr(), *geom, x.shape[-1], x_coff, cin, Wp, ps, 0, 1, self.cm_x.data_ptr(), self.stream)
+            k.tc_wgrad(cm_g[0].data_ptr(), cm_g[1].data_ptr(), cm_g[2].data_ptr(), self.cm_x.data_ptr(), *geom, Wp, ps,
+                       cin, cout, *out)
         p["gb"].zero_()
         k.nn_bias_grad(g.data_ptr(), g.shape[-1], 0, self.B, d, h, w, cout, p["gb"].data_ptr(), self.stream)
 
