@@ -206,47 +206,42 @@ __global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slic
   }
 }
 
-// db[c] += sum over interior voxels of g.  256 is a multiple of C / 8, so a
-// thread always handles the same 8 channels: it sums whole rows in registers,
-// the lanes of a warp with the same channels are added by shuffles, and one
-// of them adds to the block's shared sums.
+// db[c] += sum over interior voxels of g.  The grid stride is a multiple of
+// C / 8, so a thread always handles the same 8 channels: it sums in
+// registers and adds to the block's shared sums once.  I: 32-bit voxel indices
+// where they suffice (64-bit divisions per vector bounded it: 304 -> 245 us for
+// the 15 layers of a training iteration of 4 x 64^3).
+template <typename I>
 __global__ void __launch_bounds__(256) k_bias_grad(Slice g, int B, int D, int H, int W, int C, float *db) {
   after_previous();
   extern __shared__ float sh[];
-  for (int c = threadIdx.x; c < C; c += blockDim.x) sh[c] = 0.0f;
+  for (int c = threadIdx.x; c < C; c += 256) sh[c] = 0.0f;
   __syncthreads();
-  const int nv = C / 8, cv = threadIdx.x % nv, x0 = threadIdx.x / nv, dx = 256 / nv;
+  const int nv = C / 8, cv = threadIdx.x % nv;
+  const I voxels = (I)B * (I)D * (I)H * (I)W, step = (I)gridDim.x * (I)(256 / nv);
+  const bf16 *src = g.p + g.coff + 8 * cv;
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  // rows of voxels, several at a time where a row is shorter than the block's reach
-  const int per = W >= dx ? 1 : dx / W, sub = x0 / (W >= dx ? dx : W);
-  if (sub < per)
-    for (int row = (int)blockIdx.x * per + sub; row < B * D * H; row += (int)gridDim.x * per) {
-      int n, z, y;
-      row_of(row, D, H, n, z, y);
-      const bf16 *src = g.p + vox(n, z, y, 0, D, H, W) * g.ctot + g.coff + 8 * cv;
-      for (int x = W >= dx ? x0 : x0 - sub * W; x < W; x += dx) {
-        float v[8];
-        load8(src + (long long)x * g.ctot, v);
+#pragma unroll 4
+  for (I e = (I)blockIdx.x * (I)(256 / nv) + threadIdx.x / nv; e < voxels; e += step) {
+    const I row = e / (I)W, t = row / (I)H;
+    const int x = (int)(e - row * (I)W), y = (int)(row - t * (I)H), n = (int)(t / (I)D), z = (int)(t - (I)n * (I)D);
+    float v[8];
+    load8(src + vox(n, z, y, x, D, H, W) * g.ctot, v);
 #pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] += v[i];
-      }
-    }
-  for (int o = 16; o >= nv; o >>= 1)
+    for (int i = 0; i < 8; i++) acc[i] += v[i];
+  }
 #pragma unroll
-    for (int i = 0; i < 8; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-  if ((int)(threadIdx.x & 31) < nv)
-#pragma unroll
-    for (int i = 0; i < 8; i++) atomicAdd(&sh[8 * cv + i], acc[i]);
+  for (int i = 0; i < 8; i++) atomicAdd(&sh[8 * cv + i], acc[i]);
   __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(&db[c], sh[c]);
+  for (int c = threadIdx.x; c < C; c += 256) atomicAdd(&db[c], sh[c]);
 }
 
 // The optimiser's kernels take lists of tensors: a network has 30 of them, most
 // so small that a launch each (4.2 us) was most of their time.  A block takes
 // kListBlock elements of one tensor and finds it in the table of first blocks,
 // which comes with the launch.  Bound: HBM for the large tensors.  Measured on
-// the default network (5.7 M weights): Adam 126 -> 40 us, squares 120 -> 12 us,
-// layouts 128 -> 50 us in 62 launches before, 4 now.
+// the default network: Adam 126 -> 47 us, squares 120 -> 33 us, layouts about
+// 125 -> 37 us, scaling 30 launches -> 1 of 2.8 us.
 constexpr int kListMax = 48, kListBlock = 2048;
 
 struct TensorList {
@@ -869,9 +864,13 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
 
 int slbc_nn_bias_grad(const void *g, int ctot, int coff, int B, int D, int H, int W, int C, float *db, void *stream) {
   if (!ok8(ctot, coff, C) || C > 1024 || 256 % (C / 8)) return bad("slbc_nn_bias_grad: bad channel slice");
-  launch_pdl(k_bias_grad, std::min(rows_grid((long long)B * D * H, W * (C / 8)), 152 * 4), 256, C * sizeof(float),
-             (cudaStream_t)stream,
-      Slice{(bf16 *)g, ctot, coff}, B, D, H, W, C, db);
+  const long long voxels = (long long)B * D * H * W;
+  const auto go = [&](auto kernel) {
+    launch_pdl(kernel, std::min(grid_for(voxels * (C / 8)), 152 * 4), 256, C * sizeof(float), (cudaStream_t)stream,
+               Slice{(bf16 *)g, ctot, coff}, B, D, H, W, C, db);
+  };
+  if (voxels < (1LL << 31)) go(k_bias_grad<unsigned>);  // the grid's stride may go past the end
+  else go(k_bias_grad<unsigned long long>);
   return launched("slbc_nn_bias_grad");
 }
 

@@ -396,8 +396,8 @@ __device__ __forceinline__ void conv_rows_out(const ConvArgs &a, uint32_t acc, l
   }
 }
 
-// Convolution of 32 and 64 output channels (and of 32 to 96, the input gradient
-// of the finest level's first decoder layer), one persistent block per SM, every
+// Convolution of 32, 64 and, as two parts of 64, 128 output channels (and of 32
+// to 96), one persistent block per SM, every
 // input voxel staged once per 32-channel chunk.  An output item is 8 (x) x 16
 // (y) x up to S (z) voxels; input planes of 10 x 18 voxels (64-byte rows, x
 // fastest, halo included) go through a ring in shared memory, one TMA box
@@ -421,6 +421,10 @@ __device__ __forceinline__ void conv_rows_out(const ConvArgs &a, uint32_t acc, l
 // -> 32 1300 TFLOP/s; 64^3: 64 -> 64 channels 60 -> 44 us (1320 TFLOP/s); before,
 // a stage held the input block of one x-shift (three times the copies), the
 // issuing thread was slower than the tensor core, and a tile had 2 or 4 slices.
+// 128 channels in two parts: the six layers on 4 x 16^3 of a training iteration
+// 190 -> 125 us (64 tiles of two slices were less than half of the SMs).
+// 32 -> 96 at 4 x 64^3: 280 -> 116 us (k_conv_fwd before, whose order of
+// products, dz, dy, dx, it keeps).
 template <int COUT>
 struct ConvR {
   static constexpr int kS = 256 / COUT;                // slices of an item, at most
@@ -475,7 +479,8 @@ struct ConvRIssue {
 #pragma unroll
         for (int t = 0; t < 18; t++) {
           const int dy = t / 6, dx = t / 2 % 3, kk = t % 2;
-          const uint32_t at = az + (uint32_t)(dy * 40 + dx * 4 + 2 * kk), bt = bz + (uint32_t)(dx * stage + dy * 3 * tap + 2 * kk);
+          const uint32_t at = az + (uint32_t)(dy * 40 + dx * 4 + 2 * kk);
+          const uint32_t bt = bz + (uint32_t)(dx * stage + dy * 3 * tap + 2 * kk);
           if (t == 0 && lo == 0) {
             // the first product of the last of these slices (dz = 0) overwrites it
             if (hi > 0) mma(d, at, bt, tc::idesc_bf16(128, hi * COUT), 1);
@@ -551,7 +556,7 @@ struct ConvRIssue {
 template <int COUT>
 __global__ void __launch_bounds__(192, 1)
 k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tw, ConvArgs a, int runs,
-         int items, int *err) {
+         int items, int parts, int *err) {
   after_previous();
   using C = ConvR<COUT>;
   constexpr int NB = C::kStagesB, NP = C::kPlanes;
@@ -561,7 +566,7 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   uint8_t *const tB = smem_raw + pad, *const tA = tB + NB * C::kTileB;
   __shared__ uint64_t full_b[NB], empty_b[NB], full_p[NP], empty_p[NP], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base;
-  __shared__ float bias[COUT];
+  __shared__ float bias[128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_x = a.W / 8, tiles_y = a.H / 16, cols = tiles_x * tiles_y;
   const int nck = a.cin / 32;
@@ -585,13 +590,14 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
     }
     tc::fence_mbar_init();
   }
-  for (int c = threadIdx.x; c < COUT; c += 192) bias[c] = a.bias ? a.bias[c] : 0.0f;
+  for (int c = threadIdx.x; c < a.cout; c += 192) bias[c] = a.bias ? a.bias[c] : 0.0f;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = tmem_base;
   bool ok = true;
-  // first slice and number of slices of an item; a column is cut into `runs` almost equal runs
+  // an item is a part of the output channels of a tile; first slice and number
+  // of slices of a tile: a column is cut into `runs` almost equal runs
   const auto slices = [&](int item, int &z0) {
     const int run = (item / cols) % runs;
     z0 = run * a.D / runs;
@@ -599,24 +605,25 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   };
   if (warp == 0 && tc::elect_one()) {  // copies
     int nb = 0, np = 0;    // weight stages and planes issued
-    const auto load_b = [&](int ck, int dx) {
+    const auto load_b = [&](int ck, int dx, int part) {
       const int s = nb % NB;
       if (nb >= NB && !tc::mbar_wait(&empty_b[s], (uint32_t)(nb / NB - 1) & 1u, kWaitLimit)) return false;
       tc::mbar_expect_tx(&full_b[s], (uint32_t)C::kTileB);
       for (int dy = 0; dy < 3; dy++)
         for (int dz = 0; dz < 3; dz++)
           tc::tma_load_2d(tB + s * C::kTileB + (dy * 3 + 2 - dz) * tap_b, &tw, &full_b[s], 0,
-                          ((dz * 9 + dy * 3 + dx) * nck + ck) * COUT);
+                          ((dz * 9 + dy * 3 + dx) * nck + ck) * a.cout + part * COUT);
       nb++;
       return true;
     };
-    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+    for (int work = blockIdx.x; work < items * parts && ok; work += gridDim.x) {
+      const int item = work / parts, part = work - item * parts;
       const int x0 = (item % tiles_x) * 8, y0 = ((item / tiles_x) % tiles_y) * 16, n = item / (cols * runs);
       int z0;
       const int len = slices(item, z0);
-      const bool with_b = !keep_b || item == (int)blockIdx.x;
+      const bool with_b = !keep_b || work == (int)blockIdx.x;
       for (int ck = 0; ck < nck && ok; ck++) {
-        if (with_b) ok = load_b(ck, 0);
+        if (with_b) ok = load_b(ck, 0, part);
         for (int zi = 0; zi < len + 2 && ok; zi++) {
           const int s = np % NP;
           if (np >= NP && !tc::mbar_wait(&empty_p[s], (uint32_t)(np / NP - 1) & 1u, kWaitLimit)) {
@@ -628,8 +635,8 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
           tc::tma_load_5d(tA + s * C::kPlane, &tx, &full_p[s], a.in_coff + ck * 32, x0, y0, z0 + zi, n);
           np++;
         }
-        if (with_b && ok) ok = load_b(ck, 1);
-        if (with_b && ok) ok = load_b(ck, 2);
+        if (with_b && ok) ok = load_b(ck, 1, part);
+        if (with_b && ok) ok = load_b(ck, 2, part);
       }
     }
     // the copies issued have landed before the block ends
@@ -644,10 +651,10 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
     m.full_b = full_b; m.empty_b = empty_b; m.full_p = full_p; m.empty_p = empty_p;
     m.keep_b = keep_b;
     int g = 0;
-    for (int item = blockIdx.x; item < items && m.limit; item += gridDim.x, g++) {
+    for (int work = blockIdx.x; work < items * parts && m.limit; work += gridDim.x, g++) {
       const int set = g & 1;
       int z0;
-      const int len = slices(item, z0);
+      const int len = slices(work / parts, z0);
       m.with_b = !keep_b || g == 0;
       if (g >= 2) m.wait(&acc_empty[set], (uint32_t)((g >> 1) - 1) & 1u);
       tc::fence_after_sync();
@@ -676,8 +683,8 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   } else if (warp >= 2) {  // accumulators to memory
     const int quarter = warp & 3, row = quarter * 32 + lane;
     int g = 0;
-    for (int item = blockIdx.x; item < items; item += gridDim.x, g++) {
-      const int set = g & 1;
+    for (int work = blockIdx.x; work < items * parts; work += gridDim.x, g++) {
+      const int set = g & 1, item = work / parts, co0 = (work - item * parts) * COUT;
       int z0;
       const int len = slices(item, z0);
       ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[set], (uint32_t)(g >> 1) & 1u, kWaitLimit));
@@ -689,7 +696,7 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
       for (int sl = 0; sl < len; sl++) {
         const long long vox = (((long long)n * (a.D + 2) + z0 + sl + 1) * (a.H + 2) + vy + 1) * (a.W + 2) + vx + 1;
         conv_rows_out<COUT>(a, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(set * C::kSet + sl * COUT),
-                            vox * a.out_ctot + a.out_coff, bias);
+                            vox * a.out_ctot + a.out_coff + co0, bias + co0);
       }
       tc::fence_before_sync();
       __syncwarp();
@@ -703,16 +710,15 @@ k_conv_r(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtenso
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
 }
 
-// Convolution of 128 output channels (and of 32 and 64 on grids 8 high),
-// one persistent block per SM.  An output tile is 16 (x) x 8 (y) x 2 (z)
-// voxels.  For each 32-channel chunk and each x-shift dx, one 5-D TMA
+// Convolution of 32, 64 or 128 output channels on grids 8 high (y), where
+// k_conv_r's tiles do not fit, in its order of products; one persistent block
+// per SM.  An output tile is 16 (x) x 8 (y) x 2 (z) voxels.  For each 32-channel chunk and each x-shift dx, one 5-D TMA
 // box brings the input block x0+dx .. x0+dx+15, y0-1 .. y0+8, z0-1 .. z0+2
 // (rows of 64 B, x fastest) into shared memory, with the weights of the nine
 // taps of that dx.  The 128 rows of input plane zi shifted by dy start at row
 // (zi * 10 + dy) * 16.  Two accumulator sets alternate between tiles, so four
 // warps convert and write tile t while the copies and MMAs of tile t + 1 run.
-// 128 -> 128 channels: bound by the weights' way into shared memory (74 KB
-// per 2300 cycles of MMAs).
+// Bound: operand staging.
 template <int COUT>
 struct ConvZ {
   static constexpr int S = 2;
@@ -1857,43 +1863,45 @@ static int conv3d(const void *in, int B, int D, int H, int W, int in_ctot, int i
   a.mask = (const __nv_bfloat16 *)mask;
   a.out = out_f32 ? nullptr : (__nv_bfloat16 *)out;
   a.out_f32 = out_f32;
-  if ((cout == 32 || cout == 64 || (cout == 96 && cin == 32)) && W % 8 == 0 && H % 16 == 0) {
+  if ((cout == 32 || cout == 64 || cout == 128 || (cout == 96 && cin == 32)) && W % 8 == 0 && H % 16 == 0) {
     // A column of 8 x 16 voxels is cut into runs along z.  Fewer, longer runs
     // read fewer halo planes; the count is the one whose busiest block has the
     // least work, in MMA cycles per chunk and tap pair: 32 per input plane (its
     // A rows) and cout / 4 per slice and dz (the weights).
-    const int cols = (W / 8) * (H / 16), most = 256 / cout;
+    const int parts = cout == 128 ? 2 : 1, co = cout / parts;  // output channels in parts of `co`
+    const int cols = (W / 8) * (H / 16), most = 256 / co;
     int runs = (D + most - 1) / most;
     double best = 0.0;
     for (int k = runs; k <= D; k++) {
       const double len = (double)D / k;
-      const double work = (double)(((long long)cols * k * B + kConvSms - 1) / kConvSms) * (32.0 * (len + 2.0) + 0.75 * cout * len);
+      const long long rounds = ((long long)cols * k * B * parts + kConvSms - 1) / kConvSms;
+      const double work = (double)rounds * (32.0 * (len + 2.0) + 0.75 * co * len);
       if (k == runs || work < best) {
         best = work;
         runs = k;
       }
     }
     CUtensorMap th;
-    if (!make_map_act(&th, in, B, D, H, W, in_ctot, 10, 18, 1))
+    if (!make_map_act(&th, in, B, D, H, W, in_ctot, 10, 18, 1) ||
+        !make_map_rows32(&tw, wgt, 27LL * (cin / 32) * cout, co))
       return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
     const int items = cols * runs * B;
     static unsigned long long attr_r[3] = {0, 0, 0};
     const auto go = [&](auto kernel, int smem, int slot) {
       cudaError_t e = smem_opt_in((const void *)kernel, smem, attr_r[slot]);
       if (e != cudaSuccess) return e;
-      launch_pdl(kernel, std::min(items, kConvSms), 192, smem, (cudaStream_t)stream, th, tw, a, runs, items, err);
+      launch_pdl(kernel, std::min(items * parts, kConvSms), 192, smem, (cudaStream_t)stream, th, tw, a, runs, items,
+                 parts, err);
       slbc::count_launch();
       return cudaGetLastError();
     };
-    const cudaError_t e = cout == 32   ? go(k_conv_r<32>, ConvR<32>::kSmem, 0)
-                          : cout == 64 ? go(k_conv_r<64>, ConvR<64>::kSmem, 1)
-                                       : go(k_conv_r<96>, ConvR<96>::kSmem, 2);
+    const cudaError_t e = co == 32   ? go(k_conv_r<32>, ConvR<32>::kSmem, 0)
+                          : co == 64 ? go(k_conv_r<64>, ConvR<64>::kSmem, 1)
+                                     : go(k_conv_r<96>, ConvR<96>::kSmem, 2);
     if (e != cudaSuccess) return slbc::set_error(std::string("slbc_tc_conv3d: ") + cudaGetErrorString(e)), 1;
     return 0;
   }
   if ((cout == 32 || cout == 64 || cout == 128) && W % 16 == 0 && H % 8 == 0 && D % 2 == 0) {
-    // 128 output channels, whose accumulator sets of two slices fill the TMEM
-    // and whose weights fill the ring's memory, and grids 8 high.
     CUtensorMap th;
     if (!make_map_act(&th, in, B, D, H, W, in_ctot, 16, 10, 4))
       return slbc::set_error("slbc_tc_conv3d: tensor map encoding failed"), 1;
