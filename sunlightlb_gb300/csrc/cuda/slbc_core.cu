@@ -27,11 +27,13 @@ struct slbc_lattice {
   std::vector<unsigned char> solid_host;  // solidity per node, for body-force checks
 };
 
+constexpr int kFillBlocks = 152 * 4;  // blocks of a tracer fill, at most
+
 struct slbc_tracer {
   slbc_lattice *h = nullptr;
   int f64 = 1;
   void *p = nullptr, *p2 = nullptr;
-  double *acc = nullptr;  // tracer added by fills since creation or the last reset; the fills' block counter
+  double *acc = nullptr;  // tracer added by fills since creation or the last reset, a slot per block (kFillBlocks)
   double *objstate = nullptr;
   int objstate_cap = 0;
   // FP32 tracers: the low part of p (p = hi + lo, |lo| <= half an FP32 ulp
@@ -295,17 +297,17 @@ __device__ __forceinline__ long long plane_node(long long e, int axis, int pos, 
 
 // Tracer injection on the fluid nodes of a region (reference src/mpobjs.c).
 // Kind 2 (a wall) visits only the nodes of its plane and needs no
-// coordinates.  Each block leaves the sum of (value - old p) over the nodes
-// it set; the last block to finish adds them to acc[0] in block order, so the
-// host layer can keep count of the tracer the fills have added (a second
-// launch for that sum cost as much as the fill of a plane: a source and an
-// absorbing plane of a 256^3 lattice set again every update took 21 of its
-// 255 us).  done: a counter, zero before and after.
+// coordinates.  Each block adds the sum of (value - old p) over the nodes it
+// set to its own slot of acc, so the host layer can keep count of the tracer
+// the fills have added (slbc_mp_injected adds the slots in order).  Bound:
+// latency; flags and values are loaded together, and no block waits for
+// another.  Measured, a plane of 256^3 on a frozen flow: 10.3 -> 8.2 us, where a
+// last block added the blocks' sums behind a fence and a counter (before that,
+// in a launch of its own).
 template <typename TP>
 __global__ void __launch_bounds__(kReduceThreads)
 k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, int kind, double g0, double g1,
-          double g2, double g3, double g4, double g5, double value, int count, double *partials, unsigned *done,
-          double *acc) {
+          double g2, double g3, double g4, double g5, double value, int count, double *acc) {
   after_previous();
   double v[1] = {0.0};
   const TP nv = (TP)value;
@@ -317,7 +319,10 @@ k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, in
       else if (axis == 1) x = ((e / esk) * esj + pos) * esk + e % esk;
       else x = e * esk + pos;
     }
-    if (flags[x] & FLAG_SOLID) continue;
+    const uint16_t fl = flags[x];
+    const TP old = p[x];
+    const float old_lo = lo ? lo[x] : 0.0f;
+    if (fl & FLAG_SOLID) continue;
     bool in = true;
     if (kind == 1 || kind == 3 || kind == 4) {
       const int k = x % esk, r = x / esk, j = r % esj, i = r / esj;
@@ -335,29 +340,13 @@ k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, in
       }
     }
     if (in) {
-      v[0] += (double)nv - (double)p[x] - (lo ? (double)lo[x] : 0.0);
+      v[0] += (double)nv - (double)old - (double)old_lo;
       p[x] = nv;
       if (lo) lo[x] = 0.0f;
     }
   }
   block_sum<1>(v);
-  __shared__ bool last;
-  if (threadIdx.x == 0) {
-    partials[blockIdx.x] = v[0];
-    __threadfence();
-    last = atomicAdd(done, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  v[0] = 0.0;
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) v[0] += __ldcg(partials + b);
-  __syncthreads();
-  block_sum<1>(v);
-  if (threadIdx.x == 0) {
-    acc[0] += v[0];
-    *done = 0u;
-  }
+  if (threadIdx.x == 0) acc[blockIdx.x] += v[0];
 }
 
 // sum of p and number of fluid nodes on one plane
@@ -1593,8 +1582,8 @@ int slbc_mp_create(slbc_lattice *h, slbc_tracer **out, int use_f64) {
   if (e == cudaSuccess) e = cudaMemsetAsync(t->p2, 0, (size_t)L.nnodes * es, L.stream);
   if (e == cudaSuccess && !use_f64) e = cudaMalloc(&t->lo, (size_t)L.nnodes * sizeof(float));
   if (e == cudaSuccess && !use_f64) e = cudaMalloc(&t->lo2, (size_t)L.nnodes * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&t->acc, 2 * sizeof(double));
-  if (e == cudaSuccess) e = cudaMemsetAsync(t->acc, 0, 2 * sizeof(double), L.stream);
+  if (e == cudaSuccess) e = cudaMalloc(&t->acc, kFillBlocks * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemsetAsync(t->acc, 0, kFillBlocks * sizeof(double), L.stream);
   if (e == cudaSuccess && !L.mp_rho64) {
     e = cudaMalloc(&L.mp_rho64, (size_t)L.nnodes * sizeof(double));
     if (e == cudaSuccess) {
@@ -1840,16 +1829,13 @@ int slbc_mp_fill(slbc_tracer *t, int kind, const double *geo, double value) {
     if (axis < 0 || axis > 2 || pos < 0 || pos >= lim) return fail_msg("slbc_mp_fill: wall outside the lattice");
     count = plane_size(L, axis);
   }
-  const int nb = (int)std::max<long long>(1, std::min<long long>(blocks_for(count, kReduceThreads), 152 * 4));
-  if (ensure_partials(L, nb + 8)) return 1;
-  unsigned *done = (unsigned *)(t->acc + 1);
+  const int nb = (int)std::max<long long>(1, std::min<long long>(blocks_for(count, kReduceThreads), kFillBlocks));
   if (t->f64)
     launch_pdl(k_mp_fill<double>, nb, kReduceThreads, 0, L.stream, (double *)t->p, nullptr, L.flags, L.esi, L.esj,
-               L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, L.partials, done, t->acc);
+               L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, t->acc);
   else
     launch_pdl(k_mp_fill<float>, nb, kReduceThreads, 0, L.stream, (float *)t->p, t->lo_live ? t->lo : nullptr,
-               L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count,
-               L.partials, done, t->acc);
+               L.flags, L.esi, L.esj, L.esk, kind, g[0], g[1], g[2], g[3], g[4], g[5], value, (int)count, t->acc);
   count_launch();
   CK(cudaGetLastError());
   return 0;
@@ -1857,11 +1843,12 @@ int slbc_mp_fill(slbc_tracer *t, int kind, const double *geo, double value) {
 
 int slbc_mp_injected(slbc_tracer *t, int reset, double *out) {
   Lattice &L = t->h->L;
-  double v = 0.0;
-  CK(cudaMemcpyAsync(&v, t->acc, sizeof(double), cudaMemcpyDeviceToHost, L.stream));
+  double slot[kFillBlocks], v = 0.0;
+  CK(cudaMemcpyAsync(slot, t->acc, sizeof slot, cudaMemcpyDeviceToHost, L.stream));
   CK(cudaStreamSynchronize(L.stream));
+  for (int b = 0; b < kFillBlocks; b++) v += slot[b];
   if (out) *out = v;
-  if (reset) CK(cudaMemsetAsync(t->acc, 0, sizeof(double), L.stream));
+  if (reset) CK(cudaMemsetAsync(t->acc, 0, sizeof slot, L.stream));
   return 0;
 }
 
