@@ -311,7 +311,8 @@ k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, in
   after_previous();
   double v[1] = {0.0};
   const TP nv = (TP)value;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
+  grid_turns(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, (unsigned)count, [&](unsigned turn) {
+    const int e = (int)turn;
     int x = e;
     if (kind == 2) {
       const int axis = (int)g0, pos = (int)g1;
@@ -322,8 +323,8 @@ k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, in
     const uint16_t fl = flags[x];
     const TP old = p[x];
     const float old_lo = lo ? lo[x] : 0.0f;
-    if (fl & FLAG_SOLID) continue;
-    bool in = true;
+    if (fl & FLAG_SOLID) return;
+    bool in = kind == 0 || kind == 2;
     if (kind == 1 || kind == 3 || kind == 4) {
       const int k = x % esk, r = x / esk, j = r % esj, i = r / esj;
       if (kind == 1) {
@@ -344,7 +345,7 @@ k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, in
       p[x] = nv;
       if (lo) lo[x] = 0.0f;
     }
-  }
+  });
   block_sum<1>(v);
   if (threadIdx.x == 0) acc[blockIdx.x] += v[0];
 }
