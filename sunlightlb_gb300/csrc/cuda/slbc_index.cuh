@@ -20,6 +20,48 @@ SLBC_HD void grid_turns(unsigned first, unsigned step, unsigned count, F f) {
   for (unsigned e = first; e < count; e += step) f(e);
 }
 
+// The kernels over voxels walk the grid row by row (a row: W voxels times the
+// 16-byte vectors of a voxel): a block of 256 threads takes one long row or
+// several short ones at a time, so a thread divides once per row instead of
+// four times per vector.  I: unsigned below 2^31 rows (row + step does not
+// wrap), unsigned long long above.
+template <typename I>
+struct RowWalk {
+  I row, step;  // first row of this thread, rows between its turns
+  unsigned e;   // first element in the row
+};
+
+template <typename I>
+SLBC_HD RowWalk<I> row_walk(unsigned block, unsigned blocks, unsigned thread, unsigned rowlen) {
+  RowWalk<I> w;
+  if (rowlen >= 256) {
+    w.row = block;
+    w.step = blocks;
+    w.e = thread;
+  } else {
+    const unsigned per = 256 / rowlen, sub = thread / rowlen;
+    w.e = thread - sub * rowlen;
+    w.row = sub < per ? (I)block * per + sub : ~(I)0;  // past every row
+    w.step = (I)blocks * per;
+  }
+  return w;
+}
+
+// Blocks for `rows` rows of `rowlen` (>= 1) elements
+inline int rows_grid(long long rows, long long rowlen) {
+  const long long per = rowlen >= 256 ? 1 : 256 / rowlen, blocks = (rows + per - 1) / per;
+  return (int)(blocks < 1 ? 1 : blocks > 152LL * 16 ? 152LL * 16 : blocks);
+}
+
+// The sample n, plane z and line y of a row of B x D x H
+template <typename I>
+SLBC_HD void row_of(I row, int D, int H, int &n, int &z, int &y) {
+  const I t = row / (I)H;
+  y = (int)(row - t * (I)H);
+  n = (int)(t / (I)D);
+  z = (int)(t - (I)n * (I)D);
+}
+
 }  // namespace slbc
 
 #endif

@@ -18,6 +18,8 @@ namespace {
 
 using slbc::after_previous;
 using slbc::launch_pdl;
+using slbc::row_of;
+using slbc::rows_grid;
 
 typedef __nv_bfloat16 bf16;
 
@@ -51,60 +53,39 @@ __device__ __forceinline__ void store8(bf16 *p, const float (&v)[8]) {
 
 int grid_for(long long n) { return (int)std::min<long long>((n + 255) / 256, 152LL * 32); }
 
-// The kernels over voxels walk the grid row by row (a row: W voxels times the
-// 16-byte vectors of a voxel): a block takes one long row or several short
-// ones at a time, so a thread divides once per row in 32 bits instead of four
-// times per vector in 64 bits, which bounded these kernels at a third to a
-// fifth of the memory rate.
-struct RowWalk {
-  int row, step, e;  // first row of this thread, rows between its turns, first element in the row
-};
-
-__device__ __forceinline__ RowWalk row_walk(int rowlen) {
-  RowWalk w;
-  if (rowlen >= 256) {
-    w.row = blockIdx.x;
-    w.step = gridDim.x;
-    w.e = threadIdx.x;
-  } else {
-    const int per = 256 / rowlen, sub = (int)threadIdx.x / rowlen;
-    w.e = (int)threadIdx.x - sub * rowlen;
-    w.row = sub < per ? (int)blockIdx.x * per + sub : 0x7fffffff;
-    w.step = (int)gridDim.x * per;
-  }
-  return w;
+// A row walk and its row counts in 32 bits where the rows fit it (64-bit
+// divisions per vector bounded these kernels at a third to a fifth of the
+// memory rate), else in 64: go(I()) launches the kernel for that index type.
+template <typename F>
+void for_rows(long long rows, F go) {
+  if (rows < (1LL << 31)) go(0u);
+  else go(0ull);
 }
 
-int rows_grid(long long rows, int rowlen) {
-  const int per = rowlen >= 256 ? 1 : 256 / rowlen;
-  return (int)std::max<long long>(1, std::min<long long>((rows + per - 1) / per, 152LL * 16));
-}
-
-__device__ __forceinline__ void row_of(int row, int D, int H, int &n, int &z, int &y) {
-  const int t = row / H;
-  y = row - t * H;
-  n = t / D;
-  z = t - n * D;
+template <typename I>
+__device__ __forceinline__ slbc::RowWalk<I> walk(int rowlen) {
+  return slbc::row_walk<I>(blockIdx.x, gridDim.x, threadIdx.x, (unsigned)rowlen);
 }
 
 // 2x2x2 average of the fine interior (D, H, W) into the coarse interior
+template <typename I>
 __global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const RowWalk w = row_walk(len);
-  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+  const auto w = walk<I>(len);
+  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
     int n, z, y;
     row_of(row, Dc, Hc, n, z, y);
     const bf16 *src = in.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * in.ctot + in.coff;
     bf16 *dst = out.p + vox(n, z, y, 0, Dc, Hc, Wc) * out.ctot + out.coff;
     const long long py = (long long)(W + 2) * in.ctot, pz = (H + 2) * py;
-    for (int e = w.e; e < len; e += 256) {
-      const int x = e / nv, cv = e - x * nv;
+    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+      const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
       for (int c = 0; c < 8; c++) {
         float v[8];
-        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * in.ctot + 8 * cv, v);
+        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2LL * x + (c & 1)) * in.ctot + 8 * cv, v);
 #pragma unroll
         for (int i = 0; i < 8; i++) acc[i] += v[i];
       }
@@ -117,18 +98,19 @@ __global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D,
 
 // gradient of k_pool: dfine = (dcoarse / 8 + add) * (mask > 0); add and mask
 // optional (null pointers)
+template <typename I>
 __global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Slice add, Slice mask, int B, int D,
                                                   int H, int W, int C) {
   after_previous();
   const int nv = C / 8, len = W * nv;
-  const RowWalk w = row_walk(len);
-  for (int row = w.row; row < B * D * H; row += w.step) {
+  const auto w = walk<I>(len);
+  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
     int n, z, y;
     row_of(row, D, H, n, z, y);
     const bf16 *src = dcoarse.p + vox(n, z / 2, y / 2, 0, D / 2, H / 2, W / 2) * dcoarse.ctot + dcoarse.coff;
     const long long v0 = vox(n, z, y, 0, D, H, W);
-    for (int e = w.e; e < len; e += 256) {
-      const int x = e / nv, cv = e - x * nv;
+    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+      const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float g[8];
       load8(src + (long long)(x / 2) * dcoarse.ctot + 8 * cv, g);
 #pragma unroll
@@ -153,44 +135,46 @@ __global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Sl
 
 // nearest upsampling: fine (D, H, W) interior = coarse parent; a thread
 // reads its vector of the parent once and writes the eight children
+template <typename I>
 __global__ void __launch_bounds__(256) k_up(Slice in, Slice out, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const RowWalk w = row_walk(len);
-  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+  const auto w = walk<I>(len);
+  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
     int n, z, y;
     row_of(row, Dc, Hc, n, z, y);
     const bf16 *src = in.p + vox(n, z, y, 0, Dc, Hc, Wc) * in.ctot + in.coff;
     bf16 *dst = out.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * out.ctot + out.coff;
     const long long py = (long long)(W + 2) * out.ctot, pz = (H + 2) * py;
-    for (int e = w.e; e < len; e += 256) {
-      const int x = e / nv, cv = e - x * nv;
+    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+      const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       const uint4 v = *(const uint4 *)(src + (long long)x * in.ctot + 8 * cv);
 #pragma unroll
       for (int c = 0; c < 8; c++)
-        *(uint4 *)(dst + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * out.ctot + 8 * cv) = v;
+        *(uint4 *)(dst + (c >> 2) * pz + ((c >> 1) & 1) * py + (2LL * x + (c & 1)) * out.ctot + 8 * cv) = v;
     }
   }
 }
 
 // gradient of k_up: dcoarse = sum of the 8 children * (mask > 0) (coarse mask)
+template <typename I>
 __global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slice mask, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const RowWalk w = row_walk(len);
-  for (int row = w.row; row < B * Dc * Hc; row += w.step) {
+  const auto w = walk<I>(len);
+  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
     int n, z, y;
     row_of(row, Dc, Hc, n, z, y);
     const bf16 *src = dfine.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * dfine.ctot + dfine.coff;
     const long long py = (long long)(W + 2) * dfine.ctot, pz = (H + 2) * py;
     const long long v0 = vox(n, z, y, 0, Dc, Hc, Wc);
-    for (int e = w.e; e < len; e += 256) {
-      const int x = e / nv, cv = e - x * nv;
+    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+      const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
       for (int c = 0; c < 8; c++) {
         float v[8];
-        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2 * x + (c & 1)) * dfine.ctot + 8 * cv, v);
+        load8(src + (c >> 2) * pz + ((c >> 1) & 1) * py + (2LL * x + (c & 1)) * dfine.ctot + 8 * cv, v);
 #pragma unroll
         for (int i = 0; i < 8; i++) acc[i] += v[i];
       }
@@ -374,6 +358,7 @@ __global__ void __launch_bounds__(256) k_scale(const __grid_constant__ TensorLis
 // in FP32 channels 0..nch-1 of a padded buffer (ctot_p channels), label
 // [n][D][H][W][nch] FP32; grad (BF16, gctot channels, padded) = d loss /
 // d pred in channels 0..nch-1, 0 in the others.  loss[0] += the sum / count.
+template <typename I>
 __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, const float *label, int nch,
                                              const float *sample_w, int B, int D, int H, int W, bf16 *grad, int gctot,
                                              double *loss) {
@@ -381,13 +366,14 @@ __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, cons
   __shared__ double sh[256];
   const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   double acc = 0.0;
-  const RowWalk w = row_walk(W);
-  for (int row = w.row; row < B * D * H; row += w.step) {
+  const auto w = walk<I>(W);
+  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
     int n, z, y;
     row_of(row, D, H, n, z, y);
     const long long v0 = vox(n, z, y, 0, D, H, W), e0 = (long long)row * W;
     const float sw = sample_w ? sample_w[n] : 1.0f;
-    for (int x = w.e; x < W; x += 256) {
+    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
+      const int x = (int)turn;
       const long long v = v0 + x;
       bf16 *gp = grad + v * gctot;
       for (int c = 0; c < gctot; c += 8) *(uint4 *)(gp + c) = make_uint4(0, 0, 0, 0);
@@ -473,14 +459,15 @@ constexpr int kDistR1 = 5, kDistR2 = 12;
 // 2R + 1 neighbours instead of (2R + 1)^3.  Values stay integers, so the
 // result equals the cube search.
 // Pass 1 (along x): nearest solid node on the row, searched outwards.
-template <int R>
-__global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int rows, int W, unsigned char *a) {
+template <int R, typename I>
+__global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, I rows, int W, unsigned char *a) {
   after_previous();
-  const RowWalk w = row_walk(W);
-  for (int row = w.row; row < rows; row += w.step) {
+  const auto w = walk<I>(W);
+  for (I row = w.row; row < rows; row += w.step) {
     const unsigned char *src = solid + (long long)row * W;
     unsigned char *dst = a + (long long)row * W;
-    for (int x = w.e; x < W; x += 256) {
+    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
+      const int x = (int)turn;
       int best = src[x] ? 0 : R * R;
       if (W >= R) {
         for (int d = 1; d < R && best == R * R; d++) {
@@ -507,13 +494,14 @@ __global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, int 
 // plane.
 constexpr int kDistRun = 4;
 
-template <int R, int VEC>
-__global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int outers, int n, int inner, unsigned char *b) {
+template <int R, int VEC, typename I>
+__global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int outers, int n, long long inner,
+                                                  unsigned char *b) {
   after_previous();
-  const unsigned len = (unsigned)inner / VEC, groups = (unsigned)(n + kDistRun - 1) / kDistRun;
-  const unsigned total = (unsigned)outers * groups * len;
-  for (unsigned i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
-    const unsigned row = i / len, e = i - row * len, outer = row / groups;
+  const I len = (I)inner / VEC, groups = (I)(n + kDistRun - 1) / kDistRun;
+  const I total = (I)outers * groups * len;
+  for (I i = (I)blockIdx.x * 256u + threadIdx.x; i < total; i += (I)gridDim.x * 256u) {
+    const I row = i / len, e = i - row * len, outer = row / groups;
     const int p0 = (int)(row - outer * groups) * kDistRun;
     const unsigned char *base = a + (long long)outer * n * inner + VEC * e;
     unsigned lo[kDistRun], hi[kDistRun];
@@ -547,18 +535,19 @@ __global__ void __launch_bounds__(256) k_dist_min(const unsigned char *a, int ou
 
 // dist2: the squared distances of the passes above (null without features),
 // searched to radius R
+template <typename I>
 __global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, const unsigned char *dist2, int R, int B,
                                                 int D, int H, int W, bf16 *out, int ctot) {
   after_previous();
   const int nv = ctot / 8, len = W * nv;
-  const RowWalk w = row_walk(len);
-  for (int row = w.row; row < B * D * H; row += w.step) {
+  const auto w = walk<I>(len);
+  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
     int n, z, y;
     row_of(row, D, H, n, z, y);
     bf16 *dst = out + vox(n, z, y, 0, D, H, W) * ctot;
     const long long e0 = (long long)row * W;
-    for (int e = w.e; e < len; e += 256) {
-      const int x = e / nv, cv = e - x * nv;
+    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+      const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       uint4 u = make_uint4(0, 0, 0, 0);
       if (cv == 0) {
         bf16 *p = (bf16 *)&u;
@@ -581,17 +570,19 @@ __global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, cons
 // nodes into three FP32 arrays u[c * N + e] (0 on solid nodes), the layout
 // of lbsetveldev; shift_x is subtracted from u_x on fluid nodes.  With
 // drho, channel 3 * drho_scale into drho[e] (0 on solid nodes).
+template <typename I>
 __global__ void __launch_bounds__(256) k_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H,
                                                 int W, float scale, float shift_x, float *u, float drho_scale,
                                                 float *drho) {
   after_previous();
   const long long total = (long long)D * H * W;
-  const RowWalk w = row_walk(W);
-  for (int row = w.row; row < D * H; row += w.step) {
+  const auto w = walk<I>(W);
+  for (I row = w.row; row < (I)D * (I)H; row += w.step) {
     int n, z, y;
     row_of(row, D, H, n, z, y);
     const float *src = pred + vox(0, z, y, 0, D, H, W) * ctot_p;
-    for (int x = w.e; x < W; x += 256) {
+    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
+      const int x = (int)turn;
       const long long e = (long long)row * W + x;
       const float *v = src + (long long)x * ctot_p;
       const bool s = solid[e] != 0;
@@ -779,6 +770,8 @@ __global__ void k_cross_apply(float *u, int D, int H, int W, const double *work)
 
 bool ok8(int ctot, int coff, int C) { return ctot % 8 == 0 && coff % 8 == 0 && C % 8 == 0 && C > 0 && coff + C <= ctot; }
 
+bool empty(int B, int D, int H, int W) { return B < 1 || D < 1 || H < 1 || W < 1; }
+
 int launched(const char *what) {
   slbc::count_launch();
   const cudaError_t e = cudaGetLastError();
@@ -822,9 +815,12 @@ int slbc_nn_pool(const void *in, int in_ctot, int in_coff, void *out, int out_ct
                  int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool: channel slices must be multiples of 8 and the grid even");
-  launch_pdl(k_pool, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
-             Slice{(bf16 *)in, in_ctot, in_coff},
-                                                        Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
+  if (empty(B, D, H, W)) return bad("slbc_nn_pool: empty grid");
+  const long long rows = (long long)B * (D / 2) * (H / 2);
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_pool<decltype(i)>, rows_grid(rows, (long long)(W / 2) * (C / 8)), 256, 0, (cudaStream_t)stream,
+               Slice{(bf16 *)in, in_ctot, in_coff}, Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
+  });
   return launched("slbc_nn_pool");
 }
 
@@ -834,9 +830,13 @@ int slbc_nn_pool_bwd(const void *dcoarse, int dc_ctot, int dc_coff, void *dfine,
   if (!ok8(dc_ctot, dc_coff, C) || !ok8(df_ctot, df_coff, C) || (add && !ok8(a_ctot, a_coff, C)) ||
       (mask && !ok8(m_ctot, m_coff, C)) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_pool_bwd: channel slices must be multiples of 8 and the grid even");
-  launch_pdl(k_pool_bwd, rows_grid((long long)B * D * H, W * (C / 8)), 256, 0, (cudaStream_t)stream,
-      Slice{(bf16 *)dcoarse, dc_ctot, dc_coff}, Slice{(bf16 *)dfine, df_ctot, df_coff},
-      Slice{(bf16 *)add, a_ctot, a_coff}, Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
+  if (empty(B, D, H, W)) return bad("slbc_nn_pool_bwd: empty grid");
+  const long long rows = (long long)B * D * H;
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_pool_bwd<decltype(i)>, rows_grid(rows, (long long)W * (C / 8)), 256, 0, (cudaStream_t)stream,
+               Slice{(bf16 *)dcoarse, dc_ctot, dc_coff}, Slice{(bf16 *)dfine, df_ctot, df_coff},
+               Slice{(bf16 *)add, a_ctot, a_coff}, Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
+  });
   return launched("slbc_nn_pool_bwd");
 }
 
@@ -844,9 +844,12 @@ int slbc_nn_up(const void *in, int in_ctot, int in_coff, void *out, int out_ctot
                int W, int C, void *stream) {
   if (!ok8(in_ctot, in_coff, C) || !ok8(out_ctot, out_coff, C) || D % 2 || H % 2 || W % 2)
     return bad("slbc_nn_up: channel slices must be multiples of 8 and the grid even");
-  launch_pdl(k_up, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
-             Slice{(bf16 *)in, in_ctot, in_coff},
-                                                      Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
+  if (empty(B, D, H, W)) return bad("slbc_nn_up: empty grid");
+  const long long rows = (long long)B * (D / 2) * (H / 2);
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_up<decltype(i)>, rows_grid(rows, (long long)(W / 2) * (C / 8)), 256, 0, (cudaStream_t)stream,
+               Slice{(bf16 *)in, in_ctot, in_coff}, Slice{(bf16 *)out, out_ctot, out_coff}, B, D, H, W, C);
+  });
   return launched("slbc_nn_up");
 }
 
@@ -855,10 +858,13 @@ int slbc_nn_up_bwd(const void *dfine, int df_ctot, int df_coff, void *dcoarse, i
   if (!ok8(df_ctot, df_coff, C) || !ok8(dc_ctot, dc_coff, C) || (mask && !ok8(m_ctot, m_coff, C)) || D % 2 ||
       H % 2 || W % 2)
     return bad("slbc_nn_up_bwd: channel slices must be multiples of 8 and the grid even");
-  launch_pdl(k_up_bwd, rows_grid((long long)B * (D / 2) * (H / 2), W / 2 * (C / 8)), 256, 0, (cudaStream_t)stream,
-             Slice{(bf16 *)dfine, df_ctot, df_coff},
-                                                          Slice{(bf16 *)dcoarse, dc_ctot, dc_coff},
-                                                          Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
+  if (empty(B, D, H, W)) return bad("slbc_nn_up_bwd: empty grid");
+  const long long rows = (long long)B * (D / 2) * (H / 2);
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_up_bwd<decltype(i)>, rows_grid(rows, (long long)(W / 2) * (C / 8)), 256, 0, (cudaStream_t)stream,
+               Slice{(bf16 *)dfine, df_ctot, df_coff}, Slice{(bf16 *)dcoarse, dc_ctot, dc_coff},
+               Slice{(bf16 *)mask, m_ctot, m_coff}, B, D, H, W, C);
+  });
   return launched("slbc_nn_up_bwd");
 }
 
@@ -959,8 +965,12 @@ int slbc_nn_scale(float *g, long long n, const double *state, void *stream) {
 int slbc_nn_mse(const float *pred, int ctot_p, const float *label, int nch, const float *sample_w, int B, int D, int H,
                 int W, void *grad, int gctot, double *loss, void *stream) {
   if (nch < 1 || ctot_p < nch || gctot % 8 || gctot < 8 || gctot < nch) return bad("slbc_nn_mse: bad channel counts");
-  launch_pdl(k_mse, std::min(rows_grid((long long)B * D * H, W), 152 * 8), 256, 0, (cudaStream_t)stream,
-      pred, ctot_p, label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss);
+  if (empty(B, D, H, W)) return bad("slbc_nn_mse: empty grid");
+  const long long rows = (long long)B * D * H;
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_mse<decltype(i)>, std::min(rows_grid(rows, W), 152 * 8), 256, 0, (cudaStream_t)stream, pred, ctot_p,
+               label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss);
+  });
   return launched("slbc_nn_mse");
 }
 
@@ -983,36 +993,46 @@ int slbc_nn_proj(const float *pred, int ctot_p, const float *label, int lch, int
 int slbc_nn_encode(const unsigned char *solid, int B, int D, int H, int W, void *out, int ctot, int features,
                    void *stream) {
   if (ctot % 8 || ctot < 8) return bad("slbc_nn_encode: bad channel count");
-  if ((long long)B * D * H >= 1LL << 31) return bad("slbc_nn_encode: too many rows");
-  const long long total = (long long)B * D * H * W;
+  if (empty(B, D, H, W)) return bad("slbc_nn_encode: empty grid");
+  const long long rows = (long long)B * D * H, total = rows * W;
   const cudaStream_t st = (cudaStream_t)stream;
   unsigned char *a = nullptr;
   if (features) {
-    // two stream-ordered scratch masks of one byte per voxel
-    const cudaError_t e = cudaMallocAsync((void **)&a, 2 * ((total + 255) / 256 * 256), st);
+    // two stream-ordered scratch masks of one byte per voxel, the second on a
+    // word boundary
+    const long long mask = (total + 255) / 256 * 256;
+    const cudaError_t e = cudaMallocAsync((void **)&a, 2 * mask, st);
     if (e != cudaSuccess) return bad((std::string("slbc_nn_encode scratch: ") + cudaGetErrorString(e)).c_str());
-    // the second mask on a word boundary; whole words along x where W holds them
-    unsigned char *b = a + (total + 255) / 256 * 256;
+    unsigned char *b = a + mask;
+    for_rows(rows, [&](auto i) {
+      using I = decltype(i);
+      const auto go = [&](auto kernel) {
+        launch_pdl(kernel, rows_grid(rows, W), 256, 0, st, solid, (I)rows, W, a);
+      };
+      if (features == 2) go(k_dist_x<kDistR2, I>);
+      else go(k_dist_x<kDistR1, I>);
+    });
+    // whole words along x where W holds them
     const int vec = W % 4 == 0 ? 4 : 1;
-    const auto passes = [&](auto rx, auto ry, auto rz) {
-      launch_pdl(rx, rows_grid((long long)B * D * H, W), 256, 0, st, solid, B * D * H, W, a);
-      const long long run_y = (long long)B * D * ((H + kDistRun - 1) / kDistRun) * (W / vec);
-      const long long run_z = (long long)B * ((D + kDistRun - 1) / kDistRun) * (W * H / vec);
-      launch_pdl(ry, grid_for(run_y), 256, 0, st, a, B * D, H, W, b);
-      launch_pdl(rz, grid_for(run_z), 256, 0, st, b, B, D, W * H, a);
+    const auto pass = [&](const unsigned char *from, int outers, int n, long long inner, unsigned char *to) {
+      const long long runs = (long long)outers * ((n + kDistRun - 1) / kDistRun) * (inner / vec);
+      for_rows(runs, [&](auto i) {
+        using I = decltype(i);
+        const auto go = [&](auto kernel) { launch_pdl(kernel, grid_for(runs), 256, 0, st, from, outers, n, inner, to); };
+        if (features == 2 && vec == 4) go(k_dist_min<kDistR2, 4, I>);
+        else if (features == 2) go(k_dist_min<kDistR2, 1, I>);
+        else if (vec == 4) go(k_dist_min<kDistR1, 4, I>);
+        else go(k_dist_min<kDistR1, 1, I>);
+      });
     };
-    if (features == 2) {
-      if (vec == 4) passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 4>, k_dist_min<kDistR2, 4>);
-      else passes(k_dist_x<kDistR2>, k_dist_min<kDistR2, 1>, k_dist_min<kDistR2, 1>);
-    } else {
-      if (vec == 4) passes(k_dist_x<kDistR1>, k_dist_min<kDistR1, 4>, k_dist_min<kDistR1, 4>);
-      else passes(k_dist_x<kDistR1>, k_dist_min<kDistR1, 1>, k_dist_min<kDistR1, 1>);
-    }
+    pass(a, B * D, H, W, b);
+    pass(b, B, D, (long long)W * H, a);
     slbc::count_launch(3);
   }
-  launch_pdl(k_encode, rows_grid((long long)B * D * H, W * (ctot / 8)), 256, 0, st, solid, a,
-             features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out,
-                                            ctot);
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_encode<decltype(i)>, rows_grid(rows, (long long)W * (ctot / 8)), 256, 0, st, solid, a,
+               features == 2 ? kDistR2 : kDistR1, B, D, H, W, (bf16 *)out, ctot);
+  });
   const int rc = launched("slbc_nn_encode");
   if (a) {
     const cudaError_t e = cudaFreeAsync(a, st);
@@ -1048,9 +1068,12 @@ int slbc_nn_cross_flux(float *u, int D, int H, int W, double *work, void *stream
 int slbc_nn_decode(const float *pred, int ctot_p, const unsigned char *solid, int D, int H, int W, float scale,
                    float shift_x, float *u, float drho_scale, float *drho, void *stream) {
   if (ctot_p < (drho ? 4 : 3)) return bad("slbc_nn_decode: bad channel count");
-  launch_pdl(k_decode, rows_grid((long long)D * H, W), 256, 0, (cudaStream_t)stream, pred, ctot_p, solid, D, H, W,
-             scale,
-                                                                                       shift_x, u, drho_scale, drho);
+  if (empty(1, D, H, W)) return bad("slbc_nn_decode: empty grid");
+  const long long rows = (long long)D * H;
+  for_rows(rows, [&](auto i) {
+    launch_pdl(k_decode<decltype(i)>, rows_grid(rows, W), 256, 0, (cudaStream_t)stream, pred, ctot_p, solid, D, H, W,
+               scale, shift_x, u, drho_scale, drho);
+  });
   return launched("slbc_nn_decode");
 }
 
