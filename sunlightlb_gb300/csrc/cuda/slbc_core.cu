@@ -981,8 +981,8 @@ static int geometry_boundary(Lattice &L, int nobj, const long *bnd_node, const i
     CK(cudaMalloc(&L.bnd_node, nbnd * sizeof(int)));
     CK(cudaMalloc(&L.bnd_obj, nbnd * sizeof(int)));
     CK(cudaMalloc(&L.bnd_f, 3 * nbnd * sizeof(double)));
-    CK(cudaMemcpy(L.bnd_node, nodes.data(), nbnd * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(L.bnd_obj, bnd_obj, nbnd * sizeof(int), cudaMemcpyHostToDevice));
+    CK(upload(L.bnd_node, nodes.data(), nbnd * sizeof(int), L.stream));
+    CK(upload(L.bnd_obj, bnd_obj, nbnd * sizeof(int), L.stream));
     CK(cudaMemsetAsync(L.bnd_f, 0, 3 * nbnd * sizeof(double), L.stream));
   }
   if (nobj > 0) {
@@ -1004,16 +1004,16 @@ static int geometry_boundary(Lattice &L, int nobj, const long *bnd_node, const i
     CK(cudaMalloc(&L.obj_pos, 3 * nobj * sizeof(double)));
     CK(cudaMalloc(&L.obj_ft, (6 * nobj + 2 * nobj) * sizeof(double)));
     // first/count stored after the 6*nobj results, as ints
-    CK(cudaMemcpy((int *)(L.obj_ft + 6 * nobj), first.data(), nobj * sizeof(int), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy((int *)(L.obj_ft + 6 * nobj) + nobj, cnt.data(), nobj * sizeof(int), cudaMemcpyHostToDevice));
+    CK(upload((int *)(L.obj_ft + 6 * nobj), first.data(), nobj * sizeof(int), L.stream));
+    CK(upload((int *)(L.obj_ft + 6 * nobj) + nobj, cnt.data(), nobj * sizeof(int), L.stream));
     if (L.npiece > 0) {
       CK(cudaMalloc(&L.piece_obj, L.npiece * sizeof(int)));
       CK(cudaMalloc(&L.piece_lo, L.npiece * sizeof(int)));
       CK(cudaMalloc(&L.piece_hi, L.npiece * sizeof(int)));
       CK(cudaMalloc(&L.piece_sum, 6 * (size_t)L.npiece * sizeof(double)));
-      CK(cudaMemcpy(L.piece_obj, po.data(), L.npiece * sizeof(int), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(L.piece_lo, plo.data(), L.npiece * sizeof(int), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(L.piece_hi, phi.data(), L.npiece * sizeof(int), cudaMemcpyHostToDevice));
+      CK(upload(L.piece_obj, po.data(), L.npiece * sizeof(int), L.stream));
+      CK(upload(L.piece_lo, plo.data(), L.npiece * sizeof(int), L.stream));
+      CK(upload(L.piece_hi, phi.data(), L.npiece * sizeof(int), L.stream));
     }
   }
   L.generation++;
@@ -1244,8 +1244,7 @@ int slbc_set_bodyforce(slbc_lattice *h, const double *bx, const double *by, cons
         if (L.precision == 0) ((double *)buf.data())[x] = src[c3][x];
         else ((float *)buf.data())[x] = (float)src[c3][x];
       }
-      CK(cudaMemcpy((char *)L.bf + c3 * (size_t)L.npad * es, buf.data(), (size_t)n * es,
-                    cudaMemcpyHostToDevice));
+      CK(upload((char *)L.bf + c3 * (size_t)L.npad * es, buf.data(), (size_t)n * es, L.stream));
     }
   }
   L.generation++;
@@ -1266,8 +1265,7 @@ int slbc_set_wallvel(slbc_lattice *h, const double *ux, const double *uy, const 
         if (L.precision == 0) ((double *)buf.data())[x] = src[c3][x];
         else ((float *)buf.data())[x] = (float)src[c3][x];
       }
-      CK(cudaMemcpy((char *)L.uw + c3 * (size_t)L.npad * es, buf.data(), (size_t)n * es,
-                    cudaMemcpyHostToDevice));
+      CK(upload((char *)L.uw + c3 * (size_t)L.npad * es, buf.data(), (size_t)n * es, L.stream));
     }
   }
   L.generation++;
@@ -1317,7 +1315,8 @@ int slbc_put_pops(slbc_lattice *h, const double *a) {
   L.layout = SLBC_LAYOUT_N;
   if (L.precision == 2) {
     int unpaired = 0;
-    CK(cudaMemcpy(&unpaired, L.partials, sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(&unpaired, L.partials, sizeof(int), cudaMemcpyDeviceToHost, L.stream));
+    CK(cudaStreamSynchronize(L.stream));
     if (unpaired > 0) {
       g_err = "slbc_put_pops: " + std::to_string(unpaired) +
               " nodes hold populations whose deviations are not paired (q and opp(q) differ); "
@@ -1590,7 +1589,7 @@ int slbc_mp_create(slbc_lattice *h, slbc_tracer **out, int use_f64) {
     if (e == cudaSuccess) {
       // rho = rho0 until the first snapshot (reference src/mpmisc.c:50-52)
       std::vector<double> r0((size_t)L.nnodes, L.par.rho0);
-      e = cudaMemcpy(L.mp_rho64, r0.data(), (size_t)L.nnodes * sizeof(double), cudaMemcpyHostToDevice);
+      e = upload(L.mp_rho64, r0.data(), (size_t)L.nnodes * sizeof(double), L.stream);
     }
   }
   if (e == cudaSuccess && !use_f64 && !L.mp_rho32) {

@@ -294,6 +294,16 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Host memory to the device in the order of `stream`, complete on return, so
+// the source may be a local vector.  Not cudaMemcpy: that goes by the default
+// stream, which the library's non-blocking streams do not wait for -- from
+// pageable memory it may return before the last of the data has landed -- and
+// it waits for whatever else the program has queued there.
+inline cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+}
+
 // Launch bookkeeping and error text (defined in slbc_core.cu)
 void count_launch(int n = 1);
 void set_error(const std::string &msg);

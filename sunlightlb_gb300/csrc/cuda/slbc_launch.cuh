@@ -132,10 +132,13 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
     h[d].odd0 = B.lats[d]->layout == SLBC_LAYOUT_C0 ? 1 : 0;
     cls[d] = (h[d].a.moving ? 2 : 0) + (h[d].a.bf_uniform ? 1 : 0);
   }
-  cudaError_t e = cudaMemcpy(B.doms, h.data(), n * sizeof(BatchDom<T_>), cudaMemcpyHostToDevice);
+  cudaError_t e = upload(B.doms, h.data(), n * sizeof(BatchDom<T_>), B.stream);
   if (e != cudaSuccess) return e;
+  // the tables of every class are there before the first launch: an upload
+  // waits for the batch's stream
+  struct ClassLaunch { int c, blocks, first_off, first_work; };
+  std::vector<ClassLaunch> launches;
   std::vector<int> off, work;
-  int base_off = 0, base_work = 0;
   for (int c = 0; c < 4; c++) {
     std::vector<int> order;
     for (int d = 0; d < n; d++) if (cls[d] == c) order.push_back(d);
@@ -151,17 +154,20 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
       load[w] += B.lats[d]->nnodes;
       owned[w].push_back(d);
     }
-    std::vector<int> o(W + 1, 0), wk;
+    launches.push_back(ClassLaunch{c, W, (int)off.size(), (int)work.size()});
+    off.push_back(0);
     for (int w = 0; w < W; w++) {
-      o[w + 1] = o[w] + (int)owned[w].size();
-      wk.insert(wk.end(), owned[w].begin(), owned[w].end());
+      off.push_back(off.back() + (int)owned[w].size());
+      work.insert(work.end(), owned[w].begin(), owned[w].end());
     }
-    e = cudaMemcpy(B.work_off + base_off, o.data(), (W + 1) * sizeof(int), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(B.work + base_work, wk.data(), wk.size() * sizeof(int), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
+  }
+  e = upload(B.work_off, off.data(), off.size() * sizeof(int), B.stream);
+  if (e == cudaSuccess) e = upload(B.work, work.data(), work.size() * sizeof(int), B.stream);
+  if (e != cudaSuccess) return e;
+  for (const ClassLaunch &l : launches) {
     const BatchDom<T_> *D = (const BatchDom<T_> *)B.doms;
-    const int *O = B.work_off + base_off, *K = B.work + base_work;
-    switch (c) {
+    const int *O = B.work_off + l.first_off, *K = B.work + l.first_work, W = l.blocks;
+    switch (l.c) {
       case 0: launch_pdl(k_batch<T_, SLBC_EXACT, false, false>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
       case 1: launch_pdl(k_batch<T_, SLBC_EXACT, false, true>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
       case 2: launch_pdl(k_batch<T_, SLBC_EXACT, true, false>, W, kBatchThreads, 0, B.stream, D, O, K, nsteps); break;
@@ -171,8 +177,6 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     B.nworkers = W;
-    base_off += W + 1;
-    base_work += (int)wk.size();
   }
   return cudaSuccess;
 }
@@ -221,7 +225,7 @@ cudaError_t SLBC_FN(prepare_tiles)(BatchState &B) {
     B.sets.push_back(set);
     d0 = d1;
   }
-  cudaError_t e = cudaMemcpy(B.doms, h.data(), n * sizeof(BatchDom<T_>), cudaMemcpyHostToDevice);
+  cudaError_t e = upload(B.doms, h.data(), n * sizeof(BatchDom<T_>), B.stream);
   if (e != cudaSuccess) return e;
   if ((long long)tiles.size() > B.tiles_cap) {
     if (B.tiles) cudaFree(B.tiles);
@@ -231,7 +235,7 @@ cudaError_t SLBC_FN(prepare_tiles)(BatchState &B) {
     if (e != cudaSuccess) return e;
     B.tiles_cap = (long long)tiles.size();
   }
-  return cudaMemcpy(B.tiles, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice);
+  return upload(B.tiles, tiles.data(), tiles.size() * sizeof(int2), B.stream);
 }
 
 // Tiles mode: one step of one set (step = position in the sequence, for the
