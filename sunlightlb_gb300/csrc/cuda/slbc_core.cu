@@ -761,7 +761,7 @@ __global__ void k_mp_ratios(const double *rho64, double rho0, double *rinv, doub
   const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= n) return;
   const double r = rho64[x];
-  rinv[x] = __drcp_rn(r);
+  rinv[x] = mp_reciprocal(r);
   ratio[x] = __ddiv_rn(rho0, r);
 }
 

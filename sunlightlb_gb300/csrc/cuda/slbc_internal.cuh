@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "slb_device.h"
+#include "slbc_arith.cuh"
 #include "slbc_index.cuh"
 
 namespace slbc {

@@ -82,18 +82,6 @@ struct MpSource {
   TP fac, piece;
 };
 
-// p / rho, correctly rounded, from y = RN(1 / rho): each pair of fused
-// multiply-adds forms the remainder of the quotient and corrects it; after the
-// first the quotient is within one ulp, so the second rounds correctly
-// (Markstein).  Five FP64 operations instead of a division's ten or so.
-// Infinite and undefined quotients pass through.
-__device__ __forceinline__ double mp_quotient(double p, double rho, double y) {
-  const double q0 = __dmul_rn(p, y);
-  if ((__double2hiint(q0) & 0x7ff00000) == 0x7ff00000) return p / rho;
-  const double q1 = __fma_rn(__fma_rn(-rho, q0, p), y, q0);
-  return __fma_rn(__fma_rn(-rho, q1, p), y, q1);
-}
-
 // What a source node's values are made of: p, rho and, for FP64 tracers, the
 // snapshot's 1 / rho and rho0 / rho.
 template <typename TP>
@@ -115,7 +103,7 @@ __device__ __forceinline__ MpRaw<TP> mp_raw(const MpArgs &m, int y) {
       r.rinv = m.rinv[y];
       r.ratio = m.rratio[y];
     } else {  // no room for the two arrays
-      r.rinv = 1.0 / r.rho;
+      r.rinv = mp_reciprocal(r.rho);
       r.ratio = m.rho0 / r.rho;
     }
   }
@@ -123,16 +111,32 @@ __device__ __forceinline__ MpRaw<TP> mp_raw(const MpArgs &m, int y) {
 }
 
 template <typename TP>
-__device__ __forceinline__ MpSource<TP> mp_source(const MpRaw<TP> &v, TP rho0, TP alpha) {
+__device__ __forceinline__ MpSource<TP> mp_source(const MpRaw<TP> &v, TP rho0, TP alpha, bool &divide) {
   MpSource<TP> r;
   if constexpr (sizeof(TP) == 8) {
-    r.fac = mp_quotient(v.p, v.rho, v.rinv);
+    r.fac = mp_quotient(v.p, v.rho, v.rinv, divide);
     r.piece = v.p * TP(1.0 / 72.0) * (v.ratio - alpha);
   } else {
     r.fac = v.p / v.rho;
     r.piece = v.p * TP(1.0 / 72.0) * (rho0 / v.rho - alpha);
   }
   return r;
+}
+
+// The sources of one plane of the ring from a thread's raw values (those with
+// off >= 0), where quotients that want a division get one.
+template <typename TP>
+__device__ __forceinline__ void mp_sources(MpSource<TP> *plane, const int (&off)[kPlaneLoads],
+                                           const MpRaw<TP> (&raw)[kPlaneLoads], TP rho0, TP alpha) {
+  bool divide = false;
+#pragma unroll
+  for (int e = 0; e < kPlaneLoads; e++)
+    if (off[e] >= 0) plane[kTileThreads * e] = mp_source<TP>(raw[e], rho0, alpha, divide);
+  if (sizeof(TP) == 8 && divide) {
+#pragma unroll
+    for (int e = 0; e < kPlaneLoads; e++)
+      if (off[e] >= 0) plane[kTileThreads * e].fac = raw[e].p / raw[e].rho;
+  }
 }
 
 // One tracer update of every node.  A block of 32 (k) x 8 (j) threads walks
@@ -169,9 +173,11 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const int base = wrap_index(i0 - 1 + h, p.esi) * plane_nodes;
+    MpRaw<TP> raw[kPlaneLoads];
 #pragma unroll
     for (int e = 0; e < kPlaneLoads; e++)
-      if (off[e] >= 0) ring[h][tid + kTileThreads * e] = mp_source<TP>(mp_raw<TP>(m, base + off[e]), rho0, alpha);
+      if (off[e] >= 0) raw[e] = mp_raw<TP>(m, base + off[e]);
+    mp_sources<TP>(&ring[h][tid], off, raw, rho0, alpha);
   }
   // Register prefetch, one plane ahead of use: p and rho of the halo tile
   // of plane i+1 (for the ring) and the flag word, adsorption byte, p and
@@ -207,11 +213,7 @@ __global__ void __launch_bounds__(kTileThreads, sizeof(TP) == 8 ? 2 : 3) k_mp_st
     const int i = i0 + ii;
     const int sm = ii % 3, s0 = (ii + 1) % 3, sp = (ii + 2) % 3;  // planes i-1, i, i+1
     __syncthreads();  // slot sp held plane i-2, last read in the previous iteration
-#pragma unroll
-    for (int e = 0; e < kPlaneLoads; e++) {
-      if (off[e] < 0) continue;
-      ring[sp][tid + kTileThreads * e] = mp_source<TP>(pre[e], rho0, alpha);
-    }
+    mp_sources<TP>(&ring[sp][tid], off, pre, rho0, alpha);
     __syncthreads();
     const uint16_t fl = n_fl, al = n_al;
     const bool ads_x = n_ads != 0;
