@@ -64,6 +64,34 @@ SLBC_HD double mp_quotient(double p, double rho, double y, bool &divide) {
   return q;
 }
 
+// Correctly rounded a / b for a constant b with rb = RN(1/b), by Markstein's
+// theorem: q = RN(a rb) is within one ulp of a / b, the remainder r = a - b q is
+// exact (one fused multiply-add), and RN(q + r rb) = RN(a / b).  Three FP64
+// operations instead of a full division; a = +-0 returns a (keeps the sign of
+// zero).  Below 2^-900, where the remainder may underflow, and for infinities
+// `divide` is set: the caller divides.
+SLBC_HD double div_const(double a, double b, double rb, bool &divide) {
+  const Words w = words(a);
+  const bool zero = ((w.hi & 0x7fffffffu) | w.lo) == 0;
+  const double q = a * rb;
+  const double r = fma_rn(-q, b, a);
+  const double q1 = fma_rn(r, rb, q);
+  divide = divide || (!zero && below(w, -900)) || not_finite(w);
+  return zero ? a : q1;
+}
+
+// c * p + s for a power of two p: where c * p is exact, one fused multiply-add
+// rounds like the multiplication and the addition.  For p = 1/2 or 1/8 that is
+// so unless c * p is subnormal: for such c (zero apart) scaling_rounds is true,
+// and c = rounded_scale(c, p) makes the two agree again (c * p rounded, which
+// the division by p keeps).
+SLBC_HD double scale_add(double c, double p, double s) { return fma_rn(c, p, s); }
+SLBC_HD bool scaling_rounds(double c) {
+  const Words w = words(c);
+  return below(w, -1000) && ((w.hi & 0x7fffffffu) | w.lo) != 0;
+}
+SLBC_HD double rounded_scale(double c, double p) { return c * p * (1.0 / p); }
+
 }  // namespace slbc
 
 #endif

@@ -88,29 +88,15 @@ __device__ __forceinline__ R link_term(int q, R ux, R uy, R uz) {
   }
 }
 
-// Correctly rounded a / b for a constant b with rb = RN(1/b), by Markstein's
-// theorem (binary64, round to nearest, no underflow or overflow): q = RN(a rb)
-// is within one ulp of a / b, the remainder r = a - b q is exact (one fused
-// multiply-add), and RN(q + r rb) = RN(a / b).  Three FP64 operations instead
-// of a full division; a = +-0 returns a (keeps the sign of zero; the test
-// looks at the bits, not through the FP64 pipe).
-__device__ __forceinline__ double div_const(double a, double b, double rb) {
-  const double q = __dmul_rn(a, rb);
-  const double r = __fma_rn(-q, b, a);
-  const double q1 = __fma_rn(r, rb, q);
-  return (__double_as_longlong(a) << 1) == 0 ? a : q1;
-}
-
-// c * p + s for a power of two p: c * p is exact, so one fused multiply-add
-// rounds like the reference's multiplication and addition.
-__device__ __forceinline__ double scale_add(double c, double p, double s) { return __fma_rn(c, p, s); }
 __device__ __forceinline__ float scale_add(float c, float p, float s) { return c * p + s; }
 
 // Rebuild the 15 populations from density deviation, momentum and stress:
 // reference src/lbkernel.c:838-865, same evaluation order.  The factors 8, 2,
 // 1/2 and 1/8 are powers of two, so the products with them ride in the
 // additions that follow (same rounding); the FP64 step is bound by the FP64
-// pipe, and these are 13 of its 130 operations per node.
+// pipe, and these are 13 of its 130 operations per node.  Values near the
+// subnormal numbers, for which quotient or product would round differently,
+// are found from their bits and take the reference's operations.
 template <typename T, bool EXACT>
 __device__ __forceinline__ void rebuild(T (&t)[15], T drho, T rux, T ruy, T ruz, T sxx,
                                         T syy, T szz, T sxy, T sxz, T syz) {
@@ -118,29 +104,46 @@ __device__ __forceinline__ void rebuild(T (&t)[15], T drho, T rux, T ruy, T ruz,
   const T fdd2bybc4 = T(4.0) * dd2bybc4, edbybc2 = T(8.0) * dbybc2;
   T rhobyb, trsby3;
   if (EXACT) {  // the reference's divisions, correctly rounded
-    rhobyb = div_const(drho, 72.0, 1.0 / 72.0);
-    trsby3 = div_const(sxx + syy + szz, 3.0, 1.0 / 3.0);
+    bool divide = false;
+    const T trace = sxx + syy + szz;
+    rhobyb = div_const(drho, 72.0, 1.0 / 72.0, divide);
+    trsby3 = div_const(trace, 3.0, 1.0 / 3.0, divide);
+    if (divide) {
+      rhobyb = drho / T(72.0);
+      trsby3 = trace / T(3.0);
+    }
   } else {
     rhobyb = drho * T(1.0 / 72.0);
     trsby3 = (sxx + syy + szz) * T(1.0 / 3.0);
   }
-  T ru, st;
+  // stress parts of the populations 1-2, 3-4, 5-6, 7/14, 8/13, 9/12, 10/11
+  T st[7] = {sxx - trsby3, syy - trsby3, szz - trsby3, trsby3 + sxy + sxz + syz, trsby3 - sxy - sxz + syz,
+             trsby3 - sxy + sxz - syz, trsby3 + sxy - sxz - syz};
+  if (EXACT) {
+    bool rounds = false;
+#pragma unroll
+    for (int i = 0; i < 7; i++) rounds = rounds || scaling_rounds(st[i]);
+    if (rounds) {
+#pragma unroll
+      for (int i = 0; i < 7; i++) st[i] = rounded_scale(st[i], i < 3 ? fdd2bybc4 : dd2bybc4);
+    }
+  }
   t[0] = scale_add(rhobyb, T(16.0), -trsby3);
-  T up, dn;  // 8 rhobyb +- ru
-  ru = edbybc2 * rux; st = sxx - trsby3; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[1] = scale_add(st, fdd2bybc4, up); t[2] = scale_add(st, fdd2bybc4, dn);
-  ru = edbybc2 * ruy; st = syy - trsby3; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[3] = scale_add(st, fdd2bybc4, up); t[4] = scale_add(st, fdd2bybc4, dn);
-  ru = edbybc2 * ruz; st = szz - trsby3; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[5] = scale_add(st, fdd2bybc4, up); t[6] = scale_add(st, fdd2bybc4, dn);
-  ru = dbybc2 * (rux + ruy + ruz); st = trsby3 + sxy + sxz + syz;
-  t[7] = scale_add(st, dd2bybc4, rhobyb + ru); t[14] = scale_add(st, dd2bybc4, rhobyb - ru);
-  ru = dbybc2 * (rux - ruy - ruz); st = trsby3 - sxy - sxz + syz;
-  t[8] = scale_add(st, dd2bybc4, rhobyb - ru); t[13] = scale_add(st, dd2bybc4, rhobyb + ru);
-  ru = dbybc2 * (rux - ruy + ruz); st = trsby3 - sxy + sxz - syz;
-  t[9] = scale_add(st, dd2bybc4, rhobyb + ru); t[12] = scale_add(st, dd2bybc4, rhobyb - ru);
-  ru = dbybc2 * (rux + ruy - ruz); st = trsby3 + sxy - sxz - syz;
-  t[10] = scale_add(st, dd2bybc4, rhobyb - ru); t[11] = scale_add(st, dd2bybc4, rhobyb + ru);
+  T ru, up, dn;  // 8 rhobyb +- ru
+  ru = edbybc2 * rux; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
+  t[1] = scale_add(st[0], fdd2bybc4, up); t[2] = scale_add(st[0], fdd2bybc4, dn);
+  ru = edbybc2 * ruy; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
+  t[3] = scale_add(st[1], fdd2bybc4, up); t[4] = scale_add(st[1], fdd2bybc4, dn);
+  ru = edbybc2 * ruz; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
+  t[5] = scale_add(st[2], fdd2bybc4, up); t[6] = scale_add(st[2], fdd2bybc4, dn);
+  ru = dbybc2 * (rux + ruy + ruz);
+  t[7] = scale_add(st[3], dd2bybc4, rhobyb + ru); t[14] = scale_add(st[3], dd2bybc4, rhobyb - ru);
+  ru = dbybc2 * (rux - ruy - ruz);
+  t[8] = scale_add(st[4], dd2bybc4, rhobyb - ru); t[13] = scale_add(st[4], dd2bybc4, rhobyb + ru);
+  ru = dbybc2 * (rux - ruy + ruz);
+  t[9] = scale_add(st[5], dd2bybc4, rhobyb + ru); t[12] = scale_add(st[5], dd2bybc4, rhobyb - ru);
+  ru = dbybc2 * (rux + ruy - ruz);
+  t[10] = scale_add(st[6], dd2bybc4, rhobyb - ru); t[11] = scale_add(st[6], dd2bybc4, rhobyb + ru);
 }
 
 // Moments of one node after relaxation: density deviation, momentum (with

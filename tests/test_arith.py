@@ -18,6 +18,7 @@ HEAD = r"""
 #include <cstdint>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <limits>
 #include "slbc_arith.cuh"
 static uint64_t state = 88172645463325252ull;
@@ -53,6 +54,42 @@ int main() {
 }
 """
 
+CONSTANT = HEAD + r"""
+int main() {
+  const double special[] = {0.0, -0.0, std::numeric_limits<double>::infinity(), -std::numeric_limits<double>::infinity(),
+                            std::nan(""), 5e-324, -5e-324, 2.2250738585072014e-308, 1.7976931348623157e308};
+  long wrong = 0, count = 0;
+  const auto quotient = [&](double a, double b) {
+    const volatile double want = a / b;
+    bool divide = false;
+    const double q = slbc::div_const(a, b, 1.0 / b, divide);
+    count++;
+    wrong += divide ? std::isfinite(a) && std::fabs(a) >= 1e-270 : !same(q, want);
+  };
+  const auto product = [&](double c, double p, double s) {
+    const volatile double cp = c * p, want = cp + s;
+    const bool rounds = slbc::scaling_rounds(c);
+    count++;
+    wrong += (rounds && std::fabs(c) >= 1e-300) || !same(slbc::scale_add(rounds ? slbc::rounded_scale(c, p) : c, p, s), want);
+  };
+  for (double a : special)
+    for (double b : {72.0, 3.0}) quotient(a, b);
+  for (double c : special)
+    for (double s : special)
+      for (double p : {0.5, 0.125}) product(c, p, s);
+  for (int e = 0; e < 2047; e++)
+    for (int i = 0; i < 1000; i++) {
+      quotient(number(e), 72.0);
+      quotient(number(e), 3.0);
+      const int f = e + (int)(bits() % 121) - 60;  // an addend near c
+      const double s = number(f < 0 ? 0 : f > 2046 ? 2046 : f);
+      product(number(e), 0.5, s);
+      product(number(e), 0.125, s);
+    }
+  std::printf("%ld %ld\n", wrong, count);
+}
+"""
+
 
 def run(tmp_path, source):
     cxx = shutil.which(os.environ.get("CXX", "g++"))
@@ -67,4 +104,9 @@ def run(tmp_path, source):
 
 def test_tracer_quotients_equal_divisions(tmp_path):
     wrong, count = run(tmp_path, QUOTIENT)
+    assert count > 8_000_000 and wrong == 0
+
+
+def test_collision_quotients_and_products_equal_plain_ones(tmp_path):
+    wrong, count = run(tmp_path, CONSTANT)
     assert count > 8_000_000 and wrong == 0

@@ -6,6 +6,8 @@ densities: the GPU's bits are the CPU oracle's.
 import numpy as np
 import pytest
 
+from scenarios import two_spheres
+
 pytestmark = pytest.mark.gpu
 
 
@@ -48,4 +50,27 @@ def test_tiny_tracer_equals_oracle(gpu, orc, scale):
 def test_infinite_density_equals_oracle(gpu, orc):
     got, want = tracer(gpu, 1.0, big=True), tracer(orc, 1.0, big=True)
     assert np.isfinite(want).all()  # p over an infinite density is 0
+    assert np.array_equal(got, want), int((got != want).sum())
+
+
+def populations(L, scale, stokes, dims):
+    """Four updates of random populations around two spheres."""
+    lb = two_spheres(L, dims=dims, steps=0, measure=False, bf=(0.0, 0.0, 0.0), stokes=stokes)
+    if L.has("lbpull"):
+        L.lbpull(lb)
+    a = lb.array("a")
+    a[:] = (np.random.default_rng(5).random(a.shape) - 0.5) * scale
+    a[::7] = 0.0
+    if L.has("lbpush"):
+        L.lbpush(lb)
+    for _ in range(4):
+        L.lbstep(lb)
+    return lb.pops()
+
+
+@pytest.mark.parametrize("scale", [1e-250, 1e-270, 1e-290, 1e-300, 1e-306, 1e-308, 1e-312, 1e-318])
+@pytest.mark.parametrize("stokes", [1, 0])
+@pytest.mark.parametrize("dims", [(9, 10, 11), (5, 6, 32)])  # a plane as one run of nodes, rows of whole warps
+def test_tiny_populations_equal_oracle(gpu, orc, scale, stokes, dims):
+    got, want = populations(gpu, scale, stokes, dims), populations(orc, scale, stokes, dims)
     assert np.array_equal(got, want), int((got != want).sum())
