@@ -88,38 +88,39 @@ __device__ __forceinline__ R link_term(int q, R ux, R uy, R uz) {
   }
 }
 
+// FP32 tracers: contracted by the compiler
 __device__ __forceinline__ float scale_add(float c, float p, float s) { return c * p + s; }
 
 // Rebuild the 15 populations from density deviation, momentum and stress:
-// reference src/lbkernel.c:838-865, same evaluation order.  The factors 8, 2,
-// 1/2 and 1/8 are powers of two, so the products with them ride in the
-// additions that follow (same rounding); the FP64 step is bound by the FP64
-// pipe, and these are 13 of its 130 operations per node.  Values near the
-// subnormal numbers, for which quotient or product would round differently,
-// are found from their bits and take the reference's operations.
+// reference src/lbkernel.c:838-865, same evaluation order.
+//
+// EXACT (FP64): the bits of the reference.  The factors 8, 2, 1/2 and 1/8 are
+// powers of two, so the products with them ride in the additions that follow
+// (same rounding); the FP64 step is bound by the FP64 pipe, and these are 13 of
+// its 130 operations per node.  Values near the subnormal numbers, for which
+// quotient or product would round differently, are found from their bits and
+// take the reference's operations.
+//
+// FP32: written as the reference is, and contracted by the compiler; in the
+// form above it rounds the trace before its product with 1/3 is subtracted,
+// and an update is 2% further from 64 bits (8% in the rest population).
 template <typename T, bool EXACT>
 __device__ __forceinline__ void rebuild(T (&t)[15], T drho, T rux, T ruy, T ruz, T sxx,
                                         T syy, T szz, T sxy, T sxz, T syz) {
   const T dbybc2 = T(1.0 / 24.0), dd2bybc4 = T(1.0 / 8.0);
   const T fdd2bybc4 = T(4.0) * dd2bybc4, edbybc2 = T(8.0) * dbybc2;
-  T rhobyb, trsby3;
-  if (EXACT) {  // the reference's divisions, correctly rounded
+  if constexpr (EXACT) {
     bool divide = false;
     const T trace = sxx + syy + szz;
-    rhobyb = div_const(drho, 72.0, 1.0 / 72.0, divide);
-    trsby3 = div_const(trace, 3.0, 1.0 / 3.0, divide);
+    T rhobyb = div_const(drho, 72.0, 1.0 / 72.0, divide);
+    T trsby3 = div_const(trace, 3.0, 1.0 / 3.0, divide);
     if (divide) {
-      rhobyb = drho / T(72.0);
-      trsby3 = trace / T(3.0);
+      rhobyb = drho / 72.0;
+      trsby3 = trace / 3.0;
     }
-  } else {
-    rhobyb = drho * T(1.0 / 72.0);
-    trsby3 = (sxx + syy + szz) * T(1.0 / 3.0);
-  }
-  // stress parts of the populations 1-2, 3-4, 5-6, 7/14, 8/13, 9/12, 10/11
-  T st[7] = {sxx - trsby3, syy - trsby3, szz - trsby3, trsby3 + sxy + sxz + syz, trsby3 - sxy - sxz + syz,
-             trsby3 - sxy + sxz - syz, trsby3 + sxy - sxz - syz};
-  if (EXACT) {
+    // stress parts of the populations 1-2, 3-4, 5-6, 7/14, 8/13, 9/12, 10/11
+    T st[7] = {sxx - trsby3, syy - trsby3, szz - trsby3, trsby3 + sxy + sxz + syz, trsby3 - sxy - sxz + syz,
+               trsby3 - sxy + sxz - syz, trsby3 + sxy - sxz - syz};
     bool rounds = false;
 #pragma unroll
     for (int i = 0; i < 7; i++) rounds = rounds || scaling_rounds(st[i]);
@@ -127,23 +128,43 @@ __device__ __forceinline__ void rebuild(T (&t)[15], T drho, T rux, T ruy, T ruz,
 #pragma unroll
       for (int i = 0; i < 7; i++) st[i] = rounded_scale(st[i], i < 3 ? fdd2bybc4 : dd2bybc4);
     }
+    t[0] = scale_add(rhobyb, 16.0, -trsby3);
+    T ru, up, dn;  // 8 rhobyb +- ru
+    ru = edbybc2 * rux; up = scale_add(rhobyb, 8.0, ru); dn = scale_add(rhobyb, 8.0, -ru);
+    t[1] = scale_add(st[0], fdd2bybc4, up); t[2] = scale_add(st[0], fdd2bybc4, dn);
+    ru = edbybc2 * ruy; up = scale_add(rhobyb, 8.0, ru); dn = scale_add(rhobyb, 8.0, -ru);
+    t[3] = scale_add(st[1], fdd2bybc4, up); t[4] = scale_add(st[1], fdd2bybc4, dn);
+    ru = edbybc2 * ruz; up = scale_add(rhobyb, 8.0, ru); dn = scale_add(rhobyb, 8.0, -ru);
+    t[5] = scale_add(st[2], fdd2bybc4, up); t[6] = scale_add(st[2], fdd2bybc4, dn);
+    ru = dbybc2 * (rux + ruy + ruz);
+    t[7] = scale_add(st[3], dd2bybc4, rhobyb + ru); t[14] = scale_add(st[3], dd2bybc4, rhobyb - ru);
+    ru = dbybc2 * (rux - ruy - ruz);
+    t[8] = scale_add(st[4], dd2bybc4, rhobyb - ru); t[13] = scale_add(st[4], dd2bybc4, rhobyb + ru);
+    ru = dbybc2 * (rux - ruy + ruz);
+    t[9] = scale_add(st[5], dd2bybc4, rhobyb + ru); t[12] = scale_add(st[5], dd2bybc4, rhobyb - ru);
+    ru = dbybc2 * (rux + ruy - ruz);
+    t[10] = scale_add(st[6], dd2bybc4, rhobyb - ru); t[11] = scale_add(st[6], dd2bybc4, rhobyb + ru);
+  } else {
+    const T rhobyb = drho * T(1.0 / 72.0);
+    const T trsby3 = (sxx + syy + szz) * T(1.0 / 3.0);
+    const T erhobyb = T(8.0) * rhobyb;
+    T ru, st;
+    t[0] = T(2.0) * erhobyb - T(2.0) * fdd2bybc4 * trsby3;
+    ru = edbybc2 * rux; st = fdd2bybc4 * (sxx - trsby3);
+    t[1] = erhobyb + ru + st; t[2] = erhobyb - ru + st;
+    ru = edbybc2 * ruy; st = fdd2bybc4 * (syy - trsby3);
+    t[3] = erhobyb + ru + st; t[4] = erhobyb - ru + st;
+    ru = edbybc2 * ruz; st = fdd2bybc4 * (szz - trsby3);
+    t[5] = erhobyb + ru + st; t[6] = erhobyb - ru + st;
+    ru = dbybc2 * (rux + ruy + ruz); st = dd2bybc4 * (trsby3 + sxy + sxz + syz);
+    t[7] = rhobyb + ru + st; t[14] = rhobyb - ru + st;
+    ru = dbybc2 * (rux - ruy - ruz); st = dd2bybc4 * (trsby3 - sxy - sxz + syz);
+    t[8] = rhobyb - ru + st; t[13] = rhobyb + ru + st;
+    ru = dbybc2 * (rux - ruy + ruz); st = dd2bybc4 * (trsby3 - sxy + sxz - syz);
+    t[9] = rhobyb + ru + st; t[12] = rhobyb - ru + st;
+    ru = dbybc2 * (rux + ruy - ruz); st = dd2bybc4 * (trsby3 + sxy - sxz - syz);
+    t[10] = rhobyb - ru + st; t[11] = rhobyb + ru + st;
   }
-  t[0] = scale_add(rhobyb, T(16.0), -trsby3);
-  T ru, up, dn;  // 8 rhobyb +- ru
-  ru = edbybc2 * rux; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[1] = scale_add(st[0], fdd2bybc4, up); t[2] = scale_add(st[0], fdd2bybc4, dn);
-  ru = edbybc2 * ruy; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[3] = scale_add(st[1], fdd2bybc4, up); t[4] = scale_add(st[1], fdd2bybc4, dn);
-  ru = edbybc2 * ruz; up = scale_add(rhobyb, T(8.0), ru); dn = scale_add(rhobyb, T(8.0), -ru);
-  t[5] = scale_add(st[2], fdd2bybc4, up); t[6] = scale_add(st[2], fdd2bybc4, dn);
-  ru = dbybc2 * (rux + ruy + ruz);
-  t[7] = scale_add(st[3], dd2bybc4, rhobyb + ru); t[14] = scale_add(st[3], dd2bybc4, rhobyb - ru);
-  ru = dbybc2 * (rux - ruy - ruz);
-  t[8] = scale_add(st[4], dd2bybc4, rhobyb - ru); t[13] = scale_add(st[4], dd2bybc4, rhobyb + ru);
-  ru = dbybc2 * (rux - ruy + ruz);
-  t[9] = scale_add(st[5], dd2bybc4, rhobyb + ru); t[12] = scale_add(st[5], dd2bybc4, rhobyb - ru);
-  ru = dbybc2 * (rux + ruy - ruz);
-  t[10] = scale_add(st[6], dd2bybc4, rhobyb - ru); t[11] = scale_add(st[6], dd2bybc4, rhobyb + ru);
 }
 
 // Moments of one node after relaxation: density deviation, momentum (with
