@@ -1088,7 +1088,7 @@ __global__ void k_move_sphere(PopArgs<T> p, MoveArgs m, T *uw) {
 // host (an FP64 operation per node is what bounded this kernel).
 struct FieldArgs {
   double rho0, fac, fb[3];          // fb = fac * b (uniform body force)
-  float rho0_h, rho0_l, fac_f, fb_h[3], fb_l[3];
+  float rho0_h, rho0_l, fac_h, fac_l, fb_h[3], fb_l[3];
   int bf_uniform;
 };
 
@@ -1098,6 +1098,36 @@ __device__ __forceinline__ float ff_quotient(float nh, float nl, float rh, float
   const float q = nh * rinv;
   const float rem = __fmaf_rn(-q, rh, nh) + __fmaf_rn(-q, rl, nl);
   return __fmaf_rn(rem, rinv, q);
+}
+
+// m += fac * b, the product as a hi + lo pair
+__device__ __forceinline__ void add_force(Acc<float> &m, const FieldArgs &f, float b) {
+  const float p = f.fac_h * b;
+  m.add(p);
+  m.lo += __fmaf_rn(f.fac_h, b, -p) + f.fac_l * b;
+}
+
+// Velocity and density deviation of a node in plain FP64: infinite sums, for
+// which pairs of FP32 values would give NaN, and sums beyond FP32.
+template <typename T>
+__device__ __forceinline__ void field_plain(const FieldArgs &f, const T (&t)[15], const T *bf, long long S, int x,
+                                            float &ux, float &uy, float &uz, float &dr) {
+  double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+#pragma unroll
+  for (int q = 0; q < 15; q++) {
+    const double v = (double)t[q];
+    r += v;
+    mx += CX(q) * v;
+    my += CY(q) * v;
+    mz += CZ(q) * v;
+  }
+  double bx = f.fb[0], by = f.fb[1], bz = f.fb[2];
+  if (!f.bf_uniform) { bx = f.fac * bf[x]; by = f.fac * bf[S + x]; bz = f.fac * bf[2 * S + x]; }
+  const double inv = 1.0 / (f.rho0 + r);
+  ux = (float)((mx + bx) * inv);
+  uy = (float)((my + by) * inv);
+  uz = (float)((mz + bz) * inv);
+  dr = (float)r;
 }
 
 // Velocity field u = (sum_q c_q a_q + fac * b) / (rho0 + sum_q a_q) of the
@@ -1149,13 +1179,14 @@ __global__ void k_velocity(PopArgs<T> p, FieldArgs f, const T *bf, float *u, flo
       if (f.bf_uniform) {
         mx.add(f.fb_h[0]); my.add(f.fb_h[1]); mz.add(f.fb_h[2]);
         mx.lo += f.fb_l[0]; my.lo += f.fb_l[1]; mz.lo += f.fb_l[2];
-      } else {  // fac is +-1/2 or 0: the products are exact
-        mx.add(f.fac_f * bf[x]); my.add(f.fac_f * bf[p.npad + x]); mz.add(f.fac_f * bf[2 * p.npad + x]);
+      } else {
+        add_force(mx, f, bf[x]); add_force(my, f, bf[p.npad + x]); add_force(mz, f, bf[2 * p.npad + x]);
       }
       ux = ff_quotient(mx.hi, mx.lo, rh, rl, rinv);
       uy = ff_quotient(my.hi, my.lo, rh, rl, rinv);
       uz = ff_quotient(mz.hi, mz.lo, rh, rl, rinv);
     }
+    if (!(fabsf(ux) + fabsf(uy) + fabsf(uz) + fabsf(dr) < 1e38f)) field_plain<T>(f, t, bf, p.npad, x, ux, uy, uz, dr);
   }
   u[x] = ux;
   u[n + x] = uy;

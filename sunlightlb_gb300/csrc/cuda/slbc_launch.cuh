@@ -402,7 +402,8 @@ cudaError_t SLBC_FN(launch_velocity)(Lattice &L, double fac, float *u, float *dr
   FieldArgs f;
   f.rho0 = L.par.rho0;
   f.fac = fac;
-  f.fac_f = (float)fac;
+  f.fac_h = (float)fac;
+  f.fac_l = (float)(fac - f.fac_h);
   f.rho0_h = (float)f.rho0;
   f.rho0_l = (float)(f.rho0 - f.rho0_h);
   f.bf_uniform = L.bf_uniform;
