@@ -1108,14 +1108,17 @@ __device__ __forceinline__ void add_force(Acc<float> &m, const FieldArgs &f, flo
 }
 
 // Velocity and density deviation of a node in plain FP64: infinite sums, for
-// which pairs of FP32 values would give NaN, and sums beyond FP32.
-template <typename T>
-__device__ __forceinline__ void field_plain(const FieldArgs &f, const T (&t)[15], const T *bf, long long S, int x,
-                                            float &ux, float &uy, float &uz, float &dr) {
+// which pairs of FP32 values would give NaN, and sums beyond FP32.  The
+// populations are read again: kept for this, they cost k_velocity a quarter of
+// its time in occupancy.
+template <typename T, int LAYOUT>
+__device__ __noinline__ float4 field_plain(const PopArgs<T> &p, const FieldArgs &f, const T *bf, int x, uint16_t fl,
+                                           Nbr nb) {
+  const long long S = p.npad;
   double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
-#pragma unroll
+#pragma unroll 1
   for (int q = 0; q < 15; q++) {
-    const double v = (double)t[q];
+    const double v = (double)post_value<T>(p.pop, S, LAYOUT, q, x, fl, nb);
     r += v;
     mx += CX(q) * v;
     my += CY(q) * v;
@@ -1124,10 +1127,7 @@ __device__ __forceinline__ void field_plain(const FieldArgs &f, const T (&t)[15]
   double bx = f.fb[0], by = f.fb[1], bz = f.fb[2];
   if (!f.bf_uniform) { bx = f.fac * bf[x]; by = f.fac * bf[S + x]; bz = f.fac * bf[2 * S + x]; }
   const double inv = 1.0 / (f.rho0 + r);
-  ux = (float)((mx + bx) * inv);
-  uy = (float)((my + by) * inv);
-  uz = (float)((mz + bz) * inv);
-  dr = (float)r;
+  return make_float4((float)((mx + bx) * inv), (float)((my + by) * inv), (float)((mz + bz) * inv), (float)r);
 }
 
 // Velocity field u = (sum_q c_q a_q + fac * b) / (rho0 + sum_q a_q) of the
@@ -1138,16 +1138,28 @@ __device__ __forceinline__ void field_plain(const FieldArgs &f, const T (&t)[15]
 // with a remainder correction, all on the FP32 pipe: the first form widened
 // every population to FP64 (15 conversions and 45 multiply-adds per node on
 // a pipe 64 times narrower) and took 22.3 ms at 512^3 against 1.5 ms of
-// memory traffic.  One row of k per block row, so no index is divided.
-template <typename T, int LAYOUT>
-__global__ void k_velocity(PopArgs<T> p, FieldArgs f, const T *bf, float *u, float *drho) {
+// memory traffic.  FLAT: the nodes are one run, so no thread is idle on short
+// rows (256 x 256 x 1 FP64: 254 us with a block row per row of k, 11 as a
+// run); else one row of k per block row, and no index is divided.
+template <typename T, int LAYOUT, bool FLAT>
+__global__ void k_velocity(const __grid_constant__ PopArgs<T> p, const __grid_constant__ FieldArgs f, const T *bf, float *u,
+                           float *drho) {
   after_previous();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y, i = blockIdx.z;
-  if (k >= p.esk) return;
   const long long n = (long long)p.esi * p.esj * p.esk;
-  const Nbr nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
-  const int x = nb.at(0, 0, 0);
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= (FLAT ? n : p.esk)) return;
+  int i = blockIdx.z, j = blockIdx.y, k = (int)e, x;
+  Nbr nb{};
+  if constexpr (FLAT) {
+    x = (int)e;
+    if constexpr (LAYOUT == SLBC_LAYOUT_C1) {
+      decode(x, p.esj, p.esk, i, j, k);
+      nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
+    }
+  } else {
+    nb = make_nbr(i, j, k, p.esi, p.esj, p.esk);
+    x = nb.at(0, 0, 0);
+  }
   const uint16_t fl = p.flags[x];
   float ux = 0.f, uy = 0.f, uz = 0.f, dr = 0.f;
   if (!(fl & FLAG_SOLID)) {
@@ -1186,7 +1198,10 @@ __global__ void k_velocity(PopArgs<T> p, FieldArgs f, const T *bf, float *u, flo
       uy = ff_quotient(my.hi, my.lo, rh, rl, rinv);
       uz = ff_quotient(mz.hi, mz.lo, rh, rl, rinv);
     }
-    if (!(fabsf(ux) + fabsf(uy) + fabsf(uz) + fabsf(dr) < 1e38f)) field_plain<T>(f, t, bf, p.npad, x, ux, uy, uz, dr);
+    if (!(fabsf(ux) + fabsf(uy) + fabsf(uz) + fabsf(dr) < 1e38f)) {
+      const float4 v = field_plain<T, LAYOUT>(p, f, bf, x, fl, nb);
+      ux = v.x; uy = v.y; uz = v.z; dr = v.w;
+    }
   }
   u[x] = ux;
   u[n + x] = uy;

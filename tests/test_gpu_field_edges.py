@@ -91,3 +91,23 @@ def test_any_factor_of_a_per_node_force(gpu, precision, fac):
     wu, wr = plain(pops, force, fac)
     assert near(dr, wr).all()
     assert near(u, wu).all(), int((~near(u, wu)).sum())
+
+
+SHAPES = [  # dims: rows of 1 to 260 nodes, a line, a side beyond 65,535
+    (17, 19, 1), (700, 1, 1), (1, 700, 1), (9, 11, 3), (5, 7, 31), (6, 5, 32), (5, 6, 33), (4, 5, 48), (3, 5, 65), (3, 4, 97),
+    (3, 3, 128), (2, 3, 130), (2, 2, 260), (2, 70000, 2), (70000, 2, 1),
+]
+
+
+@pytest.mark.parametrize("precision", [1, 0])
+@pytest.mark.parametrize("dims", SHAPES, ids=lambda d: "x".join(map(str, d)))
+def test_every_shape_and_layout(gpu, dims, precision):
+    """The uploaded layout and those after one and two updates (sides beyond
+    65,535 take no update: the uploaded one)."""
+    n = int(np.prod(dims))
+    pops = ((np.random.default_rng(8).random((n, 15)) - 0.5) * 0.1).astype(np.float32).astype(float)
+    for steps in (0, 1, 2) if max(dims[:2]) <= 65535 else (0,):
+        u, dr, state = field(gpu, dims, precision, pops, fac=0.5, steps=steps)
+        wu, wr = plain(state, None, 0.0)
+        assert near(dr, wr).all(), steps
+        assert near(u, wu).all(), (steps, int((~near(u, wu)).sum()))
