@@ -141,8 +141,9 @@ int slbc_layout(slbc_lattice *h);
  * even threads along k, odd rows per thread, odd threads along k}; for BF16
  * lattices the "rows per thread" entries are planes per block (1..64),
  * threads along k is 32, and the even entries serve every step (one update
- * kernel).  The
- * first slbc_step of a lattice of 2^20 nodes or more times the candidate
+ * kernel).  Rows per thread -4 is the 128-bit form of FP32 lattices, -1 the
+ * run form of FP64 ones (the nodes of a plane as one run, in blocks of 32, 64
+ * or 128 threads).  The first slbc_step of a lattice of 2^20 nodes or more times the candidate
  * shapes on a copy of the populations and keeps the fastest (environment
  * SLB_AUTOTUNE=0 turns this off); get returns 1 tuned, -1 defaults, 0 not
  * yet decided; set pins a shape. */

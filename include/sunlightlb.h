@@ -311,11 +311,13 @@ long lbkernelcount(void);
  * rows per thread, even threads along k, odd rows per thread, odd threads
  * along k} (BF16 lattices: planes per block in place of rows per thread;
  * rows per thread -4: the 128-bit form, 4 nodes along k per thread, 128
- * threads per block); returns 1 tuned, -1 defaults, 0 not decided yet. */
+ * threads per block; -1: the run form, the nodes of a plane as one run, with
+ * the threads per block); returns 1 tuned, -1 defaults, 0 not decided yet. */
 int lbtuning(LBSys, int *);
 /* Set the launch shape of the fused step of lb (same cfg as lbtuning; rows
  * per thread -4 selects the 128-bit form, 4 nodes along k per thread and
- * 128 threads per block, FP32 populations with esk a multiple of 4);
+ * 128 threads per block, FP32 populations with esk a multiple of 4; -1 the
+ * run form in blocks of 32, 64 or 128 threads, FP64 populations);
  * returns 0, or non-zero (with a message) for a shape it does not take. */
 int lbsettuning(LBSys, int *);
 /* Storage layout of the device populations of lb: 0 the reference's order

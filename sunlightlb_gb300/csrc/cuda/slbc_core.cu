@@ -489,6 +489,19 @@ int autotune_time(Lattice &L);
 
 namespace slbc {
 bool vec4_ok(const Lattice &L) { return L.precision == 1 && L.esk % 4 == 0 && L.npad % 4 == 0; }
+bool run_ok(const Lattice &L) { return L.precision == 0 && 15LL * L.npad <= 0xFFFFFFFFLL; }
+
+// FP64 rows that leave more than 1/17 of their warps' lanes without a node go
+// as runs, in blocks of one warp where the lattice is small.  Measured, one
+// update as rows and as runs: 64 x 64 rows of 60 nodes 74.5 and 69.4 us, of 30
+// 37.8 and 38.1, of 62 74.5 and 73.0; 40 x 40 rows of 31 16.2 and 16.2, of 15
+// 16.1 and 8.8; 96 x 96 x 97 319 and 242 us.  From 2^20 nodes on both forms are
+// timed (autotune).
+StepConfig default_step(const Lattice &L) {
+  if (run_ok(L) && 17LL * L.esk < 16LL * ((L.esk + 31) / 32 * 32))
+    return {kStepRun, L.nnodes < 152LL * kRunThreads * 8 ? 32 : kRunThreads};
+  return {1, 128};
+}
 }  // namespace slbc
 
 namespace {
@@ -509,9 +522,10 @@ int autotune(Lattice &L) {
 }
 
 int autotune_time(Lattice &L) {
-  // FP64/FP32: {rows per thread, threads along k}; BF16: {planes per block, 32}
-  static const int cand_fp[][2] = {{1, 64},  {1, 128}, {2, 64}, {2, 128}, {1, 256},
-                                   {2, 256}, {4, 64},  {4, 128}, {kStepVec4, kV4Threads}};
+  // FP64/FP32: {rows per thread, threads along k}, last the form of one
+  // storage only; BF16: {planes per block, 32}
+  const int cand_fp[][2] = {{1, 64},  {1, 128}, {2, 64},  {2, 128}, {1, 256}, {2, 256}, {4, 64}, {4, 128},
+                            {run_ok(L) ? kStepRun : kStepVec4, run_ok(L) ? kRunThreads : kV4Threads}};
   const bool bf = L.precision == 2;
   // BF16: powers of two, and the plane counts that fill one or two waves of
   // three blocks per SM evenly
@@ -528,11 +542,10 @@ int autotune_time(Lattice &L) {
     }
   }
   const int (*cand)[2] = bf ? cand_bf : cand_fp;
-  const int ncand = bf ? nbf : (vec4_ok(L) ? 9 : 8);
+  const int ncand = bf ? nbf : (vec4_ok(L) || run_ok(L) ? 9 : 8);
   const char *env = getenv("SLB_AUTOTUNE");
   for (int p = 0; p < 2; p++) {
-    L.tuned[p].npt = bf ? bf16_default_planes(L) : 1;
-    L.tuned[p].block_k = bf ? 32 : 128;
+    L.tuned[p] = bf ? StepConfig{bf16_default_planes(L), 32} : default_step(L);
   }
   if ((env && env[0] == '0') || L.nnodes < (1LL << 20) || L.esk < 64) {
     L.tune_state = -1;
@@ -934,12 +947,15 @@ int slbc_set_tuning(slbc_lattice *h, const int cfg[4]) {
       if (!vec4_ok(L) || bx != kV4Threads)
         return fail_msg("slbc_set_tuning: the 4-wide form needs FP32 populations, esk a multiple of 4 and "
                         "128 threads per block");
+    } else if (npt == kStepRun) {
+      if (!run_ok(L) || (bx != 32 && bx != 64 && bx != kRunThreads))
+        return fail_msg("slbc_set_tuning: the run form needs FP64 populations of fewer than 2^32 / 15 nodes and 32, "
+                        "64 or 128 threads per block");
     } else if ((npt != 1 && npt != 2 && npt != 4) || (bx != 32 && bx != 64 && bx != 128 && bx != 256)) {
       return fail_msg("slbc_set_tuning: rows per thread must be 1, 2 or 4 and threads along k 32, 64, 128 or 256");
     }
-    L.tuned[p].npt = npt;
-    L.tuned[p].block_k = bx;
   }
+  for (int p = 0; p < 2; p++) L.tuned[p] = StepConfig{cfg[2 * p], cfg[2 * p + 1]};
   L.tune_state = 1;
   L.generation++;
   return 0;

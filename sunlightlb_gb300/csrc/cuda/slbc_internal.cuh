@@ -50,11 +50,14 @@ constexpr uint16_t FLAG_LINKS = 0x7FFEu;
 // Launch shape of the fused step (chosen by the autotuner per parity).
 // npt = kStepVec4 selects the 128-bit form (FP32 populations, esk a
 // multiple of 4): 4 nodes along k per thread, block_k threads per block.
-constexpr int kStepVec4 = -4;
-constexpr int kV4Threads = 128;  // threads per block of the 4-wide form
+// kStepRun selects the run form (FP64 populations with 32-bit indices): the
+// nodes of a plane as one run, block_k threads per block.
+constexpr int kStepVec4 = -4, kStepRun = -1;
+constexpr int kV4Threads = 128;   // threads per block of the 4-wide form
+constexpr int kRunThreads = 128;  // threads per block of the run form, at most
 struct StepConfig {
-  int npt = 0;      // rows along j per thread (1, 2 or 4), or kStepVec4; 0 = not tuned
-  int block_k = 0;  // threads along k (threads per block for kStepVec4)
+  int npt = 0;      // rows along j per thread (1, 2 or 4), kStepVec4 or kStepRun; 0 = not tuned
+  int block_k = 0;  // threads along k (threads per block for kStepVec4 and kStepRun)
 };
 
 // Device state of one lattice.
@@ -139,9 +142,11 @@ struct Lattice {
   int tune_state = 0;         // 0 not tuned, 1 tuned, -1 tuning disabled
 };
 
-// whether the 128-bit form of the fused step applies to a lattice
-struct Lattice;
+// whether the 128-bit form and the run form of the fused step apply to a
+// lattice, and the launch shape of one that is not tuned
 bool vec4_ok(const Lattice &L);
+bool run_ok(const Lattice &L);
+StepConfig default_step(const Lattice &L);
 
 // Arguments shared by the population kernels.
 template <typename T>

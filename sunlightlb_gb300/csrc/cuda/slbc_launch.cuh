@@ -82,13 +82,11 @@ static void step_variant(Lattice &L, const StepArgs<T_> &a, int npt, int bx) {
     }
     return;
   }
-  // FP64 rows that leave more than 1/16 of their warps' lanes without a node
-  // go as runs over whole planes (32-bit indices only)
-  if (std::is_same<T_, double>::value && 15LL * L.npad <= 0xFFFFFFFFLL &&
-      17 * L.esk < 16 * ((L.esk + 31) / 32 * 32)) {
-    const int bs = L.nnodes < 152LL * 128 * 8 ? 32 : 128;
-    const dim3 run((unsigned)((L.esj * L.esk + bs - 1) / bs), 1, (unsigned)L.esi);
-    launch_pdl(k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU>, run, bs, 0, L.stream, a, odd_offsets(L));
+  if (npt == kStepRun) {  // the nodes of a plane as one run, bx threads per block
+    if constexpr (std::is_same<T_, double>::value) {
+      const dim3 run((unsigned)((L.esj * L.esk + bx - 1) / bx), 1, (unsigned)L.esi);
+      launch_pdl(k_step_run<T_, ODD, SLBC_EXACT, MOVING, BFU>, run, bx, 0, L.stream, a, odd_offsets(L));
+    }
     return;
   }
   const dim3 grid((unsigned)((L.esk + bx - 1) / bx), (unsigned)((L.esj + npt - 1) / npt), (unsigned)L.esi);
@@ -268,17 +266,17 @@ cudaError_t SLBC_FN(launch_tiles)(BatchState &B, const BatchState::Set &set, int
   return cudaSuccess;
 }
 
-// One fused step with the tuned (rows per thread, threads along k) of this
-// parity; small lattices use one row per thread and the block width that
-// fits esk.
+// One fused step in the launch shape chosen for this parity, or the default
+// one; rows take the block width that fits esk.
 cudaError_t SLBC_FN(launch_step)(Lattice &L, int odd) {
-  const StepConfig &c = L.tuned[odd ? 1 : 0];
+  StepConfig c = L.tuned[odd ? 1 : 0];
+  if (c.block_k <= 0) c = default_step(L);
+  if ((c.npt == kStepVec4 && !vec4_ok(L)) || (c.npt == kStepRun && !run_ok(L))) c = {1, 128};
   int bx = c.block_k, npt = c.npt;
-  if (bx <= 0) { bx = 128; npt = 1; }
-  if (npt == kStepVec4 && !vec4_ok(L)) npt = 1;
-  if (npt != kStepVec4)
+  if (npt > 0) {
     while (bx > 32 && bx / 2 >= L.esk) bx /= 2;
-  if (L.esj < 2) npt = 1;
+    if (L.esj < 2) npt = 1;
+  }
   StepArgs<T_> a = step_args(L);
   if (odd) step_dispatch<true>(L, a, npt, bx);
   else step_dispatch<false>(L, a, npt, bx);
