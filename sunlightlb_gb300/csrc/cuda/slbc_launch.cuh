@@ -11,6 +11,7 @@
 
 #include "slbc_kernels.cuh"
 #include "slbc_mp.cuh"
+#include "slbc_sets.cuh"
 #include "slbc_step_v4.cuh"
 
 #define SLBC_CAT2(a, b) a##_##b
@@ -179,17 +180,8 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
   return cudaSuccess;
 }
 
-// Tiles mode: descriptors and the tile table (rebuilt per batch step call).
-//
-// The lattices are independent, so they need not take each step together: a
-// set of them small enough to stay in L2 goes through all the steps of the
-// call before the next set starts, and only a set's first step reads it from
-// memory.  A batch that fits the L2 as a whole (up to kBatchWhole) is one
-// set; a larger one is cut into equal sets of at most kBatchSet (64 lattices,
-// 460 MB: 183 us per step in one set, 162 in sets of 64 MB; 16 lattices, 92
-// MB: 33 us in one set, 36 in two).
-constexpr long long kBatchWhole = 112LL << 20, kBatchSet = 64LL << 20;
-
+// Tiles mode: descriptors and the tile table by sets (rebuilt per batch step
+// call).
 cudaError_t SLBC_FN(prepare_tiles)(BatchState &B) {
   const int n = (int)B.lats.size();
   std::vector<BatchDom<T_>> h(n);
@@ -198,30 +190,27 @@ cudaError_t SLBC_FN(prepare_tiles)(BatchState &B) {
     h[d].a = step_args(*B.lats[d]);
     h[d].odd0 = B.lats[d]->layout == SLBC_LAYOUT_C0 ? 1 : 0;
   }
-  const auto state_bytes = [&](int d) { return B.lats[d]->nnodes * (15LL * (long long)sizeof(T_) + 2); };
-  long long total = 0, before = 0;
-  for (int d = 0; d < n; d++) total += state_bytes(d);
-  const long long nsets = total <= kBatchWhole ? 1 : (total + kBatchSet - 1) / kBatchSet;
+  std::vector<long long> bytes((size_t)n);
+  std::vector<int> cls((size_t)n);  // moving, uniform force, starting parity
+  for (int d = 0; d < n; d++) {
+    bytes[d] = B.lats[d]->nnodes * (15LL * (long long)sizeof(T_) + 2);
+    cls[d] = (h[d].a.moving ? 4 : 0) + (h[d].a.bf_uniform ? 2 : 0) + h[d].odd0;
+  }
   B.sets.clear();
-  for (int d0 = 0; d0 < n;) {
-    // lattices whose middle lies in this set's share of the state
-    const long long upto = total * ((long long)B.sets.size() + 1) / nsets;
-    int d1 = d0;
-    while (d1 < n && (d1 == d0 || before + state_bytes(d1) / 2 < upto)) before += state_bytes(d1++);
+  for (const std::vector<int> &members : batch_sets(bytes, cls)) {
     BatchState::Set set;
     set.first_tile = (long long)tiles.size();
     for (int c = 0; c < 4; c++) {
       for (int g = 0; g < 2; g++) {
         const size_t first = tiles.size();
-        for (int d = d0; d < d1; d++) {
-          if ((h[d].a.moving ? 2 : 0) + (h[d].a.bf_uniform ? 1 : 0) != c || h[d].odd0 != g) continue;
+        for (int d : members) {
+          if (cls[d] != 2 * c + g) continue;
           for (long long e = 0; e < B.lats[d]->nnodes; e += kBatchTile) tiles.push_back(make_int2(d, (int)e));
         }
         set.class_tiles[c][g] = (int)(tiles.size() - first);
       }
     }
     B.sets.push_back(set);
-    d0 = d1;
   }
   cudaError_t e = upload(B.doms, h.data(), n * sizeof(BatchDom<T_>), B.stream);
   if (e != cudaSuccess) return e;
