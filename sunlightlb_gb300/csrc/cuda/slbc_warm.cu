@@ -1503,44 +1503,49 @@ __global__ void k_sum_splits(const float *partial, long long n, int splits, floa
 // of a training iteration of 4 x 64^3.
 constexpr int kCmPos = 256, kCmPitch = 80;  // bytes per row of 32 channels: 8 rows hit 8 different bank groups
 
-template <int NC>
+//
+// I: 32-bit voxels and positions of a sample, and blocks of work, where they
+// fit it, else 64-bit.
+template <int NC, typename I>
 __global__ void __launch_bounds__(256) k_cmajor(const __nv_bfloat16 *src, int B, int D, int H, int W, int ctot, int coff,
-                                                int nch, int Wp, int pstride, int shift, int zero_halo, int copy, int ncopy,
-                                                long long copy_stride, __nv_bfloat16 *dst) {
+                                                int nch, int Wp, long long pstride, int shift, int zero_halo, int copy,
+                                                int ncopy, long long copy_stride, __nv_bfloat16 *dst) {
   after_previous();
   __shared__ __align__(16) unsigned char rows[(kCmPos + 3) * kCmPitch];  // positions -1 .. 256, and a row of zeros
-  __shared__ int voxel[kCmPos + 2];
-  __shared__ short xs[kCmPos + 2];
+  __shared__ I voxel[kCmPos + 2];
+  __shared__ int xs[kCmPos + 2];
   constexpr int kZero = kCmPos + 2;
-  const int plane = (H + 2) * Wp, per_sample = (D + 2) * plane;
+  const I plane = (I)(H + 2) * Wp, per_sample = (I)(D + 2) * plane;
   const long long total = (long long)B * pstride;
-  const int nblk = (int)((total + kCmPos - 1) / kCmPos), nck = (nch + 31) / 32;
+  const I nck = (nch + 31) / 32, works = (I)((total + kCmPos - 1) / kCmPos) * nck;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < kCmPitch / 4) ((unsigned *)(rows + kZero * kCmPitch))[threadIdx.x] = 0u;
-  for (int work = blockIdx.x; work < nblk * nck; work += gridDim.x) {
-    const int blk = work / nck, c0 = (work - blk * nck) * 32;
-    const int cw = min(32, nch - c0);
+  for (I work = blockIdx.x; work < works; work += gridDim.x) {
+    const I blk = work / nck;
+    const int c0 = (int)(work - blk * nck) * 32, cw = min(32, nch - c0);
     const long long e0 = (long long)blk * kCmPos;
     __syncthreads();
     for (int i = threadIdx.x; i < kCmPos + 2; i += 256) {
       const long long e = e0 + i - 1;
-      int v = -1, x = -0x4000;  // no voxel there
+      I v = -1;
+      int x = -0x4000;  // no voxel there
       if (e >= 0 && e < total) {
-        const int n = (int)(e / pstride), f = (int)(e - (long long)n * pstride);
+        const I n = (I)(e / pstride), f = (I)(e - n * pstride);
         if (f < per_sample) {
-          const int z = f / plane, r = f - z * plane, y = r / Wp;
-          x = r - y * Wp;
+          const I z = f / plane, r = f - z * plane, y = r / Wp;
+          x = (int)(r - y * Wp);
           bool in = x <= W + 1;
           if (zero_halo) in = in && x >= 1 && x <= W && y >= 1 && y <= H && z >= 1 && z <= D;
           if (in) v = ((n * (D + 2) + z) * (H + 2) + y) * (W + 2) + x;
         }
       }
       voxel[i] = v;
-      xs[i] = (short)x;
+      xs[i] = x;
     }
     __syncthreads();
     for (int a = threadIdx.x; a < (kCmPos + 2) * 4; a += 256) {
-      const int i = a >> 2, cv = a & 3, v = voxel[i];
+      const int i = a >> 2, cv = a & 3;
+      const I v = voxel[i];
       uint4 u = make_uint4(0, 0, 0, 0);
       if (v >= 0 && 8 * cv < cw) u = *(const uint4 *)(src + (long long)v * ctot + coff + c0 + 8 * cv);
       *(uint4 *)(rows + i * kCmPitch + 16 * cv) = u;
@@ -1680,19 +1685,16 @@ int cmajor_launch(const char *who, const void *src, int B, int D, int H, int W, 
     return slbc::set_error(std::string(who) + ": bad geometry"), 1;
   if (nch % 8 || coff % 8 || ctot % 8 || !aligned16(src) || !aligned16(dst))
     return slbc::set_error(std::string(who) + ": channels in multiples of 8, 16-byte aligned buffers"), 1;
-  if (pstride >= 1LL << 31 || (long long)B * (D + 2) * (H + 2) * (W + 2) >= 1LL << 31 || W >= 0x3fff)
-    return slbc::set_error(std::string(who) + ": grid too large"), 1;
   const long long work = ((long long)B * pstride + kCmPos - 1) / kCmPos * ((nch + 31) / 32);
-  if (work >= 1LL << 31) return slbc::set_error(std::string(who) + ": grid too large"), 1;
   const int blocks = (int)std::min<long long>(work, 152LL * 8);
   const auto go = [&](auto kernel) {
-    launch_pdl(kernel, blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16 *)src, B, D, H, W, ctot, coff,
-               nch, Wp,
-                                                     (int)pstride, shift, zero_halo, copy, ncopy, copy_stride,
-                                                     (__nv_bfloat16 *)dst);
+    launch_pdl(kernel, blocks, 256, 0, (cudaStream_t)stream, (const __nv_bfloat16 *)src, B, D, H, W, ctot, coff, nch,
+               Wp, pstride, shift, zero_halo, copy, ncopy, copy_stride, (__nv_bfloat16 *)dst);
   };
-  if (nc == 3) go(k_cmajor<3>);
-  else go(k_cmajor<1>);
+  // below 2^30: the walk over the work adds the grid without a wrap
+  const bool fits = std::max({pstride, (long long)B * (D + 2) * (H + 2) * (W + 2), work}) < 1LL << 30;
+  if (nc == 3) fits ? go(k_cmajor<3, int>) : go(k_cmajor<3, long long>);
+  else fits ? go(k_cmajor<1, int>) : go(k_cmajor<1, long long>);
   slbc::count_launch();
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(std::string(who) + ": " + cudaGetErrorString(e)), 1;
