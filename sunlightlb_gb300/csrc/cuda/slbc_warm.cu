@@ -1124,9 +1124,10 @@ struct WgradNArgs {
 constexpr int kWgnMaxRows = 288;
 constexpr int kWgnSmem = kStages * (kWgTileA + kWgnMaxRows * 128) + 1024;
 
-// Block decomposition of k_wgrad_n for (cin, cout); false when it does not
-// apply (cout not 32, 64 or 128).
-bool wgrad_n_plan(int cin, int cout, WgradNArgs &w) {
+// Block decomposition of k_wgrad_n and k_wgrad_f for (cin, cout); false when it
+// does not apply (cout not 32, 64 or 128).  Channels per block come in multiples
+// of `step` (k_wgrad_f: 32, the channels of its boxes).
+bool wgrad_n_plan(int cin, int cout, WgradNArgs &w, int step = 16) {
   if (!(cout == 32 || cout == 64 || cout == 128) || cin < 16 || cin % 16) return false;
   w.cin = cin;
   w.cout = cout;
@@ -1134,7 +1135,7 @@ bool wgrad_n_plan(int cin, int cout, WgradNArgs &w) {
   int cc = cin;
   if (cc > 256) {
     cc = 0;
-    for (int c = 256; c >= 16; c -= 16)
+    for (int c = 256; c >= step; c -= step)
       if (cin % c == 0) { cc = c; break; }
     if (!cc) return false;
   }
@@ -2025,7 +2026,7 @@ int slbc_tc_wgrad_flat(const void *dyf, const void *xf, int B, int D, int H, int
                        int cout, float *partial, long long partial_floats, int splits, float *dw, void *stream) {
   const std::string me = "slbc_tc_wgrad_flat";
   WgradNArgs w;
-  if (cin % 32 || !wgrad_n_plan(cin, cout, w) || w.cc % 32)
+  if (cin % 32 || !wgrad_n_plan(cin, cout, w, 32))
     return slbc::set_error(me + ": cout must be 32, 64 or 128, cin a multiple of 32"), 1;
   const long long rows = (long long)B * pstride;
   if (B < 1 || Wp < W + 2 || Wp % 8 || pstride % 64 || pstride < (long long)(D + 2) * (H + 2) * Wp || splits < 1 ||
