@@ -48,6 +48,7 @@ warmstart run the full-size forms of the legs.
 """
 
 import argparse
+import ctypes
 import json
 import math
 import os
@@ -136,6 +137,13 @@ class Clocks:
                           if len(s) > 5 + i and s[5 + i].lower() == "active"})
         return {"sm_mhz": statistics.median(sm) if sm else None,
                 "sm_max_mhz": max(mx) if mx else None, "reasons": reasons, "samples": len(self.samples)}
+
+
+def emit(line):
+    """The result on a line of its own: what the C library has printed may still
+    be in its buffer, flushed up to the middle of a line, and goes out first."""
+    ctypes.CDLL(None).fflush(None)
+    print(json.dumps(line), flush=True)
 
 
 def aggregate(total_ms, nodes, steps, world, dist=None, device=None):
@@ -232,7 +240,6 @@ def time_steps(torch, L, lb, steps, warmup, flusher=None, kinds=None):
 
 
 def tuning(L, lb):
-    import ctypes
     cfg = (ctypes.c_int * 4)()
     state = L.lbtuning(lb, ctypes.addressof(cfg))
     st = {1: "tuned", -1: "default", 0: "none"}.get(state, state)
@@ -401,7 +408,7 @@ def run_mine(args):
     }
     if not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_baseline(solid, budget_s=args.cpu_seconds)
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def run_e2e(L, precision, solid, intervals):
@@ -571,7 +578,7 @@ def run_reference(args):
                  "build": "the same restatement, LBReal double (the reference's default build)"},
         "e2e": {"value": round(v32, 3), "unit": "MLUPS", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 # ---- flow + passive scalar in a large packed bed ----------------------------
@@ -718,7 +725,7 @@ def run_tracer(args):
                               args.max_converge_steps))
     if not args.no_cpu_baseline:
         line["cpu_baseline"] = cpu_tracer_baseline(args.cpu_seconds)
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def tracer_leg(torch, L, args):
@@ -934,7 +941,7 @@ def run_batch(args):
     line = {"workload": f"batched ensemble: {args.domains} periodic moving-sphere domains, sides {list(BATCH_SIDES)}",
             "metric": "MLUPS of all domains together, batched vs one domain at a time"}
     line.update(out)
-    print(json.dumps(line), flush=True)
+    emit(line)
 
 
 def batch_leg(torch, L, args):
@@ -1124,7 +1131,7 @@ def run_warmstart(args):
                                                         if r[f"check50_{name}"]["warm_wall_s"])), 3)}
             for name in variants + tuple(f"correct{n}" for n in corrections)} if 50 in checks else None,
     }
-    print(json.dumps(line), flush=True)
+    emit(line)
     if args.save_weights:
         WS.save_weights(net, args.save_weights,
                         meta={"train_samples": args.train, "train_side": side, "epochs": args.epochs,
