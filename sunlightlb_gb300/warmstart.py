@@ -105,9 +105,21 @@ def pointers(addresses):
 
 
 def flat_geometry(D, H, W_):
-    """Row pitch and sample stride of the channel-major weight-gradient copies."""
+    """Row pitch and sample stride of the copies weight gradients are formed from."""
     Wp = (W_ + 2 + 7) // 8 * 8
     return Wp, ((D + 2) * (H + 2) * Wp + 63) // 64 * 64
+
+
+def weight_gradient(k, dy, x, B, D, H, W_, Wp, ps, cin, cout, *out):
+    """Weight gradient of a layer from the copies at dy and x (addresses): flat
+    ones that keep the channels last for cout <= 128, else channel-major ones,
+    of dY three, one per x shift.  out: workspace, its floats, splits, result,
+    stream."""
+    if cout <= 128:
+        k.tc_wgrad_flat(dy, x, B, D, H, W_, Wp, ps, cin, cout, *out)
+    else:
+        n = 2 * cout * B * ps  # bytes of one copy
+        k.tc_wgrad(dy, dy + n, dy + 2 * n, x, B, D, H, W_, Wp, ps, cin, cout, *out)
 
 
 class UNet:
@@ -297,14 +309,10 @@ class UNet:
         if cout <= 128:
             k.tc_flat(g.data_ptr(), *geom, g.shape[-1], 0, cout, Wp, ps, 0, self.cm_g.data_ptr(), self.stream)
             k.tc_flat(x.data_ptr(), *geom, x.shape[-1], x_coff, cin, Wp, ps, 1, self.cm_x.data_ptr(), self.stream)
-            k.tc_wgrad_flat(self.cm_g.data_ptr(), self.cm_x.data_ptr(), *geom, Wp, ps, cin, cout, *out)
         else:
-            n = cout * self.B * ps
-            cm_g = [self.cm_g[i * n:(i + 1) * n] for i in range(3)]
             k.tc_cmajor_shifts(g.data_ptr(), *geom, g.shape[-1], 0, cout, Wp, ps, 0, self.cm_g.data_ptr(), self.stream)
             k.tc_cmajor(x.data_ptr(), *geom, x.shape[-1], x_coff, cin, Wp, ps, 0, 1, self.cm_x.data_ptr(), self.stream)
-            k.tc_wgrad(cm_g[0].data_ptr(), cm_g[1].data_ptr(), cm_g[2].data_ptr(), self.cm_x.data_ptr(), *geom, Wp, ps,
-                       cin, cout, *out)
+        weight_gradient(k, self.cm_g.data_ptr(), self.cm_x.data_ptr(), *geom, Wp, ps, cin, cout, *out)
         p["gb"].zero_()
         k.nn_bias_grad(g.data_ptr(), g.shape[-1], 0, self.B, d, h, w, cout, p["gb"].data_ptr(), self.stream)
 
@@ -741,12 +749,11 @@ def conv_layer_times(lib, side, batch, widths=(32, 64, 128, 256), reps=20):
 
 
 def wgrad_layer_times(lib, side, batch, widths=(32, 64, 128, 256), reps=20):
-    """Weight-gradient time (slbc_tc_wgrad_tiles for cout <= 128, else
-    slbc_tc_wgrad, alone, from ready copies of dY and X; the split sum
-    included) of every layer shape of the network on
-    `batch` grids of side^3, CUDA events over `reps` calls on random BF16
-    data: [(level, cin, cout, splits, ms, TFLOP/s)], FLOPs 2 * 27 * cin *
-    cout * interior voxels."""
+    """Weight-gradient time (weight_gradient, what a training step launches,
+    alone, from ready copies of dY and X; the split sum included) of every
+    layer shape of the network on `batch` grids of side^3, CUDA events over
+    `reps` calls on random BF16 data: [(level, cin, cout, splits, ms,
+    TFLOP/s)], FLOPs 2 * 27 * cin * cout * interior voxels."""
     import torch
     k = Kernels(lib.dll)
     dev = torch.device("cuda")
@@ -764,17 +771,14 @@ def wgrad_layer_times(lib, side, batch, widths=(32, 64, 128, 256), reps=20):
         dys = torch.randn(3, cout, batch * ps, device=dev).to(torch.bfloat16)
         dw = torch.empty(27 * cout * cin, device=dev, dtype=torch.float32)
         splits = k.tc_wgrad_splits(cin, cout, batch * ps // 64, ws_floats // (27 * cout * cin))
-        tail = (batch, d, d, d, Wp, ps, cin, cout, ws.data_ptr(), ws_floats, splits, dw.data_ptr(), stream)
-        if cout <= 128:  # K-tile blocks, as UNet lays them out
-            fn, args = k.tc_wgrad_tiles, (dys.data_ptr(), xt.data_ptr()) + tail
-        else:
-            fn, args = k.tc_wgrad, (dys[0].data_ptr(), dys[1].data_ptr(), dys[2].data_ptr(), xt.data_ptr()) + tail
+        args = (k, dys.data_ptr(), xt.data_ptr(), batch, d, d, d, Wp, ps, cin, cout, ws.data_ptr(), ws_floats, splits,
+                dw.data_ptr(), stream)
         for _ in range(3):
-            fn(*args)
+            weight_gradient(*args)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         for _ in range(reps):
-            fn(*args)
+            weight_gradient(*args)
         e1.record()
         torch.cuda.synchronize()
         ms = e0.elapsed_time(e1) / reps
