@@ -122,6 +122,12 @@ def weight_gradient(k, dy, x, B, D, H, W_, Wp, ps, cin, cout, *out):
         k.tc_wgrad(dy, dy + n, dy + 2 * n, x, B, D, H, W_, Wp, ps, cin, cout, *out)
 
 
+def copy_elements(cin, cout, B, D, H, W_):
+    """Elements of the copies of a layer's input and of its output gradient."""
+    positions = B * flat_geometry(D, H, W_)[1]
+    return cin * positions, (1 if cout <= 128 else 3) * cout * positions
+
+
 class UNet:
     """The encoder-decoder on a batch of B grids D x H x W (powers of two,
     the coarsest level D*H*W/512 >= 128 voxels)."""
@@ -278,12 +284,9 @@ class UNet:
             "gB3": (3, w3), "gA3": (3, w3), "gP3": (3, w2),
         }
         self.grad = {n: self._act(lv, c) for n, (lv, c) in self.grad_spec.items()}
-        Wp, ps = flat_geometry(self.D, self.H, self.W)
-        maxc = max(c for _, c in self.buf_spec.values())
-        self.cm_x = torch.empty(maxc * self.B * ps, device=self.dev, dtype=torch.bfloat16)
-        # the flat copy of an output gradient (cout <= 128), else three
-        # channel-major copies, one per x shift
-        self.cm_g = torch.empty(3 * w3 * self.B * ps, device=self.dev, dtype=torch.bfloat16)
+        x, g = zip(*(copy_elements(cin, cout, self.B, *self.dims(lv)) for _, lv, cin, cout, *_ in self.layers))
+        self.cm_x = torch.empty(max(x), device=self.dev, dtype=torch.bfloat16)
+        self.cm_g = torch.empty(max(g), device=self.dev, dtype=torch.bfloat16)
         self.ws_floats = 1 << 26
         self.ws = torch.empty(self.ws_floats, device=self.dev, dtype=torch.float32)
         self.loss_acc = torch.zeros(1, device=self.dev, dtype=torch.float64)
