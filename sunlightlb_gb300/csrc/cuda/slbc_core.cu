@@ -778,18 +778,29 @@ __global__ void k_mp_ratios(const double *rho64, double rho0, double *rinv, doub
   ratio[x] = __ddiv_rn(rho0, r);
 }
 
+// Made with the first FP64 tracer, and filled with the density snapshot, so that
+// an update neither allocates nor depends on what was filled when it was last
+// called: it may be captured in a graph and replayed after another snapshot.
+// Without room on the GPU the update divides instead.
+cudaError_t alloc_mp_ratios(Lattice &L) {
+  if (L.mp_ratio64) return cudaSuccess;
+  cudaError_t e = cudaMalloc(&L.mp_rinv64, (size_t)L.nnodes * sizeof(double));
+  if (e == cudaSuccess) {
+    e = cudaMalloc(&L.mp_ratio64, (size_t)L.nnodes * sizeof(double));
+    if (e != cudaSuccess) cudaFree(L.mp_rinv64);
+  }
+  if (e == cudaSuccess) return e;
+  L.mp_rinv64 = L.mp_ratio64 = nullptr;
+  cudaGetLastError();
+  return e == cudaErrorMemoryAllocation ? cudaSuccess : e;
+}
+
 cudaError_t ensure_mp_ratios(Lattice &L) {
-  if (L.mp_rinv64 && L.mp_ratio64 && L.mp_ratio_gen == L.mp_rho_gen && L.mp_ratio_rho0 == L.par.rho0) return cudaSuccess;
-  if (!L.mp_rho64) return cudaErrorInvalidValue;
-  cudaError_t e = cudaSuccess;
-  if (!L.mp_rinv64) e = cudaMalloc(&L.mp_rinv64, (size_t)L.nnodes * sizeof(double));
-  if (e == cudaSuccess && !L.mp_ratio64) e = cudaMalloc(&L.mp_ratio64, (size_t)L.nnodes * sizeof(double));
-  if (e != cudaSuccess) return e;
+  if (!L.mp_ratio64 || (L.mp_ratio_gen == L.mp_rho_gen && L.mp_ratio_rho0 == L.par.rho0)) return cudaSuccess;
   launch_pdl(k_mp_ratios, (int)((L.nnodes + 255) / 256), 256, 0, L.stream, L.mp_rho64, L.par.rho0, L.mp_rinv64,
-             L.mp_ratio64,
-                                                                   L.nnodes);
+             L.mp_ratio64, L.nnodes);
   g_launches += 1;
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
     L.mp_ratio_gen = L.mp_rho_gen;
     L.mp_ratio_rho0 = L.par.rho0;
@@ -1617,6 +1628,8 @@ int slbc_mp_create(slbc_lattice *h, slbc_tracer **out, int use_f64) {
       e = cudaGetLastError();
     }
   }
+  if (e == cudaSuccess && use_f64) e = alloc_mp_ratios(L);
+  if (e == cudaSuccess) e = ensure_mp_ratios(L);
   if (e == cudaSuccess) e = cudaStreamSynchronize(L.stream);
   if (e != cudaSuccess) {
     slbc_mp_destroy(t);
@@ -1643,6 +1656,7 @@ int slbc_mp_rhoinit(slbc_lattice *h) {
   if (!L.mp_rho64) CK(cudaMalloc(&L.mp_rho64, (size_t)L.nnodes * sizeof(double)));
   CK(DISPATCH3(L, launch_mp_rhoinit, L));
   L.mp_rho_gen++;
+  CK(ensure_mp_ratios(L));
   return 0;
 }
 

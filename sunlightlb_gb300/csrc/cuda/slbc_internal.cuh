@@ -260,7 +260,8 @@ cudaError_t launch_mp_rhoinit_bf16(Lattice &L);
 // 1/rho of the density snapshot for FP32 tracers, rebuilt when stale
 // (slbc_core.cu)
 cudaError_t ensure_mp_rinv(Lattice &L);
-// 1/rho and rho0/rho of the snapshot for FP64 tracers, likewise
+// 1/rho and rho0/rho of the snapshot for FP64 tracers, where there was room for
+// them (null else)
 cudaError_t ensure_mp_ratios(Lattice &L);
 // planes a tracer block marches over
 int march_planes(const Lattice &L, int blocks_per_sm);

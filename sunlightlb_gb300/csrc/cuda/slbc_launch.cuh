@@ -533,15 +533,10 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
     attr_set[tp_f64 ? 1 : 0] |= bit;
   }
   if (tp_f64) {
-    const cudaError_t e = ensure_mp_ratios(L);
-    if (e == cudaSuccess) {
-      m.rinv = L.mp_rinv64;
-      m.rratio = L.mp_ratio64;
-    } else if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();  // the kernel divides instead
-    } else {
-      return e;
-    }
+    const cudaError_t e = ensure_mp_ratios(L);  // rho0 may have changed
+    if (e != cudaSuccess) return e;
+    m.rinv = L.mp_rinv64;
+    m.rratio = L.mp_ratio64;
   }
   const dim3 grid = tiling(tp_f64 ? 2 : 3);
   if (tp_f64)
