@@ -808,24 +808,9 @@ cudaError_t ensure_mp_ratios(Lattice &L) {
   return e;
 }
 
-// The march with the least work in whole waves of resident blocks, a block
-// costing its planes and the two it reads for its halo.  (Up to 8 planes with
-// four blocks per SM before: 96^3 in 864 blocks of 4 + 2 planes, now 288 of
-// 12 + 2 in one wave.)
 int march_planes(const Lattice &L, int blocks_per_sm) {
   const long long tiles = (long long)((L.esk + kTileK - 1) / kTileK) * ((L.esj + kTileJ - 1) / kTileJ);
-  const long long slots = 152LL * blocks_per_sm;
-  long long best = 0;
-  int planes = 1;
-  for (int chunks = 1; chunks <= L.esi; chunks++) {
-    const int p = (L.esi + chunks - 1) / chunks;
-    const long long waves = (tiles * ((L.esi + p - 1) / p) + slots - 1) / slots, cost = waves * (p + 2);
-    if (best == 0 || cost < best) {
-      best = cost;
-      planes = p;
-    }
-  }
-  return planes;
+  return march_planes(L.esi, tiles, 152LL * blocks_per_sm);
 }
 
 void count_launch(int n) { g_launches += n; }
