@@ -496,8 +496,7 @@ cudaError_t launch_get_bf16(Lattice &L, double *stage, long long x0, long long n
 
 cudaError_t launch_vsum_bf16(Lattice &L, double fac, const double *psi, double *partials, int nblocks) {
   launch_pdl(k_vsum_pair, nblocks, kReduceThreads, 0, L.stream, pair_args(L), L.par.rho0, fac, L.bf_uniform,
-                                                         L.bf_const[0], L.bf_const[1], L.bf_const[2],
-                                                         (const float *)L.bf, psi, partials);
+             L.bf_const[0], L.bf_const[1], L.bf_const[2], (const float *)L.bf, psi, partials);
   count_launch();
   return cudaGetLastError();
 }
@@ -513,9 +512,8 @@ cudaError_t launch_force_bf16(Lattice &L) {
 
 cudaError_t launch_setvel_bf16(Lattice &L, const double *stage, long long x0, long long n, int has_rho,
                                int skip_solid) {
-  launch_pdl(k_setvel_pair, fblocks(n, 256), 256, 0, L.stream, pair_args_inplace(L), stage, x0, n, has_rho,
-             L.par.rho0,
-                                                       L.par.stokes_flow, skip_solid);
+  launch_pdl(k_setvel_pair, fblocks(n, 256), 256, 0, L.stream, pair_args_inplace(L), stage, x0, n, has_rho, L.par.rho0,
+             L.par.stokes_flow, skip_solid);
   count_launch();
   return cudaGetLastError();
 }
@@ -535,7 +533,7 @@ cudaError_t launch_collide_bf16(Lattice &L) {
 
 cudaError_t launch_mp_rhoinit_bf16(Lattice &L) {
   launch_pdl(k_mp_rhoinit_pair, fblocks(L.nnodes, 256), 256, 0, L.stream, pair_args(L), L.par.rho0, L.mp_rho64,
-                                                                  L.mp_rho32);
+             L.mp_rho32);
   count_launch();
   return cudaGetLastError();
 }

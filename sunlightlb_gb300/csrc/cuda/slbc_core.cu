@@ -742,7 +742,7 @@ __global__ void k_mp_coef_norm(float *coef, const uint16_t *flags, int esi, int 
 
 cudaError_t launch_mp_coef_norm(Lattice &L) {
   launch_pdl(k_mp_coef_norm, (int)((L.nnodes + 255) / 256), 256, 0, L.stream, L.mp_coef, L.flags, L.esi, L.esj, L.esk,
-                                                                      (unsigned)L.npad);
+             (unsigned)L.npad);
   g_launches += 1;
   return cudaGetLastError();
 }
@@ -750,8 +750,7 @@ cudaError_t launch_mp_coef_norm(Lattice &L) {
 cudaError_t launch_mp_apply(Lattice &L, const float *pin, const float *lin, float *pout, float *lout, dim3 grid,
                             dim3 block, int planes) {
   launch_pdl(k_mp_apply, grid, block, 0, L.stream, L.mp_coef, pin, lin, pout, lout, L.esi, L.esj, L.esk,
-             (unsigned)L.npad,
-                                           planes);
+             (unsigned)L.npad, planes);
   g_launches += 1;
   return cudaGetLastError();
 }
@@ -1512,15 +1511,14 @@ int slbc_distribf(slbc_lattice *h, const double *pos, double *ft) {
   if (L.nobj == 0) return 0;
   CK(cudaMemcpyAsync(L.obj_pos, pos, 3 * (size_t)L.nobj * sizeof(double), cudaMemcpyHostToDevice, L.stream));
   if (L.npiece > 0) {
-    launch_pdl(k_distrib_piece, L.npiece, 256, 0, L.stream, L.bnd_node, L.bnd_f, L.nbnd, L.piece_obj,
-                                                   L.piece_lo, L.piece_hi, L.obj_pos, L.esj,
-                                                   L.esk, L.piece_sum);
+    launch_pdl(k_distrib_piece, L.npiece, 256, 0, L.stream, L.bnd_node, L.bnd_f, L.nbnd, L.piece_obj, L.piece_lo,
+               L.piece_hi, L.obj_pos, L.esj, L.esk, L.piece_sum);
     count_launch();
     CK(cudaGetLastError());
   }
   const int *first = (const int *)(L.obj_ft + 6 * L.nobj);
-  launch_pdl(k_distrib_obj, blocks_for(L.nobj, 4), 128, 0, L.stream, first, first + L.nobj, L.piece_sum,
-                                                               L.nobj, L.obj_ft);
+  launch_pdl(k_distrib_obj, blocks_for(L.nobj, 4), 128, 0, L.stream, first, first + L.nobj, L.piece_sum, L.nobj,
+             L.obj_ft);
   count_launch();
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(ft, L.obj_ft, 6 * (size_t)L.nobj * sizeof(double), cudaMemcpyDeviceToHost, L.stream));

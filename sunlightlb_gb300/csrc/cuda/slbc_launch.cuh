@@ -278,8 +278,7 @@ cudaError_t SLBC_FN(launch_force)(Lattice &L) {
   ForceArgs f{L.nbnd, L.bnd_node, L.bnd_f};
   const int bs = 128;
   const int moving = L.par.objects_moving && L.uw != nullptr;
-  launch_pdl(k_force<T_>, flat_blocks(L.nbnd, bs), bs, 0, L.stream, pop_args(L), L.layout, moving,
-                                                           (const T_ *)L.uw, f);
+  launch_pdl(k_force<T_>, flat_blocks(L.nbnd, bs), bs, 0, L.stream, pop_args(L), L.layout, moving, (const T_ *)L.uw, f);
   count_launch();
   return cudaGetLastError();
 }
@@ -287,9 +286,8 @@ cudaError_t SLBC_FN(launch_force)(Lattice &L) {
 cudaError_t SLBC_FN(launch_vsum)(Lattice &L, double fac, const double *psi, double *partials,
                                  int nblocks) {
   const auto go = [&](auto kernel) {
-    launch_pdl(kernel, nblocks, kReduceThreads, 0, L.stream, pop_args(L), L.par.rho0, fac, L.bf_uniform,
-               L.bf_const[0],
-                                                     L.bf_const[1], L.bf_const[2], (const T_ *)L.bf, psi, partials);
+    launch_pdl(kernel, nblocks, kReduceThreads, 0, L.stream, pop_args(L), L.par.rho0, fac, L.bf_uniform, L.bf_const[0],
+               L.bf_const[1], L.bf_const[2], (const T_ *)L.bf, psi, partials);
   };
   if (L.layout == SLBC_LAYOUT_N) go(k_vsum<T_, SLBC_LAYOUT_N>);
   else if (L.layout == SLBC_LAYOUT_C0) go(k_vsum<T_, SLBC_LAYOUT_C0>);
@@ -341,8 +339,8 @@ cudaError_t SLBC_FN(launch_bbl)(Lattice &L, int with_force) {
   if (L.nbnd == 0) return cudaSuccess;
   ForceArgs f{L.nbnd, L.bnd_node, L.bnd_f};
   const int moving = L.par.objects_moving && L.uw != nullptr;
-  launch_pdl(k_bbl_n<T_>, flat_blocks(L.nbnd, 128), 128, 0, L.stream, pop_args(L), moving,
-                                                              (const T_ *)L.uw, with_force, f);
+  launch_pdl(k_bbl_n<T_>, flat_blocks(L.nbnd, 128), 128, 0, L.stream, pop_args(L), moving, (const T_ *)L.uw, with_force,
+             f);
   count_launch();
   return cudaGetLastError();
 }
@@ -362,8 +360,8 @@ cudaError_t SLBC_FN(launch_collide)(Lattice &L) {
 
 cudaError_t SLBC_FN(launch_setvel)(Lattice &L, const double *stage, long long x0, long long n,
                                    int has_rho, int skip_solid) {
-  launch_pdl(k_setvel<T_, SLBC_EXACT>, flat_blocks(n, 256), 256, 0, L.stream,
-      pop_args(L), stage, x0, n, has_rho, L.par.rho0, L.par.stokes_flow, skip_solid);
+  launch_pdl(k_setvel<T_, SLBC_EXACT>, flat_blocks(n, 256), 256, 0, L.stream, pop_args(L), stage, x0, n, has_rho,
+             L.par.rho0, L.par.stokes_flow, skip_solid);
   count_launch();
   return cudaGetLastError();
 }
@@ -371,8 +369,7 @@ cudaError_t SLBC_FN(launch_setvel)(Lattice &L, const double *stage, long long x0
 cudaError_t SLBC_FN(launch_vacf_sums)(Lattice &L, double *p, const double *p2, const double *psi, double pmean,
                                       int axis, double *partials, int nblocks) {
   launch_pdl(k_vacf_sums<T_>, nblocks, kReduceThreads, 0, L.stream, pop_args(L), L.layout, L.mp_rho64, p, p2, psi,
-             pmean,
-                                                             axis, partials);
+             pmean, axis, partials);
   count_launch();
   return cudaGetLastError();
 }
@@ -420,8 +417,8 @@ cudaError_t SLBC_FN(launch_velocity)(Lattice &L, double fac, float *u, float *dr
 }
 
 cudaError_t SLBC_FN(launch_mp_rhoinit)(Lattice &L) {
-  launch_pdl(k_mp_rhoinit<T_>, flat_blocks(L.nnodes, 256), 256, 0, L.stream,
-      pop_args(L), L.layout, L.par.rho0, L.mp_rho64, L.mp_rho32);
+  launch_pdl(k_mp_rhoinit<T_>, flat_blocks(L.nnodes, 256), 256, 0, L.stream, pop_args(L), L.layout, L.par.rho0,
+             L.mp_rho64, L.mp_rho32);
   count_launch();
   return cudaGetLastError();
 }

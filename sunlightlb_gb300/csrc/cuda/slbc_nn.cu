@@ -984,9 +984,8 @@ int slbc_nn_proj(const float *pred, int ctot_p, const float *label, int lch, int
   const dim3 g1((unsigned)std::min<long long>((per + 255) / 256, 152), (unsigned)B);
   launch_pdl(k_proj_dot, g1, 256, 0, st, pred, ctot_p, label, lch, nch, D, H, W, dot);
   if (launched("slbc_nn_proj")) return 1;
-  launch_pdl(k_proj_grad, std::min(grid_for((long long)B * per), 152 * 4), 256, 0, st, label, lch, nch, lab_sq, dot,
-             B, D, H,
-                                                                                W, weight, (bf16 *)grad, gctot, loss);
+  launch_pdl(k_proj_grad, std::min(grid_for((long long)B * per), 152 * 4), 256, 0, st, label, lch, nch, lab_sq, dot, B,
+             D, H, W, weight, (bf16 *)grad, gctot, loss);
   return launched("slbc_nn_proj");
 }
 

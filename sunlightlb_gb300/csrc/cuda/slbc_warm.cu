@@ -1764,7 +1764,7 @@ int wgrad_launch(const char *who, const void *dy0, const void *dy1, const void *
     if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
     const long long n = 27LL * cout * cin;
     launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream,
-        partial, n, splits, dw);
+               partial, n, splits, dw);
     slbc::count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
@@ -1801,8 +1801,8 @@ int wgrad_launch(const char *who, const void *dy0, const void *dy1, const void *
   e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
   const long long n = 27LL * cout * cin;
-  launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream,
-      partial, n, splits, dw);
+  launch_pdl(k_sum_splits, (int)std::min<long long>((n + 255) / 256, 152LL * 8), 256, 0, (cudaStream_t)stream, partial,
+             n, splits, dw);
   slbc::count_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess) return slbc::set_error(me + ": " + cudaGetErrorString(e)), 1;
