@@ -301,9 +301,8 @@ __device__ __forceinline__ long long plane_node(long long e, int axis, int pos, 
 // set to its own slot of acc, so the host layer can keep count of the tracer
 // the fills have added (slbc_mp_injected adds the slots in order).  Bound:
 // latency; flags and values are loaded together, and no block waits for
-// another.  Measured, a plane of 256^3 on a frozen flow: 10.3 -> 8.2 us, where a
-// last block added the blocks' sums behind a fence and a counter (before that,
-// in a launch of its own).
+// another.  Measured, a plane of 256^3 on a frozen flow: 8.2 us, 10.3 with a last
+// block that adds the blocks' sums behind a fence.
 template <typename TP>
 __global__ void __launch_bounds__(kReduceThreads)
 k_mp_fill(TP *p, float *lo, const uint16_t *flags, int esi, int esj, int esk, int kind, double g0, double g1,

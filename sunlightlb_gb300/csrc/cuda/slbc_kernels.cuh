@@ -508,10 +508,12 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(const BatchDom<T> *d
 // domain's first step, so one launch has one parity (ODD) and carries the
 // code of that parity only (64 registers, four blocks per SM).  The domain's
 // arguments come in a word per thread, and the pull-and-push update keeps
-// each 32-bit index for both directions (odd_places): 187 -> 162 us per step
-// of 64 FP32 lattices of sides 24 to 64 with the sets of prepare_tiles.
-// Slower: blocks that walk through the tiles with a barrier per tile (169),
-// all arguments in the tile table (180).
+// each 32-bit index for both directions (odd_places).  Bound: latency, in a set
+// that stays in L2 as in one read from memory (39-41% of the warps, no unit above
+// 41%).  Measured, 64 FP32 lattices of sides 24 to 64: 187 -> 162 us per step with
+// the sets of batch_sets, before launches overlapped; slower then were blocks that
+// walk through the tiles with a barrier per tile (169) and all arguments in the
+// tile table (180).  Now 105 in sets, 148 in one.
 constexpr int kBatchTile = 256;
 
 template <typename T, bool ODD, bool EXACT, bool MOVING, bool BFU>

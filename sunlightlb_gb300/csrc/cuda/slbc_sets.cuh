@@ -14,9 +14,11 @@ namespace slbc {
 // together: a set of them small enough to stay in L2 goes through all the steps
 // of the call before the next set starts, and only a set's first step reads it
 // from memory.  A batch that fits the L2 as a whole (up to kBatchWhole) is one
-// set; a larger one is cut into equal sets of at most kBatchSet (64 lattices,
-// 460 MB: 183 us per step in one set, 162 in sets of 64 MB; 16 lattices, 92
-// MB: 33 us in one set, 36 in two).
+// set, whose steps are replayed from a graph; a larger one is cut into equal sets
+// of at most kBatchSet.  Measured, FP32, per step: 64 lattices of 48^3 (419 MB)
+// 161 us in one set, 134 in sets of 96 MB, 115 in sets of 64 MB; 16 of 45^3 (86
+// MB) 29.0 in one set, 25.5 in two (before launches overlapped 16 lattices of 92
+// MB took 33 in one and 36 in two, where the line comes from).
 constexpr long long kBatchWhole = 112LL << 20, kBatchSet = 64LL << 20;
 
 // The members of each set from the bytes of state per member and the member's

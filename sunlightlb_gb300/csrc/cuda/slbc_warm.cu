@@ -1314,8 +1314,10 @@ k_wgrad_n(const __grid_constant__ CUtensorMap a0, const __grid_constant__ CUtens
 //
 // Against k_wgrad_n it stages 40 instead of 48 KB per K tile at 32 channels, and
 // the copies are one pass each without a transpose, one of dY instead of three.
-// Bound: staging (L2 to shared memory).  Measured, the 13 layers of a training
-// iteration of 4 x 64^3: 1228 -> 735 us, their copies 835 -> 451 us.
+// Bound: the tensor pipe (71-83% active at 32 output channels on 4 x 64^3, with
+// L2 at 69% and shared memory at 67-78%; 61% at 64 on 4 x 32^3).  Measured, the
+// 13 layers of a training iteration of 4 x 64^3: 1228 -> 735 us, their copies 835
+// -> 451 us.
 constexpr int kWgfTileA = 72 * 128 * 2;
 constexpr int kWgfSmem = kStages * (kWgfTileA + kWgnMaxRows * 128) + 1024;
 
