@@ -823,7 +823,7 @@ def advance(L, lbs, specs, steps, every, batch=None):
 
 def batch_result(torch, L, ndom, steps, cpu_subset=0, persistent=True, clocks=True, translate_every=0):
     """Many independent moving-sphere domains advanced together (batchsteps,
-    packed tiles, one launch per step from a CUDA graph) against the same
+    packed tiles, in sets that fit the L2) against the same
     domains one at a time (lbsteps per domain), per-domain drag compared;
     optionally the other batch mode and a seeded subset against the CPU
     oracle (FP64).  With translate_every > 0 the spheres really move: every
@@ -879,7 +879,7 @@ def batch_result(torch, L, ndom, steps, cpu_subset=0, persistent=True, clocks=Tr
                                (f", spheres re-rasterised at their new centres every {translate_every} steps "
                                 "(lbtranslate)" if translate_every > 0 else " on the fixed node map")},
         "build_s": round(t_build, 1),
-        "batched": {"mode": "packed tiles, one launch per step, CUDA graph", "wall_s": round(t_batch, 3),
+        "batched": {"mode": "packed tiles, sets that fit the L2, one launch per class and step", "wall_s": round(t_batch, 3),
                     "MLUPS": round(nodes * steps / t_batch / 1e6, 1), "hbm_gbs": round(gbs, 1),
                     "frac_of_measured_hbm": round(gbs / peak, 4), "gpu_launches": launches,
                     "clocks": clk.summary() if clk else None},

@@ -407,8 +407,9 @@ LBBatch newbatch(void);
 void batchadd(LBBatch, LBSys);
 void batchsteps(LBBatch, int);
 int batchsize(LBBatch);
-/* 0 (default): one launch per step over the packed cell index of all the
- * lattices, replayed from a CUDA graph; 1: one persistent launch for all
+/* 0 (default): launches over the packed cell index of all the lattices, a step
+ * at a time (a batch larger than the L2 goes through the steps of a call set by
+ * set); 1: one persistent launch for all
  * the steps, every GPU block owning whole lattices. */
 void batchmode(LBBatch, int);
 void freebatch(LBBatch);
