@@ -63,8 +63,8 @@ void for_rows(long long rows, F go) {
 }
 
 template <typename I>
-__device__ __forceinline__ slbc::RowWalk<I> walk(int rowlen) {
-  return slbc::row_walk<I>(blockIdx.x, gridDim.x, threadIdx.x, (unsigned)rowlen);
+__device__ __forceinline__ slbc::RowTurns<I> walk(I rows, int rowlen) {
+  return slbc::row_turns<I>(blockIdx.x, gridDim.x, threadIdx.x, rows, (unsigned)rowlen);
 }
 
 // 2x2x2 average of the fine interior (D, H, W) into the coarse interior
@@ -72,14 +72,15 @@ template <typename I>
 __global__ void __launch_bounds__(256) k_pool(Slice in, Slice out, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const auto w = walk<I>(len);
-  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
+  const auto w = walk<I>((I)B * (I)Dc * (I)Hc, len);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, Dc, Hc, n, z, y);
+    row_of(part.row, Dc, Hc, n, z, y);
     const bf16 *src = in.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * in.ctot + in.coff;
     bf16 *dst = out.p + vox(n, z, y, 0, Dc, Hc, Wc) * out.ctot + out.coff;
     const long long py = (long long)(W + 2) * in.ctot, pz = (H + 2) * py;
-    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+    for (unsigned e = part.e; e < part.end; e += 256) {
       const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -103,13 +104,14 @@ __global__ void __launch_bounds__(256) k_pool_bwd(Slice dcoarse, Slice dfine, Sl
                                                   int H, int W, int C) {
   after_previous();
   const int nv = C / 8, len = W * nv;
-  const auto w = walk<I>(len);
-  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
+  const auto w = walk<I>((I)B * (I)D * (I)H, len);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, D, H, n, z, y);
+    row_of(part.row, D, H, n, z, y);
     const bf16 *src = dcoarse.p + vox(n, z / 2, y / 2, 0, D / 2, H / 2, W / 2) * dcoarse.ctot + dcoarse.coff;
     const long long v0 = vox(n, z, y, 0, D, H, W);
-    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+    for (unsigned e = part.e; e < part.end; e += 256) {
       const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float g[8];
       load8(src + (long long)(x / 2) * dcoarse.ctot + 8 * cv, g);
@@ -139,14 +141,15 @@ template <typename I>
 __global__ void __launch_bounds__(256) k_up(Slice in, Slice out, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const auto w = walk<I>(len);
-  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
+  const auto w = walk<I>((I)B * (I)Dc * (I)Hc, len);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, Dc, Hc, n, z, y);
+    row_of(part.row, Dc, Hc, n, z, y);
     const bf16 *src = in.p + vox(n, z, y, 0, Dc, Hc, Wc) * in.ctot + in.coff;
     bf16 *dst = out.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * out.ctot + out.coff;
     const long long py = (long long)(W + 2) * out.ctot, pz = (H + 2) * py;
-    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+    for (unsigned e = part.e; e < part.end; e += 256) {
       const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       const uint4 v = *(const uint4 *)(src + (long long)x * in.ctot + 8 * cv);
 #pragma unroll
@@ -161,14 +164,15 @@ template <typename I>
 __global__ void __launch_bounds__(256) k_up_bwd(Slice dfine, Slice dcoarse, Slice mask, int B, int D, int H, int W, int C) {
   after_previous();
   const int Dc = D / 2, Hc = H / 2, Wc = W / 2, nv = C / 8, len = Wc * nv;
-  const auto w = walk<I>(len);
-  for (I row = w.row; row < (I)B * (I)Dc * (I)Hc; row += w.step) {
+  const auto w = walk<I>((I)B * (I)Dc * (I)Hc, len);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, Dc, Hc, n, z, y);
+    row_of(part.row, Dc, Hc, n, z, y);
     const bf16 *src = dfine.p + vox(n, 2 * z, 2 * y, 0, D, H, W) * dfine.ctot + dfine.coff;
     const long long py = (long long)(W + 2) * dfine.ctot, pz = (H + 2) * py;
     const long long v0 = vox(n, z, y, 0, Dc, Hc, Wc);
-    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+    for (unsigned e = part.e; e < part.end; e += 256) {
       const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -366,14 +370,15 @@ __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, cons
   __shared__ double sh[256];
   const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   double acc = 0.0;
-  const auto w = walk<I>(W);
-  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
+  const auto w = walk<I>((I)B * (I)D * (I)H, W);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, D, H, n, z, y);
-    const long long v0 = vox(n, z, y, 0, D, H, W), e0 = (long long)row * W;
+    row_of(part.row, D, H, n, z, y);
+    const long long v0 = vox(n, z, y, 0, D, H, W), e0 = (long long)part.row * W;
     const float sw = sample_w ? sample_w[n] : 1.0f;
-    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
-      const int x = (int)turn;
+    for (unsigned e = part.e; e < part.end; e += 256) {
+      const int x = (int)e;
       const long long v = v0 + x;
       bf16 *gp = grad + v * gctot;
       for (int c = 0; c < gctot; c += 8) *(uint4 *)(gp + c) = make_uint4(0, 0, 0, 0);
@@ -462,12 +467,13 @@ constexpr int kDistR1 = 5, kDistR2 = 12;
 template <int R, typename I>
 __global__ void __launch_bounds__(256) k_dist_x(const unsigned char *solid, I rows, int W, unsigned char *a) {
   after_previous();
-  const auto w = walk<I>(W);
-  for (I row = w.row; row < rows; row += w.step) {
-    const unsigned char *src = solid + (long long)row * W;
-    unsigned char *dst = a + (long long)row * W;
-    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
-      const int x = (int)turn;
+  const auto w = walk<I>(rows, W);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
+    const unsigned char *src = solid + (long long)part.row * W;
+    unsigned char *dst = a + (long long)part.row * W;
+    for (unsigned e = part.e; e < part.end; e += 256) {
+      const int x = (int)e;
       int best = src[x] ? 0 : R * R;
       if (W >= R) {
         for (int d = 1; d < R && best == R * R; d++) {
@@ -540,13 +546,14 @@ __global__ void __launch_bounds__(256) k_encode(const unsigned char *solid, cons
                                                 int D, int H, int W, bf16 *out, int ctot) {
   after_previous();
   const int nv = ctot / 8, len = W * nv;
-  const auto w = walk<I>(len);
-  for (I row = w.row; row < (I)B * (I)D * (I)H; row += w.step) {
+  const auto w = walk<I>((I)B * (I)D * (I)H, len);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, D, H, n, z, y);
+    row_of(part.row, D, H, n, z, y);
     bf16 *dst = out + vox(n, z, y, 0, D, H, W) * ctot;
-    const long long e0 = (long long)row * W;
-    for (unsigned e = w.e; e < (unsigned)len; e += 256) {
+    const long long e0 = (long long)part.row * W;
+    for (unsigned e = part.e; e < part.end; e += 256) {
       const int x = (int)(e / (unsigned)nv), cv = (int)e - x * nv;
       uint4 u = make_uint4(0, 0, 0, 0);
       if (cv == 0) {
@@ -576,14 +583,15 @@ __global__ void __launch_bounds__(256) k_decode(const float *pred, int ctot_p, c
                                                 float *drho) {
   after_previous();
   const long long total = (long long)D * H * W;
-  const auto w = walk<I>(W);
-  for (I row = w.row; row < (I)D * (I)H; row += w.step) {
+  const auto w = walk<I>((I)D * (I)H, W);
+  for (I turn = w.first; turn < w.turns; turn += w.step) {
+    const auto part = w.piece(turn);
     int n, z, y;
-    row_of(row, D, H, n, z, y);
+    row_of(part.row, D, H, n, z, y);
     const float *src = pred + vox(0, z, y, 0, D, H, W) * ctot_p;
-    for (unsigned turn = w.e; turn < (unsigned)W; turn += 256) {
-      const int x = (int)turn;
-      const long long e = (long long)row * W + x;
+    for (unsigned turn_e = part.e; turn_e < part.end; turn_e += 256) {
+      const int x = (int)turn_e;
+      const long long e = (long long)part.row * W + x;
       const float *v = src + (long long)x * ctot_p;
       const bool s = solid[e] != 0;
 #pragma unroll
