@@ -361,14 +361,15 @@ __global__ void __launch_bounds__(256) k_scale(const __grid_constant__ TensorLis
 // loss = mean over voxels and the nch components of (pred - label)^2, pred
 // in FP32 channels 0..nch-1 of a padded buffer (ctot_p channels), label
 // [n][D][H][W][nch] FP32; grad (BF16, gctot channels, padded) = d loss /
-// d pred in channels 0..nch-1, 0 in the others.  loss[0] += the sum / count.
+// d pred in channels 0..nch-1, 0 in the others.  loss[0] += the sum / count (inv:
+// 1 / count).  Bound: the FP64 sums, so no thread divides in FP64 and the blocks
+// are few (a division per thread and twice the blocks: 67 us on 4 x 64^3, 55 so).
 template <typename I>
 __global__ void __launch_bounds__(256) k_mse(const float *pred, int ctot_p, const float *label, int nch,
                                              const float *sample_w, int B, int D, int H, int W, bf16 *grad, int gctot,
-                                             double *loss) {
+                                             double *loss, double inv) {
   after_previous();
   __shared__ double sh[256];
-  const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   double acc = 0.0;
   const auto w = walk<I>((I)B * (I)D * (I)H, W);
   for (I turn = w.first; turn < w.turns; turn += w.step) {
@@ -975,9 +976,10 @@ int slbc_nn_mse(const float *pred, int ctot_p, const float *label, int nch, cons
   if (nch < 1 || ctot_p < nch || gctot % 8 || gctot < 8 || gctot < nch) return bad("slbc_nn_mse: bad channel counts");
   if (empty(B, D, H, W)) return bad("slbc_nn_mse: empty grid");
   const long long rows = (long long)B * D * H;
+  const double inv = 1.0 / ((double)nch * ((double)B * D * H * W));
   for_rows(rows, [&](auto i) {
-    launch_pdl(k_mse<decltype(i)>, std::min(rows_grid(rows, W), 152 * 8), 256, 0, (cudaStream_t)stream, pred, ctot_p,
-               label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss);
+    launch_pdl(k_mse<decltype(i)>, std::min(rows_grid(rows, W), 152 * 4), 256, 0, (cudaStream_t)stream, pred, ctot_p,
+               label, nch, sample_w, B, D, H, W, (bf16 *)grad, gctot, loss, inv);
   });
   return launched("slbc_nn_mse");
 }
