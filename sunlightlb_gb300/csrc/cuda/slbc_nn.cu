@@ -226,27 +226,40 @@ __global__ void __launch_bounds__(256) k_bias_grad(Slice g, int B, int D, int H,
 
 // The optimiser's kernels take lists of tensors: a network has 30 of them, most
 // so small that a launch each (4.2 us) was most of their time.  A block takes
-// kListBlock elements of one tensor and finds it in the table of first blocks,
-// which comes with the launch.  Bound: HBM for the large tensors.  Measured on
-// the default network: Adam 126 -> 47 us, squares 120 -> 33 us, layouts about
-// 125 -> 37 us, scaling 30 launches -> 1 of 2.8 us.
+// `block` elements of one tensor and finds it in the table of first blocks,
+// which comes with the launch: kListBlock of them, or 256 where the blocks of the
+// whole list then fit the GPU at once (Adam on 27,648 elements: 4.0 us, 4.8 in
+// blocks of 2048).  Bound: HBM for the large tensors.  Measured on the default
+// network: Adam 126 -> 47 us, squares 120 -> 33 us, layouts about 125 -> 37 us,
+// scaling 30 launches -> 1 of 2.8 us.
 constexpr int kListMax = 48, kListBlock = 2048;
 
 struct TensorList {
   float *p[4][kListMax];
   long long n[kListMax];
   unsigned first[kListMax];  // first block of each tensor
-  int count;
+  int count, block;
 };
 
 // Block decomposition of `count` (<= kListMax) element counts; the blocks in all.
-unsigned list_blocks(int count, const long long *n, unsigned *first) {
-  unsigned blocks = 0;
+// Where blocks end in a sum (most: blocks it should not exceed, 0 for none), large
+// lists take more elements per block: 30 M squares 152 -> 116 us.
+unsigned list_blocks(int count, const long long *n, unsigned *first, int &block, long long most = 0) {
+  const auto cut = [&](long long elements) {
+    long long blocks = 0;
+    for (int t = 0; t < count; t++) blocks += (n[t] + elements - 1) / elements;
+    return blocks;
+  };
+  const long long blocks = cut(kListBlock);
+  block = kListBlock;
+  if (cut(256) <= 152 * 8) block = 256;
+  else if (most > 0 && blocks > most) block = (int)std::min<long long>((blocks + most - 1) / most, 1024) * kListBlock;
+  unsigned at = 0;
   for (int t = 0; t < count; t++) {
-    first[t] = blocks;
-    blocks += (unsigned)((n[t] + kListBlock - 1) / kListBlock);
+    first[t] = at;
+    at += (unsigned)((n[t] + block - 1) / block);
   }
-  return blocks;
+  return at;
 }
 
 __device__ __forceinline__ int list_tensor(const unsigned *first, int count) {
@@ -257,12 +270,14 @@ __device__ __forceinline__ int list_tensor(const unsigned *first, int count) {
 
 // f(i) for the elements of this block of its tensor
 template <typename F>
-__device__ __forceinline__ void list_elements(unsigned first, long long n, F f) {
-  const long long i0 = (long long)(blockIdx.x - first) * kListBlock;
+__device__ __forceinline__ void list_elements(unsigned first, long long n, int block, F f) {
+  const long long i0 = (long long)(blockIdx.x - first) * block + threadIdx.x;
+  for (int k0 = 0; k0 < block; k0 += kListBlock) {
 #pragma unroll
-  for (int k = 0; k < kListBlock / 256; k++) {
-    const long long i = i0 + k * 256 + threadIdx.x;
-    if (i < n) f(i);
+    for (int k = 0; k < kListBlock; k += 256) {
+      const long long i = i0 + k0 + k;
+      if (k0 + k < block && i < n) f(i);
+    }
   }
 }
 
@@ -275,7 +290,7 @@ struct LayoutList {
   bf16 *w[kListMax];
   int cout[kListMax], cin[kListMax], ci0[kListMax], nci[kListMax];  // nci 0: forward
   unsigned first[kListMax];
-  int count;
+  int count, block;
 };
 
 __global__ void __launch_bounds__(256) k_layouts(const __grid_constant__ LayoutList L) {
@@ -284,7 +299,7 @@ __global__ void __launch_bounds__(256) k_layouts(const __grid_constant__ LayoutL
   const float *m = L.m[t];
   bf16 *w = L.w[t];
   const unsigned cout = L.cout[t], cin = L.cin[t], ci0 = L.ci0[t], nci = L.nci[t];
-  list_elements(L.first[t], 27LL * cout * (nci ? nci : cin), [&](long long e) {
+  list_elements(L.first[t], 27LL * cout * (nci ? nci : cin), L.block, [&](long long e) {
     const unsigned j = (unsigned)e & 31u;
     unsigned r = (unsigned)(e >> 5);
     const unsigned c = r % (nci ? nci : cout);
@@ -301,7 +316,7 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ TensorList
   const int t = list_tensor(L.first, L.count);
   float *p = L.p[0][t], *m = L.p[2][t], *v = L.p[3][t];
   const float *g = L.p[1][t];
-  list_elements(L.first[t], L.n[t], [&](long long i) {
+  list_elements(L.first[t], L.n[t], L.block, [&](long long i) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
@@ -317,17 +332,17 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ TensorList
 // running norm (0 before the first call); state[2]: the scale to apply.
 __global__ void __launch_bounds__(256) k_sqsum(const __grid_constant__ TensorList L, double *state) {
   after_previous();
-  __shared__ double sh[8];
+  __shared__ double sh[256];
   const int t = list_tensor(L.first, L.count);
   const float *g = L.p[0][t];
   double s = 0.0;
-  list_elements(L.first[t], L.n[t], [&](long long i) { s += (double)g[i] * g[i]; });
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  list_elements(L.first[t], L.n[t], L.block, [&](long long i) { s += (double)g[i] * g[i]; });
+  sh[threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < 8; i++) s += sh[i];
-    atomicAdd(state, s);
+  if (threadIdx.x < 32) {  // one warp adds for all: the FP64 pipe is what this kernel waits for
+    for (int i = 32; i < 256; i += 32) s += sh[threadIdx.x + i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) atomicAdd(state, s);
   }
 }
 
@@ -355,7 +370,7 @@ __global__ void __launch_bounds__(256) k_scale(const __grid_constant__ TensorLis
   if (sc == 1.0f) return;
   const int t = list_tensor(L.first, L.count);
   float *g = L.p[0][t];
-  list_elements(L.first[t], L.n[t], [&](long long i) { g[i] = sc == 0.0f ? 0.0f : g[i] * sc; });
+  list_elements(L.first[t], L.n[t], L.block, [&](long long i) { g[i] = sc == 0.0f ? 0.0f : g[i] * sc; });
 }
 
 // loss = mean over voxels and the nch components of (pred - label)^2, pred
@@ -799,7 +814,8 @@ int bad(const char *msg) {
 // `arrays` pointer arrays of `count` tensors each, in launches of kListMax:
 // go(list, blocks)
 template <typename F>
-int tensor_lists(const char *who, int count, const long long *n, int arrays, const void *const *const *ptrs, F go) {
+int tensor_lists(const char *who, int count, const long long *n, int arrays, const void *const *const *ptrs, F go,
+                 long long most = 0) {
   for (int t = 0; t < count; t++)
     if (n[t] <= 0) return bad((std::string(who) + ": empty tensor").c_str());
   for (int t0 = 0; t0 < count; t0 += kListMax) {
@@ -809,7 +825,7 @@ int tensor_lists(const char *who, int count, const long long *n, int arrays, con
       for (int a = 0; a < arrays; a++) L.p[a][t] = (float *)ptrs[a][t0 + t];
       L.n[t] = n[t0 + t];
     }
-    const unsigned blocks = list_blocks(L.count, L.n, L.first);
+    const unsigned blocks = list_blocks(L.count, L.n, L.first, L.block, most);
     go(L, blocks);
     if (launched(who)) return 1;
   }
@@ -909,7 +925,7 @@ int slbc_nn_layouts(int count, const float *const *master, const int *cout, cons
       L.nci[t] = nci[t0 + t];
       n[t] = 27LL * L.cout[t] * (L.nci[t] ? L.nci[t] : L.cin[t]);
     }
-    const unsigned blocks = list_blocks(L.count, n, L.first);
+    const unsigned blocks = list_blocks(L.count, n, L.first, L.block);
     launch_pdl(k_layouts, blocks, 256, 0, (cudaStream_t)stream, L);
     if (launched("slbc_nn_layouts")) return 1;
   }
@@ -947,7 +963,7 @@ int slbc_nn_sqsum_list(int count, const float *const *g, const long long *n, dou
   const void *const *ptrs[1] = {(const void *const *)g};
   return tensor_lists("slbc_nn_sqsum", count, n, 1, ptrs, [&](const TensorList &L, unsigned blocks) {
     launch_pdl(k_sqsum, blocks, 256, 0, (cudaStream_t)stream, L, state);
-  });
+  }, 152 * 32);
 }
 
 int slbc_nn_sqsum(const float *g, long long n, double *state, void *stream) {
