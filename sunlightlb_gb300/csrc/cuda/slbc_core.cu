@@ -806,9 +806,20 @@ cudaError_t ensure_mp_ratios(Lattice &L) {
   return e;
 }
 
-int march_planes(const Lattice &L, int blocks_per_sm) {
+// FP32 tracers between fixed walls take whole waves of long marches (160 x 120 x
+// 140: 304 us, with at most 8 planes 322), on a frozen flow twice the waves where
+// they cost little more (128^3 34.0 us with 15 planes, 33.8 so;
+// the other lattice 43.6 with 20 and 45.4 with 10).  FP64 ones
+// take at most 4 planes: their blocks differ more (ragged tiles, the sorted sums
+// of the faces), and one wave of long marches waits for the longest (126 x 110 x
+// 97: 595 us with 26 planes, 492 with 8, 480 so; 96^3 303, 297, 293).  Moving
+// walls make a few blocks several times longer than the rest, so marches are
+// short: FP64 at 96^3 622 us with 12 planes, 422 with 4, 350 so; FP32 180, 159, 145.
+int march_planes(const Lattice &L, int blocks_per_sm, bool f64, bool moving, bool frozen) {
   const long long tiles = (long long)((L.esk + kTileK - 1) / kTileK) * ((L.esj + kTileJ - 1) / kTileJ);
-  return march_planes(L.esi, tiles, 152LL * blocks_per_sm);
+  const long long slots = 152LL * blocks_per_sm;
+  if (moving) return march_planes(L.esi, tiles, slots, 1 << 30, 1, 12);
+  return march_planes(L.esi, tiles, slots, f64 ? 4 : 1 << 30, 2, frozen ? 1 : 0);
 }
 
 void count_launch(int n) { g_launches += n; }

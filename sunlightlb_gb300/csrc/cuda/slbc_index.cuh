@@ -105,22 +105,23 @@ SLBC_HD void row_of(I row, int D, int H, int &n, int &z, int &y) {
   z = (int)(t - (I)n * (I)D);
 }
 
-// Planes a tracer block marches over: the march with the least work in whole
-// waves of `slots` resident blocks, a block costing its planes and the two it
-// reads for its halo, for `tiles` tiles of a plane.  (Up to 8 planes with four
-// blocks per SM before: 96^3 in 864 blocks of 4 + 2 planes, now 288 of 12 + 2 in
-// one wave.)  Of the many counts of blocks along i that give the same march only
-// the first is looked at: the rule runs at every update (60,000 x 4 x 4 in FP32: 351 us per
-// update with all, 118 so).
-inline int march_planes(int esi, long long tiles, long long slots) {
+// Planes a tracer block marches over, at most `most`: the least of (waves of
+// `slots` resident blocks + tail / 6) x (planes + halo) for `tiles` tiles of a
+// plane, where a block costs its planes and what it does once, and `tail` sixths
+// of a wave stand for blocks that take longer than the others.  Of the many counts of blocks along i
+// that give the same march only the first is looked at: the rule runs at every
+// update (60,000 x 4 x 4 in FP32: 351 us per update with all, 118 so).
+inline int march_planes(int esi, long long tiles, long long slots, int most = 1 << 30, int halo = 2, int tail = 0) {
   long long best = 0;
   int planes = 1;
   for (long long chunks = 1; chunks <= esi;) {
     const int p = (int)((esi + chunks - 1) / chunks);
-    const long long waves = (tiles * ((esi + p - 1) / p) + slots - 1) / slots, cost = waves * (p + 2);
-    if (best == 0 || cost < best) {
-      best = cost;
-      planes = p;
+    if (p <= most) {
+      const long long waves = (tiles * ((esi + p - 1) / p) + slots - 1) / slots, cost = (6 * waves + tail) * (p + halo);
+      if (best == 0 || cost < best || (tail > 0 && cost == best)) {
+        best = cost;
+        planes = p;
+      }
     }
     if (p == 1) break;
     chunks = (esi + p - 2) / (p - 1);  // the fewest with a shorter march

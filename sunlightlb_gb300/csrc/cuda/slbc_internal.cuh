@@ -264,7 +264,7 @@ cudaError_t ensure_mp_rinv(Lattice &L);
 // them (null else)
 cudaError_t ensure_mp_ratios(Lattice &L);
 // planes a tracer block marches over
-int march_planes(const Lattice &L, int blocks_per_sm);
+int march_planes(const Lattice &L, int blocks_per_sm, bool f64, bool moving, bool frozen);
 // column sums of the tracer stencil set to 1 (mass conservation)
 cudaError_t launch_mp_coef_norm(Lattice &L);
 // one FP32 tracer update from the lattice's stencil coefficients

@@ -427,8 +427,8 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
                                     double alpha, double adprob, int moving,
                                     const double *objstate, float *lo_in, float *lo_out, int *lo_live) {
   int planes = 1;
-  const auto tiling = [&](int blocks_per_sm) {
-    planes = march_planes(L, blocks_per_sm);
+  const auto tiling = [&](int blocks_per_sm, bool frozen = false) {
+    planes = march_planes(L, blocks_per_sm, tp_f64 != 0, moving != 0, frozen);
     return dim3((unsigned)((L.esk + kTileK - 1) / kTileK), (unsigned)((L.esj + kTileJ - 1) / kTileJ),
                 (unsigned)((L.esi + planes - 1) / planes));
   };
@@ -491,7 +491,7 @@ cudaError_t SLBC_FN(launch_mp_step)(Lattice &L, const void *p_in, void *p_out, i
           if (me != cudaSuccess) return me;
         }
         *lo_live = 1;
-        const dim3 grid = tiling(4);
+        const dim3 grid = tiling(4, true);
         return launch_mp_apply(L, (const float *)p_in, lo_in, (float *)p_out, lo_out, grid, block, planes);
       }
     }
