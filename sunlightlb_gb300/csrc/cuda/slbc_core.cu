@@ -28,6 +28,7 @@ struct slbc_lattice {
 };
 
 constexpr int kFillBlocks = 152 * 4;  // blocks of a tracer fill, at most
+constexpr int kHostSums = 64;  // page-locked results of a lattice's sums; a tracer's fill slots come behind them
 
 struct slbc_tracer {
   slbc_lattice *h = nullptr;
@@ -896,7 +897,7 @@ int slbc_create(slbc_lattice **out, int esi, int esj, int esk, int precision) {
   if (e == cudaSuccess) e = cudaMemsetAsync(L.flags, 0, (size_t)n * sizeof(uint16_t), L.stream);
   if (e == cudaSuccess) e = cudaMalloc(&L.objidx, (size_t)n * sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(L.objidx, 0xff, (size_t)n * sizeof(int), L.stream);
-  if (e == cudaSuccess) e = cudaMallocHost(&L.host_out, 64 * sizeof(double));
+  if (e == cudaSuccess) e = cudaMallocHost(&L.host_out, (kHostSums + kFillBlocks) * sizeof(double));
   for (int b = 0; b < 2 && e == cudaSuccess && precision == 2; b++) {
     e = cudaMalloc(&L.mom[b], (size_t)L.npad * 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMemsetAsync(L.mom[b], 0, (size_t)L.npad * 4 * sizeof(float), L.stream);
@@ -1878,12 +1879,12 @@ int slbc_mp_fill(slbc_tracer *t, int kind, const double *geo, double value) {
 
 int slbc_mp_injected(slbc_tracer *t, int reset, double *out) {
   Lattice &L = t->h->L;
-  double slot[kFillBlocks], v = 0.0;
-  CK(cudaMemcpyAsync(slot, t->acc, sizeof slot, cudaMemcpyDeviceToHost, L.stream));
+  double *const slot = L.host_out + kHostSums, v = 0.0;
+  CK(cudaMemcpyAsync(slot, t->acc, kFillBlocks * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
   CK(cudaStreamSynchronize(L.stream));
   for (int b = 0; b < kFillBlocks; b++) v += slot[b];
   if (out) *out = v;
-  if (reset) CK(cudaMemsetAsync(t->acc, 0, sizeof slot, L.stream));
+  if (reset) CK(cudaMemsetAsync(t->acc, 0, kFillBlocks * sizeof(double), L.stream));
   return 0;
 }
 
