@@ -131,10 +131,8 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
     h[d].odd0 = B.lats[d]->layout == SLBC_LAYOUT_C0 ? 1 : 0;
     cls[d] = (h[d].a.moving ? 2 : 0) + (h[d].a.bf_uniform ? 1 : 0);
   }
-  cudaError_t e = upload(B.doms, h.data(), n * sizeof(BatchDom<T_>), B.stream);
-  if (e != cudaSuccess) return e;
-  // the tables of every class are there before the first launch: an upload
-  // waits for the batch's stream
+  // the tables of every class are there before the first launch: uploads wait
+  // for the batch's stream, once for all three
   struct ClassLaunch { int c, blocks, first_off, first_work; };
   std::vector<ClassLaunch> launches;
   std::vector<int> off, work;
@@ -160,8 +158,10 @@ cudaError_t SLBC_FN(launch_batch)(BatchState &B, int nsteps) {
       work.insert(work.end(), owned[w].begin(), owned[w].end());
     }
   }
-  e = upload(B.work_off, off.data(), off.size() * sizeof(int), B.stream);
-  if (e == cudaSuccess) e = upload(B.work, work.data(), work.size() * sizeof(int), B.stream);
+  cudaError_t e = cudaMemcpyAsync(B.doms, h.data(), n * sizeof(BatchDom<T_>), cudaMemcpyHostToDevice, B.stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(B.work_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, B.stream);
+  const cudaError_t u = upload(B.work, work.data(), work.size() * sizeof(int), B.stream);
+  if (e == cudaSuccess) e = u;
   if (e != cudaSuccess) return e;
   for (const ClassLaunch &l : launches) {
     const BatchDom<T_> *D = (const BatchDom<T_> *)B.doms;
@@ -212,17 +212,17 @@ cudaError_t SLBC_FN(prepare_tiles)(BatchState &B) {
     }
     B.sets.push_back(set);
   }
-  cudaError_t e = upload(B.doms, h.data(), n * sizeof(BatchDom<T_>), B.stream);
-  if (e != cudaSuccess) return e;
   if ((long long)tiles.size() > B.tiles_cap) {
     if (B.tiles) cudaFree(B.tiles);
     B.tiles = nullptr;
     B.tiles_cap = 0;
-    e = cudaMalloc(&B.tiles, tiles.size() * sizeof(int2));
+    const cudaError_t e = cudaMalloc(&B.tiles, tiles.size() * sizeof(int2));
     if (e != cudaSuccess) return e;
     B.tiles_cap = (long long)tiles.size();
   }
-  return upload(B.tiles, tiles.data(), tiles.size() * sizeof(int2), B.stream);
+  const cudaError_t e = cudaMemcpyAsync(B.doms, h.data(), n * sizeof(BatchDom<T_>), cudaMemcpyHostToDevice, B.stream);
+  const cudaError_t u = upload(B.tiles, tiles.data(), tiles.size() * sizeof(int2), B.stream);  // waits for both
+  return e != cudaSuccess ? e : u;
 }
 
 // Tiles mode: one step of one set (step = position in the sequence, for the
