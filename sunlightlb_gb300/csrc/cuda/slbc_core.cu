@@ -181,26 +181,35 @@ __global__ void k_distrib_piece(const int *bnd_node, const double *f, long long 
     for (int c = 0; c < 6; c++) piece_sum[6 * pc + c] = v[c];
 }
 
-// distribf, level 2: one warp per object, lane l adding the object's pieces
-// l, l + 32, ... in order, then a fixed-shape tree (one thread adding the
-// 5,000 pieces of a 512^3 bed held as one object took 1.17 ms; the warp 15 us).
+// distribf, level 2: the pieces of an object added in order by a thread, or (WARP)
+// by a warp, lane l adding pieces l, l + 32, ... in order, then a fixed-shape tree.
+template <bool WARP>
 __global__ void __launch_bounds__(128) k_distrib_obj(const int *obj_first_piece, const int *obj_npiece,
                                                      const double *piece_sum, int nobj, double *ft) {
   after_previous();
-  const int o = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, o = WARP ? t >> 5 : t, lane = WARP ? threadIdx.x & 31 : 0;
   if (o >= nobj) return;
   double v[6] = {0, 0, 0, 0, 0, 0};
-  for (int pc = obj_first_piece[o] + lane; pc < obj_first_piece[o] + obj_npiece[o]; pc += 32)
+  for (int pc = obj_first_piece[o] + lane; pc < obj_first_piece[o] + obj_npiece[o]; pc += WARP ? 32 : 1)
 #pragma unroll
     for (int c = 0; c < 6; c++) v[c] += piece_sum[6 * pc + c];
+  if constexpr (WARP) {
 #pragma unroll
-  for (int c = 0; c < 6; c++)
+    for (int c = 0; c < 6; c++)
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], d);
+      for (int d = 16; d > 0; d >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], d);
+  }
   if (lane == 0)
 #pragma unroll
     for (int c = 0; c < 6; c++) ft[6 * o + c] = v[c];
 }
+
+// A warp for an object where the longest sum of one thread would take longer than
+// the trees of all warps: a piece is some 0.23 us of a thread (5,000 pieces of a
+// 512^3 bed held as one object 1.17 ms, by a warp 15 us), a tree 30 FP64 additions
+// of a warp (32,768 objects of one piece: distribf 1,218 us so, 1,021 by
+// threads).
+static bool distrib_by_warps(int nobj, int most_pieces) { return 150LL * most_pieces > 300LL + nobj; }
 
 // Per fluid node, the boundary links whose solid end adsorbs (bit q: the
 // solid node x - c_q has its adsorption byte set).
@@ -1033,6 +1042,7 @@ static int geometry_boundary(Lattice &L, int nobj, const long *bnd_node, const i
     }
     if (e != nbnd) return fail_msg("slbc_set_geometry: boundary list not sorted by object");
     L.npiece = (int)po.size();
+    L.most_pieces = *std::max_element(cnt.begin(), cnt.end());
     CK(cudaMalloc(&L.obj_pos, 3 * nobj * sizeof(double)));
     CK(cudaMalloc(&L.obj_ft, (6 * nobj + 2 * nobj) * sizeof(double)));
     // first/count stored after the 6*nobj results, as ints
@@ -1538,8 +1548,12 @@ int slbc_distribf(slbc_lattice *h, const double *pos, double *ft) {
     CK(cudaGetLastError());
   }
   const int *first = (const int *)(L.obj_ft + 6 * L.nobj);
-  launch_pdl(k_distrib_obj, blocks_for(L.nobj, 4), 128, 0, L.stream, first, first + L.nobj, L.piece_sum, L.nobj,
-             L.obj_ft);
+  const auto go = [&](auto kernel, int per_block) {
+    launch_pdl(kernel, blocks_for(L.nobj, per_block), 128, 0, L.stream, first, first + L.nobj, L.piece_sum, L.nobj,
+               L.obj_ft);
+  };
+  if (distrib_by_warps(L.nobj, L.most_pieces)) go(k_distrib_obj<true>, 4);
+  else go(k_distrib_obj<false>, 128);
   count_launch();
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(ft, L.obj_ft, 6 * (size_t)L.nobj * sizeof(double), cudaMemcpyDeviceToHost, L.stream));

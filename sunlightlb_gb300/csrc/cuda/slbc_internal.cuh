@@ -77,6 +77,7 @@ struct Lattice {
   int *bnd_obj = nullptr;
   double *bnd_f = nullptr;    // 3 * nbnd node forces (x block, y block, z block)
   int npiece = 0;             // distribf work pieces
+  int most_pieces = 0;        // of one object
   int *piece_obj = nullptr, *piece_lo = nullptr, *piece_hi = nullptr;
   double *piece_sum = nullptr;  // 6 * npiece
   double *obj_pos = nullptr;    // 3 * nobj
